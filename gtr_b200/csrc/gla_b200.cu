@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "gla_kernel.cuh"
+#include "gla_step.cuh"
 #include "swiglu_dwconv.cuh"
 #include "gla_bwd.cuh"
 
@@ -183,6 +184,10 @@ int relay_segments(int NT, int nseq, int slots, size_t workspace_bytes, double* 
     *cost_out = best_cost;
     return best;
 }
+
+// A few tokens per sequence go token by token through the state in registers (gla_step.cuh), unless the caller asks for
+// the chunk kernel's decomposition or the fused epilogue.
+bool step_serves(int T, bool gated, int segments) { return T <= gla::kStepMaxTokens && !gated && segments == 0; }
 
 // ---- tensor maps ------------------------------------------------------------------------
 struct MapKey {
@@ -516,11 +521,33 @@ int gla_b200_forward(const gla_b200_args* a, void* stream_v) {
     if (!a->workspace || (reinterpret_cast<uintptr_t>(a->workspace) & 255u) || a->workspace_bytes < L.total)
         return GLA_B200_ERR_WORKSPACE;
 
+    uint8_t* ws = static_cast<uint8_t*>(a->workspace);
+    if (step_serves(a->T, gated, a->segments)) {
+        gla::StepParams S;
+        S.q = static_cast<const __half*>(a->q); S.k = static_cast<const __half*>(a->k);
+        S.v = static_cast<const __half*>(a->v); S.g = static_cast<const __half*>(a->g);
+        S.o = static_cast<__half*>(a->o);
+        S.s0 = a->initial_state; S.sT = a->final_state;
+        S.ctrl = reinterpret_cast<uint32_t*>(ws + L.ctrl);
+        for (int i = 0; i < 3; ++i) {
+            S.q_s[i] = key.stride[gla::TQ][i]; S.k_s[i] = key.stride[gla::TK][i]; S.v_s[i] = key.stride[gla::TV][i];
+            S.g_s[i] = key.stride[gla::TG][i]; S.o_s[i] = key.stride[gla::TO][i];
+        }
+        S.T = a->T; S.H = a->H; S.Hc = key.Hc; S.Wc = key.Wc; S.rev = a->direction & 1;
+        S.scale = a->scale;
+        S.inv_norm = a->gk_normalizer > 0.f ? 1.f / a->gk_normalizer : 0.f;
+        cudaStream_t st = static_cast<cudaStream_t>(stream_v);
+        if (a->K == 64) gla::gla_step_kernel<64><<<nseq, gla::kStepThreads, 0, st>>>(S);
+        else gla::gla_step_kernel<32><<<nseq, gla::kStepThreads, 0, st>>>(S);
+        ce = cudaPeekAtLastError();
+        if (ce != cudaSuccess) { note_cuda("step kernel launch", ce); return GLA_B200_ERR_CUDA; }
+        return GLA_B200_OK;
+    }
+
     gla::Maps maps;
     rc = get_maps(key, &maps);
     if (rc != GLA_B200_OK) return rc;
 
-    uint8_t* ws = static_cast<uint8_t*>(a->workspace);
     gla::Params P;
     memset(&P, 0, sizeof(P));
     P.B = a->B; P.T = a->T; P.H = a->H; P.NT = NT; P.K = a->K;
