@@ -57,6 +57,7 @@ EXPORTS = (
 )
 
 _lib = None
+_front = None
 
 
 class GlaError(RuntimeError):
@@ -108,6 +109,21 @@ def lib() -> ctypes.CDLL:
     L.gla_b200_version.restype = ctypes.c_int
     _lib = L
     return L
+
+
+def front():
+    """The native face of the library (csrc/torch_front.cpp): the operator's calls without the ctypes round trip."""
+    global _front
+    if _front is None:
+        L = lib()
+        path = os.path.join(PKG, "_front.so")
+        if not os.path.exists(path):
+            raise ImportError(f"{path} is missing: build it with `python -m gtr_b200.build`")
+        from . import _front as F
+        address = lambda fn: ctypes.cast(fn, ctypes.c_void_p).value
+        F.bind(address(L.gla_b200_forward), address(L.gla_b200_workspace_bytes))
+        _front = F
+    return _front
 
 
 def check(code: int) -> None:

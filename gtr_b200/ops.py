@@ -26,6 +26,9 @@ from typing import Optional, Tuple
 import torch
 
 from . import _lib
+from ._lib import front as _front
+
+_SLOW = 1               # the native face's answer to arguments it leaves to the Python path, which names what is wrong
 
 kK = 64                 # widest key head; SUPPORTED_K lists every key head size served
 kV = 64
@@ -129,15 +132,25 @@ def _forward(q, k, v, gk, o, ws, scale, gk_normalizer, direction, grid_hw, initi
 def chunk_gla_run(q, k, v, gk, scale, ws, o, gk_normalizer: float = 0.0, *, direction=0, grid_hw=None,
                   initial_state=None, final_state=None, segments: int = 0, wait_limit: int = 0) -> None:
     """o <- GLA(q, k, v, gk) on the current stream.  Reference: ext.chunk_gla_run (gla_torch_ext.cu:40-90)."""
-    _forward(q, k, v, gk, o, ws, scale, gk_normalizer, direction, grid_hw, initial_state, final_state,
-             segments=segments, wait_limit=wait_limit)
+    rc = _front().run(q, k, v, gk, o, ws, scale, gk_normalizer, direction, grid_hw, initial_state, final_state, None, None,
+                      0.0, segments, wait_limit)
+    if rc == _SLOW:
+        _forward(q, k, v, gk, o, ws, scale, gk_normalizer, direction, grid_hw, initial_state, final_state,
+                 segments=segments, wait_limit=wait_limit)
+    elif rc:
+        _lib.check(rc)
 
 
 def chunk_gla_run_gated(q, k, v, gk, g, rms_w, scale, eps, ws, y, gk_normalizer: float = 0.0, *, direction=0,
                         grid_hw=None, initial_state=None, final_state=None, segments: int = 0) -> None:
     """y <- RMSNorm(GLA(q,k,v,gk)) * rms_w * silu(g).  Reference: ext.chunk_gla_run_gated (gla_torch_ext.cu:92-154)."""
-    _forward(q, k, v, gk, y, ws, scale, gk_normalizer, direction, grid_hw, initial_state, final_state,
-             out_gate=g, rms_w=rms_w, eps=eps, segments=segments)
+    rc = _front().run(q, k, v, gk, y, ws, scale, gk_normalizer, direction, grid_hw, initial_state, final_state, g, rms_w,
+                      eps, segments, 0)
+    if rc == _SLOW:
+        _forward(q, k, v, gk, y, ws, scale, gk_normalizer, direction, grid_hw, initial_state, final_state,
+                 out_gate=g, rms_w=rms_w, eps=eps, segments=segments)
+    elif rc:
+        _lib.check(rc)
 
 
 def chunk_gla_with_ws(q, k, v, gk, scale, ws, **kw) -> torch.Tensor:
@@ -310,6 +323,12 @@ def chunk_gla(q, k, v, g, scale: Optional[float] = None, initial_state: Optional
     `chunk_gla_backward` -- as FLA's operator does for the reference in training.  The gradient kernels serve the
     row-major scan with log-space gates (what FLA's signature expresses); for the other scan directions the backward
     gathers the tokens into scan order around them, and for raw gate logits it applies logsigmoid's derivative."""
+    if cu_seqlens is None:
+        done = _front().gla(q, k, v, g, scale, initial_state, output_final_state, direction, grid_hw, gk_normalizer, segments)
+        if type(done) is tuple:
+            return done
+        if done != _SLOW:
+            _lib.check(done)
     tensors = [x for x in (q, k, v, g, initial_state) if x is not None]
     if not (torch.is_grad_enabled() and any(x.requires_grad for x in tensors)):
         return _chunk_gla_forward(q, k, v, g, scale, initial_state, output_final_state, cu_seqlens, direction=direction,
