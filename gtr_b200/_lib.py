@@ -49,11 +49,18 @@ class BwdArgs(ctypes.Structure):
     ]
 
 
+class BwdScan(ctypes.Structure):
+    """Mirror of `gla_b200_bwd_scan`."""
+    _fields_ = [("grid_h", ctypes.c_int32), ("grid_w", ctypes.c_int32), ("direction", ctypes.c_int32),
+                ("dg_is_half", ctypes.c_int32)]
+
+
 EXPORTS = (
     "gla_b200_forward", "gla_b200_workspace_bytes", "gla_b200_check_status", "gla_b200_rmsnorm_gated",
     "gla_b200_trt_enqueue", "gla_b200_strerror", "gla_b200_last_cuda_error", "gla_b200_version",
     "gla_b200_forward_static", "gla_b200_selftest_wait_timeout", "gla_b200_swiglu_dwconv", "gla_b200_layernorm",
     "gla_b200_stream_probe", "gla_b200_backward", "gla_b200_backward_workspace_bytes",
+    "gla_b200_backward_scan",
 )
 
 _lib = None
@@ -85,6 +92,8 @@ def lib() -> ctypes.CDLL:
     L.gla_b200_stream_probe.restype = ctypes.c_int
     L.gla_b200_backward.argtypes = [ctypes.POINTER(BwdArgs), ctypes.c_void_p]
     L.gla_b200_backward.restype = ctypes.c_int
+    L.gla_b200_backward_scan.argtypes = [ctypes.POINTER(BwdArgs), ctypes.POINTER(BwdScan), ctypes.c_void_p]
+    L.gla_b200_backward_scan.restype = ctypes.c_int
     L.gla_b200_backward_workspace_bytes.argtypes = [ctypes.c_int32] * 5
     L.gla_b200_backward_workspace_bytes.restype = ctypes.c_size_t
     L.gla_b200_workspace_bytes.argtypes = [ctypes.c_int32] * 5
@@ -121,7 +130,8 @@ def front():
             raise ImportError(f"{path} is missing: build it with `python -m gtr_b200.build`")
         from . import _front as F
         address = lambda fn: ctypes.cast(fn, ctypes.c_void_p).value
-        F.bind(address(L.gla_b200_forward), address(L.gla_b200_workspace_bytes))
+        F.bind(*(address(fn) for fn in (L.gla_b200_forward, L.gla_b200_workspace_bytes, L.gla_b200_backward_scan,
+                                        L.gla_b200_backward_workspace_bytes, L.gla_b200_strerror)))
         _front = F
     return _front
 

@@ -8,6 +8,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <utility>
 #include <vector>
 
 #include "gla_kernel.cuh"
@@ -73,6 +74,14 @@ int device_info(int dev, DeviceInfo* out) {
         }
         for (int v = 0; v < 8 && e == cudaSuccess; ++v)
             e = cudaFuncSetAttribute(fwd_kernel(v), cudaFuncAttributeMaxDynamicSharedMemorySize, gla::kSmemBytes);
+        if (e != cudaSuccess) { note_cuda("cudaFuncSetAttribute", e); return GLA_B200_ERR_CUDA; }
+        const std::pair<const void*, int> bwd[] = {
+            {reinterpret_cast<const void*>(&gla::gla_bwd_state_kernel<64>), gla::BwdStateSmem::kBytes},
+            {reinterpret_cast<const void*>(&gla::gla_bwd_state_kernel<32>), gla::BwdStateSmem::kBytes},
+            {reinterpret_cast<const void*>(&gla::gla_bwd_chunk_kernel<64>), gla::BwdChunkSmem::kBytes},
+            {reinterpret_cast<const void*>(&gla::gla_bwd_chunk_kernel<32>), gla::BwdChunkSmem::kBytes}};
+        for (const auto& k : bwd)
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(k.first, cudaFuncAttributeMaxDynamicSharedMemorySize, k.second);
         if (e != cudaSuccess) { note_cuda("cudaFuncSetAttribute", e); return GLA_B200_ERR_CUDA; }
         // The warpgroups of the kernel re-divide the registers the CTA was launched with (setmaxnreg); a group that
         // asks for more than the others release would wait for ever, so the budgets are checked against what this
@@ -673,76 +682,119 @@ int gla_b200_check_status(const void* workspace, void* stream) {
     return ctrl[1] == 0 ? GLA_B200_OK : GLA_B200_ERR_TIMEOUT;
 }
 
-// Segments per sequence for the gradient sweeps: enough CTAs to give every SM several (the sweeps hide latency by
-// occupancy), segments of at least 256 tokens.  A pure function of the shape, so the workspace size can be asked ahead.
-static int bwd_segments(int B, int T, int H, int* seg_len) {
-    const int64_t ctas = 3LL * B * H;
-    int nseg = static_cast<int>((600 + ctas - 1) / ctas);
-    nseg = std::max(1, std::min(nseg, T / 256));
-    int len = ((T + nseg - 1) / nseg + 31) / 32 * 32;
-    nseg = (T + len - 1) / len;
-    *seg_len = nseg > 1 ? len : std::max(T, 1);
-    return nseg;
+// Segments per sequence for the gradient: two CTAs per SM walk one segment each, so the split that costs least is the one
+// whose rounds x (chunks per segment, plus what a segment costs once) are fewest; more than one segment per sequence also
+// needs the state gradients of the segments (a quarter of a chunk's work each).  A pure function of the shape, so the
+// workspace size can be asked ahead; 296 = 2 x 148 SMs.
+static int bwd_segments(int64_t nseq, int NT, int* cps_out) {
+    constexpr int64_t kSlots = 296;
+    int best_cps = NT;
+    double best = 1e300;
+    for (int want = 1; want <= NT && want <= 64; ++want) {
+        const int cps = (NT + want - 1) / want, nseg = (NT + cps - 1) / cps;
+        if (nseg != want) continue;
+        const double rounds = static_cast<double>((nseq * nseg + kSlots - 1) / kSlots);
+        const double cost = rounds * (cps * (nseg > 1 ? 1.25 : 1.0) + 1.5 + 0.1 * nseg);
+        if (cost < best - 1e-9) { best = cost; best_cps = cps; }
+    }
+    *cps_out = best_cps;
+    return (NT + best_cps - 1) / best_cps;
+}
+
+struct BwdLayout { size_t chunk_state, chunk_decay, seg_grad, seg_decay, park, total; };
+static BwdLayout bwd_layout(int64_t nseq, int NT, int nseg) {
+    BwdLayout L;
+    const size_t chunks = static_cast<size_t>(nseq) * NT, segs = static_cast<size_t>(nseq) * nseg;
+    L.chunk_state = 256;
+    L.chunk_decay = L.chunk_state + chunks * 64 * 64 * sizeof(float);
+    L.seg_grad = L.chunk_decay + chunks * 64 * sizeof(float);
+    L.seg_decay = L.seg_grad + segs * 64 * 64 * sizeof(float);
+    L.park = L.seg_decay + segs * 64 * sizeof(float);
+    L.total = L.park + 2 * segs * 64 * 64 * sizeof(float);
+    return L;
 }
 
 size_t gla_b200_backward_workspace_bytes(int32_t B, int32_t T, int32_t H, int32_t K, int32_t V) {
     if (B <= 0 || T <= 0 || H <= 0 || (K != 32 && K != 64) || V != 64) return 0;
-    const size_t per = align_up(static_cast<size_t>(B) * T * H * K * sizeof(float), 256);
-    int seg_len = 0;
-    const size_t nseg = static_cast<size_t>(bwd_segments(B, T, H, &seg_len));
-    const size_t seg = nseg > 1 ? align_up(2 * static_cast<size_t>(B) * H * nseg * K * (2 * 64 + 1) * sizeof(float), 256) : 0;
-    return 2 * per + align_up(static_cast<size_t>(B) * H * K * sizeof(float), 256) + seg;
+    int cps = 0;
+    const int64_t nseq = static_cast<int64_t>(B) * H;
+    // never less than two fp32 [B,T,H,K] arrays and one [B,H,K], which callers may have sized pools by
+    const size_t arrays = 2 * align_up(static_cast<size_t>(B) * T * H * K * sizeof(float), 256) +
+                          align_up(static_cast<size_t>(nseq) * K * sizeof(float), 256);
+    return std::max(arrays, bwd_layout(nseq, num_chunks(T), bwd_segments(nseq, num_chunks(T), &cps)).total);
 }
 
-int gla_b200_backward(const gla_b200_bwd_args* a, void* stream_v) {
+int gla_b200_backward(const gla_b200_bwd_args* a, void* stream) { return gla_b200_backward_scan(a, nullptr, stream); }
+
+int gla_b200_backward_scan(const gla_b200_bwd_args* a, const gla_b200_bwd_scan* o, void* stream_v) {
     if (!a) return GLA_B200_ERR_NULL;
     if (a->B < 0 || a->T < 0 || a->H <= 0 || (a->K != 32 && a->K != 64) || a->V != 64) return GLA_B200_ERR_SHAPE;
-    if (static_cast<int64_t>(a->B) * a->H > 0x7fffffffLL) return GLA_B200_ERR_SHAPE;
+    const int64_t nseq = static_cast<int64_t>(a->B) * a->H;
+    if (nseq > 0x7fffffffLL) return GLA_B200_ERR_SHAPE;
+    if (o) {
+        if (o->direction < 0 || o->direction > 3) return GLA_B200_ERR_DIRECTION;
+        if (o->direction >= 2 && (o->grid_h <= 0 || o->grid_w <= 0)) return GLA_B200_ERR_SHAPE;
+        if ((o->grid_h != 0 || o->grid_w != 0) && (o->grid_h < 0 || o->grid_w < 0 || static_cast<int64_t>(o->grid_h) * o->grid_w != a->T))
+            return GLA_B200_ERR_SHAPE;
+    }
     if (a->B == 0 || a->T == 0) return GLA_B200_OK;
     if (!a->q || !a->k || !a->v || !a->g || !a->d_o || !a->dq || !a->dk || !a->dv || !a->dg) return GLA_B200_ERR_NULL;
     const void* ptrs[] = {a->q, a->k, a->v, a->g, a->d_o, a->dq, a->dk, a->dv, a->dg, a->initial_state, a->d_final_state,
                           a->d_initial_state, a->workspace};
     for (const void* p : ptrs)
         if (p && !aligned16(p)) return GLA_B200_ERR_ALIGN;
-    const size_t need = gla_b200_backward_workspace_bytes(a->B, a->T, a->H, a->K, a->V);
-    if (!a->workspace || a->workspace_bytes < need) return GLA_B200_ERR_WORKSPACE;
+    const int NT = num_chunks(a->T);
+    gla::BwdParams P{};
+    P.nseg = bwd_segments(nseq, NT, &P.cps);
+    const BwdLayout L = bwd_layout(nseq, NT, P.nseg);
+    if (!a->workspace || a->workspace_bytes < L.total) return GLA_B200_ERR_WORKSPACE;
+    if (nseq * P.nseg > 0x7fffffffLL) return GLA_B200_ERR_SHAPE;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) { note_cuda("cudaGetDevice", e); return GLA_B200_ERR_CUDA; }
+    if (dev < 0 || dev >= 64) return GLA_B200_ERR_DEVICE;
     DeviceInfo info;
     if (int rc = device_info(dev, &info)) return rc;
 
-    gla::BwdParams P{};
-    P.q = static_cast<const __half*>(a->q); P.k = static_cast<const __half*>(a->k); P.v = static_cast<const __half*>(a->v);
-    P.g = static_cast<const __half*>(a->g); P.d_o = static_cast<const __half*>(a->d_o);
+    MapKey key;
+    memset(&key, 0, sizeof(key));
+    const bool col = o && o->direction >= 2;
+    key.B = a->B; key.T = a->T; key.H = a->H; key.K = a->K; key.dev = dev;
+    key.col = col ? 1 : 0;
+    key.Hc = col ? o->grid_h : a->T;
+    key.Wc = col ? o->grid_w : 1;
+    const std::pair<int, const void*> tensors[] = {{gla::TQ, a->q}, {gla::TK, a->k}, {gla::TG, a->g}, {gla::TV, a->v}, {gla::TO, a->d_o}};
+    for (const auto& t : tensors) {
+        const int64_t D = t.first == gla::TV || t.first == gla::TO ? gla::kD : a->K;
+        key.ptr[t.first] = t.second;
+        key.stride[t.first][0] = static_cast<int64_t>(a->T) * a->H * D;
+        key.stride[t.first][1] = static_cast<int64_t>(a->H) * D;
+        key.stride[t.first][2] = D;
+    }
+    gla::Maps maps;
+    if (int rc = get_maps(key, &maps)) return rc;
     P.dq = static_cast<__half*>(a->dq); P.dk = static_cast<__half*>(a->dk); P.dv = static_cast<__half*>(a->dv);
-    P.dg = a->dg; P.h0 = a->initial_state; P.dht = a->d_final_state; P.dh0 = a->d_initial_state;
-    const size_t per = align_up(static_cast<size_t>(a->B) * a->T * a->H * a->K * sizeof(float), 256);
+    if (o && o->dg_is_half) P.dg_half = reinterpret_cast<__half*>(a->dg);
+    else P.dg = a->dg;
+    P.h0 = a->initial_state; P.dht = a->d_final_state; P.dh0 = a->d_initial_state;
     unsigned char* ws = static_cast<unsigned char*>(a->workspace);
-    P.qdq = reinterpret_cast<float*>(ws); P.kdk = reinterpret_cast<float*>(ws + per);
-    P.g_last = a->d_final_state ? reinterpret_cast<float*>(ws + 2 * per) : nullptr;
-    P.B = a->B; P.T = a->T; P.H = a->H; P.scale = a->scale;
-    P.nseg = bwd_segments(a->B, a->T, a->H, &P.seg_len);
-    const size_t last = align_up(static_cast<size_t>(a->B) * a->H * a->K * sizeof(float), 256);
-    P.seg_state = reinterpret_cast<float*>(ws + 2 * per + last);
-    P.seg_start = P.seg_state + 2 * static_cast<size_t>(a->B) * a->H * P.nseg * a->K * 64;
-    P.seg_decay = P.seg_start + 2 * static_cast<size_t>(a->B) * a->H * P.nseg * a->K * 64;
+    P.ctrl = reinterpret_cast<uint32_t*>(ws);
+    P.chunk_state = reinterpret_cast<float*>(ws + L.chunk_state); P.chunk_decay = reinterpret_cast<float*>(ws + L.chunk_decay);
+    P.seg_grad = reinterpret_cast<float*>(ws + L.seg_grad); P.seg_decay = reinterpret_cast<float*>(ws + L.seg_decay);
+    P.park = reinterpret_cast<float*>(ws + L.park);
+    P.B = a->B; P.T = a->T; P.H = a->H; P.NT = NT;
+    P.Hc = key.Hc; P.Wc = key.Wc; P.rev = o ? (o->direction & 1) : 0;
+    P.scale = a->scale;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
-    const unsigned bh = static_cast<unsigned>(a->B * a->H);
-    if (static_cast<int64_t>(bh) * P.nseg > 0x7fffffffLL) return GLA_B200_ERR_SHAPE;
-#define GLA_BWD_LAUNCH(KK)                                                                                            \
-    do {                                                                                                              \
-        if (P.nseg > 1) {                                                                                             \
-            gla::gla_bwd_state_kernel<KK><<<dim3(bh * (P.nseg - 1), 2), gla::kBwdThreads, 0, stream>>>(P);            \
-            gla::gla_bwd_combine_kernel<KK><<<dim3(bh, 2, KK / 4), 256, 0, stream>>>(P);                                   \
-        }                                                                                                             \
-        gla::gla_bwd_sweep_kernel<KK><<<dim3(bh * P.nseg, 3), gla::kBwdThreads, 0, stream>>>(P);                      \
-        if (bh >= 256) gla::gla_bwd_dg_kernel<KK, KK><<<dim3(bh, 1), 1024, 0, stream>>>(P);                           \
-        else gla::gla_bwd_dg_kernel<KK, 16><<<dim3(bh, KK / 16), 1024, 0, stream>>>(P);                               \
-    } while (0)
-    if (a->K == 64) GLA_BWD_LAUNCH(64);
-    else GLA_BWD_LAUNCH(32);
-#undef GLA_BWD_LAUNCH
+    const unsigned ctas = static_cast<unsigned>(nseq * P.nseg);
+    const dim3 states(ctas, P.nseg > 1 ? 2 : 1);
+    if (a->K == 64) {
+        gla::gla_bwd_state_kernel<64><<<states, gla::kBwdThreads, gla::BwdStateSmem::kBytes, stream>>>(maps, P);
+        gla::gla_bwd_chunk_kernel<64><<<ctas, gla::kBwdChunkThreads, gla::BwdChunkSmem::kBytes, stream>>>(maps, P);
+    } else {
+        gla::gla_bwd_state_kernel<32><<<states, gla::kBwdThreads, gla::BwdStateSmem::kBytes, stream>>>(maps, P);
+        gla::gla_bwd_chunk_kernel<32><<<ctas, gla::kBwdChunkThreads, gla::BwdChunkSmem::kBytes, stream>>>(maps, P);
+    }
     e = cudaPeekAtLastError();
     if (e != cudaSuccess) { note_cuda("backward launch", e); return GLA_B200_ERR_CUDA; }
     return GLA_B200_OK;

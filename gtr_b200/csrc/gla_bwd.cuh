@@ -1,4 +1,4 @@
-// Gradient of the gated-linear-attention operator, token by token with the state in registers.
+// Gradient of the gated-linear-attention operator, chunk by chunk on the tensor cores.
 //
 //   forward    S_t = exp(g_t) S_{t-1} + k_t v_t^T ,  o_t = scale q_t^T S_t
 //   gradient   dS_t = exp(g_{t+1}) dS_{t+1} + scale q_t do_t^T
@@ -6,43 +6,165 @@
 //              dg_t = sum_{s >= t} (q_s dq_s - k_s dk_s)   (+ the final state's term at the last token)
 //
 // The reference trains through the third-party FLA operator (engine/gtr/backbone/vit_adapter.py:441,560-568); its
-// own CUDA extension has no gradient.  Three independent sweeps run as three kinds of CTA per (batch, head):
-//   kind 0  walks forward with S and emits dq;
-//   kind 1  walks backward with dS and emits dk (and d initial_state);
-//   kind 2  walks backward with a second copy of dS, blocked the other way round, and emits dv.
-// A thread owns a small block of the state, so a token costs it 6 or 7 shared-memory reads of 16 bytes, and every
-// per-token reduction is inside the thread plus a 3-step butterfly over 8 lanes.  Tokens are staged 32 at a time:
-// the next chunk's fp16 rows are fetched into registers while the current chunk is worked from fp32 tiles in
-// shared memory.  A last kernel turns the per-token products q dq - k dk into dg by a reverse running sum.
-// All arithmetic is fp32 on CUDA cores, two lanes per instruction (fma.rn.f32x2): 1.5 instructions per state element and
-// token, so the sweeps are bound by instruction issue, not by memory.
+// own CUDA extension has no gradient.
+//
+// With G the inclusive gate sum inside a 64-token chunk, G_L its last value, R = G_L / 2 per channel, S the state at the
+// chunk's start and dS the state gradient at its end:
+//   qt = q e^(G-R)    kt = k e^(R-G)    St = e^R S    dSt = e^(G_L-R) dS    P = tril(qt kt^T)    dP = tril(do v^T)
+//   dq = scale e^(G-R) (do St^T + dP kt)        dk = e^(R-G) (v dSt^T + scale dP^T qt)
+//   dv = kt dSt + scale P^T do                  dS at the chunk's start = e^R (dSt + scale qt^T do)
+//   dg_t = sum over the chunk's tokens s >= t of (q_s dq_s - k_s dk_s)  +  sum_v S_end dS   (S_end: state after the chunk)
+// The last line closes the sum over all later tokens with two states at hand: no pass over the sequence is needed for dg.
+//
+// Precision.  The gradient is fp32 arithmetic on fp16 inputs, as a token recurrence in fp32 would be: every operand of the
+// tensor cores that is not an input itself (qt, kt, P, dP, St, dSt) is the sum of two fp16 tiles, high and low part, and a
+// product of two such operands is three MMAs (high high, high low, low high) into one fp32 accumulator: 22 bits.  Each
+// operand carries a power-of-two scale of its own per chunk, taken from the largest magnitudes of the tiles at hand, that
+// puts it where fp16 has both parts normal, so neither tiny nor huge gradients lose bits.  Measured against the float64
+// recurrence: dg 1e-6 relative, the same as the token-by-token kernels these replace.
+// A chunk in which some channel decays by more than 2^(2 kBwdRefLimit) has no common reference that keeps both operands in
+// range; its products within the chunk are computed pair by pair in fp32 from gate differences (bwd_wide_chunk).
+//
+// Measured (B200): B4 H12 T6400 K64 238 us (states 74, chunks 164) against 1080 us for three recurrent sweeps in fp32, whose
+// bound was the FMA pipe (500 us); B8 H6 T1600 75 against 285.  HBM alone would take about 115 us at 6.5 TB/s (96 KB per
+// chunk and head in the chunk kernel, 40 KB in the states'); what is left is the latency of the chunk's five dependent
+// tensor-core round trips with two CTAs per SM.
+//
+// Two kernels.  gla_bwd_state_kernel walks the segments of every sequence and leaves the local state after every chunk
+// (forward) and the local state gradient of a segment (backward); gla_bwd_chunk_kernel chains the segments' totals into its
+// own start, then walks its segment backwards and emits everything.  Several CTAs share an SM and hide one another's
+// tensor-core and memory latencies; the work of one chunk stays in one CTA.
 #pragma once
 #include <cuda_fp16.h>
 #include <cstdint>
 
+#include "gla_kernel.cuh"
+
 namespace gla {
 
-constexpr int kBwdThreads = 128;
-constexpr int kBwdChunk = 32;
+constexpr int kBwdThreads = 256;
+constexpr float kBwdRefLimit = 8.f;       // log2: qt and kt carry factors up to 2^8, see bwd_scale() for the room they have
 
 struct BwdParams {
-    const __half *q, *k, *v, *g, *d_o;
-    __half *dq, *dk, *dv;
-    float* dg;
+    __half *dq, *dk, *dv;                 // contiguous [B,T,H,K|64], as q, k, v, g, do (which come through tensor maps)
+    float* dg;            // [B,T,H,K] fp32, or null when dg_half is set
+    __half* dg_half;
     const float* h0;      // [B,H,K,64] or null
     const float* dht;     // [B,H,K,64] or null
     float* dh0;           // [B,H,K,64] or null
-    float *qdq, *kdk;     // scratch [B,T,H,K]
-    float* g_last;        // scratch [B,H,K]: sum_v dht * final_state
-    float* seg_state;     // scratch [2][B*H][nseg][K,64]: a segment's own contribution (forward S, backward dS)
-    float* seg_start;     // scratch, same shape: the state a segment starts from
-    float* seg_decay;     // scratch [2][B*H][nseg][K]: product of the gates over a segment
-    int B, T, H;
-    int nseg, seg_len;    // a sequence is cut into nseg pieces of seg_len tokens (a multiple of 32), each its own CTA
+    // States in scratch lie in the order of the threads that hold them: float4 e of thread t at [e][t].
+    float* chunk_state;   // scratch [B*H][NT][4096]: forward state after a chunk, from a zero state at its segment's start
+    float* chunk_decay;   // scratch [B*H][NT][64]: log2 decay from the segment's start to the chunk's end
+    float* seg_grad;      // scratch [B*H][nseg][4096]: state gradient at a segment's start, from zero at its end
+    float* seg_decay;     // scratch [B*H][nseg][64]: log2 decay over the segment
+    float* park;          // scratch [B*H][nseg][2][4096]: what a thread holds (dS; q and k) while a wide chunk has the registers
+    uint32_t* ctrl;       // [1] status: a bounded wait expired
+    int B, T, H, NT;
+    int nseg, cps;        // segments per sequence, chunks per segment
+    int Hc, Wc, rev;      // scan order as in Params
     float scale;
 };
 
-// Two fp32 lanes per instruction (the packed FMA pipe of sm_100): the sweeps are bound by instruction issue.
+// ------------------------------------------------------------------------------------------ shared pieces
+// One M = 64 accumulator per slot: 64 columns, lanes 0-15 (even slots) or 16-31 (odd) of every quadrant.
+__device__ __forceinline__ uint32_t bwd_slot(uint32_t tmem, int slot) {
+    return tmem + (static_cast<uint32_t>(16 * (slot & 1)) << 16) + 64u * static_cast<uint32_t>(slot >> 1);
+}
+// 16 columns of one accumulator row: lanes 0-15 of warp w columns 32 (w / 4) .. +15 of rows 16 (w % 4) + lane, lanes 16-31
+// columns +16 .. +31 of the same rows.
+__device__ __forceinline__ void bwd_read(uint32_t tmem, int slot, int w, float* x) {
+    const uint32_t a = bwd_slot(tmem, slot) + (static_cast<uint32_t>(32 * (w & 3)) << 16) + 32u * static_cast<uint32_t>(w >> 2);
+    uint32_t* r = reinterpret_cast<uint32_t*>(x);
+    asm volatile(
+        "tcgen05.ld.sync.aligned.16x32bx2.x16.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16], 16;"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(a)
+        : "memory");
+}
+// columns `off` .. +7 of the same piece
+__device__ __forceinline__ void bwd_read8(uint32_t tmem, int slot, int w, uint32_t off, float* x) {
+    const uint32_t a = bwd_slot(tmem, slot) + (static_cast<uint32_t>(32 * (w & 3)) << 16) + 32u * static_cast<uint32_t>(w >> 2) + off;
+    uint32_t* r = reinterpret_cast<uint32_t*>(x);
+    asm volatile("tcgen05.ld.sync.aligned.16x32bx2.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8], 16;"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(a)
+                 : "memory");
+}
+__device__ __forceinline__ void bwd_write(uint32_t tmem, int slot, int w, const float* x) {
+    const uint32_t a = bwd_slot(tmem, slot) + (static_cast<uint32_t>(32 * (w & 3)) << 16) + 32u * static_cast<uint32_t>(w >> 2);
+    const uint32_t* r = reinterpret_cast<const uint32_t*>(x);
+    asm volatile(
+        "tcgen05.st.sync.aligned.16x32bx2.x16.b32 [%0], 16, "
+        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+        ::"r"(a), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+          "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+}
+
+// D (+)= A B over K = 64 from two swizzled tiles; kA / kB: 1 when the tile's rows are the contraction index.
+template <uint32_t kA, uint32_t kB>
+__device__ __forceinline__ void bwd_mma(uint32_t d, uint32_t a, uint32_t b, bool accumulate) {
+    constexpr uint32_t id = umma_idesc(FMT_F16, kA, kB, 64, 64);
+    const uint64_t da = umma_desc_sw128(a, 8192), db = umma_desc_sw128(b, 8192);
+#pragma unroll
+    for (uint32_t ks = 0; ks < 4; ++ks)
+        umma_f16(d, da + ks * (kA ? 128u : 2u), db + ks * (kB ? 128u : 2u), id, (accumulate || ks > 0) ? 1u : 0u);
+}
+
+// Bounded wait for an MMA batch; on expiry the status word is set and the kernel goes on (its result is undefined).
+__device__ __forceinline__ void bwd_wait(uint32_t* ctrl, uint32_t bar, uint32_t parity) {
+    if (mbar_try_wait(bar, parity)) return;
+    const uint64_t t0 = globaltimer_ns();
+    for (uint32_t n = 0;; ++n) {
+        if (mbar_try_wait(bar, parity)) return;
+        if ((n & 63u) == 63u && globaltimer_ns() - t0 > 2000000000ull) {
+            atomicCAS(ctrl + 1, 0u, static_cast<uint32_t>(WHERE_MBAR));
+            return;
+        }
+    }
+}
+
+// token (row of the [B,T,...] tensors) at scan position p, or -1 past the end
+__device__ __forceinline__ int bwd_token(const BwdParams& P, int p) {
+    if (p >= P.T) return -1;
+    const int u = P.rev ? P.T - 1 - p : p;
+    if (P.Wc == 1) return u;
+    const int c = u / P.Hc;
+    return (u - c * P.Hc) * P.Wc + c;
+}
+
+// One chunk of `n` tensors into tiles, in the order the rows lie in memory (a reversed scan's chunk is mirrored: its first
+// token along the scan is row 63).  Rows past the sequence are filled with zeros, channels a K = 32 head does not have too.
+__device__ __forceinline__ void bwd_load(const Maps& maps, const BwdParams& P, int chunk, int b, int h, uint32_t bar, int n,
+                                         const int* tensors, const uint32_t* tiles) {
+    const BoxWalker bw(P, chunk * kChunk);
+    bw.for_each(P, [&](int id, int r, int c, int row) {
+        for (int i = 0; i < n; ++i) tma_load_5d(tiles[i] + 128u * row, &maps.m[tensors[i]][id], bar, 0, h, r, c, b);
+    });
+    bw.for_each_missing(P, [&](int id, int row) {
+        for (int i = 0; i < n; ++i) tma_load_5d(tiles[i] + 128u * row, &maps.m[tensors[i]][id], bar, 0, h, P.Hc, 0, b);
+    });
+}
+__device__ __forceinline__ void bwd_bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void bwd_bar_arrive(uint32_t id, uint32_t threads) {
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+// 16 columns of one row of a swizzled fp16 tile as they lie there
+__device__ __forceinline__ void bwd_row16(uint32_t tile, uint32_t row, uint32_t unit, uint32_t* r) {
+    const uint4 a = ld_shared_v4(sw_unit(tile, row, unit)), b = ld_shared_v4(sw_unit(tile, row, unit + 1));
+    r[0] = a.x; r[1] = a.y; r[2] = a.z; r[3] = a.w; r[4] = b.x; r[5] = b.y; r[6] = b.z; r[7] = b.w;
+}
+__device__ __forceinline__ void bwd_put16(uint32_t tile, uint32_t row, uint32_t unit, const uint32_t* r) {
+    st_shared_v4(sw_unit(tile, row, unit), r[0], r[1], r[2], r[3]);
+    st_shared_v4(sw_unit(tile, row, unit + 1), r[4], r[5], r[6], r[7]);
+}
+// Two fp32 lanes per instruction: these kernels are bound by instruction issue first.
 __device__ __forceinline__ float2 bwd_fma2(float2 a, float2 b, float2 c) {
     unsigned long long d;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d)
@@ -56,432 +178,794 @@ __device__ __forceinline__ float2 bwd_mul2(float2 a, float2 b) {
         : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)));
     return reinterpret_cast<const float2&>(d);
 }
+__device__ __forceinline__ float2 bwd_two(float x) { return make_float2(x, x); }
+__device__ __forceinline__ float2 bwd_pair(const float* x, int e) { return make_float2(x[2 * e], x[2 * e + 1]); }
+__device__ __forceinline__ float2 bwd_ex2(float2 x) { return make_float2(ex2(x.x), ex2(x.y)); }
 
-// 32 tokens x W halves of one head, 16 bytes per thread and step; rows past the sequence read as zero, which makes
-// a padded token the identity (gate 1, no update).
-template <int W>
-__device__ __forceinline__ void bwd_fetch(uint4 (&r)[W / 32], const __half* base, int64_t tok_stride, int t0, int T, int tid) {
+// a pair as a high and a low fp16 part
+__device__ __forceinline__ void bwd_split(float2 x, uint32_t& h, uint32_t& l) {
+    h = pack_half2(x.x, x.y);
+    const float2 d = bwd_fma2(unpack_half2(h), make_float2(-1.f, -1.f), x);
+    l = pack_half2(d.x, d.y);
+}
+// x[0..15] * f as a high and a low fp16 part, one row piece of two tiles
+__device__ __forceinline__ void bwd_put_split(uint32_t hi, uint32_t lo, uint32_t row, uint32_t unit, const float* x, float f = 1.f) {
+    uint32_t h[8], l[8];
 #pragma unroll
-    for (int i = 0; i < W / 32; ++i) {
-        const int idx = tid + kBwdThreads * i, row = idx / (W / 8), c8 = idx % (W / 8), t = t0 + row;
-        r[i] = t < T ? __ldg(reinterpret_cast<const uint4*>(base + t * tok_stride + c8 * 8)) : make_uint4(0u, 0u, 0u, 0u);
-    }
+    for (int i = 0; i < 8; ++i) bwd_split(bwd_mul2(bwd_pair(x, i), bwd_two(f)), h[i], l[i]);
+    bwd_put16(hi, row, unit, h);
+    bwd_put16(lo, row, unit, l);
+}
+// in[0..15] * 2^(x * mul + add) likewise: the gated operands
+__device__ __forceinline__ void bwd_put_gated(uint32_t hi, uint32_t lo, uint32_t row, uint32_t unit, const uint32_t* in, const float* x,
+                                              float mul, float add) {
+    uint32_t h[8], l[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+        bwd_split(bwd_mul2(unpack_half2(in[i]), bwd_ex2(bwd_fma2(bwd_pair(x, i), bwd_two(mul), bwd_two(add)))), h[i], l[i]);
+    bwd_put16(hi, row, unit, h);
+    bwd_put16(lo, row, unit, l);
 }
 
-template <int W, bool kExp>
-__device__ __forceinline__ void bwd_spread(float* tile, const uint4 (&r)[W / 32], float mul, int tid) {
+// largest |x| of 16 packed halves, as the bits of a half2 (both halves)
+__device__ __forceinline__ uint32_t bwd_max16(const uint32_t* r) {
+    __half2 m = __habs2(*reinterpret_cast<const __half2*>(&r[0]));
 #pragma unroll
-    for (int i = 0; i < W / 32; ++i) {
-        const int idx = tid + kBwdThreads * i, row = idx / (W / 8), c8 = idx % (W / 8);
-        const __half2* h = reinterpret_cast<const __half2*>(&r[i]);
-        float f[8];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const float2 x = __half22float2(h[e]);
-            f[2 * e] = kExp ? __expf(x.x) : x.x * mul;
-            f[2 * e + 1] = kExp ? __expf(x.y) : x.y * mul;
-        }
-        float4* dst = reinterpret_cast<float4*>(tile + row * W + c8 * 8);
-        dst[0] = make_float4(f[0], f[1], f[2], f[3]);
-        dst[1] = make_float4(f[4], f[5], f[6], f[7]);
+    for (int i = 1; i < 8; ++i) m = __hmax2(m, __habs2(*reinterpret_cast<const __half2*>(&r[i])));
+    return *reinterpret_cast<uint32_t*>(&m);
+}
+__device__ __forceinline__ float bwd_half_max(uint32_t m) {
+    const float2 f = unpack_half2(m);
+    return fmaxf(f.x, f.y);
+}
+__device__ __forceinline__ float bwd_warp_max(float x) {          // x >= 0: ordered like its bits
+    return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(x)));
+}
+// the power of two that brings m to [2^(to-1), 2^to); 1 for zero and for what is not finite
+__device__ __forceinline__ float bwd_scale(float m, int to) {
+    const int e = static_cast<int>(__float_as_uint(m) >> 23);     // biased exponent: m in [2^(e-127), 2^(e-126))
+    if (e == 0 || e == 255) return 1.f;
+    return __uint_as_float(static_cast<uint32_t>(min(max(127 + to - 1 - (e - 127), 1), 254)) << 23);
+}
+__device__ __forceinline__ float bwd_log2(float f) { return static_cast<float>(static_cast<int>(__float_as_uint(f) >> 23) - 127); }  // of a power of two
+__device__ __forceinline__ float bwd_inverse(float f) { return __uint_as_float((254u << 23) - __float_as_uint(f)); }   // of a power of two
+
+// A [64 x 64] constant operand of the gate-sum MMA: out-of-place K-major tile, entry (r, s) = value(r, s)
+template <class F>
+__device__ __forceinline__ void bwd_constant(uint8_t* tile, F value) {
+    for (int e = threadIdx.x; e < 64 * 64; e += blockDim.x) {
+        const uint32_t r = static_cast<uint32_t>(e) >> 6, s = static_cast<uint32_t>(e) & 63u;
+        *reinterpret_cast<__half*>(tile + sw_f16(r, s)) = __float2half(value(r, s));
     }
 }
-
-template <int W>
-__device__ __forceinline__ void bwd_keep(__half* tile, const uint4 (&r)[W / 32], int tid) {
-#pragma unroll
-    for (int i = 0; i < W / 32; ++i) {
-        const int idx = tid + kBwdThreads * i;
-        reinterpret_cast<uint4*>(tile)[idx] = r[i];
-    }
-}
-
-struct BwdSmem {
-    float tile[4][kBwdChunk * 64];
-    float out[kBwdChunk * 64];
-    __half raw[kBwdChunk * 64];
+// ------------------------------------------------------------------------------------------ segments' states
+// blockIdx.y 0: S after every chunk of a segment, from zero at its start:     S' = 2^G_L S + (k 2^(G_L-G))^T v
+// blockIdx.y 1: dS at a segment's start, from zero at its end (walked backwards): dS' = 2^G_L dS + scale (q 2^G)^T do
+// Bound by latency (a chunk is two dependent MMA round trips and two block barriers with little between them), then by memory:
+// hence three CTAs per SM (66 KB each) and the next chunk's tiles in flight meanwhile.  3.9 TB/s at B4 H12 T6400.
+struct BwdStateSmem {
+    static constexpr int kStage = 3 * kTileBytes;                                      // a (k or q), b (v or do), g
+    static constexpr int kLow = 2 * kStage, kMat = kLow + kTileBytes, kMisc = kMat + kTileBytes;
+    static constexpr int kBytes = kMisc + 1024 + 1024;                                 // misc, alignment
 };
+struct BwdStateMisc {
+    uint64_t full[2], bar_x, bar_inc;
+    uint32_t tmem;
+    uint32_t top[8];                  // per warp: largest |a|, as half2 bits
+    alignas(16) float gl[64];         // log2 decay of the chunk per channel
+};
+static_assert(sizeof(BwdStateMisc) <= 1024, "misc block too large");
 
-// Sum over the 8 lanes of a group (lane bits 0..2) of R values each lane holds, by a butterfly that halves the values
-// kept at every exchange: 4 shuffles for R = 4, 3 for R = 2.  Every lane ends with the complete sum of value `which`.
-template <int R>
-__device__ __forceinline__ float bwd_reduce8(const float (&v)[R], int lane, int& which) {
-    constexpr unsigned kAll = 0xffffffffu;
-    const bool b2 = (lane & 4) != 0, b1 = (lane & 2) != 0;
-    float k;
-    if (R == 4) {
-        float k0 = b2 ? v[R - 2] : v[0], k1 = b2 ? v[R - 1] : v[1];
-        const float s0 = b2 ? v[0] : v[R - 2], s1 = b2 ? v[1] : v[R - 1];
-        k0 += __shfl_xor_sync(kAll, s0, 4);
-        k1 += __shfl_xor_sync(kAll, s1, 4);
-        k = b1 ? k1 : k0;
-        k += __shfl_xor_sync(kAll, b1 ? k0 : k1, 2);
-        which = (b2 ? 2 : 0) + (b1 ? 1 : 0);
-    } else {
-        k = b2 ? v[R - 1] : v[0];
-        k += __shfl_xor_sync(kAll, b2 ? v[0] : v[R - 1], 4);
-        k += __shfl_xor_sync(kAll, k, 2);
-        which = b2 ? 1 : 0;
+template <int K>
+__global__ void __launch_bounds__(kBwdThreads, 3) gla_bwd_state_kernel(const __grid_constant__ Maps maps, const __grid_constant__ BwdParams P) {
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t raw = smem_u32(smem_raw), base = (raw + 1023u) & ~1023u;
+    uint8_t* base_ptr = smem_raw + (base - raw);
+    BwdStateMisc& M = *reinterpret_cast<BwdStateMisc*>(base_ptr + BwdStateSmem::kMisc);
+    const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
+    const bool back = blockIdx.y != 0;
+    const int bh = blockIdx.x / P.nseg, seg = blockIdx.x - bh * P.nseg;
+    const int first = seg * P.cps, n = min(P.cps, P.NT - first);
+    if (back && seg == 0) return;                                  // nothing before it needs its gradient
+    if (blockIdx.x == 0 && tid < 2) P.ctrl[tid] = 0u;
+
+    const int b = bh / P.H, h = bh - b * P.H;
+    const bool rev = P.rev != 0;
+
+    if (tid == 0) {
+        mbar_init(smem_u32(&M.full[0]), 1);
+        mbar_init(smem_u32(&M.full[1]), 1);
+        mbar_init(smem_u32(&M.bar_x), 1);
+        mbar_init(smem_u32(&M.bar_inc), 1);
+        fence_mbar_init();
     }
-    k += __shfl_xor_sync(kAll, k, 1);
-    return k;
-}
-
-template <int N>
-__device__ __forceinline__ void bwd_lds(float (&d)[N], const float* src) {
-    if (N == 2) {
-        const float2 u = *reinterpret_cast<const float2*>(src);
-        d[0] = u.x; d[1] = u.y;
-    } else {
-#pragma unroll
-        for (int i = 0; i < N / 4; ++i) {
-            const float4 u = reinterpret_cast<const float4*>(src)[i];
-            d[4 * i] = u.x; d[4 * i + 1] = u.y; d[4 * i + 2] = u.z; d[4 * i + 3] = u.w;
-        }
+    if (w == 0) {
+        tmem_alloc(smem_u32(&M.tmem), 64);
+        tmem_relinquish();
     }
-}
-
-// Kinds 0 and 1.  A thread owns an R x 8 block of the K x 64 state (R = K / 16): 16 row groups x 8 column groups, the 8
-// column groups of a row group in neighbouring lanes.  Per token it reads its R gates and key-side factors and its 8 + 8
-// value-side entries (6 shared-memory reads of 16 bytes), and the R row sums are completed across the 8 lanes.
-//   kind 0 (forward in t):   S = a S + b x ,  acc = S . y     a = exp(g_t), b = k_t,        x = v_t,  y = do_t
-//   kind 1 (backward in t):  S = S + b x ,    acc = S . y ,  S = a S     a = exp(g_t), b = scale q_t, x = do_t, y = v_t
-// With kStateOnly the sweep starts from zero, emits nothing per token and leaves the segment's own contribution to the
-// state, and the product of its gates, for gla_bwd_combine_kernel.
-template <int K, int kKind, bool kStateOnly>
-__device__ void bwd_row_sweep(const BwdParams& P, BwdSmem& sm, int bh, int seg) {
-    constexpr int R = K / 16;
-    constexpr bool kFwd = kKind == 0;
-    const int tid = threadIdx.x, lane = tid & 31, cg = tid & 7, rg = tid >> 3;
-    const int b = bh / P.H, h = bh % P.H;
-    const int t_begin = seg * P.seg_len, T = min(P.T, t_begin + P.seg_len);        // this CTA's tokens: [t_begin, T)
-    const int64_t strideK = static_cast<int64_t>(P.H) * K, strideV = static_cast<int64_t>(P.H) * 64;
-    const int64_t offK = (static_cast<int64_t>(b) * P.T * P.H + h) * K, offV = (static_cast<int64_t>(b) * P.T * P.H + h) * 64;
-    const __half* pa = P.g + offK;                                  // gate
-    const __half* pb = (kFwd ? P.k : P.q) + offK;                   // the rank-one update's key-side factor
-    const __half* px = (kFwd ? P.v : P.d_o) + offV;                 // its value-side factor
-    const __half* py = (kFwd ? P.d_o : P.v) + offV;                 // what the state is contracted with
-    const __half* pr = (kFwd ? P.q : P.k) + offK;                   // the factor of the gate-gradient product
-    __half* pout = (kFwd ? P.dq : P.dk) + offK;
-    float* pprod = (kFwd ? P.qdq : P.kdk) + offK;
-    const int block_off = R * rg * 64 + 8 * cg;                     // this thread's block inside a [K,64] state
-    const int64_t state_off = static_cast<int64_t>(bh) * K * 64 + block_off;
-    const int64_t seg_slot = (static_cast<int64_t>(kFwd ? 0 : P.B * P.H) + bh) * P.nseg + seg;
-
-    float2 S[R][4];
-    float decay[R];
-    const float* init = kStateOnly ? nullptr
-                        : P.nseg > 1 ? P.seg_start + seg_slot * K * 64 + block_off
-                        : (kFwd ? P.h0 : P.dht) ? (kFwd ? P.h0 : P.dht) + state_off : nullptr;
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        decay[r] = 1.f;
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-            S[r][c] = init ? *reinterpret_cast<const float2*>(init + r * 64 + 2 * c) : make_float2(0.f, 0.f);
-    }
-
-    const int nchunks = (T - t_begin + kBwdChunk - 1) / kBwdChunk;
-    uint4 ra[K / 32], rb[K / 32], rr[K / 32], rx[2], ry[2];
-    auto fetch = [&](int ci) {
-        const int t0 = t_begin + (kFwd ? ci : nchunks - 1 - ci) * kBwdChunk;
-        bwd_fetch<K>(ra, pa, strideK, t0, T, tid);
-        bwd_fetch<K>(rb, pb, strideK, t0, T, tid);
-        bwd_fetch<64>(rx, px, strideV, t0, T, tid);
-        if (!kStateOnly) {
-            bwd_fetch<K>(rr, pr, strideK, t0, T, tid);
-            bwd_fetch<64>(ry, py, strideV, t0, T, tid);
-        }
+    // log factor of a row: the gates after it (forward), its own and those before it (backward), along the scan
+    bwd_constant(base_ptr + BwdStateSmem::kMat, [&](uint32_t r, uint32_t s) { return (back ? (rev ? s >= r : s <= r) : (rev ? s < r : s > r)) ? 1.f : 0.f; });
+    fence_proxy_async_smem();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = M.tmem;
+    auto chunk_of = [&](int i) { return first + (back ? n - 1 - i : i); };
+    auto load = [&](int i) {
+        const uint32_t s = base + (i & 1) * BwdStateSmem::kStage, bar = smem_u32(&M.full[i & 1]);
+        const int tensors[3] = {TG, back ? TQ : TK, back ? TO : TV};
+        const uint32_t tiles[3] = {s + 2 * kTileBytes, s, s + kTileBytes};
+        mbar_arrive_expect_tx(bar, 3 * kTileBytes);
+        bwd_load(maps, P, chunk_of(i), b, h, bar, 3, tensors, tiles);
     };
-    if (nchunks > 0) fetch(0);
-    for (int ci = 0; ci < nchunks; ++ci) {
-        const int t0 = t_begin + (kFwd ? ci : nchunks - 1 - ci) * kBwdChunk;
-        bwd_spread<K, true>(sm.tile[0], ra, 1.f, tid);
-        bwd_spread<K, false>(sm.tile[1], rb, kFwd ? 1.f : P.scale, tid);
-        bwd_spread<64, false>(sm.tile[2], rx, 1.f, tid);
-        if (!kStateOnly) {
-            bwd_spread<64, false>(sm.tile[3], ry, 1.f, tid);
-            bwd_keep<K>(sm.raw, rr, tid);
+    if (w == 0 && elect_one()) load(0);
+
+    const uint32_t row = 16u * (w & 3) + (l & 15u), c0 = 32u * (w >> 2) + 16u * (static_cast<uint32_t>(l) >> 4), u0 = c0 >> 3;
+    float S[16], total = 0.f;          // a state row piece: channel `row`, columns c0 .. +15
+#pragma unroll
+    for (int e = 0; e < 16; ++e) S[e] = 0.f;
+    const size_t cslot = static_cast<size_t>(bh) * P.NT;
+    const uint32_t low = base + BwdStateSmem::kLow, mat = base + BwdStateSmem::kMat;
+
+    for (int i = 0; i < n; ++i) {
+        const int st = i & 1;
+        const uint32_t ta = base + st * BwdStateSmem::kStage, tb = ta + kTileBytes, tg = tb + kTileBytes;
+        bwd_wait(P.ctrl, smem_u32(&M.full[st]), (i >> 1) & 1);
+        if (w == 0 && elect_one()) {
+            tc_fence_after();
+            bwd_mma<0, 1>(bwd_slot(tmem, 0), mat, tg, false);
+            umma_commit(smem_u32(&M.bar_x));
+            if (i + 1 < n) load(i + 1);
         }
-        __syncthreads();
-        if (ci + 1 < nchunks) fetch(ci + 1);
-#pragma unroll 4
-        for (int tt = 0; tt < kBwdChunk; ++tt) {
-            const int t = kFwd ? tt : kBwdChunk - 1 - tt;
-            float a[R], bq[R], x[8], y[8], v[R];
-            bwd_lds<R>(a, &sm.tile[0][t * K + R * rg]);
-            bwd_lds<R>(bq, &sm.tile[1][t * K + R * rg]);
-            bwd_lds<8>(x, &sm.tile[2][t * 64 + 8 * cg]);
-            if (kStateOnly) {
+        uint32_t a[8];
+        bwd_row16(ta, row, u0, a);
+        {
+            const uint32_t m = __reduce_max_sync(0xffffffffu, __float_as_uint(bwd_half_max(bwd_max16(a))));
+            if (l == 0) M.top[w] = m;
+        }
+        bwd_wait(P.ctrl, smem_u32(&M.bar_x), i & 1);
+        tc_fence_after();
+        float x[16];
+        bwd_read(tmem, 0, w, x);
+        tmem_ld_wait();
+        __syncthreads();                                            // every warp's maximum is there
+        uint32_t m = M.top[0];
 #pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    const float2 aa = make_float2(a[r], a[r]), bb = make_float2(bq[r], bq[r]);
-                    decay[r] *= a[r];
+        for (int j = 1; j < 8; ++j) m = max(m, M.top[j]);
+        const float f = bwd_scale(__uint_as_float(m), 15);
+        if (row == ((back != rev) ? 63u : 0u)) {                             // x + own gate (forward), x (backward) = G_L
+            uint32_t gr[8];
+            bwd_row16(tg, row, u0, gr);
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        const float2 x2 = make_float2(x[2 * c], x[2 * c + 1]);
-                        if (kFwd) S[r][c] = bwd_fma2(S[r][c], aa, bwd_mul2(bb, x2));
-                        else S[r][c] = bwd_mul2(bwd_fma2(bb, x2, S[r][c]), aa);
-                    }
-                }
-                continue;
+            for (int e = 0; e < 8; ++e) {
+                const float2 gf = unpack_half2(gr[e]);
+                M.gl[c0 + 2 * e] = (x[2 * e] + (back ? 0.f : gf.x)) * kLog2e;
+                M.gl[c0 + 2 * e + 1] = (x[2 * e + 1] + (back ? 0.f : gf.y)) * kLog2e;
             }
-            bwd_lds<8>(y, &sm.tile[3][t * 64 + 8 * cg]);
-#pragma unroll
-            for (int r = 0; r < R; ++r) {
-                const float2 aa = make_float2(a[r], a[r]), bb = make_float2(bq[r], bq[r]);
-                float2 acc = make_float2(0.f, 0.f);
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const float2 x2 = make_float2(x[2 * c], x[2 * c + 1]), y2 = make_float2(y[2 * c], y[2 * c + 1]);
-                    if (kFwd) S[r][c] = bwd_fma2(S[r][c], aa, bwd_mul2(bb, x2));
-                    else S[r][c] = bwd_fma2(bb, x2, S[r][c]);
-                    acc = bwd_fma2(S[r][c], y2, acc);
-                    if (!kFwd) S[r][c] = bwd_mul2(S[r][c], aa);
-                }
-                v[r] = acc.x + acc.y;
-            }
-            int which;
-            const float sum = bwd_reduce8<R>(v, lane, which);
-            if (!(lane & 1)) sm.out[t * K + R * rg + which] = sum;
         }
-        if (kStateOnly) {
-            __syncthreads();
-            continue;
-        }
+        bwd_put_gated(ta, low, row, u0, a, x, kLog2e, bwd_log2(f));
+        fence_proxy_async_smem();
+        tc_fence_before();
         __syncthreads();
-        // the chunk's gradient rows, and their products with q (k) for the gate gradient
+        if (w == 0 && elect_one()) {
+            tc_fence_after();
+            bwd_mma<1, 1>(bwd_slot(tmem, 1), ta, tb, false);
+            bwd_mma<1, 1>(bwd_slot(tmem, 1), low, tb, true);
+            umma_commit(smem_u32(&M.bar_inc));
+        }
+        const float gl = M.gl[row], decay = ex2(gl), c = (back ? P.scale : 1.f) * bwd_inverse(f);
+        total += gl;
+        bwd_wait(P.ctrl, smem_u32(&M.bar_inc), i & 1);
+        tc_fence_after();
+        bwd_read(tmem, 1, w, x);
+        tmem_ld_wait();
+        tc_fence_before();
 #pragma unroll
-        for (int i = 0; i < K / 32; ++i) {
-            const int idx = tid + kBwdThreads * i, r = idx / (K / 8), c8 = idx % (K / 8), t = t0 + r;
-            if (t < T) {
-                const float4 u0 = *reinterpret_cast<const float4*>(&sm.out[r * K + c8 * 8]);
-                const float4 u1 = *reinterpret_cast<const float4*>(&sm.out[r * K + c8 * 8 + 4]);
-                const float mul = kFwd ? P.scale : 1.f;
-                const float d[8] = {u0.x * mul, u0.y * mul, u0.z * mul, u0.w * mul, u1.x * mul, u1.y * mul, u1.z * mul, u1.w * mul};
-                const uint4 rw = reinterpret_cast<const uint4*>(sm.raw)[idx];
-                const __half2* hr = reinterpret_cast<const __half2*>(&rw);
-                uint4 packed;
-                __half2* hp = reinterpret_cast<__half2*>(&packed);
-                float pr8[8];
+        for (int e = 0; e < 8; ++e) {
+            const float2 s = bwd_fma2(bwd_two(decay), bwd_pair(S, e), bwd_mul2(bwd_two(c), bwd_pair(x, e)));
+            S[2 * e] = s.x; S[2 * e + 1] = s.y;
+        }
+        if (!back) {
+            const size_t at = cslot + chunk_of(i);
+            float4* dst = reinterpret_cast<float4*>(P.chunk_state + at * 4096) + tid;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) dst[e * kBwdThreads] = make_float4(S[4 * e], S[4 * e + 1], S[4 * e + 2], S[4 * e + 3]);
+            if (c0 == 0) P.chunk_decay[at * 64 + row] = total;
+        }
+    }
+    if (back) {
+        const size_t at = static_cast<size_t>(bh) * P.nseg + seg;
+        float4* dst = reinterpret_cast<float4*>(P.seg_grad + at * 4096) + tid;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) dst[e * kBwdThreads] = make_float4(S[4 * e], S[4 * e + 1], S[4 * e + 2], S[4 * e + 3]);
+        if (c0 == 0) P.seg_decay[at * 64 + row] = total;
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (w == 0) tmem_dealloc(tmem, 64);
+}
+
+// ------------------------------------------------------------------------------------------ the gradient
+struct BwdChunkSmem {
+    static constexpr int kG = 0, kQ = kTileBytes, kK = 2 * kTileBytes, kV = 3 * kTileBytes, kDo = 4 * kTileBytes;
+    static constexpr int kQl = 5 * kTileBytes, kKl = 6 * kTileBytes;
+    // four tiles, used in turn for St and dSt, for P and dP (high and low parts each), and, as 64 x 64 fp32, for the terms of dg
+    static constexpr int kR = 7 * kTileBytes, kMat = 11 * kTileBytes;
+    static constexpr int kS0 = 12 * kTileBytes;                       // the state the segment starts from, fp32, each thread's own piece
+    static constexpr int kMisc = 14 * kTileBytes;
+    // no slack: dynamic shared memory starts on a 1024-byte boundary when a kernel has no other (checked at run time), and two
+    // CTAs of 113 KB fill an SM
+    static constexpr int kBytes = kMisc + 1024;
+};
+struct BwdChunkMisc {
+    uint64_t full, bar_x, bar_a, bar_s, bar_o;
+    uint32_t tmem;
+    // per chunk: largest |q|, |k|, |v|, |do|, |S|, |dS| as float bits, and whether the chunk needs the pair-by-pair path
+    uint32_t top[2][8];
+    alignas(16) float vec[64];        // log2: half the chunk's total decay per channel
+    int tok[64];                      // the chunk's tokens by row, -1 past the end
+    alignas(16) float decay[64];      // log2 decay from the segment's start to the chunk's start
+};
+static_assert(sizeof(BwdChunkMisc) <= 1024, "misc block too large");
+enum { BWD_BAR_COMPUTE = 1, BWD_BAR_GATED = 2, BWD_BAR_STATES = 3, BWD_BAR_SCORES = 4, BWD_BAR_READ = 5 };     // named barriers
+enum { BWD_X = 0, BWD_P = 1, BWD_DP = 2, BWD_DQ_S = 3, BWD_DK_S = 4, BWD_DV_S = 5, BWD_INC = 6, BWD_DQ_I = 7 };
+
+// a 64 x 64 fp32 tile whose 16-byte units are permuted by the row, so that both row pieces and columns are read without
+// bank conflicts
+__device__ __forceinline__ uint32_t bwd_f32(uint32_t tile, uint32_t row, uint32_t col) {
+    return tile + row * 256u + ((((col >> 2) ^ row) & 15u) << 4) + ((col & 3u) << 2);
+}
+__device__ __forceinline__ void bwd_f32_put16(uint32_t tile, uint32_t row, uint32_t c0, const float* x) {
+#pragma unroll
+    for (uint32_t e = 0; e < 4; ++e) st_shared_f4(bwd_f32(tile, row, c0 + 4 * e), x[4 * e], x[4 * e + 1], x[4 * e + 2], x[4 * e + 3]);
+}
+__device__ __forceinline__ void bwd_f32_row16(uint32_t tile, uint32_t row, uint32_t c0, float* x) {
+#pragma unroll
+    for (uint32_t e = 0; e < 4; ++e) {
+        const float4 v = ld_shared_f4(bwd_f32(tile, row, c0 + 4 * e));
+        x[4 * e] = v.x; x[4 * e + 1] = v.y; x[4 * e + 2] = v.z; x[4 * e + 3] = v.w;
+    }
+}
+
+// A chunk with a strong decay, pair by pair in fp32: P (scaled by fq fk, into its accumulator), and the part of dq and dk that
+// comes from within the chunk (into BWD_DQ_I and BWD_DP, complete); q and k are then rewritten with the references 0 and G_L,
+// whose exponents are never positive.  Out of line; about 30 k cycles a chunk, so a sequence of nothing but such chunks takes
+// some five times the usual time.
+__device__ __noinline__ void bwd_wide_chunk(uint32_t base, const float* vec, uint32_t tmem, float fq, float fk, float scale,
+                                            bool rev) {
+    const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
+    const uint32_t row = 16u * (w & 3) + (l & 15u), c0 = 32u * (w >> 2) + 16u * (static_cast<uint32_t>(l) >> 4), u0 = c0 >> 3;
+    const uint32_t tg = base + BwdChunkSmem::kG, tq = base + BwdChunkSmem::kQ, tk = base + BwdChunkSmem::kK;
+    const uint32_t dp = base + BwdChunkSmem::kR, out = dp + 2 * kTileBytes;
+    float x[16];
+    auto sync = [] { named_bar_sync(BWD_BAR_COMPUTE, kBwdThreads); };
+    auto at = [&](int t) { return static_cast<uint32_t>(rev ? 63 - t : t); };     // row of the chunk's t-th token
+    uint32_t qr[8], kr[8];
+    bwd_row16(tq, row, u0, qr);
+    bwd_row16(tk, row, u0, kr);
+    bwd_read(tmem, BWD_DP, w, x);
+    tmem_ld_wait();
+    bwd_f32_put16(dp, row, c0, x);
+    sync();
+    // four neighbouring lanes share a row, 16 channels each
+    const int i = tid >> 2;                                // the i-th token
+    const uint32_t ch = 16u * (tid & 3), cu = ch >> 3;
+    float acc[16], D[16];
+    {
+        uint32_t own[8];
+        bwd_row16(tq, at(i), cu, own);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) acc[e] = D[e] = 0.f;
+        for (int s = 0; s < 64; ++s) {
+            const int j = i - s;
+            float a = 0.f;
+            if (j >= 0) {
+                uint32_t kk[8], gg[8];
+                bwd_row16(tk, at(j), cu, kk);
+                bwd_row16(tg, at(j), cu, gg);
+                const float d = ld_shared_f(bwd_f32(dp, at(i), at(j)));
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    const float2 kf = unpack_half2(kk[e]), qf = unpack_half2(own[e]), gf = unpack_half2(gg[e]);
+                    const float k0 = kf.x * ex2(D[2 * e]), k1 = kf.y * ex2(D[2 * e + 1]);
+                    a = fmaf(qf.x, k0, fmaf(qf.y, k1, a));
+                    acc[2 * e] = fmaf(d, k0, acc[2 * e]);
+                    acc[2 * e + 1] = fmaf(d, k1, acc[2 * e + 1]);
+                    D[2 * e] = fmaf(gf.x, kLog2e, D[2 * e]);
+                    D[2 * e + 1] = fmaf(gf.y, kLog2e, D[2 * e + 1]);
+                }
+            }
+            a += __shfl_xor_sync(0xffffffffu, a, 1);
+            a += __shfl_xor_sync(0xffffffffu, a, 2);
+            if ((tid & 3) == 0)
+                asm volatile("st.shared.f32 [%0], %1;" ::"r"(bwd_f32(out, at(i), at(j >= 0 ? j : s))), "f"(a * fq * fk) : "memory");
+        }
+    }
+    sync();
+    bwd_f32_row16(out, row, c0, x);
+    bwd_write(tmem, BWD_P, w, x);
+    sync();
+#pragma unroll
+    for (int e = 0; e < 16; ++e) acc[e] *= scale;
+    bwd_f32_put16(out, at(i), ch, acc);
+    sync();
+    bwd_f32_row16(out, row, c0, x);
+    bwd_write(tmem, BWD_DQ_I, w, x);
+#pragma unroll
+    for (int e = 0; e < 16; ++e) acc[e] = D[e] = 0.f;
+    for (int t = i; t < 64; ++t) {
+        uint32_t qq[8], gg[8];
+        if (t > i) {
+            bwd_row16(tg, at(t), cu, gg);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const float2 gf = unpack_half2(gg[e]);
+                D[2 * e] = fmaf(gf.x, kLog2e, D[2 * e]);
+                D[2 * e + 1] = fmaf(gf.y, kLog2e, D[2 * e + 1]);
+            }
+        }
+        bwd_row16(tq, at(t), cu, qq);
+        const float d = ld_shared_f(bwd_f32(dp, at(t), at(i))) * scale;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const float2 qf = unpack_half2(qq[e]);
+            acc[2 * e] = fmaf(d, qf.x * ex2(D[2 * e]), acc[2 * e]);
+            acc[2 * e + 1] = fmaf(d, qf.y * ex2(D[2 * e + 1]), acc[2 * e + 1]);
+        }
+    }
+    sync();
+    bwd_f32_put16(out, at(i), ch, acc);
+    sync();
+    bwd_f32_row16(out, row, c0, x);
+    bwd_write(tmem, BWD_DP, w, x);
+    float gsum[16];
+    bwd_read(tmem, BWD_X, w, gsum);
+    tmem_ld_wait();
+#pragma unroll
+    for (int e = 0; e < 16; ++e) x[e] = fmaf(gsum[e], kLog2e, vec[c0 + e]);
+    bwd_put_gated(tq, base + BwdChunkSmem::kQl, row, u0, qr, x, 1.f, bwd_log2(fq));
+#pragma unroll
+    for (int e = 0; e < 16; ++e) x[e] = fmaf(gsum[e], -kLog2e, vec[c0 + e]);
+    bwd_put_gated(tk, base + BwdChunkSmem::kKl, row, u0, kr, x, 1.f, bwd_log2(fk));
+    tmem_st_wait();
+}
+
+constexpr int kBwdChunkThreads = kBwdThreads + 32;       // eight compute warps, one that issues MMAs and copies
+
+// Per chunk (walked from the segment's last to its first), compute warps | issuing warp:
+//   tiles landed:  maxima of the tiles and states    | X = G - G_L/2 and dP = do v^T
+//   St, dSt as split operands                        | do St^T, v dSt^T
+//   qt, kt as split operands                         | P = qt kt^T, qt^T do, kt dSt
+//   P, dP masked, as split operands                  | P^T do, dP kt, dP^T qt
+//   dS to the chunk's start                          | next chunk's copies once those have run
+//   outputs; dg                                      |
+// The compute warps hand operands over with an arrival and never wait for one another to do so.
+template <int K>
+__global__ void __launch_bounds__(kBwdChunkThreads, 2) gla_bwd_chunk_kernel(const __grid_constant__ Maps maps, const __grid_constant__ BwdParams P) {
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t base = smem_u32(smem_raw);
+    uint8_t* base_ptr = smem_raw;
+    if ((base & 1023u) != 0u) {                                        // never with this kernel's shared memory, see kBytes
+        if (threadIdx.x == 0) atomicCAS(P.ctrl + 1, 0u, static_cast<uint32_t>(WHERE_MBAR));
+        return;
+    }
+    BwdChunkMisc& M = *reinterpret_cast<BwdChunkMisc*>(base_ptr + BwdChunkSmem::kMisc);
+    const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
+    const int bh = blockIdx.x / P.nseg, seg = blockIdx.x - bh * P.nseg;
+    const int first = seg * P.cps, n = min(P.cps, P.NT - first);
+    const int b = bh / P.H, h = bh - b * P.H;
+    const bool rev = P.rev != 0;
+    const size_t cslot = static_cast<size_t>(bh) * P.NT;
+    const uint32_t tg = base + BwdChunkSmem::kG, tq = base + BwdChunkSmem::kQ, tk = base + BwdChunkSmem::kK, tv = base + BwdChunkSmem::kV,
+                   tdo = base + BwdChunkSmem::kDo, ql = base + BwdChunkSmem::kQl, kl = base + BwdChunkSmem::kKl,
+                   r0 = base + BwdChunkSmem::kR, r1 = r0 + kTileBytes, r2 = r1 + kTileBytes, r3 = r2 + kTileBytes;
+
+    if (tid == 0) {
+        mbar_init(smem_u32(&M.full), 1);
+        mbar_init(smem_u32(&M.bar_x), 1);
+        mbar_init(smem_u32(&M.bar_a), 1);
+        mbar_init(smem_u32(&M.bar_s), 1);
+        mbar_init(smem_u32(&M.bar_o), 1);
+        fence_mbar_init();
+    }
+    if (w == 0) {
+        tmem_alloc(smem_u32(&M.tmem), 256);
+        tmem_relinquish();
+    }
+    bwd_constant(base_ptr + BwdChunkSmem::kMat, [&](uint32_t r, uint32_t s) { return (rev ? s >= r : s <= r) ? 0.5f : -0.5f; });      // G - G_L / 2
+    if (tid < 16) M.top[tid >> 3][tid & 7] = 0u;
+    fence_proxy_async_smem();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = M.tmem;
+
+    if (w == kBwdThreads / 32) {
+        // ==================================================================== issuing warp
+        const uint32_t sx = bwd_slot(tmem, BWD_X), sp = bwd_slot(tmem, BWD_P), sdp = bwd_slot(tmem, BWD_DP), sdq = bwd_slot(tmem, BWD_DQ_S),
+                       sdk = bwd_slot(tmem, BWD_DK_S), sdv = bwd_slot(tmem, BWD_DV_S), sinc = bwd_slot(tmem, BWD_INC), sdqi = bwd_slot(tmem, BWD_DQ_I);
+        // chunk i's tiles, and the state after chunk i - 1 (relative to the segment's start) into r2, r3
+        auto load = [&](int i) {
+            const uint32_t bar = smem_u32(&M.full);
+            mbar_arrive_expect_tx(bar, i > 0 ? 7 * kTileBytes + 256 : 5 * kTileBytes);
+            const int tensors[5] = {TG, TO, TV, TQ, TK};
+            const uint32_t tiles[5] = {tg, tdo, tv, tq, tk};
+            bwd_load(maps, P, first + i, b, h, bar, 5, tensors, tiles);
+            if (i > 0) {
+                bwd_bulk_load(r2, P.chunk_state + (cslot + first + i - 1) * 4096, 2 * kTileBytes, bar);
+                bwd_bulk_load(smem_u32(M.decay), P.chunk_decay + (cslot + first + i - 1) * 64, 256, bar);
+            }
+        };
+        if (elect_one()) load(n - 1);
+        __syncwarp();
+        for (int i = n - 1, it = 0; i >= 0; --i, ++it) {
+            const uint32_t ph = it & 1;
+            bwd_wait(P.ctrl, smem_u32(&M.full), ph);
+            if (it > 0) named_bar_sync(BWD_BAR_READ, kBwdChunkThreads);            // the previous chunk's accumulators are read
+            tc_fence_after();
+            if (elect_one()) {
+                bwd_mma<0, 1>(sx, base + BwdChunkSmem::kMat, tg, false);
+                bwd_mma<0, 0>(sdp, tdo, tv, false);
+                umma_commit(smem_u32(&M.bar_x));
+            }
+            named_bar_sync(BWD_BAR_STATES, kBwdChunkThreads);
+            tc_fence_after();
+            const bool wide = M.top[i & 1][6] != 0u;
+            if (elect_one()) {
+                bwd_mma<0, 0>(sdq, tdo, r0, false);
+                bwd_mma<0, 0>(sdq, tdo, r1, true);
+                bwd_mma<0, 0>(sdk, tv, r2, false);
+                bwd_mma<0, 0>(sdk, tv, r3, true);
+            }
+            named_bar_sync(BWD_BAR_GATED, kBwdChunkThreads);
+            tc_fence_after();
+            if (elect_one()) {
+                if (!wide) {
+                    bwd_mma<0, 0>(sp, tq, tk, false);
+                    bwd_mma<0, 0>(sp, tq, kl, true);
+                    bwd_mma<0, 0>(sp, ql, tk, true);
+                }
+                umma_commit(smem_u32(&M.bar_a));
+                bwd_mma<1, 1>(sinc, tq, tdo, false);
+                bwd_mma<1, 1>(sinc, ql, tdo, true);
+                bwd_mma<0, 1>(sdv, tk, r2, false);
+                bwd_mma<0, 1>(sdv, tk, r3, true);
+                bwd_mma<0, 1>(sdv, kl, r2, true);
+                umma_commit(smem_u32(&M.bar_s));
+            }
+            named_bar_sync(BWD_BAR_SCORES, kBwdChunkThreads);
+            tc_fence_after();
+            if (elect_one()) {
+                const uint32_t dv = wide ? sp : sdp;
+                bwd_mma<1, 1>(dv, r0, tdo, false);
+                bwd_mma<1, 1>(dv, r1, tdo, true);
+                if (!wide) {
+                    bwd_mma<0, 1>(sdqi, r2, tk, false);
+                    bwd_mma<0, 1>(sdqi, r2, kl, true);
+                    bwd_mma<0, 1>(sdqi, r3, tk, true);
+                    bwd_mma<1, 1>(sp, r2, tq, false);
+                    bwd_mma<1, 1>(sp, r2, ql, true);
+                    bwd_mma<1, 1>(sp, r3, tq, true);
+                }
+                umma_commit(smem_u32(&M.bar_o));
+            }
+            __syncwarp();
+            bwd_wait(P.ctrl, smem_u32(&M.bar_o), ph);
+            if (i > 0 && elect_one()) load(i - 1);
+            __syncwarp();
+        }
+    } else {
+        // ==================================================================== compute warps
+        // This thread's piece of every 64 x 64 array: row `row`, columns c0 .. c0 + 15.  A row is a token (scores, gradients) or
+        // a key channel (states).
+        const uint32_t row = 16u * (w & 3) + (l & 15u), c0 = 32u * (w >> 2) + 16u * (static_cast<uint32_t>(l) >> 4), u0 = c0 >> 3;
+        const bool real_row = row < K;
+        auto sync = [] { named_bar_sync(BWD_BAR_COMPUTE, kBwdThreads); };
+        auto hand_over = [](uint32_t id) {                   // operands written by this thread may be read by the tensor core
+            fence_proxy_async_smem();
+            tc_fence_before();
+            bwd_bar_arrive(id, kBwdChunkThreads);
+        };
+        float dS[16];                 // the state gradient at the end of the current chunk
+        const uint32_t s0_at = base + BwdChunkSmem::kS0 + 16u * tid;           // float4 e of this thread 4096 bytes apart
+        auto own = [&](uint32_t at, float* x) {
+#pragma unroll
+            for (uint32_t e = 0; e < 4; ++e) {
+                const float4 v = ld_shared_f4(at + 16u * kBwdThreads * e);
+                x[4 * e] = v.x; x[4 * e + 1] = v.y; x[4 * e + 2] = v.z; x[4 * e + 3] = v.w;
+            }
+        };
+        auto get = [&](const float* src, int step, float* x) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float4 v = __ldcg(reinterpret_cast<const float4*>(src) + e * step);
+                x[4 * e] = v.x; x[4 * e + 1] = v.y; x[4 * e + 2] = v.z; x[4 * e + 3] = v.w;
+            }
+        };
+        auto chain = [&](float* x, float f, const float* y) {                // x = f x + y
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const float2 z = bwd_fma2(bwd_two(f), bwd_pair(x, e), bwd_pair(y, e));
+                x[2 * e] = z.x; x[2 * e + 1] = z.y;
+            }
+        };
+        const size_t state_off = (static_cast<size_t>(bh) * K + row) * 64 + c0;
+        {
+            float S0[16];
+#pragma unroll
+            for (int e = 0; e < 16; ++e) S0[e] = dS[e] = 0.f;
+            if (P.h0 != nullptr && real_row) get(P.h0 + state_off, 1, S0);
+            if (P.dht != nullptr && real_row) get(P.dht + state_off, 1, dS);
+#pragma unroll 2
+            for (int j = 0; j < seg; ++j) {
+                const size_t at = cslot + static_cast<size_t>(j + 1) * P.cps - 1;
+                float y[16];
+                get(P.chunk_state + at * 4096 + 4 * tid, kBwdThreads, y);
+                chain(S0, ex2(__ldcg(P.chunk_decay + at * 64 + row)), y);
+            }
+#pragma unroll 2
+            for (int j = P.nseg - 1; j > seg; --j) {
+                const size_t at = static_cast<size_t>(bh) * P.nseg + j;
+                float y[16];
+                get(P.seg_grad + at * 4096 + 4 * tid, kBwdThreads, y);
+                chain(dS, ex2(__ldcg(P.seg_decay + at * 64 + row)), y);
+            }
+#pragma unroll
+            for (uint32_t e = 0; e < 4; ++e) st_shared_f4(s0_at + 16u * kBwdThreads * e, S0[4 * e], S0[4 * e + 1], S0[4 * e + 2], S0[4 * e + 3]);
+            float later = 0.f;
+            if (P.dht != nullptr || seg + 1 < P.nseg) {                  // dS is not zero at the segment's end
+                float y[16];
+                const size_t at = cslot + first + n - 1;
+                get(P.chunk_state + at * 4096 + 4 * tid, kBwdThreads, y);
+                chain(S0, ex2(__ldcg(P.chunk_decay + at * 64 + row)), y);          // now the state after the segment
+#pragma unroll
+                for (int e = 0; e < 16; ++e) later = fmaf(S0[e], dS[e], later);
+                later += __shfl_xor_sync(0xffffffffu, later, 16);
+            }
+            // halves of the sum, per channel, by way of a tile that is not in use yet
+            if (l < 16) asm volatile("st.shared.f32 [%0], %1;" ::"r"(kl + 256u * (w >> 2) + 4u * row), "f"(later) : "memory");
+        }
+        sync();
+        float later = ld_shared_f(kl + 4u * (tid & 63)) + ld_shared_f(kl + 256u + 4u * (tid & 63));         // dg's share of all later tokens, channel tid & 63
+        const uint32_t decay_at = smem_u32(M.decay);
+        const uint32_t tok_at = smem_u32(M.tok);
+        const long long head_row = (static_cast<long long>(b) * P.T * P.H + h) * K;
+        const uint32_t last_row = rev ? 0u : 63u;
+        const int above = 32 * (w >> 2) - 16 * (w & 3);                  // first column - first row of this warp's piece
+        const bool on_diagonal = above == 0 || above == -16;
+        const bool beyond = rev ? above < -16 : above > 0;               // wholly on the masked side of the diagonal
+
+        for (int i = n - 1, it = 0; i >= 0; --i, ++it) {
+            const int p = i & 1;
+            const uint32_t ph = it & 1;
+            bwd_wait(P.ctrl, smem_u32(&M.full), ph);
+            uint32_t qr[8], kr[8];
+            float S[16], x[16];
+            own(s0_at, S);
+            if (i > 0) {
+                own(r2 + 16u * tid, x);
+                chain(S, ex2(ld_shared_f(decay_at + 4u * row)), x);
+            }
+            bwd_row16(tq, row, u0, qr);
+            bwd_row16(tk, row, u0, kr);
+            {
+                float m[6];
+                uint32_t t[8];
+                m[0] = bwd_half_max(bwd_max16(qr));
+                m[1] = bwd_half_max(bwd_max16(kr));
+                bwd_row16(tv, row, u0, t);
+                m[2] = bwd_half_max(bwd_max16(t));
+                bwd_row16(tdo, row, u0, t);
+                m[3] = bwd_half_max(bwd_max16(t));
+                m[4] = m[5] = 0.f;
+#pragma unroll
+                for (int e = 0; e < 16; ++e) {
+                    m[4] = fmaxf(m[4], fabsf(S[e]));
+                    m[5] = fmaxf(m[5], fabsf(dS[e]));
+                }
+                uint32_t mine = 0u;
+#pragma unroll
+                for (int j = 0; j < 6; ++j) {
+                    const uint32_t r = __reduce_max_sync(0xffffffffu, __float_as_uint(m[j]));
+                    if (l == j) mine = r;
+                }
+                if (l < 6) atomicMax(&M.top[p][l], mine);
+            }
+            bwd_wait(P.ctrl, smem_u32(&M.bar_x), ph);
+            tc_fence_after();
+            bwd_read(tmem, BWD_X, w, x);
+            tmem_ld_wait();
+            if (row == last_row) {                                      // X of the last row is half the chunk's decay
+                bool far = false;
+#pragma unroll
+                for (int e = 0; e < 16; ++e) {
+                    const float half_decay = x[e] * kLog2e;
+                    M.vec[c0 + e] = half_decay;
+                    far = far || !(-half_decay <= kBwdRefLimit);
+                }
+                if (far) M.top[p][6] = 1u;
+            }
+            sync();                                                     // maxima, decay and the wide flag are complete
+            const float fq = bwd_scale(__uint_as_float(M.top[p][0]), 6), fk = bwd_scale(__uint_as_float(M.top[p][1]), 6);
+            const float fp = 0.125f, fd = bwd_scale(__uint_as_float(M.top[p][2]), 5) * bwd_scale(__uint_as_float(M.top[p][3]), 4);
+            const float fS = bwd_scale(__uint_as_float(M.top[p][4]), 15), fdS = bwd_scale(__uint_as_float(M.top[p][5]), 15);
+            const bool wide = M.top[p][6] != 0u;
+            if (wide) {
+                // out of line, and everything a register holds across the call is fetched again afterwards: the ordinary chunk
+                // must not pay for it with spills (the SM's shared memory leaves no L1 to catch them)
+                float* park = P.park + (static_cast<size_t>(bh) * P.nseg + seg) * 8192 + 4 * tid;
+                uint4* raw = reinterpret_cast<uint4*>(park + 4096);
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    *reinterpret_cast<float4*>(park + 4 * kBwdThreads * e) = make_float4(dS[4 * e], dS[4 * e + 1], dS[4 * e + 2], dS[4 * e + 3]);
+                raw[0] = make_uint4(qr[0], qr[1], qr[2], qr[3]);
+                raw[kBwdThreads] = make_uint4(qr[4], qr[5], qr[6], qr[7]);
+                raw[2 * kBwdThreads] = make_uint4(kr[0], kr[1], kr[2], kr[3]);
+                raw[3 * kBwdThreads] = make_uint4(kr[4], kr[5], kr[6], kr[7]);
+                bwd_wide_chunk(base, M.vec, tmem, fq, fk, P.scale, rev);
+                sync();
+                get(park, kBwdThreads, dS);
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    const float2 f = __half22float2(hr[e]);
-                    hp[e] = __floats2half2_rn(d[2 * e], d[2 * e + 1]);
-                    pr8[2 * e] = f.x * d[2 * e];
-                    pr8[2 * e + 1] = f.y * d[2 * e + 1];
+                    const uint4 v = __ldcg(raw + e * kBwdThreads);
+                    uint32_t* to = e < 2 ? qr + 4 * e : kr + 4 * (e - 2);
+                    to[0] = v.x; to[1] = v.y; to[2] = v.z; to[3] = v.w;
                 }
-                *reinterpret_cast<uint4*>(pout + t * strideK + c8 * 8) = packed;
-                float4* pp = reinterpret_cast<float4*>(pprod + t * strideK + c8 * 8);
-                pp[0] = make_float4(pr8[0], pr8[1], pr8[2], pr8[3]);
-                pp[1] = make_float4(pr8[4], pr8[5], pr8[6], pr8[7]);
+                own(s0_at, S);
+                if (i > 0) {
+                    get(P.chunk_state + (cslot + first + i - 1) * 4096 + 4 * tid, kBwdThreads, x);
+                    chain(S, ex2(__ldcg(P.chunk_decay + (cslot + first + i - 1) * 64 + row)), x);
+                }
             }
-        }
-        __syncthreads();
-    }
-    if (kStateOnly) {
+            const float half_decay = M.vec[row], eR = ex2(half_decay);
+            bwd_put_split(r0, r1, row, u0, S, (wide ? 1.f : eR) * fS);
+            bwd_put_split(r2, r3, row, u0, dS, (wide ? 1.f : eR) * fdS);
+            hand_over(BWD_BAR_STATES);
+            if (!wide) {
+                bwd_read(tmem, BWD_X, w, x);
+                tmem_ld_wait();
+                bwd_put_gated(tq, ql, row, u0, qr, x, kLog2e, bwd_log2(fq));
+                bwd_put_gated(tk, kl, row, u0, kr, x, -kLog2e, bwd_log2(fk));
+            }
+            hand_over(BWD_BAR_GATED);
+            // ---- within the chunk: P and dP, causal, as split operands
+            bwd_wait(P.ctrl, smem_u32(&M.bar_a), ph);
+            tc_fence_after();
+            if (!beyond) {
+                float y[16];
+                bwd_read(tmem, BWD_P, w, x);
+                bwd_read(tmem, BWD_DP, w, y);                           // (of no use in a wide chunk)
+                tmem_ld_wait();
+                if (on_diagonal) {
+                    const int lim = static_cast<int>(row) - static_cast<int>(c0);
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-                *reinterpret_cast<float2*>(P.seg_state + seg_slot * K * 64 + block_off + r * 64 + 2 * c) = S[r][c];
-            if (cg == 0) P.seg_decay[seg_slot * K + R * rg + r] = decay[r];
-        }
-    } else if (kFwd) {
-        if (P.g_last && seg == P.nseg - 1) {                      // S is the final state here
-            float v[R];
-#pragma unroll
-            for (int r = 0; r < R; ++r) {
-                float acc = 0.f;
-                if (P.dht) {
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        const float2 d = *reinterpret_cast<const float2*>(P.dht + state_off + r * 64 + 2 * c);
-                        acc = fmaf(d.x, S[r][c].x, fmaf(d.y, S[r][c].y, acc));
+                    for (int e = 0; e < 16; ++e) {
+                        const bool keep = rev ? e >= lim : e <= lim;
+                        x[e] = keep ? x[e] : 0.f;
+                        y[e] = keep ? y[e] : 0.f;
                     }
                 }
-                v[r] = acc;
+                bwd_put_split(r0, r1, row, u0, x, fp);                  // St has been read since bar_a, dSt will have with bar_s
+                bwd_wait(P.ctrl, smem_u32(&M.bar_s), ph);
+                bwd_put_split(r2, r3, row, u0, y, fd);
+            } else {
+                const uint32_t z[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+                bwd_put16(r0, row, u0, z); bwd_put16(r1, row, u0, z);
+                bwd_wait(P.ctrl, smem_u32(&M.bar_s), ph);
+                bwd_put16(r2, row, u0, z); bwd_put16(r3, row, u0, z);
             }
-            int which;
-            const float sum = bwd_reduce8<R>(v, lane, which);
-            if (!(lane & 1)) P.g_last[static_cast<int64_t>(bh) * K + R * rg + which] = sum;
-        }
-    } else if (P.dh0 && seg == 0) {
+            hand_over(BWD_BAR_SCORES);
+            // ---- the state gradient moves to the chunk's start
+            if (tid < 8) M.top[p ^ 1][tid] = 0u;
+            bwd_read(tmem, BWD_INC, w, x);
+            tmem_ld_wait();
+            {
+                const float keep = eR * eR, c = (wide ? 1.f : eR) * P.scale * bwd_inverse(fq);
 #pragma unroll
-        for (int r = 0; r < R; ++r)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) *reinterpret_cast<float2*>(P.dh0 + state_off + r * 64 + 2 * c) = S[r][c];
-    }
-}
-
-// Kind 2.  A thread owns a (K / 8) x 4 block of dS: 8 row groups in neighbouring lanes x 16 column groups.  Its rows are
-// 4 rg .. 4 rg + 3 (and 32 + the same for K = 64), so that the 8 lanes' 16-byte reads of the key-side tiles fall on distinct
-// banks.  The 4 column sums are completed across the 8 lanes.
-//   S = S + bq x ,  acc = S^T kk ,  S = a S      a = exp(g_t), bq = scale q_t, kk = k_t (over the rows),  x = do_t (over the columns)
-template <int K>
-__device__ void bwd_col_sweep(const BwdParams& P, BwdSmem& sm, int bh, int seg) {
-    constexpr int RC = K / 8;
-    const int tid = threadIdx.x, lane = tid & 31, rg = tid & 7, cg = tid >> 3;
-    const int b = bh / P.H, h = bh % P.H;
-    const int t_begin = seg * P.seg_len, T = min(P.T, t_begin + P.seg_len);
-    const int64_t strideK = static_cast<int64_t>(P.H) * K, strideV = static_cast<int64_t>(P.H) * 64;
-    const int64_t offK = (static_cast<int64_t>(b) * P.T * P.H + h) * K, offV = (static_cast<int64_t>(b) * P.T * P.H + h) * 64;
-    const __half *pa = P.g + offK, *pq = P.q + offK, *pk = P.k + offK, *px = P.d_o + offV;
-    __half* pout = P.dv + offV;
-
-    float2 S[RC][2];
-    const float* init = P.nseg > 1 ? P.seg_start + ((static_cast<int64_t>(P.B) * P.H + bh) * P.nseg + seg) * K * 64
-                        : P.dht ? P.dht + static_cast<int64_t>(bh) * K * 64 : nullptr;
-#pragma unroll
-    for (int r = 0; r < RC; ++r) {
-        const int row = (r / 4) * 32 + 4 * rg + (r % 4);
-#pragma unroll
-        for (int c = 0; c < 2; ++c)
-            S[r][c] = init ? *reinterpret_cast<const float2*>(init + row * 64 + 4 * cg + 2 * c) : make_float2(0.f, 0.f);
-    }
-
-    const int nchunks = (T - t_begin + kBwdChunk - 1) / kBwdChunk;
-    uint4 ra[K / 32], rq[K / 32], rk[K / 32], rx[2];
-    auto fetch = [&](int ci) {
-        const int t0 = t_begin + (nchunks - 1 - ci) * kBwdChunk;
-        bwd_fetch<K>(ra, pa, strideK, t0, T, tid);
-        bwd_fetch<K>(rq, pq, strideK, t0, T, tid);
-        bwd_fetch<K>(rk, pk, strideK, t0, T, tid);
-        bwd_fetch<64>(rx, px, strideV, t0, T, tid);
-    };
-    if (nchunks > 0) fetch(0);
-    for (int ci = 0; ci < nchunks; ++ci) {
-        const int t0 = t_begin + (nchunks - 1 - ci) * kBwdChunk;
-        bwd_spread<K, true>(sm.tile[0], ra, 1.f, tid);
-        bwd_spread<K, false>(sm.tile[1], rq, P.scale, tid);
-        bwd_spread<K, false>(sm.tile[2], rk, 1.f, tid);
-        bwd_spread<64, false>(sm.tile[3], rx, 1.f, tid);
-        __syncthreads();
-        if (ci + 1 < nchunks) fetch(ci + 1);
-#pragma unroll 4
-        for (int tt = 0; tt < kBwdChunk; ++tt) {
-            const int t = kBwdChunk - 1 - tt;
-            float a[RC], qq[RC], kk[RC], x[4];
-#pragma unroll
-            for (int i = 0; i < RC / 4; ++i) {
-                bwd_lds<4>(reinterpret_cast<float(&)[4]>(a[4 * i]), &sm.tile[0][t * K + 32 * i + 4 * rg]);
-                bwd_lds<4>(reinterpret_cast<float(&)[4]>(qq[4 * i]), &sm.tile[1][t * K + 32 * i + 4 * rg]);
-                bwd_lds<4>(reinterpret_cast<float(&)[4]>(kk[4 * i]), &sm.tile[2][t * K + 32 * i + 4 * rg]);
-            }
-            bwd_lds<4>(x, &sm.tile[3][t * 64 + 4 * cg]);
-            const float2 x2[2] = {make_float2(x[0], x[1]), make_float2(x[2], x[3])};
-            float2 acc[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-#pragma unroll
-            for (int r = 0; r < RC; ++r) {
-                const float2 q2 = make_float2(qq[r], qq[r]), k2 = make_float2(kk[r], kk[r]), a2 = make_float2(a[r], a[r]);
-#pragma unroll
-                for (int c = 0; c < 2; ++c) {
-                    S[r][c] = bwd_fma2(q2, x2[c], S[r][c]);
-                    acc[c] = bwd_fma2(S[r][c], k2, acc[c]);
-                    S[r][c] = bwd_mul2(S[r][c], a2);
+                for (int e = 0; e < 8; ++e) {
+                    const float2 z = bwd_fma2(bwd_two(keep), bwd_pair(dS, e), bwd_mul2(bwd_two(c), bwd_pair(x, e)));
+                    dS[2 * e] = z.x; dS[2 * e + 1] = z.y;
                 }
             }
-            const float v[4] = {acc[0].x, acc[0].y, acc[1].x, acc[1].y};
-            int which;
-            const float sum = bwd_reduce8<4>(v, lane, which);
-            if (!(lane & 1)) sm.out[t * 64 + 4 * cg + which] = sum;
-        }
-        __syncthreads();
+            const int tok = bwd_token(P, (first + i) * kChunk + (rev ? 63 - static_cast<int>(row) : static_cast<int>(row)));
+            const bool live = tok >= 0 && c0 < K;
+            if (c0 == 0) st_shared_u32(tok_at + 4u * row, static_cast<uint32_t>(tok));
+            const long long at = (static_cast<long long>(b) * P.T + max(tok, 0)) * P.H + h;          // in units of one head's row
+            const float iS = bwd_inverse(fS), idS = bwd_inverse(fdS), ifd = bwd_inverse(fd), ifq = bwd_inverse(fq), ifk = bwd_inverse(fk);
+            bwd_wait(P.ctrl, smem_u32(&M.bar_o), ph);
+            tc_fence_after();
+            // ---- outputs, eight columns at a time
+            const int slot_dv = wide ? BWD_P : BWD_DP, slot_dk = wide ? BWD_DP : BWD_P;
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const int idx = tid + kBwdThreads * i, r = idx / 8, c8 = idx % 8, t = t0 + r;
-            if (t < T) {
-                const float4 u0 = *reinterpret_cast<const float4*>(&sm.out[r * 64 + c8 * 8]);
-                const float4 u1 = *reinterpret_cast<const float4*>(&sm.out[r * 64 + c8 * 8 + 4]);
-                uint4 packed;
-                __half2* hp = reinterpret_cast<__half2*>(&packed);
-                hp[0] = __floats2half2_rn(u0.x, u0.y); hp[1] = __floats2half2_rn(u0.z, u0.w);
-                hp[2] = __floats2half2_rn(u1.x, u1.y); hp[3] = __floats2half2_rn(u1.z, u1.w);
-                *reinterpret_cast<uint4*>(pout + t * strideV + c8 * 8) = packed;
+            for (int hf = 0; hf < 2; ++hf) {
+                float a[8], y[8], g[8], D[8];
+                uint32_t o[4];
+                // one of dk, dq: gate factor 2^(sign X) (2^(sign X + R) for the state part alone in a wide chunk) times the sum
+                // of state part and chunk part
+                auto finish = [&](int slot_s, int slot_i, float cs, float ci, float sign, const uint32_t* in, __half* out) {
+                    bwd_read8(tmem, slot_s, w, 8 * hf, a);
+                    bwd_read8(tmem, slot_i, w, 8 * hf, y);
+                    if (sign < 0.f) bwd_read8(tmem, BWD_X, w, 8 * hf, g);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        float2 z;
+                        if (!wide) {
+                            z = bwd_fma2(bwd_two(cs), bwd_pair(a, e), bwd_mul2(bwd_two(ci), bwd_pair(y, e)));
+                            z = bwd_mul2(z, bwd_ex2(bwd_mul2(bwd_pair(g, e), bwd_two(sign * kLog2e))));
+                        } else {
+                            const float2 r = make_float2(M.vec[c0 + 8 * hf + 2 * e], M.vec[c0 + 8 * hf + 2 * e + 1]);
+                            z = bwd_mul2(bwd_pair(a, e), bwd_two(cs));
+                            z = bwd_fma2(z, bwd_ex2(bwd_fma2(bwd_pair(g, e), bwd_two(sign * kLog2e), r)), bwd_pair(y, e));
+                        }
+                        o[e] = pack_half2(z.x, z.y);
+                        const float2 f = unpack_half2(sign > 0.f ? in[4 * hf + e] : in[4 * hf + e] ^ 0x80008000u);
+                        z = sign > 0.f ? bwd_fma2(f, z, bwd_pair(D, e)) : bwd_mul2(f, z);
+                        D[2 * e] = z.x; D[2 * e + 1] = z.y;
+                    }
+                    if (live) *reinterpret_cast<uint4*>(out + at * K + c0 + 8 * hf) = make_uint4(o[0], o[1], o[2], o[3]);
+                };
+                finish(BWD_DK_S, slot_dk, idS, P.scale * ifd * ifq, -1.f, kr, P.dk);
+                finish(BWD_DQ_S, BWD_DQ_I, P.scale * iS, P.scale * ifd * ifk, 1.f, qr, P.dq);
+                st_shared_f4(bwd_f32(r0, row, c0 + 8 * hf), D[0], D[1], D[2], D[3]);
+                st_shared_f4(bwd_f32(r0, row, c0 + 8 * hf + 4), D[4], D[5], D[6], D[7]);
+                bwd_read8(tmem, BWD_DV_S, w, 8 * hf, a);
+                bwd_read8(tmem, slot_dv, w, 8 * hf, y);
+                tmem_ld_wait();
+                const float2 cs = bwd_two(ifk * idS), ci = bwd_two(P.scale * ifq * ifk * 8.f);      // 8 = 1 / fp
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float2 z = bwd_fma2(cs, bwd_pair(a, e), bwd_mul2(ci, bwd_pair(y, e)));
+                    o[e] = pack_half2(z.x, z.y);
+                }
+                if (tok >= 0) *reinterpret_cast<uint4*>(P.dv + at * 64 + c0 + 8 * hf) = make_uint4(o[0], o[1], o[2], o[3]);
+            }
+            tc_fence_before();
+            if (i > 0) bwd_bar_arrive(BWD_BAR_READ, kBwdChunkThreads);
+            sync();
+            // ---- dg: sums of the terms of the tokens at and after each token, a quarter of the rows per thread and channel,
+            // handed back to the rows' owners through the tiles of the low parts
+            {
+                const uint32_t c = tid & 63u, q4 = static_cast<uint32_t>(tid) >> 6;
+                float t[16], run = 0.f;
+                if (!rev) {
+#pragma unroll
+                    for (int r = 15; r >= 0; --r) t[r] = run += ld_shared_f(bwd_f32(r0, 16u * q4 + r, c));
+                } else {
+#pragma unroll
+                    for (int r = 0; r < 16; ++r) t[r] = run += ld_shared_f(bwd_f32(r0, 16u * q4 + r, c));
+                }
+                const uint32_t part = kl + 4u * c;                      // [4][64] sums of 16 rows
+                asm volatile("st.shared.f32 [%0], %1;" ::"r"(part + 256u * q4), "f"(run) : "memory");
+                sync();
+                float add = later;
+#pragma unroll
+                for (uint32_t j = 0; j < 4; ++j) {
+                    const float s = ld_shared_f(part + 256u * j);
+                    add += (rev ? j < q4 : j > q4) ? s : 0.f;
+                    later += s;
+                }
+                if (c < K) {
+#pragma unroll
+                    for (int r = 0; r < 16; ++r) {
+                        const int o = static_cast<int>(ld_shared_u32(tok_at + 4u * (16u * q4 + r)));
+                        if (o < 0) continue;
+                        const long long at = head_row + static_cast<long long>(o) * (P.H * K) + c;
+                        if (P.dg_half != nullptr) P.dg_half[at] = __float2half_rn(t[r] + add);
+                        else P.dg[at] = t[r] + add;
+                    }
+                }
             }
         }
-        __syncthreads();
-    }
-}
-
-template <int K>
-__global__ void __launch_bounds__(kBwdThreads) gla_bwd_sweep_kernel(const BwdParams P) {
-    __shared__ __align__(16) BwdSmem sm;
-    const int bh = blockIdx.x / P.nseg, seg = blockIdx.x % P.nseg, kind = blockIdx.y;
-    if (kind == 0) bwd_row_sweep<K, 0, false>(P, sm, bh, seg);
-    else if (kind == 1) bwd_row_sweep<K, 1, false>(P, sm, bh, seg);
-    else bwd_col_sweep<K>(P, sm, bh, seg);
-}
-
-// Sequences cut into segments (few sequences, many tokens): every segment but the last in sweep order first runs alone
-// from a zero state (this kernel: S of segments 0 .. nseg-2 forward, dS of segments 1 .. nseg-1 backward) ...
-template <int K>
-__global__ void __launch_bounds__(kBwdThreads) gla_bwd_state_kernel(const BwdParams P) {
-    __shared__ __align__(16) BwdSmem sm;
-    const int bh = blockIdx.x / (P.nseg - 1), i = blockIdx.x % (P.nseg - 1);
-    if (blockIdx.y == 0) bwd_row_sweep<K, 0, true>(P, sm, bh, i);
-    else bwd_row_sweep<K, 1, true>(P, sm, bh, i + 1);
-}
-
-// ... then the segments' contributions are chained, S' = decay * S + own, into the state each segment starts from
-// (seg_start, laid out like seg_state), which gla_bwd_sweep_kernel picks up.  blockIdx.y: 0 forward states, 1 backward;
-// one state element per thread, so the loads of a thread do not depend on one another.
-template <int K>
-__global__ void __launch_bounds__(256) gla_bwd_combine_kernel(const BwdParams P) {
-    const int bh = blockIdx.x, back = blockIdx.y, nseg = P.nseg;
-    const int e = blockIdx.z * 256 + threadIdx.x, row = e / 64;
-    const int64_t slot0 = (static_cast<int64_t>(back ? P.B * P.H : 0) + bh) * nseg;
-    const float* __restrict__ own = P.seg_state + slot0 * K * 64 + e;
-    float* __restrict__ start = P.seg_start + slot0 * K * 64 + e;
-    const float* __restrict__ dec = P.seg_decay + slot0 * K + row;
-    const float* init = back ? P.dht : P.h0;
-    float S = init ? init[static_cast<int64_t>(bh) * K * 64 + e] : 0.f;
-    if (!back) {
-#pragma unroll 4
-        for (int j = 0; j < nseg - 1; ++j) {
-            start[static_cast<int64_t>(j) * K * 64] = S;
-            S = fmaf(__ldg(dec + j * K), S, __ldg(own + static_cast<int64_t>(j) * K * 64));
+        if (P.dh0 != nullptr && seg == 0 && real_row) {
+            float4* dst = reinterpret_cast<float4*>(P.dh0 + state_off);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) dst[e] = make_float4(dS[4 * e], dS[4 * e + 1], dS[4 * e + 2], dS[4 * e + 3]);
         }
-        start[static_cast<int64_t>(nseg - 1) * K * 64] = S;
-    } else {
-#pragma unroll 4
-        for (int j = nseg - 1; j > 0; --j) {
-            start[static_cast<int64_t>(j) * K * 64] = S;
-            S = fmaf(__ldg(dec + j * K), S, __ldg(own + static_cast<int64_t>(j) * K * 64));
-        }
-        start[0] = S;
     }
-}
-
-// dg_t = sum_{s >= t} (q_s dq_s - k_s dk_s), per (batch, head, channel).  One CTA per (batch, head, kCh channels):
-// 1024 / kCh slices of the sequence, each summed on its own first, then walked backwards from the total of the slices
-// after it.  kCh = K reads whole rows (many sequences); kCh = 16 gives four times the CTAs (few, long sequences).
-template <int K, int kCh>
-__global__ void __launch_bounds__(1024) gla_bwd_dg_kernel(const BwdParams P) {
-    constexpr int kSlices = 1024 / kCh;
-    __shared__ float total[kSlices][kCh];
-    const int bh = blockIdx.x, b = bh / P.H, h = bh % P.H, T = P.T;
-    const int cl = threadIdx.x % kCh, c = blockIdx.y * kCh + cl, s = threadIdx.x / kCh;
-    const int64_t stride = static_cast<int64_t>(P.H) * K, off = (static_cast<int64_t>(b) * T * P.H + h) * K + c;
-    const float* __restrict__ pq = P.qdq + off;
-    const float* __restrict__ pk = P.kdk + off;
-    float* __restrict__ pg = P.dg + off;
-    const int per = (T + kSlices - 1) / kSlices, lo = s * per, hi = min(T, lo + per);
-    const float last = P.g_last ? P.g_last[static_cast<int64_t>(bh) * K + c] : 0.f;
-    float sum = 0.f;
-#pragma unroll 8
-    for (int t = lo; t < hi; ++t) sum += __ldg(pq + t * stride) - __ldg(pk + t * stride);
-    if (lo < T && hi == T) sum += last;
-    total[s][cl] = sum;
+    tc_fence_before();
     __syncthreads();
-    float run = 0.f;
-    for (int j = s + 1; j < kSlices; ++j) run += total[j][cl];
-    if (lo < T && hi == T) run += last;
-#pragma unroll 8
-    for (int t = hi - 1; t >= lo; --t) {
-        run += __ldg(pq + t * stride) - __ldg(pk + t * stride);
-        pg[t * stride] = run;
-    }
+    if (w == 0) tmem_dealloc(tmem, 256);
 }
 
 }  // namespace gla

@@ -241,15 +241,16 @@ __device__ __forceinline__ void warp_arrive(uint64_t* bar, int lane) {
 struct BoxWalker {
     int u_lo;     // scan position of the chunk's first row (may be negative for the ragged chunk of a reversed scan)
     int c, r;     // column and row inside the column of max(u_lo, 0)
-    __device__ __forceinline__ BoxWalker(const Params& P, int p0) {
+    template <class P_t>
+    __device__ __forceinline__ BoxWalker(const P_t& P, int p0) {
         u_lo = P.rev ? (P.T - p0 - kChunk) : p0;
         const int u0 = max(u_lo, 0);
         c = u0 / P.Hc;
         r = u0 - c * P.Hc;
     }
     // boxes over the rows the sequence has
-    template <class F>
-    __device__ __forceinline__ void for_each(const Params& P, F f) const {
+    template <class P_t, class F>
+    __device__ __forceinline__ void for_each(const P_t& P, F f) const {
         int u0 = max(u_lo, 0);
         const int u1 = min(u_lo + kChunk, P.T);
         int cc = c, rr = r;
@@ -268,8 +269,8 @@ struct BoxWalker {
     }
     // boxes over the rows of the tile the sequence does not have (loads only): placed out of bounds, the copy
     // engine fills them with zeros.  f(box_id, smem_row)
-    template <class F>
-    __device__ __forceinline__ void for_each_missing(const Params& P, F f) const {
+    template <class P_t, class F>
+    __device__ __forceinline__ void for_each_missing(const P_t& P, F f) const {
         int row = u_lo < 0 ? 0 : min(u_lo + kChunk, P.T) - u_lo;        // first missing tile row
         int len = u_lo < 0 ? -u_lo : kChunk - row;
         while (len > 0) {
@@ -281,7 +282,8 @@ struct BoxWalker {
         }
     }
     // one chunk back along the scan
-    __device__ __forceinline__ void retreat(const Params& P) {
+    template <class P_t>
+    __device__ __forceinline__ void retreat(const P_t& P) {
         if (!P.rev) {
             u_lo -= kChunk;
             r -= kChunk;
@@ -294,7 +296,8 @@ struct BoxWalker {
             while (r >= P.Hc) { r -= P.Hc; ++c; }
         }
     }
-    __device__ __forceinline__ void advance(const Params& P) {
+    template <class P_t>
+    __device__ __forceinline__ void advance(const P_t& P) {
         if (!P.rev) {
             u_lo += kChunk;
             r += kChunk;

@@ -9,10 +9,13 @@
 #include <ATen/core/grad_mode.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <cmath>
 #include <cstring>
+#include <optional>
+#include <stdexcept>
 
 #include "gla_b200.h"
 
@@ -23,6 +26,9 @@ constexpr int64_t kV = GLA_B200_HEAD_V;
 
 decltype(&gla_b200_forward) g_forward = nullptr;
 decltype(&gla_b200_workspace_bytes) g_workspace_bytes = nullptr;
+decltype(&gla_b200_backward_scan) g_backward = nullptr;
+decltype(&gla_b200_backward_workspace_bytes) g_backward_workspace_bytes = nullptr;
+decltype(&gla_b200_strerror) g_strerror = nullptr;
 
 // The tensor inside a Python object, or null when it is not a plain torch.Tensor / Parameter.
 const at::Tensor* tensor(PyObject* o) {
@@ -137,9 +143,106 @@ PyObject* run(PyObject*, PyObject* const* v, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
+struct LibraryError : std::runtime_error {
+    int code;
+    explicit LibraryError(int c) : std::runtime_error(g_strerror(c)), code(c) {}
+};
+void check(int rc) {
+    if (rc != GLA_B200_OK) throw LibraryError(rc);
+}
+void* stream_of(const at::Tensor& x) { return c10::cuda::getCurrentCUDAStream(x.device().index()).stream(); }
+
+// What a call is besides its tensors.
+struct Call {
+    double scale, norm;
+    int32_t direction, grid_h, grid_w, segments;
+    bool final_wanted;
+};
+
+// Output, final state (undefined unless wanted) and scratch of one call; the scratch need not be cleared.
+std::pair<at::Tensor, at::Tensor> forward(gla_b200_args& a, const at::Tensor& q, const at::Tensor* s0, const Call& c) {
+    const c10::cuda::CUDAGuard guard(q.device());
+    const auto opts = at::TensorOptions().device(q.device());
+    a.direction = c.direction; a.grid_h = c.grid_h; a.grid_w = c.grid_w;
+    a.segments = c.segments;
+    a.scale = static_cast<float>(c.scale);
+    a.gk_normalizer = static_cast<float>(c.norm);
+    if (s0) a.initial_state = static_cast<const float*>(s0->data_ptr());
+    at::Tensor o = at::empty({a.B, a.T, a.H, kV}, opts.dtype(at::kHalf)), final_state;
+    if (c.final_wanted) {
+        final_state = at::empty({a.B, a.H, a.K, kV}, opts.dtype(at::kFloat));
+        a.final_state = static_cast<float*>(final_state.data_ptr());
+    }
+    a.o = o.data_ptr();
+    a.workspace_bytes = g_workspace_bytes(a.B, a.T, a.H, a.K, a.V);
+    const at::Tensor ws = at::empty({static_cast<int64_t>(a.workspace_bytes)}, opts.dtype(at::kByte));
+    a.workspace = ws.data_ptr();
+    check(g_forward(&a, stream_of(q)));
+    return {o, final_state};
+}
+
+// The call under autograd: the gradient is gla_b200_backward_scan on the same tokens in the same scan order.
+struct ChunkGLA : torch::autograd::Function<ChunkGLA> {
+    static torch::autograd::variable_list forward(torch::autograd::AutogradContext* ctx, const at::Tensor& q, const at::Tensor& k,
+                                                  const at::Tensor& v, const at::Tensor& g, const std::optional<at::Tensor>& s0,
+                                                  const Call* c) {
+        gla_b200_args a;
+        std::memset(&a, 0, sizeof(a));
+        if (!operands(a, q, k, v, g)) throw LibraryError(GLA_B200_ERR_ARG);
+        const auto r = ::forward(a, q, s0 ? &*s0 : nullptr, *c);
+        ctx->save_for_backward({q, k, v, g, s0 ? *s0 : at::Tensor()});
+        ctx->saved_data["scale"] = c->scale;
+        ctx->saved_data["norm"] = c->norm;
+        ctx->saved_data["scan"] = at::IValue(c10::List<int64_t>({c->direction, c->grid_h, c->grid_w}));
+        ctx->saved_data["state"] = s0 && s0->requires_grad();
+        if (!c->final_wanted) return {r.first};
+        return {r.first, r.second};
+    }
+
+    static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
+        const auto saved = ctx->get_saved_variables();
+        const at::Tensor &q = saved[0], &k = saved[1], &v = saved[2], &s0 = saved[4];
+        at::Tensor g = saved[3], logits;
+        const c10::cuda::CUDAGuard guard(q.device());
+        const double norm = ctx->saved_data["norm"].toDouble();
+        const auto scan = ctx->saved_data["scan"].toIntList();
+        const bool state_wanted = ctx->saved_data["state"].toBool();
+        if (norm > 0.0) {                        // the forward kernel turned raw logits into log-space gates itself
+            logits = g.to(at::kFloat);
+            g = (at::log_sigmoid(logits) / norm).to(at::kHalf);
+        }
+        const at::Tensor qc = q.contiguous(), kc = k.contiguous(), vc = v.contiguous(), gc = g.contiguous();
+        const at::Tensor d_o = grads[0].to(at::kHalf).contiguous();
+        const at::Tensor d_final = grads.size() > 1 ? grads[1].to(at::kFloat).contiguous() : at::Tensor();
+        gla_b200_bwd_args a;
+        std::memset(&a, 0, sizeof(a));
+        a.B = static_cast<int32_t>(q.size(0)); a.T = static_cast<int32_t>(q.size(1)); a.H = static_cast<int32_t>(q.size(2));
+        a.K = static_cast<int32_t>(q.size(3)); a.V = static_cast<int32_t>(kV);
+        const auto opts = qc.options();
+        at::Tensor dq = at::empty(qc.sizes(), opts), dk = at::empty(qc.sizes(), opts), dv = at::empty(vc.sizes(), opts);
+        at::Tensor dg = at::empty(qc.sizes(), logits.defined() ? opts.dtype(at::kFloat) : opts), ds0;
+        if (state_wanted) ds0 = at::empty(s0.sizes(), opts.dtype(at::kFloat));
+        const size_t bytes = g_backward_workspace_bytes(a.B, a.T, a.H, a.K, a.V);
+        const at::Tensor ws = at::empty({static_cast<int64_t>(bytes)}, opts.dtype(at::kByte));
+        a.q = qc.data_ptr(); a.k = kc.data_ptr(); a.v = vc.data_ptr(); a.g = gc.data_ptr(); a.d_o = d_o.data_ptr();
+        a.dq = dq.data_ptr(); a.dk = dk.data_ptr(); a.dv = dv.data_ptr(); a.dg = static_cast<float*>(dg.data_ptr());
+        a.initial_state = s0.defined() ? static_cast<const float*>(s0.data_ptr()) : nullptr;
+        a.d_final_state = d_final.defined() ? static_cast<const float*>(d_final.data_ptr()) : nullptr;
+        a.d_initial_state = state_wanted ? static_cast<float*>(ds0.data_ptr()) : nullptr;
+        a.workspace = ws.data_ptr();
+        a.workspace_bytes = bytes;
+        a.scale = static_cast<float>(ctx->saved_data["scale"].toDouble());
+        gla_b200_bwd_scan o;
+        o.direction = static_cast<int32_t>(scan[0]); o.grid_h = static_cast<int32_t>(scan[1]); o.grid_w = static_cast<int32_t>(scan[2]);
+        o.dg_is_half = logits.defined() ? 0 : 1;
+        check(g_backward(&a, &o, stream_of(q)));
+        if (logits.defined()) dg = (dg * at::sigmoid(-logits) / norm).to(at::kHalf);      // d logsigmoid(x) / dx = sigmoid(-x)
+        return {dq, dk, dv, dg, ds0, at::Tensor()};
+    }
+};
+
 // gla(q, k, v, g, scale, initial_state, output_final_state, direction, grid_hw, gk_normalizer, segments) ->
-// (o, final_state or None), a library error, or kSlow.  The FLA-style call outside autograd: allocates output, scratch and
-// final state.  The scratch need not be cleared (the launch clears what must be).
+// (o, final_state or None), a library error, or kSlow.  The FLA-style call, recorded for autograd where a gradient is wanted.
 PyObject* gla(PyObject*, PyObject* const* v, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     if (n != 11) return PyLong_FromLong(kSlow);
@@ -149,43 +252,39 @@ PyObject* gla(PyObject*, PyObject* const* v, Py_ssize_t n) {
     const at::Tensor& q = *t[0];
     const at::Tensor* s0 = v[5] == Py_None ? nullptr : tensor(v[5]);
     if (v[5] != Py_None && !s0) return PyLong_FromLong(kSlow);
-    if (at::GradMode::is_enabled()) {
-        bool wanted = s0 && s0->requires_grad();
-        for (const at::Tensor* x : t) wanted = wanted || x->requires_grad();
-        if (wanted) return PyLong_FromLong(kSlow);
-    }
     gla_b200_args a;
     std::memset(&a, 0, sizeof(a));
-    double scale, norm;
+    Call c;
     long segments;
-    if (!operands(a, q, *t[1], *t[2], *t[3]) || !scan_order(v[7], &a.direction) || !grid_pair(v[8], &a.grid_h, &a.grid_w) ||
-        !number(v[9], &norm) || !integer(v[10], &segments) || (s0 && !state(*s0, q)))
+    if (!operands(a, q, *t[1], *t[2], *t[3]) || !scan_order(v[7], &c.direction) || !grid_pair(v[8], &c.grid_h, &c.grid_w) ||
+        !number(v[9], &c.norm) || !integer(v[10], &segments) || (s0 && !state(*s0, q)))
         return PyLong_FromLong(kSlow);
-    if (v[4] == Py_None) scale = 1.0 / std::sqrt(static_cast<double>(a.K));
-    else if (!number(v[4], &scale)) return PyLong_FromLong(kSlow);
+    c.segments = static_cast<int32_t>(segments);
+    if (v[4] == Py_None) c.scale = 1.0 / std::sqrt(static_cast<double>(a.K));
+    else if (!number(v[4], &c.scale)) return PyLong_FromLong(kSlow);
     const int final_wanted = PyObject_IsTrue(v[6]);
     if (final_wanted < 0) return nullptr;
-    if (s0) a.initial_state = static_cast<const float*>(s0->data_ptr());
-    a.segments = static_cast<int32_t>(segments);
-    a.scale = static_cast<float>(scale);
-    a.gk_normalizer = static_cast<float>(norm);
-
-    const c10::cuda::CUDAGuard guard(q.device());
-    const auto opts = at::TensorOptions().device(q.device());
-    at::Tensor o = at::empty({a.B, a.T, a.H, kV}, opts.dtype(at::kHalf)), final_state;
-    if (final_wanted) {
-        final_state = at::empty({a.B, a.H, a.K, kV}, opts.dtype(at::kFloat));
-        a.final_state = static_cast<float*>(final_state.data_ptr());
+    c.final_wanted = final_wanted != 0;
+    bool grad = false;
+    if (at::GradMode::is_enabled()) {
+        grad = s0 && s0->requires_grad();
+        for (const at::Tensor* x : t) grad = grad || x->requires_grad();
     }
-    a.o = o.data_ptr();
-    a.workspace_bytes = g_workspace_bytes(a.B, a.T, a.H, a.K, a.V);
-    const at::Tensor ws = at::empty({static_cast<int64_t>(a.workspace_bytes)}, opts.dtype(at::kByte));
-    a.workspace = ws.data_ptr();
-    const int rc = g_forward(&a, c10::cuda::getCurrentCUDAStream(q.device().index()).stream());
-    if (rc != GLA_B200_OK) return PyLong_FromLong(rc);
+    at::Tensor o, final_state;
+    try {
+        if (grad) {
+            const auto r = ChunkGLA::apply(q, *t[1], *t[2], *t[3], s0 ? std::optional<at::Tensor>(*s0) : std::nullopt, &c);
+            o = r[0];
+            if (c.final_wanted) final_state = r[1];
+        } else {
+            std::tie(o, final_state) = forward(a, q, s0, c);
+        }
+    } catch (const LibraryError& e) {
+        return PyLong_FromLong(e.code);
+    }
     PyObject* po = THPVariable_Wrap(o);
     if (!po) return nullptr;
-    PyObject* pf = final_wanted ? THPVariable_Wrap(final_state) : Py_NewRef(Py_None);
+    PyObject* pf = c.final_wanted ? THPVariable_Wrap(final_state) : Py_NewRef(Py_None);
     if (!pf) { Py_DECREF(po); return nullptr; }
     PyObject* out = PyTuple_Pack(2, po, pf);
     Py_DECREF(po);
@@ -194,17 +293,20 @@ PyObject* gla(PyObject*, PyObject* const* v, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
-// bind(address of gla_b200_forward, address of gla_b200_workspace_bytes)
+// bind(addresses of gla_b200_forward, _workspace_bytes, _backward_scan, _backward_workspace_bytes, _strerror)
 PyObject* bind(PyObject*, PyObject* const* v, Py_ssize_t n) {
-    if (n != 2) { PyErr_SetString(PyExc_TypeError, "bind takes 2 addresses"); return nullptr; }
-    void* p[2];
-    for (int i = 0; i < 2; ++i)
+    if (n != 5) { PyErr_SetString(PyExc_TypeError, "bind takes 5 addresses"); return nullptr; }
+    void* p[5];
+    for (int i = 0; i < 5; ++i)
         if (!(p[i] = PyLong_AsVoidPtr(v[i]))) {
             if (!PyErr_Occurred()) PyErr_SetString(PyExc_ValueError, "null address");
             return nullptr;
         }
     g_forward = reinterpret_cast<decltype(g_forward)>(p[0]);
     g_workspace_bytes = reinterpret_cast<decltype(g_workspace_bytes)>(p[1]);
+    g_backward = reinterpret_cast<decltype(g_backward)>(p[2]);
+    g_backward_workspace_bytes = reinterpret_cast<decltype(g_backward_workspace_bytes)>(p[3]);
+    g_strerror = reinterpret_cast<decltype(g_strerror)>(p[4]);
     Py_RETURN_NONE;
 }
 

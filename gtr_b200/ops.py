@@ -207,8 +207,9 @@ def backward_workspace_bytes(B: int, T: int, H: int, K: int = kK) -> int:
 
 
 def chunk_gla_backward(q, k, v, g, do, scale: Optional[float] = None, initial_state: Optional[torch.Tensor] = None,
-                       d_final_state: Optional[torch.Tensor] = None, want_d_initial_state: bool = False):
-    """Gradients of `chunk_gla` (row-major scan, log-space gates): returns (dq, dk, dv, dg, d_initial_state) with
+                       d_final_state: Optional[torch.Tensor] = None, want_d_initial_state: bool = False, *, direction=0,
+                       grid_hw=None):
+    """Gradients of `chunk_gla` (log-space gates): returns (dq, dk, dv, dg, d_initial_state) with
     dq, dk, dv in fp16, dg and the state gradient in fp32.  The reference gets these from FLA's autograd
     (vit_adapter.py:441,560-568)."""
     B, T, H, K = q.shape
@@ -246,19 +247,12 @@ def chunk_gla_backward(q, k, v, g, do, scale: Optional[float] = None, initial_st
     a.scale = float(scale)
     with torch.cuda.device(dev):
         stream = torch.cuda.current_stream(dev).cuda_stream
-        _lib.check(_lib.lib().gla_b200_backward(ctypes.byref(a), ctypes.c_void_p(stream)))
+        scan = _lib.BwdScan()
+        scan.direction = _direction_id(direction)
+        if grid_hw is not None:
+            scan.grid_h, scan.grid_w = int(grid_hw[0]), int(grid_hw[1])
+        _lib.check(_lib.lib().gla_b200_backward_scan(ctypes.byref(a), ctypes.byref(scan), ctypes.c_void_p(stream)))
     return dq, dk, dv, dg, dh0
-
-
-def _scan_order(direction: int, grid_hw, T: int, device) -> torch.Tensor:
-    """perm[p] = canonical (row-major) index of the token the scan reads at step p
-    (vit_adapter_spatial_swiglu.py:88-94: flip after every block, transpose the grid after odd ones)."""
-    hg, wg = (1, T) if grid_hw is None else (int(grid_hw[0]), int(grid_hw[1]))
-    idx = torch.arange(hg * wg, device=device).reshape(hg, wg)
-    if direction >= 2:
-        idx = idx.t()
-    perm = idx.reshape(-1)
-    return perm.flip(0) if direction & 1 else perm.contiguous()
 
 
 class _ChunkGLA(torch.autograd.Function):
@@ -289,14 +283,9 @@ class _ChunkGLA(torch.autograd.Function):
         if ctx.gk_normalizer > 0.0:          # the forward kernel turned raw logits into log-space gates itself
             logits = g.float()
             g = (torch.nn.functional.logsigmoid(logits) / ctx.gk_normalizer).to(torch.float16)
-        inverse = None
-        if ctx.direction != 0:               # the gradient kernels walk tokens in memory order: put them in scan order
-            perm = _scan_order(ctx.direction, ctx.grid_hw, q.shape[1], q.device)
-            inverse = torch.empty_like(perm)
-            inverse[perm] = torch.arange(perm.numel(), device=perm.device)
-            q, k, v, g, do = (x.index_select(1, perm) for x in (q, k, v, g, do))
         if ctx.offs is None:
-            dq, dk, dv, dg, ds0 = chunk_gla_backward(q, k, v, g, do, ctx.scale, s0, d_final, want_s0)
+            dq, dk, dv, dg, ds0 = chunk_gla_backward(q, k, v, g, do, ctx.scale, s0, d_final, want_s0, direction=ctx.direction,
+                                                     grid_hw=ctx.grid_hw)
         else:
             dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
             dg = torch.empty(q.shape, dtype=torch.float32, device=q.device)
@@ -308,8 +297,6 @@ class _ChunkGLA(torch.autograd.Function):
                 dq[:, a:b], dk[:, a:b], dv[:, a:b], dg[:, a:b] = part[:4]
                 if want_s0:
                     ds0[i:i + 1] = part[4]
-        if inverse is not None:
-            dq, dk, dv, dg = (x.index_select(1, inverse) for x in (dq, dk, dv, dg))
         if logits is not None:               # d logsigmoid(x) / dx = sigmoid(-x)
             dg = dg * torch.sigmoid(-logits) / ctx.gk_normalizer
         return dq, dk, dv, dg.to(ctx.saved_tensors[3].dtype), ds0, None, None, None, None, None, None, None
@@ -320,9 +307,9 @@ def chunk_gla(q, k, v, g, scale: Optional[float] = None, initial_state: Optional
               gk_normalizer: float = 0.0, segments: int = 0) -> Tuple[torch.Tensor, Optional[torch.Tensor]]:
     """FLA-style call (vit_adapter.py:566-568): returns (o, final_state); `_chunk_gla_forward` documents the arguments.
     When gradients are enabled and an input requires one, the call is recorded for autograd and its backward runs
-    `chunk_gla_backward` -- as FLA's operator does for the reference in training.  The gradient kernels serve the
-    row-major scan with log-space gates (what FLA's signature expresses); for the other scan directions the backward
-    gathers the tokens into scan order around them, and for raw gate logits it applies logsigmoid's derivative."""
+    `chunk_gla_backward` -- as FLA's operator does for the reference in training -- in the same scan order; for raw gate
+    logits it applies logsigmoid's derivative around it.  (The native face records the call; `_ChunkGLA` serves packed
+    sequences and arguments that need converting.)"""
     if cu_seqlens is None:
         done = _front().gla(q, k, v, g, scale, initial_state, output_final_state, direction, grid_hw, gk_normalizer, segments)
         if type(done) is tuple:

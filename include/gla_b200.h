@@ -145,7 +145,8 @@ int gla_b200_stream_probe(const void* buf, int64_t rows, int32_t heads, int32_t 
  *   dS_t = exp(g_{t+1}) dS_{t+1} + scale q_t do_t^T,  dq_t = scale S_t do_t,  dk_t = dS_t v_t,  dv_t = dS_t^T k_t,
  *   dg_t = sum_{s>=t} (q_s dq_s - k_s dk_s) (+ sum_v d_final_state * final_state at the last token),
  *   d_initial_state = exp(g_1) dS_1.
- * Never synchronises or allocates; the workspace needs no clearing. */
+ * Never synchronises or allocates; the workspace needs no clearing.  (A wait inside the kernels is bounded as in the forward;
+ * gla_b200_check_status reads this workspace's status word too.) */
 typedef struct gla_b200_bwd_args {
     const void* q;
     const void* k;
@@ -167,6 +168,15 @@ typedef struct gla_b200_bwd_args {
 
 size_t gla_b200_backward_workspace_bytes(int32_t B, int32_t T, int32_t H, int32_t K, int32_t V);
 int gla_b200_backward(const gla_b200_bwd_args* args, void* stream);
+
+/* The same for the other scan directions (tokens stay where they are, as in gla_b200_forward), and with dg in fp16 for
+ * callers whose gates are fp16.  `scan` == NULL: row-major, fp32 dg. */
+typedef struct gla_b200_bwd_scan {
+    int32_t grid_h, grid_w;          /* patch grid; needed for directions 2,3; 0,0 means 1 x T */
+    int32_t direction;
+    int32_t dg_is_half;              /* args->dg points to fp16 [B,T,H,K] */
+} gla_b200_bwd_scan;
+int gla_b200_backward_scan(const gla_b200_bwd_args* args, const gla_b200_bwd_scan* scan, void* stream);
 
 /* Replaces rmsnorm_gated (gla_torch_ext.cu:156-196, kernel gla_norm_gate.cuh:13-75):
  * y = x * rsqrt(mean(x^2) + eps) * w * silu(g) over rows of D = 64 fp16 values; y may alias x. */
