@@ -60,7 +60,7 @@ EXPORTS = (
     "gla_b200_trt_enqueue", "gla_b200_strerror", "gla_b200_last_cuda_error", "gla_b200_version",
     "gla_b200_forward_static", "gla_b200_selftest_wait_timeout", "gla_b200_swiglu_dwconv", "gla_b200_layernorm",
     "gla_b200_stream_probe", "gla_b200_backward", "gla_b200_backward_workspace_bytes",
-    "gla_b200_backward_scan",
+    "gla_b200_backward_scan", "gla_b200_forward_packed", "gla_b200_packed_workspace_bytes",
 )
 
 _lib = None
@@ -84,6 +84,10 @@ def lib() -> ctypes.CDLL:
     L = ctypes.CDLL(LIB_PATH)
     L.gla_b200_forward.argtypes = [ctypes.POINTER(Args), ctypes.c_void_p]
     L.gla_b200_forward.restype = ctypes.c_int
+    L.gla_b200_forward_packed.argtypes = [ctypes.POINTER(Args), ctypes.POINTER(ctypes.c_int32), ctypes.c_int32, ctypes.c_void_p]
+    L.gla_b200_forward_packed.restype = ctypes.c_int
+    L.gla_b200_packed_workspace_bytes.argtypes = [ctypes.POINTER(ctypes.c_int32), ctypes.c_int32, ctypes.c_int32]
+    L.gla_b200_packed_workspace_bytes.restype = ctypes.c_size_t
     L.gla_b200_forward_static.argtypes = [ctypes.POINTER(Args), ctypes.c_void_p]
     L.gla_b200_forward_static.restype = ctypes.c_int
     L.gla_b200_selftest_wait_timeout.argtypes = [ctypes.c_void_p, ctypes.c_size_t, ctypes.c_uint32, ctypes.c_void_p]
@@ -131,7 +135,8 @@ def front():
         from . import _front as F
         address = lambda fn: ctypes.cast(fn, ctypes.c_void_p).value
         F.bind(*(address(fn) for fn in (L.gla_b200_forward, L.gla_b200_workspace_bytes, L.gla_b200_backward_scan,
-                                        L.gla_b200_backward_workspace_bytes, L.gla_b200_strerror)))
+                                        L.gla_b200_backward_workspace_bytes, L.gla_b200_strerror, L.gla_b200_forward_packed,
+                                        L.gla_b200_packed_workspace_bytes)))
         _front = F
     return _front
 

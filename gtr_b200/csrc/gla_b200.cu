@@ -52,6 +52,12 @@ const void* fwd_kernel(int variant) {
     return table[variant & 7];
 }
 
+const void* packed_kernel(bool logits) {
+    using gla::gla_fwd_kernel;
+    return logits ? reinterpret_cast<const void*>(&gla_fwd_kernel<false, true, false, gla::PackedTable>)
+                  : reinterpret_cast<const void*>(&gla_fwd_kernel<false, false, false, gla::PackedTable>);
+}
+
 struct DeviceInfo {
     bool ok = false;
     int sms = 0;
@@ -74,6 +80,8 @@ int device_info(int dev, DeviceInfo* out) {
         }
         for (int v = 0; v < 8 && e == cudaSuccess; ++v)
             e = cudaFuncSetAttribute(fwd_kernel(v), cudaFuncAttributeMaxDynamicSharedMemorySize, gla::kSmemBytes);
+        for (int v = 0; v < 2 && e == cudaSuccess; ++v)
+            e = cudaFuncSetAttribute(packed_kernel(v != 0), cudaFuncAttributeMaxDynamicSharedMemorySize, gla::kSmemBytes);
         if (e != cudaSuccess) { note_cuda("cudaFuncSetAttribute", e); return GLA_B200_ERR_CUDA; }
         const std::pair<const void*, int> bwd[] = {
             {reinterpret_cast<const void*>(&gla::gla_bwd_state_kernel<64>), gla::BwdStateSmem::kBytes},
@@ -192,6 +200,76 @@ int relay_segments(int NT, int nseq, int slots, size_t workspace_bytes, double* 
     }
     *cost_out = best_cost;
     return best;
+}
+
+// q and k each carry sqrt(scale) / 4 (head-room for the gate factors in fp16); the 16 comes back in the epilogue
+void fold_scale(float scale, gla::Params* P) {
+    if (scale > 0.f && scale < 3.0e38f) { P->q_exp = log2f(scale) - 4.f; P->q_mul = scale * 0.0625f; P->o_mul = 16.f; }
+    else { P->q_exp = -4.f; P->q_mul = 0.0625f; P->o_mul = scale * 16.f; }
+}
+
+// Packed sequences: how each is cut and in which order their items are handed out.  In units of one chunk's output pass a
+// one-segment sequence of n chunks costs n + kItem, one that r CTAs share (1 + pre) n / (r + pre) + kItem + 1 on each of them
+// (staggered_plan).  The target cost is the smallest at which all the work fits the SMs and no sequence is above it; dearest items
+// first, so that the cheap ones fill the ends.
+constexpr double kItem = 2.5;              // start and drain of one item
+int packed_plan(const int32_t* off, int n, int H, int slots, gla::PackedTable* tab, int* items_out) {
+    constexpr double pre = kPlanPrePassPlain;
+    auto shares = [&](int chunks, double target) {                   // CTAs for one sequence
+        if (chunks + kItem <= target || chunks < 3 * kMinAutoCps) return 1;
+        const int most = std::min(gla::kMaxPlanSegments - 1, chunks / kMinAutoCps - 1);
+        const int r = static_cast<int>(chunks * (1.0 + pre) / std::max(target - kItem - 1.0, 1.0) - pre + 0.999);
+        return std::max(2, std::min(r, most));
+    };
+    auto cost = [&](int chunks, int r) { return r == 1 ? chunks + kItem : (1.0 + pre) * chunks / (r + pre) + kItem + 1.0; };
+    int longest = 1;
+    double work = 0.0;
+    for (int i = 0; i < n; ++i) {
+        const int c = num_chunks(off[i + 1] - off[i]);
+        longest = std::max(longest, c);
+        work += c;
+    }
+    double lo = std::max(work * H / slots, 1.0), hi = longest + kItem;
+    auto fits = [&](double target) {
+        double sum = 0.0;
+        for (int i = 0; i < n; ++i) {
+            const int c = num_chunks(off[i + 1] - off[i]);
+            if (c == 0) continue;
+            const int r = shares(c, target);
+            if (cost(c, r) > target * 1.001 + 1e-9) return false;
+            sum += r == 1 ? c + kItem : c + (r - 1) * pre * c / (r + pre) + (r + 1) * kItem;
+        }
+        return sum * H <= slots * target;
+    };
+    if (hi > lo)
+        for (int it = 0; it < 12; ++it) {
+            const double mid = 0.5 * (lo + hi);
+            if (fits(mid)) hi = mid;
+            else lo = mid;
+        }
+    struct Entry { double cost; int i, r, c; };
+    Entry e[gla::kMaxPacked];
+    int m = 0;
+    for (int i = 0; i < n; ++i) {
+        const int c = num_chunks(off[i + 1] - off[i]);
+        if (c == 0) continue;
+        const int r = shares(c, hi);
+        e[m++] = {cost(c, r), i, r, c};
+    }
+    std::sort(e, e + m, [](const Entry& a, const Entry& b) { return a.cost != b.cost ? a.cost > b.cost : a.i < b.i; });
+    int item = 0, slot = 0;
+    tab->n = m;
+    for (int j = 0; j < m; ++j) {
+        gla::PackedSeq& q = tab->seq[j];
+        const int r = e[j].r, ns = r == 1 ? 1 : r + 1;
+        q.item0 = item; q.tok0 = off[e[j].i]; q.len = off[e[j].i + 1] - q.tok0; q.state = e[j].i;
+        q.ns = ns; q.slot0 = slot;
+        q.n0 = r == 1 ? e[j].c : std::max(1, static_cast<int>(pre * e[j].c / (r + pre) + 0.5));
+        item += ns * H;
+        slot += ns;
+    }
+    *items_out = item;
+    return slot;
 }
 
 // A few tokens per sequence go token by token through the state in registers (gla_step.cuh), unless the caller asks for
@@ -567,9 +645,7 @@ int gla_b200_forward(const gla_b200_args* a, void* stream_v) {
     for (int i = 0; i <= gla::kMaxPlanSegments; ++i) P.seg_start[i] = plan_start[i];
     P.num_items = nseq * NS;
     P.gated = gated ? 1 : 0;
-    // q and k each carry sqrt(scale) / 4 (head-room for the gate factors in fp16); the 16 comes back in the epilogue
-    if (a->scale > 0.f && a->scale < 3.0e38f) { P.q_exp = log2f(a->scale) - 4.f; P.q_mul = a->scale * 0.0625f; P.o_mul = 16.f; }
-    else { P.q_exp = -4.f; P.q_mul = 0.0625f; P.o_mul = a->scale * 16.f; }
+    fold_scale(a->scale, &P);
     P.inv_norm = a->gk_normalizer > 0.f ? 1.f / a->gk_normalizer : 0.f;
     P.rms_eps = a->rms_eps;
     P.rms_w = gated ? static_cast<const __half*>(a->rms_weight) : nullptr;
@@ -596,11 +672,93 @@ int gla_b200_forward(const gla_b200_args* a, void* stream_v) {
     if (ce != cudaSuccess) { note_cuda("cudaMemsetAsync", ce); return GLA_B200_ERR_CUDA; }
     const int grid = P.num_items < slots ? P.num_items : slots;
     const int variant = (P.gated ? 4 : 0) | (P.inv_norm > 0.f ? 2 : 0) | (P.rev ? 1 : 0);
-    void* kargs[2] = {const_cast<gla::Maps*>(&maps), &P};
+    gla::NoTable table;
+    void* kargs[3] = {const_cast<gla::Maps*>(&maps), &P, &table};
     ce = cudaLaunchKernel(fwd_kernel(variant), dim3(grid), dim3(gla::kThreads), kargs, gla::kSmemBytes, stream);
     if (ce != cudaSuccess) { note_cuda("cudaLaunchKernel", ce); return GLA_B200_ERR_CUDA; }
     ce = cudaPeekAtLastError();
     if (ce != cudaSuccess) { note_cuda("kernel launch", ce); return GLA_B200_ERR_CUDA; }
+    return GLA_B200_OK;
+}
+
+size_t gla_b200_packed_workspace_bytes(const int32_t* offsets, int32_t n, int32_t H) {
+    if (!offsets || n < 0 || H <= 0) return 0;
+    size_t most = 512;
+    for (int at = 0; at < n; at += gla::kMaxPacked) {
+        gla::PackedTable tab;
+        int items = 0;
+        const int slots = packed_plan(offsets + at, std::min(n - at, gla::kMaxPacked), H, 148, &tab, &items);
+        most = std::max(most, ws_layout(static_cast<size_t>(H), static_cast<size_t>(std::max(slots, 2))).total);
+    }
+    return most;
+}
+
+int gla_b200_forward_packed(const gla_b200_args* a, const int32_t* offsets, int32_t n, void* stream_v) {
+    if (!a || !offsets) return GLA_B200_ERR_NULL;
+    if ((a->K != 32 && a->K != gla::kD) || a->V != gla::kD || a->B != 1 || a->T < 0 || a->H <= 0 || n < 0) return GLA_B200_ERR_SHAPE;
+    if (a->direction != 0 || a->out_gate || a->rms_weight || a->segments != 0) return GLA_B200_ERR_ARG;
+    if (a->scale != a->scale || a->gk_normalizer < 0.f) return GLA_B200_ERR_ARG;
+    for (int i = 0; i < n; ++i)
+        if (offsets[i + 1] < offsets[i]) return GLA_B200_ERR_SHAPE;
+    if (n > 0 && (offsets[0] != 0 || offsets[n] != a->T)) return GLA_B200_ERR_SHAPE;
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
+    const size_t state_floats = static_cast<size_t>(a->H) * a->K * gla::kD;
+    if ((a->initial_state && !aligned16(a->initial_state)) || (a->final_state && !aligned16(a->final_state))) return GLA_B200_ERR_ALIGN;
+    cudaError_t ce = cudaSuccess;
+    for (int i = 0; i < n && a->final_state; ++i) {                  // an empty sequence leaves the state as it came in
+        if (offsets[i + 1] != offsets[i]) continue;
+        float* to = a->final_state + i * state_floats;
+        ce = a->initial_state ? cudaMemcpyAsync(to, a->initial_state + i * state_floats, state_floats * 4, cudaMemcpyDeviceToDevice, stream)
+                              : cudaMemsetAsync(to, 0, state_floats * 4, stream);
+        if (ce != cudaSuccess) { note_cuda("final state of an empty sequence", ce); return GLA_B200_ERR_CUDA; }
+    }
+    if (a->T == 0 || n == 0) return GLA_B200_OK;
+    if (!a->q || !a->k || !a->v || !a->g || !a->o) return GLA_B200_ERR_NULL;
+    MapKey key;
+    memset(&key, 0, sizeof(key));
+    const void* ptrs[gla::kNumTensors] = {a->q, a->k, a->g, a->v, a->o, nullptr};
+    const int64_t* strides[gla::kNumTensors] = {a->q_stride, a->k_stride, a->g_stride, a->v_stride, a->o_stride, a->gate_stride};
+    for (int t = 0; t < gla::kNumTensors; ++t) {
+        key.ptr[t] = ptrs[t];
+        if (!ptrs[t]) continue;
+        if (!aligned16(ptrs[t])) return GLA_B200_ERR_ALIGN;
+        const bool key_side = t == gla::TQ || t == gla::TK || t == gla::TG;
+        if (int rc = resolve_strides(strides[t], a->T, a->H, key_side ? a->K : gla::kD, key.stride[t])) return rc;
+    }
+    int dev = 0;
+    ce = cudaGetDevice(&dev);
+    if (ce != cudaSuccess) { note_cuda("cudaGetDevice", ce); return GLA_B200_ERR_CUDA; }
+    if (dev < 0 || dev >= 64) return GLA_B200_ERR_DEVICE;
+    DeviceInfo di;
+    if (int rc = device_info(dev, &di)) return rc;
+    key.B = 1; key.T = a->T; key.H = a->H; key.K = a->K; key.Hc = a->T; key.Wc = 1; key.dev = dev;
+    gla::Maps maps;
+    if (int rc = get_maps(key, &maps)) return rc;
+    uint8_t* ws = static_cast<uint8_t*>(a->workspace);
+    if (!ws || (reinterpret_cast<uintptr_t>(ws) & 255u)) return GLA_B200_ERR_WORKSPACE;
+    for (int at = 0; at < n; at += gla::kMaxPacked) {
+        gla::PackedTable tab;
+        gla::Params P;
+        memset(&P, 0, sizeof(P));
+        const int slots = packed_plan(offsets + at, std::min(n - at, gla::kMaxPacked), a->H, 148, &tab, &P.num_items);
+        if (P.num_items == 0) continue;
+        const WsLayout L = ws_layout(static_cast<size_t>(a->H), static_cast<size_t>(std::max(slots, 2)));
+        if (a->workspace_bytes < L.total) return GLA_B200_ERR_WORKSPACE;
+        P.B = 1; P.T = a->T; P.H = a->H; P.K = a->K; P.Hc = a->T; P.Wc = 1;
+        fold_scale(a->scale, &P);
+        P.inv_norm = a->gk_normalizer > 0.f ? 1.f / a->gk_normalizer : 0.f;
+        P.s0 = a->initial_state ? a->initial_state + at * state_floats : nullptr;
+        P.sT = a->final_state ? a->final_state + at * state_floats : nullptr;
+        P.ctrl = reinterpret_cast<uint32_t*>(ws + L.ctrl); P.flags = reinterpret_cast<uint32_t*>(ws + L.flags);
+        P.agg = reinterpret_cast<float*>(ws + L.agg); P.incl = reinterpret_cast<float*>(ws + L.incl);
+        P.wait_limit_us = a->wait_limit ? a->wait_limit : 2000000u;
+        ce = cudaMemsetAsync(ws, 0, L.clear_bytes, stream);
+        if (ce != cudaSuccess) { note_cuda("cudaMemsetAsync", ce); return GLA_B200_ERR_CUDA; }
+        void* kargs[3] = {&maps, &P, &tab};
+        ce = cudaLaunchKernel(packed_kernel(P.inv_norm > 0.f), dim3(std::min(P.num_items, di.sms)), dim3(gla::kThreads), kargs,
+                              gla::kSmemBytes, stream);
+        if (ce != cudaSuccess) { note_cuda("cudaLaunchKernel", ce); return GLA_B200_ERR_CUDA; }
+    }
     return GLA_B200_OK;
 }
 

@@ -162,6 +162,14 @@ constexpr int kMiscBytes = 4 * 1024;
 constexpr int kSmemBytes = kOffMisc + kMiscBytes + 1024;  // + alignment slack
 static_assert(kSmemBytes <= 227 * 1024, "shared memory budget");
 
+struct ItemInfo {
+    int seq, seg, b, h, first_chunk, nchunks, state_pass;
+    int publish_end;     // the state after the segment's output pass is what its successors start from
+    int ns;              // segments of the sequence; segment j keeps its states in slot slot0 + j
+    int T, tok0;         // tokens of the sequence, and its first one in the row (0 unless sequences are packed)
+    size_t slot0;
+};
+
 struct Misc {
     uint64_t full[kNumStages];
     uint64_t empty[kNumStages];
@@ -180,6 +188,7 @@ struct Misc {
     uint32_t wide[kSlots];
     // per chunk and key channel, log2 units: half the chunk's total decay G_L / 2 (output pass) or G_L itself (pre-pass)
     alignas(16) float vec[kSlots][kD];
+    ItemInfo info;       // packed sequences: the item at hand, decoded once
 };
 static_assert(sizeof(Misc) <= kMiscBytes, "misc block too large");
 
@@ -504,18 +513,62 @@ __global__ void wait_timeout_selftest_kernel(Params P) {
     if (threadIdx.x == 0) P.ctrl[2] = M.abort;     // 1: the CTA noticed the time-out
 }
 
-struct ItemInfo {
-    int seq, seg, b, h, first_chunk, nchunks, state_pass;
-    int publish_end;     // the state after the segment's output pass is what its successors start from
+// Sequences of different lengths back to back in one row (batch of one, forward row scan).  Each is cut as the staggered plan
+// cuts sequences: one segment, or a short first one that hands its state on, ns - 2 with a pre-pass and a last one without.
+// Items of a sequence are consecutive, segment-major with the heads inside, so that what an item waits for has a smaller ticket.
+struct PackedSeq {
+    int item0, tok0, len, state, ns, n0, slot0;      // n0: chunks of segment 0; the rest is split evenly over the others
 };
+constexpr int kMaxPacked = 96;                       // sequences per launch: the table is a kernel parameter
+struct PackedTable {
+    int n;
+    PackedSeq seq[kMaxPacked];
+};
+struct NoTable {};
+
+__device__ __forceinline__ ItemInfo decode_packed(const PackedTable& tab, const Params& P, int item) {
+    int lo = 0, hi = tab.n - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (tab.seq[mid].item0 <= item) lo = mid;
+        else hi = mid - 1;
+    }
+    const PackedSeq q = tab.seq[lo];
+    ItemInfo it;
+    const int i = item - q.item0, nt = (q.len + kChunk - 1) / kChunk;
+    it.seg = i / P.H;
+    it.h = i - it.seg * P.H;
+    it.b = 0;
+    it.seq = q.state * P.H + it.h;
+    it.ns = q.ns;
+    it.T = q.len;
+    it.tok0 = q.tok0;
+    it.slot0 = static_cast<size_t>(q.slot0) * P.H + static_cast<size_t>(it.h) * q.ns;
+    const int r = q.ns - 1, rest = nt - q.n0;
+    if (it.seg == 0) {
+        it.first_chunk = 0;
+        it.nchunks = q.n0;
+    } else {
+        const int each = rest / r, more = rest - each * r, k = it.seg - 1;
+        it.first_chunk = q.n0 + k * each + min(k, more);
+        it.nchunks = each + (k < more ? 1 : 0);
+    }
+    it.state_pass = (it.seg > 0 && it.seg < r) ? 1 : 0;
+    it.publish_end = (it.seg == 0 && q.ns > 1) ? 1 : 0;
+    return it;
+}
 
 __device__ __forceinline__ ItemInfo decode_item(const Params& P, int item) {
     ItemInfo it;
+    it.ns = P.NS;
+    it.T = P.T;
+    it.tok0 = 0;
     const int nseq = P.B * P.H;
     it.seg = item / nseq;
     it.seq = item - it.seg * nseq;
     it.b = it.seq / P.H;
     it.h = it.seq - it.b * P.H;
+    it.slot0 = static_cast<size_t>(it.seq) * P.NS;
     if (P.plan == 2) {
         it.first_chunk = it.seg * P.cps;
         it.nchunks = min(P.cps, P.NT - it.first_chunk);
@@ -567,9 +620,10 @@ template <int N> __device__ __forceinline__ void reg_budget() {
 
 // One instantiation per combination of fused epilogue, raw-logit gates and scan sense: each holds only the code of its
 // own case, which keeps the instruction working set of the concurrently running roles small.
-template <bool kGated, bool kLogits, bool kRev>
+template <bool kGated, bool kLogits, bool kRev, class Table = NoTable>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm)
-gla_fwd_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Params P) {
+gla_fwd_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Params P, const __grid_constant__ Table table) {
+    constexpr bool kPacked = !std::is_same<Table, NoTable>::value;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
@@ -654,15 +708,26 @@ gla_fwd_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Params
     // A barrier of a ring of R entries used for the u-th time is waited for with parity (u / R) & 1; "the entry is free
     // for its u-th use" is the completion of the release of use u - R, parity ((u / R) & 1) ^ 1 (true at once for u < R).
     uint32_t ctr = 0, c2 = 0;
+    struct Scan { int T, Hc, rev; };                 // what the tile walkers need to know
     // Work items come from a ticket counter; all roles fetch the same item at the same two block barriers.
     auto next_item = [&]() -> int {
-        if (tid == 0) M.item = static_cast<int>(atomicAdd(P.ctrl, 1u));
+        if (tid == 0) {
+            M.item = static_cast<int>(atomicAdd(P.ctrl, 1u));
+            if constexpr (kPacked) {
+                if (M.item < P.num_items) M.info = decode_packed(table, P, M.item);
+            }
+        }
         __syncthreads();
         GLA_TRACE_PICK(M.item);
         GLA_EVV(9, trace_t0);
         GLA_EV(3);
         GLA_EVV(6, M.item);
         return __shfl_sync(0xffffffffu, M.item, 0);   // known to be warp-uniform
+    };
+
+    auto item_info = [&](int item) -> ItemInfo {
+        if constexpr (kPacked) return M.info;
+        else return decode_item(P, item);
     };
 
     if (w < kStateWarps) {
@@ -682,11 +747,11 @@ gla_fwd_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Params
         while (true) {
             const int item = next_item();
             if (item >= P.num_items) break;
-            const ItemInfo it = decode_item(P, item);
+            const ItemInfo it = item_info(item);
             const int npass = it.state_pass ? 2 : 1;
             const size_t srow = (static_cast<size_t>(it.seq) * P.K + my_c) * kD + 32 * hf;   // this thread's half row of the state
             const bool real_row = my_c < P.K;      // rows of channels a K = 32 head does not have are zero throughout
-            const size_t slot = static_cast<size_t>(it.seq) * P.NS + it.seg;
+            const size_t slot = it.slot0 + it.seg;
             const size_t hoff = static_cast<size_t>(my_c) * kD + 32 * hf;                    // the same inside one 64 x 64 state
             float gsum = 0.f;       // log2 of the segment's total decay for channel my_c
 
@@ -733,7 +798,7 @@ gla_fwd_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Params
                     int j = it.seg - 1;
                     const uint64_t t0 = globaltimer_ns();
                     while (true) {
-                        const size_t sj = static_cast<size_t>(it.seq) * P.NS + j;
+                        const size_t sj = it.slot0 + j;
                         // one lane per warp polls (the CTAs of later segments wait here for a whole pre-pass of
                         // their predecessors), the warp barrier of the shuffle passes the acquired view on
                         uint32_t f = 0u;
@@ -874,7 +939,7 @@ gla_fwd_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Params
                 }
             }
             if (it.publish_end) publish(P.incl + slot * (kD * kD) + hoff, 2u);
-            if (it.seg == P.NS - 1 && P.sT != nullptr && real_row) {
+            if (it.seg == it.ns - 1 && P.sT != nullptr && real_row) {
                 float4* dst = reinterpret_cast<float4*>(P.sT + srow);
 #pragma unroll
                 for (int x4 = 0; x4 < 8; ++x4)
@@ -902,7 +967,7 @@ gla_fwd_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Params
         while (true) {
             const int item = next_item();
             if (item >= P.num_items) break;
-            const ItemInfo it = decode_item(P, item);
+            const ItemInfo it = item_info(item);
             const int npass = it.state_pass ? 2 : 1;
             for (int pass = 0; pass < npass; ++pass) {
                 const bool state_only = it.state_pass && pass == 0;
@@ -917,7 +982,7 @@ gla_fwd_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Params
                     GLA_EV(12);
                     if (logits) {
                         const int ci = it.first_chunk + ((state_only && kBackwardPrePass) ? it.nchunks - 1 - i : i);
-                        logits_to_log_gates(tg, P.inv_norm, rev, chunk_valid(ci * kChunk, P.T), tw, l);
+                        logits_to_log_gates(tg, P.inv_norm, rev, chunk_valid(ci * kChunk, it.T), tw, l);
                         warp_arrive(&M.g_ready[s], l);
                     }
                     // ---- gate sums of this thread's row and channel half
@@ -1125,8 +1190,10 @@ gla_fwd_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Params
                     named_bar_sync(bar_id, kTeamThreads);
                     GLA_EV(17);
                     if (storer && elect_one()) {
-                        const BoxWalker bw(P, (it.first_chunk + i) * kChunk);
-                        bw.for_each(P, [&](int id, int r, int c, int row) {
+                        const Scan scan = {it.T, P.Hc, P.rev};
+                        const BoxWalker bw(scan, (it.first_chunk + i) * kChunk);
+                        bw.for_each(scan, [&](int id, int r, int c, int row) {
+                            if constexpr (kPacked) r += it.tok0;
                             if (kL2Hints)
                                 tma_store_5d_hint(&maps.m[TO][id], out_tile + static_cast<uint32_t>(row) * 128u, 0, it.h, r, c, it.b,
                                                   pol_stream);
@@ -1151,7 +1218,7 @@ gla_fwd_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Params
         while (true) {
             const int item = next_item();
             if (item >= P.num_items) break;
-            const ItemInfo it = decode_item(P, item);
+            const ItemInfo it = item_info(item);
             const int npass = it.state_pass ? 2 : 1;
             if (w == kWarpProducer) {
                 // ------------------------------------------------------------ TMA producer
@@ -1159,7 +1226,8 @@ gla_fwd_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Params
                 for (int pass = 0; pass < npass; ++pass) {
                     const bool state_only = it.state_pass && pass == 0;
                     const bool back = state_only && kBackwardPrePass;
-                    BoxWalker bw(P, (it.first_chunk + (back ? it.nchunks - 1 : 0)) * kChunk);
+                    const Scan scan = {it.T, P.Hc, P.rev};
+                    BoxWalker bw(scan, (it.first_chunk + (back ? it.nchunks - 1 : 0)) * kChunk);
                     // tiles of a pre-pass are read again by the output pass; everything else is read once
                     const uint64_t pol = state_only ? pol_keep : pol_stream;
                     auto load = [&](uint32_t dst, int tensor, int id, uint32_t bar, int r, int c) {
@@ -1175,7 +1243,8 @@ gla_fwd_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Params
                             const uint32_t bar = smem_u32(&M.full[s]);
                             mbar_arrive_expect_tx(bar, static_cast<uint32_t>(kChunk * 128 * ntens));
                             const uint32_t stage = base + kOffStage + s * kStageBytes;
-                            bw.for_each(P, [&](int id, int r, int c, int row) {
+                            bw.for_each(scan, [&](int id, int r, int c, int row) {
+                                if constexpr (kPacked) r += it.tok0;
                                 const uint32_t off = static_cast<uint32_t>(row) * 128u;
                                 load(stage + 2 * kTileBytes + off, TG, id, bar, r, c);
                                 load(stage + 1 * kTileBytes + off, TK, id, bar, r, c);
@@ -1184,7 +1253,7 @@ gla_fwd_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Params
                             });
                             // rows the sequence does not have: boxes whose row coordinate lies past the column's end
                             // read nothing and fill their part of the tile with zeros
-                            bw.for_each_missing(P, [&](int id, int row) {
+                            bw.for_each_missing(scan, [&](int id, int row) {
                                 const uint32_t off = static_cast<uint32_t>(row) * 128u;
                                 tma_load_5d(stage + 2 * kTileBytes + off, &maps.m[TG][id], bar, 0, it.h, P.Hc, 0, it.b);
                                 tma_load_5d(stage + 1 * kTileBytes + off, &maps.m[TK][id], bar, 0, it.h, P.Hc, 0, it.b);
@@ -1194,8 +1263,8 @@ gla_fwd_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Params
                             });
                         }
                         __syncwarp();
-                        if (back) bw.retreat(P);
-                        else bw.advance(P);
+                        if (back) bw.retreat(scan);
+                        else bw.advance(scan);
                     }
                 }
             } else if (w == kWarpX) {

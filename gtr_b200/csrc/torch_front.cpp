@@ -9,6 +9,7 @@
 #include <ATen/core/grad_mode.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <pybind11/pybind11.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -29,6 +30,8 @@ decltype(&gla_b200_workspace_bytes) g_workspace_bytes = nullptr;
 decltype(&gla_b200_backward_scan) g_backward = nullptr;
 decltype(&gla_b200_backward_workspace_bytes) g_backward_workspace_bytes = nullptr;
 decltype(&gla_b200_strerror) g_strerror = nullptr;
+decltype(&gla_b200_forward_packed) g_forward_packed = nullptr;
+decltype(&gla_b200_packed_workspace_bytes) g_packed_workspace_bytes = nullptr;
 
 // The tensor inside a Python object, or null when it is not a plain torch.Tensor / Parameter.
 const at::Tensor* tensor(PyObject* o) {
@@ -151,6 +154,18 @@ void check(int rc) {
     if (rc != GLA_B200_OK) throw LibraryError(rc);
 }
 void* stream_of(const at::Tensor& x) { return c10::cuda::getCurrentCUDAStream(x.device().index()).stream(); }
+
+// (o, final_state or None)
+PyObject* result(const at::Tensor& o, const at::Tensor& final_state, bool final_wanted) {
+    PyObject* po = THPVariable_Wrap(o);
+    if (!po) return nullptr;
+    PyObject* pf = final_wanted ? THPVariable_Wrap(final_state) : Py_NewRef(Py_None);
+    if (!pf) { Py_DECREF(po); return nullptr; }
+    PyObject* out = PyTuple_Pack(2, po, pf);
+    Py_DECREF(po);
+    Py_DECREF(pf);
+    return out;
+}
 
 // What a call is besides its tensors.
 struct Call {
@@ -282,22 +297,69 @@ PyObject* gla(PyObject*, PyObject* const* v, Py_ssize_t n) {
     } catch (const LibraryError& e) {
         return PyLong_FromLong(e.code);
     }
-    PyObject* po = THPVariable_Wrap(o);
-    if (!po) return nullptr;
-    PyObject* pf = c.final_wanted ? THPVariable_Wrap(final_state) : Py_NewRef(Py_None);
-    if (!pf) { Py_DECREF(po); return nullptr; }
-    PyObject* out = PyTuple_Pack(2, po, pf);
-    Py_DECREF(po);
-    Py_DECREF(pf);
-    return out;
+    return result(o, final_state, c.final_wanted);
     END_HANDLE_TH_ERRORS
 }
 
-// bind(addresses of gla_b200_forward, _workspace_bytes, _backward_scan, _backward_workspace_bytes, _strerror)
+// packed(q, k, v, g, scale, initial_state, output_final_state, cu_seqlens, gk_normalizer) -> (o, final_state or None), a library
+// error, or kSlow.  The FLA-style call on packed sequences, outside autograd.
+PyObject* packed(PyObject*, PyObject* const* v, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    if (n != 9) return PyLong_FromLong(kSlow);
+    const at::Tensor* t[4];
+    for (int i = 0; i < 4; ++i)
+        if (!(t[i] = tensor(v[i]))) return PyLong_FromLong(kSlow);
+    const at::Tensor& q = *t[0];
+    const at::Tensor* s0 = v[5] == Py_None ? nullptr : tensor(v[5]);
+    const at::Tensor* ends = tensor(v[7]);
+    if ((v[5] != Py_None && !s0) || !ends || ends->dim() != 1) return PyLong_FromLong(kSlow);
+    gla_b200_args a;
+    std::memset(&a, 0, sizeof(a));
+    double norm, scale;
+    if (!operands(a, q, *t[1], *t[2], *t[3]) || a.B != 1 || !number(v[8], &norm)) return PyLong_FromLong(kSlow);
+    if (v[4] == Py_None) scale = 1.0 / std::sqrt(static_cast<double>(a.K));
+    else if (!number(v[4], &scale)) return PyLong_FromLong(kSlow);
+    const int final_wanted = PyObject_IsTrue(v[6]);
+    if (final_wanted < 0) return nullptr;
+    // outputs first, the offsets afterwards: reading them from the GPU waits for what is queued there
+    const c10::cuda::CUDAGuard guard(q.device());
+    const auto opts = at::TensorOptions().device(q.device());
+    at::Tensor o = at::empty({1, a.T, a.H, kV}, opts.dtype(at::kHalf)), final_state;
+    const int64_t count = ends->numel() - 1;
+    if (count < 1 || count > (1 << 24)) return PyLong_FromLong(kSlow);
+    if (s0 && (s0->scalar_type() != at::kFloat || s0->dim() != 4 || s0->size(0) != count || s0->size(1) != a.H || s0->size(2) != a.K ||
+               s0->size(3) != kV || !s0->is_contiguous() || s0->device() != q.device()))
+        return PyLong_FromLong(kSlow);
+    if (final_wanted) final_state = at::empty({count, a.H, a.K, kV}, opts.dtype(at::kFloat));
+    at::Tensor off;
+    {
+        pybind11::gil_scoped_release release;
+        off = ends->to(at::kCPU, at::kInt).contiguous();
+    }
+    const int32_t* p = off.const_data_ptr<int32_t>();
+    bool rising = p[0] == 0 && p[count] == a.T;
+    for (int64_t i = 0; i < count && rising; ++i) rising = p[i + 1] >= p[i];
+    if (!rising) return PyLong_FromLong(kSlow);
+    a.scale = static_cast<float>(scale);
+    a.gk_normalizer = static_cast<float>(norm);
+    a.o = o.data_ptr();
+    if (s0) a.initial_state = static_cast<const float*>(s0->data_ptr());
+    if (final_wanted) a.final_state = static_cast<float*>(final_state.data_ptr());
+    a.workspace_bytes = g_packed_workspace_bytes(p, static_cast<int32_t>(count), a.H);
+    const at::Tensor ws = at::empty({static_cast<int64_t>(a.workspace_bytes)}, opts.dtype(at::kByte));
+    a.workspace = ws.data_ptr();
+    const int rc = g_forward_packed(&a, p, static_cast<int32_t>(count), stream_of(q));
+    if (rc != GLA_B200_OK) return PyLong_FromLong(rc);
+    return result(o, final_state, final_wanted != 0);
+    END_HANDLE_TH_ERRORS
+}
+
+// bind(addresses of gla_b200_forward, _workspace_bytes, _backward_scan, _backward_workspace_bytes, _strerror, _forward_packed,
+//      _packed_workspace_bytes)
 PyObject* bind(PyObject*, PyObject* const* v, Py_ssize_t n) {
-    if (n != 5) { PyErr_SetString(PyExc_TypeError, "bind takes 5 addresses"); return nullptr; }
-    void* p[5];
-    for (int i = 0; i < 5; ++i)
+    if (n != 7) { PyErr_SetString(PyExc_TypeError, "bind takes 7 addresses"); return nullptr; }
+    void* p[7];
+    for (int i = 0; i < 7; ++i)
         if (!(p[i] = PyLong_AsVoidPtr(v[i]))) {
             if (!PyErr_Occurred()) PyErr_SetString(PyExc_ValueError, "null address");
             return nullptr;
@@ -307,12 +369,15 @@ PyObject* bind(PyObject*, PyObject* const* v, Py_ssize_t n) {
     g_backward = reinterpret_cast<decltype(g_backward)>(p[2]);
     g_backward_workspace_bytes = reinterpret_cast<decltype(g_backward_workspace_bytes)>(p[3]);
     g_strerror = reinterpret_cast<decltype(g_strerror)>(p[4]);
+    g_forward_packed = reinterpret_cast<decltype(g_forward_packed)>(p[5]);
+    g_packed_workspace_bytes = reinterpret_cast<decltype(g_packed_workspace_bytes)>(p[6]);
     Py_RETURN_NONE;
 }
 
 PyMethodDef methods[] = {
     {"bind", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(bind)), METH_FASTCALL, nullptr},
     {"run", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(run)), METH_FASTCALL, nullptr},
+    {"packed", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(packed)), METH_FASTCALL, nullptr},
     {"gla", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(gla)), METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_front", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

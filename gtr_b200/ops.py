@@ -175,19 +175,28 @@ def _chunk_gla_forward(q, k, v, g, scale: Optional[float] = None, initial_state:
     """FLA-style call: returns (o, final_state).  Allocates output, workspace and final state.
 
     `cu_seqlens` (the FLA convention the reference block passes through, vit_adapter.py:448-451,566-568): a batch of
-    one row holding N sequences back to back, `cu_seqlens` their N + 1 cumulative offsets.  Every sequence is one
-    launch on its slice of the row (the operator takes strided views, so nothing is copied); states are [N, H, K, 64]."""
+    one row holding N sequences back to back, `cu_seqlens` their N + 1 cumulative offsets; states are [N, H, K, 64].  One
+    launch serves them all; with an explicit `segments` every sequence is a launch on its slice of the row."""
     B, T, H, K = q.shape
     if scale is None:
         scale = K ** -0.5
-    o = torch.empty(B, T, H, kV, dtype=torch.float16, device=q.device)
-    if cu_seqlens is not None:
+    if cu_seqlens is None:
+        o = torch.empty(B, T, H, kV, dtype=torch.float16, device=q.device)
+    else:
         if direction != 0 or grid_hw is not None:
             raise ValueError("cu_seqlens describes plain forward scans")
+        if segments == 0:
+            ends = cu_seqlens if isinstance(cu_seqlens, torch.Tensor) else torch.tensor(cu_seqlens, dtype=torch.int32)
+            done = _front().packed(q, k, v, g, scale, initial_state, output_final_state, ends, gk_normalizer)
+            if type(done) is tuple:
+                return done
+            if done != _SLOW:
+                _lib.check(done)
         offs = _sequence_bounds(cu_seqlens, B, T)
         n = len(offs) - 1
         if initial_state is not None and initial_state.shape[0] != n:
             raise ValueError("initial_state needs one state per sequence")
+        o = torch.empty(B, T, H, kV, dtype=torch.float16, device=q.device)
         final = torch.empty(n, H, K, kV, dtype=torch.float32, device=q.device) if output_final_state else None
         ws = make_workspace(1, max(b - a for a, b in zip(offs, offs[1:])), H, q.device)
         for i, (a, b) in enumerate(zip(offs, offs[1:])):

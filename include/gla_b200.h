@@ -107,6 +107,13 @@ int gla_b200_forward(const gla_b200_args* args, void* stream);
 #define GLA_B200_STATIC_SCRATCH_BYTES (24u << 20)
 int gla_b200_forward_static(const gla_b200_args* args, void* stream);
 
+/* The operator on n sequences of different lengths packed back to back in one row (the cu_seqlens convention of the FLA call
+ * the reference block makes, vit_adapter.py:448-451,566-568): args->B = 1, args->T their total length, `offsets` their n + 1
+ * cumulative offsets in HOST memory, states [n,H,K,V].  Forward row scan, plain operator, automatic decomposition.  One launch
+ * for up to 96 sequences. */
+int gla_b200_forward_packed(const gla_b200_args* args, const int32_t* offsets, int32_t n, void* stream);
+size_t gla_b200_packed_workspace_bytes(const int32_t* offsets, int32_t n, int32_t H);
+
 /* Replaces workspace_floats (gla_torch_ext.cu:24-33); bytes, not floats.  0 on bad shape. */
 size_t gla_b200_workspace_bytes(int32_t B, int32_t T, int32_t H, int32_t K, int32_t V);
 
