@@ -120,9 +120,8 @@ class GatedLinearAttention(nn.Module):
             gk = self.gk_high_proj(gkl)                           # raw gate logits [B, T, key_dim]
         view = lambda t: t.unflatten(-1, (H, -1))                 # strided views, no copies
         ws, out = self._gla_buffers(B, T, x.device)
-        ops.chunk_gla_run_gated(view(q), view(k), view(v), view(gk), view(g), self.g_norm_weight, self.scale,
-                                self.norm_eps, ws, out, self.gate_logit_normalizer, direction=direction,
-                                grid_hw=grid_hw)
+        ops.block_gla_gated(view(q), view(k), view(v), view(gk), view(g), self.g_norm_weight, self.scale, self.norm_eps, ws, out,
+                            self.gate_logit_normalizer, direction=direction, grid_hw=grid_hw)
         return _project_add(out.flatten(-2), self.o_proj.weight, residual, keep_residual)
 
 

@@ -13,6 +13,7 @@
 
 #include "gla_kernel.cuh"
 #include "gla_step.cuh"
+#include "gla_block.cuh"
 #include "swiglu_dwconv.cuh"
 #include "gla_bwd.cuh"
 
@@ -41,21 +42,35 @@ EncodeTiledFn encode_tiled() {
     return fn;
 }
 
-// The forward kernel's instantiations: bit 2 fused epilogue, bit 1 raw-logit gates, bit 0 reversed scan.
-const void* fwd_kernel(int variant) {
-    using gla::gla_fwd_kernel;
-    static const void* const table[8] = {
-        reinterpret_cast<const void*>(&gla_fwd_kernel<false, false, false>), reinterpret_cast<const void*>(&gla_fwd_kernel<false, false, true>),
-        reinterpret_cast<const void*>(&gla_fwd_kernel<false, true, false>),  reinterpret_cast<const void*>(&gla_fwd_kernel<false, true, true>),
-        reinterpret_cast<const void*>(&gla_fwd_kernel<true, false, false>),  reinterpret_cast<const void*>(&gla_fwd_kernel<true, false, true>),
-        reinterpret_cast<const void*>(&gla_fwd_kernel<true, true, false>),   reinterpret_cast<const void*>(&gla_fwd_kernel<true, true, true>)};
-    return table[variant & 7];
+// The forward's instantiations: outputs by (fused epilogue, raw-logit gates), span increments by raw-logit gates; packed
+// sequences have no fused epilogue.
+const void* out_kernel(bool gated, bool logits, bool packed) {
+    using namespace gla;
+    if (packed)
+        return logits ? reinterpret_cast<const void*>(&gla_out_kernel<false, true, PackedTable>)
+                      : reinterpret_cast<const void*>(&gla_out_kernel<false, false, PackedTable>);
+    if (gated)
+        return logits ? reinterpret_cast<const void*>(&gla_out_kernel<true, true, NoTable>)
+                      : reinterpret_cast<const void*>(&gla_out_kernel<true, false, NoTable>);
+    return logits ? reinterpret_cast<const void*>(&gla_out_kernel<false, true, NoTable>)
+                  : reinterpret_cast<const void*>(&gla_out_kernel<false, false, NoTable>);
+}
+const void* state_kernel(bool logits, bool packed) {
+    using namespace gla;
+    if (packed)
+        return logits ? reinterpret_cast<const void*>(&gla_state_kernel<true, PackedTable>)
+                      : reinterpret_cast<const void*>(&gla_state_kernel<false, PackedTable>);
+    return logits ? reinterpret_cast<const void*>(&gla_state_kernel<true, NoTable>)
+                  : reinterpret_cast<const void*>(&gla_state_kernel<false, NoTable>);
 }
 
-const void* packed_kernel(bool logits) {
-    using gla::gla_fwd_kernel;
-    return logits ? reinterpret_cast<const void*>(&gla_fwd_kernel<false, true, false, gla::PackedTable>)
-                  : reinterpret_cast<const void*>(&gla_fwd_kernel<false, false, false, gla::PackedTable>);
+// The block kernel's: bit 1 raw-logit gates, bit 0 reversed scan.
+const void* block_kernel(int variant) {
+    using gla::block::gla_block_kernel;
+    static const void* const table[4] = {
+        reinterpret_cast<const void*>(&gla_block_kernel<false, false>), reinterpret_cast<const void*>(&gla_block_kernel<false, true>),
+        reinterpret_cast<const void*>(&gla_block_kernel<true, false>), reinterpret_cast<const void*>(&gla_block_kernel<true, true>)};
+    return table[variant & 3];
 }
 
 struct DeviceInfo {
@@ -79,10 +94,28 @@ int device_info(int dev, DeviceInfo* out) {
             return GLA_B200_ERR_DEVICE;
         }
         for (int v = 0; v < 8 && e == cudaSuccess; ++v)
-            e = cudaFuncSetAttribute(fwd_kernel(v), cudaFuncAttributeMaxDynamicSharedMemorySize, gla::kSmemBytes);
-        for (int v = 0; v < 2 && e == cudaSuccess; ++v)
-            e = cudaFuncSetAttribute(packed_kernel(v != 0), cudaFuncAttributeMaxDynamicSharedMemorySize, gla::kSmemBytes);
+            e = cudaFuncSetAttribute(out_kernel((v & 1) != 0, (v & 2) != 0, (v & 4) != 0), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     gla::OutSmem::kBytes);
+        for (int v = 0; v < 4 && e == cudaSuccess; ++v)
+            e = cudaFuncSetAttribute(state_kernel((v & 1) != 0, (v & 2) != 0), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     gla::StateSmem::kBytes);
         if (e != cudaSuccess) { note_cuda("cudaFuncSetAttribute", e); return GLA_B200_ERR_CUDA; }
+        for (int v = 0; v < 4 && e == cudaSuccess; ++v)
+            e = cudaFuncSetAttribute(block_kernel(v), cudaFuncAttributeMaxDynamicSharedMemorySize, gla::block::kSmemBytes);
+        if (e != cudaSuccess) { note_cuda("cudaFuncSetAttribute", e); return GLA_B200_ERR_CUDA; }
+        // The warpgroups of that kernel re-divide the registers the CTA was launched with (setmaxnreg); a group that
+        // asks for more than the others release would wait for ever, so the budgets are checked against what this
+        // build of the kernel really gets at launch.
+        for (int v = 0; v < 4; ++v) {
+            cudaFuncAttributes fa;
+            e = cudaFuncGetAttributes(&fa, block_kernel(v));
+            if (e != cudaSuccess) { note_cuda("cudaFuncGetAttributes", e); return GLA_B200_ERR_CUDA; }
+            if (fa.numRegs * gla::block::kThreads < gla::block::kRegBudgetTotal) {
+                snprintf(g_cuda_err, sizeof(g_cuda_err), "kernel launches with %d registers per thread, its register budgets need %d",
+                         fa.numRegs, (gla::block::kRegBudgetTotal + gla::block::kThreads - 1) / gla::block::kThreads);
+                return GLA_B200_ERR_DEVICE;
+            }
+        }
         const std::pair<const void*, int> bwd[] = {
             {reinterpret_cast<const void*>(&gla::gla_bwd_state_kernel<64>), gla::BwdStateSmem::kBytes},
             {reinterpret_cast<const void*>(&gla::gla_bwd_state_kernel<32>), gla::BwdStateSmem::kBytes},
@@ -91,17 +124,6 @@ int device_info(int dev, DeviceInfo* out) {
         for (const auto& k : bwd)
             if (e == cudaSuccess) e = cudaFuncSetAttribute(k.first, cudaFuncAttributeMaxDynamicSharedMemorySize, k.second);
         if (e != cudaSuccess) { note_cuda("cudaFuncSetAttribute", e); return GLA_B200_ERR_CUDA; }
-        // The warpgroups of the kernel re-divide the registers the CTA was launched with (setmaxnreg); a group that
-        // asks for more than the others release would wait for ever, so the budgets are checked against what this
-        // build of the kernel really gets at launch.
-        cudaFuncAttributes fa;
-        e = cudaFuncGetAttributes(&fa, fwd_kernel(0));
-        if (e != cudaSuccess) { note_cuda("cudaFuncGetAttributes", e); return GLA_B200_ERR_CUDA; }
-        if (fa.numRegs * gla::kThreads < gla::kRegBudgetTotal) {
-            snprintf(g_cuda_err, sizeof(g_cuda_err), "kernel launches with %d registers per thread, its register budgets need %d",
-                     fa.numRegs, (gla::kRegBudgetTotal + gla::kThreads - 1) / gla::kThreads);
-            return GLA_B200_ERR_DEVICE;
-        }
         d.ok = true;
         d.sms = sms;
         d.attr_set = true;
@@ -112,11 +134,101 @@ int device_info(int dev, DeviceInfo* out) {
 
 // ---- workspace layout ------------------------------------------------------------------
 struct WsLayout {
-    size_t ctrl, flags, agg, incl, total;
-    size_t clear_bytes;   // ctrl + flags, zeroed before every launch
+    size_t ctrl, agg, decay, total;
 };
 
 size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
+
+// `spans`: those that exchange a state increment; unsegmented sequences need none
+WsLayout ws_layout(size_t spans) {
+    WsLayout L;
+    L.ctrl = 0;
+    L.agg = 512;
+    L.decay = L.agg + spans * gla::kD * gla::kD * sizeof(float);
+    L.total = L.decay + align_up(spans * gla::kD * sizeof(float), 256);
+    return L;
+}
+
+constexpr int kAdvertisedCps = 4;   // explicit segments down to this length fit the advertised workspace
+
+int num_chunks(int T) { return (T + gla::kChunk - 1) / gla::kChunk; }
+
+// How the chunks are dealt out (gla::Params): `per` equal spans per sequence, or (per == 0) `spans` equal ones over everything.
+struct Split { int per, spans; };
+size_t exchange_spans(const Split& s) { return s.per == 1 ? 0 : static_cast<size_t>(s.spans); }
+
+// What a split costs, in units of the time one output chunk takes a CTA that has its SM to itself (3.2 us).  Up to four CTAs share
+// an SM and slow one another down: a chunk takes kOut[m] with m of them, kState[m] in the state kernel (measured at 4800 chunks
+// of 48 sequences; the sums below then rank the splits of 150 to 12288 chunks as they were timed, to within a few percent).  A span
+// costs its chunks, kStart once, and kChain for each span of its sequence before it.
+constexpr double kStart = 0.6, kChain = 0.05, kOut[5] = {0.0, 1.0, 1.29, 1.63, 1.95}, kState[5] = {0.0, 0.375, 0.53, 0.75, 1.05};
+double split_cost(int64_t chunks, int64_t nseq, int per, int64_t spans, int sms) {
+    auto run = [&](int64_t ctas, const double* each, double mean, double most) {
+        const int64_t full = ctas / (4 * sms), rest = ctas - full * 4 * sms, m = (rest + sms - 1) / sms;
+        return full * each[4] * mean + (m > 0 ? each[m] * ((m - 1) * mean + most) / m : 0.0);
+    };
+    const double mean = static_cast<double>(chunks) / spans;
+    const double most = per > 0 ? static_cast<double>((chunks / nseq + per - 1) / per) : static_cast<double>((chunks + spans - 1) / spans);
+    const double chain = kChain * (per > 0 ? per - 1 : std::max(0.0, static_cast<double>(chunks) / nseq / mean - 1.0));
+    double cost = run(spans, kOut, mean + kStart + chain, most + kStart + chain);
+    const int64_t states = per > 0 ? nseq * (per - 1) : spans - 1;
+    if (states > 0) cost += run(states, kState, mean, most) + kStart;
+    return cost;
+}
+// A split whose scratch does not fit the caller's workspace is not a candidate.
+Split choose_split(int64_t chunks, int NT, int64_t nseq, int sms, size_t workspace_bytes) {
+    Split best = NT > 0 ? Split{1, static_cast<int>(nseq)} : Split{0, static_cast<int>(std::min<int64_t>(chunks, sms))};
+    double least = 1e300;
+    auto consider = [&](int per, int64_t spans) {
+        const Split s = {per, static_cast<int>(spans)};
+        if (spans > 0x3fffffff || (exchange_spans(s) > 0 && ws_layout(exchange_spans(s)).total > workspace_bytes)) return;
+        const double c = split_cost(chunks, nseq, per, spans, sms);
+        if (c < least - 1e-9) { least = c; best = s; }
+    };
+    if (NT > 0)
+        for (int per = 1; per <= NT && per <= 128; ++per) consider(per, nseq * per);
+    for (int m = 1; m <= 4; ++m)
+        if (static_cast<int64_t>(m) * sms <= chunks) consider(0, static_cast<int64_t>(m) * sms);
+    return best;
+}
+
+// Packed sequences differ in length: flat spans only.
+Split packed_split(int64_t chunks, int64_t nseq, int sms) { return choose_split(chunks, 0, nseq, sms, ~static_cast<size_t>(0)); }
+
+void set_split(const Split& s, int64_t chunks, gla::Params* P) {
+    P->chunks = static_cast<int>(chunks);
+    P->spans = s.spans;
+    P->per = s.per;
+    P->len_ = static_cast<int>(chunks / s.spans);
+    P->longer = static_cast<int>(chunks % s.spans);
+}
+
+// q and k each carry sqrt(scale) / 4 (head-room for the gate factors in fp16); the 16 comes back in the epilogue
+template <class P_t>
+void fold_scale(float scale, P_t* P) {
+    if (scale > 0.f && scale < 3.0e38f) { P->q_exp = log2f(scale) - 4.f; P->q_mul = scale * 0.0625f; P->o_mul = 16.f; }
+    else { P->q_exp = -4.f; P->q_mul = 0.0625f; P->o_mul = scale * 16.f; }
+}
+
+// The table of packed sequences [0, n) and the number of their chunks; empty ones are left out.
+int64_t packed_table(const int32_t* off, int n, int H, gla::PackedTable* tab) {
+    int64_t chunks = 0;
+    tab->n = 0;
+    for (int i = 0; i < n; ++i) {
+        const int len = off[i + 1] - off[i];
+        if (len == 0) continue;
+        tab->seq[tab->n++] = {static_cast<int>(chunks), off[i], len, i};
+        chunks += static_cast<int64_t>(num_chunks(len)) * H;
+    }
+    return chunks;
+}
+
+// ---- the block kernel's work decomposition -----------------------------------------------
+namespace block_plan {
+struct WsLayout {
+    size_t ctrl, flags, agg, incl, total;
+    size_t clear_bytes;   // ctrl + flags, zeroed before every launch
+};
 
 WsLayout ws_layout(size_t nseq, size_t ns) {
     WsLayout L;
@@ -127,14 +239,12 @@ WsLayout ws_layout(size_t nseq, size_t ns) {
     // unsegmented sequences (ns == 1) need none, whatever their number
     const size_t slots = ns > 1 ? nseq * ns : 0;
     L.agg = L.clear_bytes;
-    L.incl = L.agg + align_up(slots * gla::kAggStride * 4, 256);
+    L.incl = L.agg + align_up(slots * gla::block::kAggStride * 4, 256);
     L.total = L.incl + align_up(slots * gla::kD * gla::kD * 4, 256);
     return L;
 }
 
-constexpr int kMinAutoCps = 4;   // smallest automatic segment length; also sizes the advertised workspace
-
-int num_chunks(int T) { return (T + gla::kChunk - 1) / gla::kChunk; }
+constexpr int kMinAutoCps = 4;   // smallest automatic segment length
 
 // Segment length that minimises a simple cost model of the persistent kernel: the work items
 // (sequences x segments) run in rounds of `slots` CTAs; an item costs its chunks once for the
@@ -160,7 +270,7 @@ int auto_chunks_per_segment(int NT, int nseq, int slots, size_t workspace_bytes)
     return best_cps;
 }
 
-// Staggered plan for r = slots / nseq CTAs per sequence, 2 <= r < kMaxPlanSegments (gla::Params::plan): segment 0 of
+// Staggered plan for r = slots / nseq CTAs per sequence, 2 <= r < kMaxPlanSegments (gla::block::Params::plan): segment 0 of
 // `pre` x the length of the others, r equal ones after it.  `pre` is what a pre-pass chunk costs next to an output-pass
 // chunk while both kinds run side by side; measured on 100 chunks with three CTAs per sequence, the fastest splits are
 // 18 + 28 + 27 + 27 for the plain operator (and with raw gate logits, which cost both passes) and 14 + 29 + 29 + 28 with
@@ -170,7 +280,7 @@ int auto_chunks_per_segment(int NT, int nseq, int slots, size_t workspace_bytes)
 constexpr double kPlanPrePassPlain = 0.68, kPlanPrePassGated = 0.48;
 double staggered_plan(int NT, int nseq, int slots, size_t workspace_bytes, double pre, int* seg_start, int* ns_out) {
     const int r = nseq > 0 ? slots / nseq : 0;
-    if (r < 2 || r + 1 > gla::kMaxPlanSegments || NT < kMinAutoCps * (r + 1)) return -1.0;
+    if (r < 2 || r + 1 > gla::block::kMaxPlanSegments || NT < kMinAutoCps * (r + 1)) return -1.0;
     if (ws_layout(static_cast<size_t>(nseq), static_cast<size_t>(r + 1)).total > workspace_bytes) return -1.0;
     const double mid = NT / (r + pre);
     int n0 = static_cast<int>(pre * mid + 0.5);
@@ -185,7 +295,7 @@ double staggered_plan(int NT, int nseq, int slots, size_t workspace_bytes, doubl
     return (with_pass > relay ? with_pass : relay) + 1.0;
 }
 
-// Relay plan (gla::Params::plan == 2) for more sequences than CTAs: the number of equal segments, without pre-passes,
+// Relay plan (gla::block::Params::plan == 2) for more sequences than CTAs: the number of equal segments, without pre-passes,
 // that minimises rounds x (segment length + one chunk's worth of look-back); 1 when whole sequences are as good.
 int relay_segments(int NT, int nseq, int slots, size_t workspace_bytes, double* cost_out) {
     int best = 1;
@@ -201,76 +311,7 @@ int relay_segments(int NT, int nseq, int slots, size_t workspace_bytes, double* 
     *cost_out = best_cost;
     return best;
 }
-
-// q and k each carry sqrt(scale) / 4 (head-room for the gate factors in fp16); the 16 comes back in the epilogue
-void fold_scale(float scale, gla::Params* P) {
-    if (scale > 0.f && scale < 3.0e38f) { P->q_exp = log2f(scale) - 4.f; P->q_mul = scale * 0.0625f; P->o_mul = 16.f; }
-    else { P->q_exp = -4.f; P->q_mul = 0.0625f; P->o_mul = scale * 16.f; }
-}
-
-// Packed sequences: how each is cut and in which order their items are handed out.  In units of one chunk's output pass a
-// one-segment sequence of n chunks costs n + kItem, one that r CTAs share (1 + pre) n / (r + pre) + kItem + 1 on each of them
-// (staggered_plan).  The target cost is the smallest at which all the work fits the SMs and no sequence is above it; dearest items
-// first, so that the cheap ones fill the ends.
-constexpr double kItem = 2.5;              // start and drain of one item
-int packed_plan(const int32_t* off, int n, int H, int slots, gla::PackedTable* tab, int* items_out) {
-    constexpr double pre = kPlanPrePassPlain;
-    auto shares = [&](int chunks, double target) {                   // CTAs for one sequence
-        if (chunks + kItem <= target || chunks < 3 * kMinAutoCps) return 1;
-        const int most = std::min(gla::kMaxPlanSegments - 1, chunks / kMinAutoCps - 1);
-        const int r = static_cast<int>(chunks * (1.0 + pre) / std::max(target - kItem - 1.0, 1.0) - pre + 0.999);
-        return std::max(2, std::min(r, most));
-    };
-    auto cost = [&](int chunks, int r) { return r == 1 ? chunks + kItem : (1.0 + pre) * chunks / (r + pre) + kItem + 1.0; };
-    int longest = 1;
-    double work = 0.0;
-    for (int i = 0; i < n; ++i) {
-        const int c = num_chunks(off[i + 1] - off[i]);
-        longest = std::max(longest, c);
-        work += c;
-    }
-    double lo = std::max(work * H / slots, 1.0), hi = longest + kItem;
-    auto fits = [&](double target) {
-        double sum = 0.0;
-        for (int i = 0; i < n; ++i) {
-            const int c = num_chunks(off[i + 1] - off[i]);
-            if (c == 0) continue;
-            const int r = shares(c, target);
-            if (cost(c, r) > target * 1.001 + 1e-9) return false;
-            sum += r == 1 ? c + kItem : c + (r - 1) * pre * c / (r + pre) + (r + 1) * kItem;
-        }
-        return sum * H <= slots * target;
-    };
-    if (hi > lo)
-        for (int it = 0; it < 12; ++it) {
-            const double mid = 0.5 * (lo + hi);
-            if (fits(mid)) hi = mid;
-            else lo = mid;
-        }
-    struct Entry { double cost; int i, r, c; };
-    Entry e[gla::kMaxPacked];
-    int m = 0;
-    for (int i = 0; i < n; ++i) {
-        const int c = num_chunks(off[i + 1] - off[i]);
-        if (c == 0) continue;
-        const int r = shares(c, hi);
-        e[m++] = {cost(c, r), i, r, c};
-    }
-    std::sort(e, e + m, [](const Entry& a, const Entry& b) { return a.cost != b.cost ? a.cost > b.cost : a.i < b.i; });
-    int item = 0, slot = 0;
-    tab->n = m;
-    for (int j = 0; j < m; ++j) {
-        gla::PackedSeq& q = tab->seq[j];
-        const int r = e[j].r, ns = r == 1 ? 1 : r + 1;
-        q.item0 = item; q.tok0 = off[e[j].i]; q.len = off[e[j].i + 1] - q.tok0; q.state = e[j].i;
-        q.ns = ns; q.slot0 = slot;
-        q.n0 = r == 1 ? e[j].c : std::max(1, static_cast<int>(pre * e[j].c / (r + pre) + 0.5));
-        item += ns * H;
-        slot += ns;
-    }
-    *items_out = item;
-    return slot;
-}
+}  // namespace block_plan
 
 // A few tokens per sequence go token by token through the state in registers (gla_step.cuh), unless the caller asks for
 // the chunk kernel's decomposition or the fused epilogue.
@@ -486,6 +527,124 @@ int static_scratch(void** out) {
 }
 }  // namespace
 
+namespace {
+void fill_params(const gla_b200_args* a, const int64_t* o_stride, uint8_t* ws, const WsLayout& L, gla::Params* P) {
+    fold_scale(a->scale, P);
+    P->inv_norm = a->gk_normalizer > 0.f ? 1.f / a->gk_normalizer : 0.f;
+    P->o = static_cast<__half*>(a->o);
+    for (int i = 0; i < 3; ++i) P->o_s[i] = o_stride[i];
+    P->sectors = (reinterpret_cast<uintptr_t>(a->o) | (o_stride[0] * 2) | (o_stride[1] * 2) | (o_stride[2] * 2)) % 32 == 0 ? 1 : 0;
+    P->s0 = a->initial_state;
+    P->sT = a->final_state;
+    P->ctrl = reinterpret_cast<uint32_t*>(ws + L.ctrl);
+    P->agg = reinterpret_cast<float*>(ws + L.agg);
+    P->agg_decay = reinterpret_cast<float*>(ws + L.decay);
+    P->wait_limit_us = a->wait_limit ? a->wait_limit : 2000000u;
+}
+
+// A kernel whose blocks may start while its predecessor in the stream drains; it waits (gla::pdl_wait) before it touches memory
+// that anything before it in the stream reads or writes.
+int launch_overlapped(const void* kernel, unsigned ctas, unsigned threads, size_t smem, void** args, cudaStream_t stream) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelExC(&cfg, kernel, args);
+    if (e != cudaSuccess) { note_cuda("cudaLaunchKernelExC", e); return GLA_B200_ERR_CUDA; }
+    return GLA_B200_OK;
+}
+
+constexpr int64_t kL2Keep = 120ll << 20;
+// The spans' increments (where spans end inside sequences), then the outputs.
+template <class Table>
+int launch_forward(bool gated, const gla::Maps& maps, gla::Params& P, const Table& table, cudaStream_t stream) {
+    constexpr bool packed = std::is_same<Table, gla::PackedTable>::value;
+    const bool logits = P.inv_norm > 0.f;
+    const int states = P.per > 0 ? P.spans / P.per * (P.per - 1) : P.spans - 1;
+    P.alone = states == 0 ? 1 : 0;
+    P.keep = static_cast<int64_t>(P.chunks) * (4 * P.K + 128) * gla::kChunk <= kL2Keep ? 1 : 0;
+    void* args[3] = {const_cast<gla::Maps*>(&maps), &P, const_cast<Table*>(&table)};
+    if (states > 0)
+        if (int rc = launch_overlapped(state_kernel(logits, packed), states, gla::kFwdThreads, gla::StateSmem::kBytes, args, stream)) return rc;
+    return launch_overlapped(out_kernel(gated, logits, packed), P.spans, gla::kFwdThreads, gla::OutSmem::kBytes, args, stream);
+}
+
+// The fused operator on the block kernel (gla_block.cuh).
+int forward_block(const gla_b200_args* a, const MapKey& key, int sms, cudaStream_t stream) {
+    using namespace block_plan;
+    const int NT = num_chunks(a->T), nseq = a->B * a->H;
+    const int slots = sms;
+    int cps;
+    int plan_start[gla::block::kMaxPlanSegments + 1] = {0}, plan_ns = 0;
+    bool plan = false, relay = false;
+    if (a->segments > 0) cps = a->segments;
+    else {
+        const size_t have = a->workspace ? a->workspace_bytes : 0;
+        cps = auto_chunks_per_segment(NT, nseq, slots, have);
+        const int ns_u = (NT + cps - 1) / cps;
+        const long rounds = (static_cast<long>(nseq) * ns_u + slots - 1) / slots;
+        // what the slowest item of the equal split costs, in the plan's units: every segment but the last pays the pre-pass
+        const double pre = kPlanPrePassGated;
+        const double uniform_cost = rounds * (cps * (1.0 + (ns_u > 1 ? pre : 0.0)) + (ns_u > 1 ? 1.0 : 0.0));
+        const double plan_cost = staggered_plan(NT, nseq, slots, have, pre, plan_start, &plan_ns);
+        plan = plan_cost > 0.0 && plan_cost < uniform_cost;
+        if (!plan && 2 * nseq > slots) {
+            double relay_cost = 0.0;
+            const int ns_r = relay_segments(NT, nseq, slots, have, &relay_cost);
+            if (ns_r > 1 && relay_cost < 0.97 * uniform_cost) { relay = true; cps = (NT + ns_r - 1) / ns_r; }
+        }
+    }
+    if (cps > NT) cps = NT;
+    const int NS = plan ? plan_ns : (NT + cps - 1) / cps;
+    const block_plan::WsLayout L = block_plan::ws_layout(static_cast<size_t>(nseq), static_cast<size_t>(NS));
+    if (!a->workspace || (reinterpret_cast<uintptr_t>(a->workspace) & 255u) || a->workspace_bytes < L.total)
+        return GLA_B200_ERR_WORKSPACE;
+
+    uint8_t* ws = static_cast<uint8_t*>(a->workspace);
+    gla::Maps maps;
+    if (int rc = get_maps(key, &maps)) return rc;
+
+    gla::block::Params P;
+    memset(&P, 0, sizeof(P));
+    P.B = a->B; P.T = a->T; P.H = a->H; P.NT = NT; P.K = a->K;
+    P.Hc = key.Hc; P.Wc = key.Wc;
+    P.rev = a->direction & 1;
+    P.NS = NS; P.cps = cps;
+    P.plan = plan ? 1 : relay ? 2 : 0;
+    for (int i = 0; i <= gla::block::kMaxPlanSegments; ++i) P.seg_start[i] = plan_start[i];
+    P.num_items = nseq * NS;
+    fold_scale(a->scale, &P);
+    P.inv_norm = a->gk_normalizer > 0.f ? 1.f / a->gk_normalizer : 0.f;
+    P.rms_eps = a->rms_eps;
+    P.rms_w = static_cast<const __half*>(a->rms_weight);
+    P.gate = static_cast<const __half*>(a->out_gate);
+    int64_t gs[3];
+    if (int rc = resolve_strides(a->gate_stride, a->T, a->H, gla::kD, gs)) return rc;
+    P.gate_sb = gs[0]; P.gate_st = gs[1]; P.gate_sh = gs[2];
+    P.s0 = a->initial_state;
+    P.sT = a->final_state;
+    P.ctrl = reinterpret_cast<uint32_t*>(ws + L.ctrl);
+    P.flags = reinterpret_cast<uint32_t*>(ws + L.flags);
+    P.agg = reinterpret_cast<float*>(ws + L.agg);
+    P.incl = reinterpret_cast<float*>(ws + L.incl);
+    P.wait_limit_us = a->wait_limit ? a->wait_limit : 2000000u;
+
+
+    int words = static_cast<int>((L.clear_bytes - L.flags) / sizeof(uint32_t));
+    void* clear[3] = {&P.ctrl, &P.flags, &words};
+    if (int rc = launch_overlapped(reinterpret_cast<const void*>(&gla::clear_kernel), 1, 256, 0, clear, stream)) return rc;
+    void* args[2] = {&maps, &P};
+    return launch_overlapped(block_kernel((P.inv_norm > 0.f ? 2 : 0) | (P.rev ? 1 : 0)), std::min(P.num_items, slots), gla::block::kThreads,
+                             gla::block::kSmemBytes, args, stream);
+}
+}  // namespace
+
 extern "C" {
 
 int gla_b200_version(void) { return GLA_B200_VERSION; }
@@ -513,12 +672,17 @@ const char* gla_b200_last_cuda_error(void) { return g_cuda_err; }
 
 size_t gla_b200_workspace_bytes(int32_t B, int32_t T, int32_t H, int32_t K, int32_t V) {
     if (B < 0 || T < 0 || H < 0 || (K != 32 && K != gla::kD) || V != gla::kD) return 0;
-    const size_t nseq = static_cast<size_t>(B) * H;
-    const size_t ns = static_cast<size_t>((num_chunks(T) + kMinAutoCps - 1) / kMinAutoCps);
-    return ws_layout(nseq, ns ? ns : 1).total;
+    const int64_t nseq = static_cast<int64_t>(B) * H;
+    const int NT = num_chunks(T);
+    if (nseq * NT == 0) return ws_layout(0).total;
+    const Split s = choose_split(nseq * NT, NT, nseq, 148, ~static_cast<size_t>(0));
+    const size_t explicit_spans = NT > kAdvertisedCps ? static_cast<size_t>(nseq) * ((NT + kAdvertisedCps - 1) / kAdvertisedCps) : 0;
+    const size_t block_segments = static_cast<size_t>((NT + block_plan::kMinAutoCps - 1) / block_plan::kMinAutoCps);
+    return std::max(ws_layout(std::max(exchange_spans(s), explicit_spans)).total,
+                    block_plan::ws_layout(static_cast<size_t>(nseq), block_segments).total);
 }
 
-int gla_b200_forward(const gla_b200_args* a, void* stream_v) {
+static int forward(const gla_b200_args* a, bool block, void* stream_v) {
     if (!a) return GLA_B200_ERR_NULL;
     if ((a->K != 32 && a->K != gla::kD) || a->V != gla::kD || a->B < 0 || a->T < 0 || a->H < 0) return GLA_B200_ERR_SHAPE;
     if (a->direction < 0 || a->direction > 3) return GLA_B200_ERR_DIRECTION;
@@ -577,34 +741,22 @@ int gla_b200_forward(const gla_b200_args* a, void* stream_v) {
     key.Hc = col ? gh : a->T;
     key.Wc = col ? gw : 1;
     key.dev = dev;
+    if (block) return forward_block(a, key, di.sms, static_cast<cudaStream_t>(stream_v));
+    int64_t o_stride[3];
+    memcpy(o_stride, key.stride[gla::TO], sizeof(o_stride));
 
-    // segmentation
     const int NT = num_chunks(a->T);
     const int nseq = a->B * a->H;
-    const int slots = gla::kCtasPerSm * di.sms;
-    int cps;
-    int plan_start[gla::kMaxPlanSegments + 1] = {0}, plan_ns = 0;
-    bool plan = false, relay = false;
-    if (a->segments > 0) cps = a->segments;
-    else {
-        const size_t have = a->workspace ? a->workspace_bytes : 0;
-        cps = auto_chunks_per_segment(NT, nseq, slots, have);
-        const int ns_u = (NT + cps - 1) / cps;
-        const long rounds = (static_cast<long>(nseq) * ns_u + slots - 1) / slots;
-        // what the slowest item of the equal split costs, in the plan's units: every segment but the last pays the pre-pass
-        const double pre = gated ? kPlanPrePassGated : kPlanPrePassPlain;
-        const double uniform_cost = rounds * (cps * (1.0 + (ns_u > 1 ? pre : 0.0)) + (ns_u > 1 ? 1.0 : 0.0));
-        const double plan_cost = staggered_plan(NT, nseq, slots, have, pre, plan_start, &plan_ns);
-        plan = plan_cost > 0.0 && plan_cost < uniform_cost;
-        if (!plan && 2 * nseq > slots) {
-            double relay_cost = 0.0;
-            const int ns_r = relay_segments(NT, nseq, slots, have, &relay_cost);
-            if (ns_r > 1 && relay_cost < 0.97 * uniform_cost) { relay = true; cps = (NT + ns_r - 1) / ns_r; }
-        }
+    const int64_t chunks = static_cast<int64_t>(nseq) * NT;
+    if (chunks > 0x3fffffff) return GLA_B200_ERR_SHAPE;
+    Split split;
+    if (a->segments > 0) {
+        split.per = (NT + a->segments - 1) / a->segments;
+        split.spans = nseq * split.per;
+    } else {
+        split = choose_split(chunks, NT, nseq, di.sms, a->workspace ? a->workspace_bytes : 0);
     }
-    if (cps > NT) cps = NT;
-    const int NS = plan ? plan_ns : (NT + cps - 1) / cps;
-    const WsLayout L = ws_layout(static_cast<size_t>(nseq), static_cast<size_t>(NS));
+    const WsLayout L = ws_layout(exchange_spans(split));
     if (!a->workspace || (reinterpret_cast<uintptr_t>(a->workspace) & 255u) || a->workspace_bytes < L.total)
         return GLA_B200_ERR_WORKSPACE;
 
@@ -618,7 +770,7 @@ int gla_b200_forward(const gla_b200_args* a, void* stream_v) {
         S.ctrl = reinterpret_cast<uint32_t*>(ws + L.ctrl);
         for (int i = 0; i < 3; ++i) {
             S.q_s[i] = key.stride[gla::TQ][i]; S.k_s[i] = key.stride[gla::TK][i]; S.v_s[i] = key.stride[gla::TV][i];
-            S.g_s[i] = key.stride[gla::TG][i]; S.o_s[i] = key.stride[gla::TO][i];
+            S.g_s[i] = key.stride[gla::TG][i]; S.o_s[i] = o_stride[i];
         }
         S.T = a->T; S.H = a->H; S.Hc = key.Hc; S.Wc = key.Wc; S.rev = a->direction & 1;
         S.scale = a->scale;
@@ -631,6 +783,8 @@ int gla_b200_forward(const gla_b200_args* a, void* stream_v) {
         return GLA_B200_OK;
     }
 
+    key.ptr[gla::TO] = nullptr;                       // outputs are stored from registers
+    memset(key.stride[gla::TO], 0, sizeof(key.stride[gla::TO]));
     gla::Maps maps;
     rc = get_maps(key, &maps);
     if (rc != GLA_B200_OK) return rc;
@@ -640,57 +794,36 @@ int gla_b200_forward(const gla_b200_args* a, void* stream_v) {
     P.B = a->B; P.T = a->T; P.H = a->H; P.NT = NT; P.K = a->K;
     P.Hc = key.Hc; P.Wc = key.Wc;
     P.rev = a->direction & 1;
-    P.NS = NS; P.cps = cps;
-    P.plan = plan ? 1 : relay ? 2 : 0;
-    for (int i = 0; i <= gla::kMaxPlanSegments; ++i) P.seg_start[i] = plan_start[i];
-    P.num_items = nseq * NS;
-    P.gated = gated ? 1 : 0;
-    fold_scale(a->scale, &P);
-    P.inv_norm = a->gk_normalizer > 0.f ? 1.f / a->gk_normalizer : 0.f;
-    P.rms_eps = a->rms_eps;
-    P.rms_w = gated ? static_cast<const __half*>(a->rms_weight) : nullptr;
-    P.gate = gated ? static_cast<const __half*>(a->out_gate) : nullptr;
+    set_split(split, chunks, &P);
+    fill_params(a, o_stride, ws, L, &P);
     if (gated) {
+        P.rms_eps = a->rms_eps;
+        P.rms_w = static_cast<const __half*>(a->rms_weight);
+        P.gate = static_cast<const __half*>(a->out_gate);
         int64_t gs[3];
         rc = resolve_strides(a->gate_stride, a->T, a->H, gla::kD, gs);
         if (rc != GLA_B200_OK) return rc;
-        P.gate_sb = gs[0]; P.gate_st = gs[1]; P.gate_sh = gs[2];
+        for (int i = 0; i < 3; ++i) P.gate_s[i] = gs[i];
     }
-    P.s0 = a->initial_state;
-    P.sT = a->final_state;
-    P.ctrl = reinterpret_cast<uint32_t*>(ws + L.ctrl);
-    P.flags = reinterpret_cast<uint32_t*>(ws + L.flags);
-    P.agg = reinterpret_cast<float*>(ws + L.agg);
-    P.incl = reinterpret_cast<float*>(ws + L.incl);
-    P.wait_limit_us = a->wait_limit ? a->wait_limit : 2000000u;
-#ifdef GLA_TRACE
-    P.trace = gla::g_trace_buffer;
-#endif
+    return launch_forward(gated, maps, P, gla::NoTable{}, static_cast<cudaStream_t>(stream_v));
+}
 
-    cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
-    ce = cudaMemsetAsync(ws, 0, L.clear_bytes, stream);
-    if (ce != cudaSuccess) { note_cuda("cudaMemsetAsync", ce); return GLA_B200_ERR_CUDA; }
-    const int grid = P.num_items < slots ? P.num_items : slots;
-    const int variant = (P.gated ? 4 : 0) | (P.inv_norm > 0.f ? 2 : 0) | (P.rev ? 1 : 0);
-    gla::NoTable table;
-    void* kargs[3] = {const_cast<gla::Maps*>(&maps), &P, &table};
-    ce = cudaLaunchKernel(fwd_kernel(variant), dim3(grid), dim3(gla::kThreads), kargs, gla::kSmemBytes, stream);
-    if (ce != cudaSuccess) { note_cuda("cudaLaunchKernel", ce); return GLA_B200_ERR_CUDA; }
-    ce = cudaPeekAtLastError();
-    if (ce != cudaSuccess) { note_cuda("kernel launch", ce); return GLA_B200_ERR_CUDA; }
-    return GLA_B200_OK;
+int gla_b200_forward(const gla_b200_args* a, void* stream) { return forward(a, false, stream); }
+
+int gla_b200_forward_block(const gla_b200_args* a, void* stream) {
+    if (a && !a->out_gate && !a->rms_weight) return GLA_B200_ERR_NULL;
+    return forward(a, true, stream);
 }
 
 size_t gla_b200_packed_workspace_bytes(const int32_t* offsets, int32_t n, int32_t H) {
     if (!offsets || n < 0 || H <= 0) return 0;
-    size_t most = 512;
+    size_t most = 0;
     for (int at = 0; at < n; at += gla::kMaxPacked) {
         gla::PackedTable tab;
-        int items = 0;
-        const int slots = packed_plan(offsets + at, std::min(n - at, gla::kMaxPacked), H, 148, &tab, &items);
-        most = std::max(most, ws_layout(static_cast<size_t>(H), static_cast<size_t>(std::max(slots, 2))).total);
+        const int64_t chunks = packed_table(offsets + at, std::min(n - at, gla::kMaxPacked), H, &tab);
+        if (chunks > 0) most = std::max(most, exchange_spans(packed_split(chunks, static_cast<int64_t>(tab.n) * H, 148)));
     }
-    return most;
+    return ws_layout(most).total;
 }
 
 int gla_b200_forward_packed(const gla_b200_args* a, const int32_t* offsets, int32_t n, void* stream_v) {
@@ -732,6 +865,10 @@ int gla_b200_forward_packed(const gla_b200_args* a, const int32_t* offsets, int3
     DeviceInfo di;
     if (int rc = device_info(dev, &di)) return rc;
     key.B = 1; key.T = a->T; key.H = a->H; key.K = a->K; key.Hc = a->T; key.Wc = 1; key.dev = dev;
+    int64_t o_stride[3];
+    memcpy(o_stride, key.stride[gla::TO], sizeof(o_stride));
+    key.ptr[gla::TO] = nullptr;                       // outputs are stored from registers
+    memset(key.stride[gla::TO], 0, sizeof(key.stride[gla::TO]));
     gla::Maps maps;
     if (int rc = get_maps(key, &maps)) return rc;
     uint8_t* ws = static_cast<uint8_t*>(a->workspace);
@@ -740,24 +877,18 @@ int gla_b200_forward_packed(const gla_b200_args* a, const int32_t* offsets, int3
         gla::PackedTable tab;
         gla::Params P;
         memset(&P, 0, sizeof(P));
-        const int slots = packed_plan(offsets + at, std::min(n - at, gla::kMaxPacked), a->H, 148, &tab, &P.num_items);
-        if (P.num_items == 0) continue;
-        const WsLayout L = ws_layout(static_cast<size_t>(a->H), static_cast<size_t>(std::max(slots, 2)));
+        const int64_t chunks = packed_table(offsets + at, std::min(n - at, gla::kMaxPacked), a->H, &tab);
+        if (chunks == 0) continue;
+        if (chunks > 0x3fffffff) return GLA_B200_ERR_SHAPE;
+        const Split split = packed_split(chunks, static_cast<int64_t>(tab.n) * a->H, 148);
+        const WsLayout L = ws_layout(exchange_spans(split));
         if (a->workspace_bytes < L.total) return GLA_B200_ERR_WORKSPACE;
         P.B = 1; P.T = a->T; P.H = a->H; P.K = a->K; P.Hc = a->T; P.Wc = 1;
-        fold_scale(a->scale, &P);
-        P.inv_norm = a->gk_normalizer > 0.f ? 1.f / a->gk_normalizer : 0.f;
+        set_split(split, chunks, &P);
+        fill_params(a, o_stride, ws, L, &P);
         P.s0 = a->initial_state ? a->initial_state + at * state_floats : nullptr;
         P.sT = a->final_state ? a->final_state + at * state_floats : nullptr;
-        P.ctrl = reinterpret_cast<uint32_t*>(ws + L.ctrl); P.flags = reinterpret_cast<uint32_t*>(ws + L.flags);
-        P.agg = reinterpret_cast<float*>(ws + L.agg); P.incl = reinterpret_cast<float*>(ws + L.incl);
-        P.wait_limit_us = a->wait_limit ? a->wait_limit : 2000000u;
-        ce = cudaMemsetAsync(ws, 0, L.clear_bytes, stream);
-        if (ce != cudaSuccess) { note_cuda("cudaMemsetAsync", ce); return GLA_B200_ERR_CUDA; }
-        void* kargs[3] = {&maps, &P, &tab};
-        ce = cudaLaunchKernel(packed_kernel(P.inv_norm > 0.f), dim3(std::min(P.num_items, di.sms)), dim3(gla::kThreads), kargs,
-                              gla::kSmemBytes, stream);
-        if (ce != cudaSuccess) { note_cuda("cudaLaunchKernel", ce); return GLA_B200_ERR_CUDA; }
+        if (int rc = launch_forward(false, maps, P, tab, stream)) return rc;
     }
     return GLA_B200_OK;
 }
@@ -818,7 +949,6 @@ int gla_b200_selftest_wait_timeout(void* workspace, size_t workspace_bytes, uint
     gla::Params P;
     memset(&P, 0, sizeof(P));
     P.ctrl = static_cast<uint32_t*>(workspace);
-    P.flags = P.ctrl + 64;
     P.wait_limit_us = limit_us;
     gla::wait_timeout_selftest_kernel<<<1, 32, 0, stream>>>(P);
     e = cudaPeekAtLastError();
@@ -859,7 +989,7 @@ static int bwd_segments(int64_t nseq, int NT, int* cps_out) {
     return (NT + best_cps - 1) / best_cps;
 }
 
-struct BwdLayout { size_t chunk_state, chunk_decay, seg_grad, seg_decay, park, total; };
+struct BwdLayout { size_t chunk_state, chunk_decay, seg_grad, seg_decay, total; };
 static BwdLayout bwd_layout(int64_t nseq, int NT, int nseg) {
     BwdLayout L;
     const size_t chunks = static_cast<size_t>(nseq) * NT, segs = static_cast<size_t>(nseq) * nseg;
@@ -867,8 +997,7 @@ static BwdLayout bwd_layout(int64_t nseq, int NT, int nseg) {
     L.chunk_decay = L.chunk_state + chunks * 64 * 64 * sizeof(float);
     L.seg_grad = L.chunk_decay + chunks * 64 * sizeof(float);
     L.seg_decay = L.seg_grad + segs * 64 * 64 * sizeof(float);
-    L.park = L.seg_decay + segs * 64 * sizeof(float);
-    L.total = L.park + 2 * segs * 64 * 64 * sizeof(float);
+    L.total = L.seg_decay + segs * 64 * sizeof(float);
     return L;
 }
 
@@ -939,18 +1068,18 @@ int gla_b200_backward_scan(const gla_b200_bwd_args* a, const gla_b200_bwd_scan* 
     P.ctrl = reinterpret_cast<uint32_t*>(ws);
     P.chunk_state = reinterpret_cast<float*>(ws + L.chunk_state); P.chunk_decay = reinterpret_cast<float*>(ws + L.chunk_decay);
     P.seg_grad = reinterpret_cast<float*>(ws + L.seg_grad); P.seg_decay = reinterpret_cast<float*>(ws + L.seg_decay);
-    P.park = reinterpret_cast<float*>(ws + L.park);
     P.B = a->B; P.T = a->T; P.H = a->H; P.NT = NT;
     P.Hc = key.Hc; P.Wc = key.Wc; P.rev = o ? (o->direction & 1) : 0;
+    P.wait_limit_us = 2000000u;
     P.scale = a->scale;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
     const unsigned ctas = static_cast<unsigned>(nseq * P.nseg);
     const dim3 states(ctas, P.nseg > 1 ? 2 : 1);
     if (a->K == 64) {
-        gla::gla_bwd_state_kernel<64><<<states, gla::kBwdThreads, gla::BwdStateSmem::kBytes, stream>>>(maps, P);
+        gla::gla_bwd_state_kernel<64><<<states, gla::kComputeThreads, gla::BwdStateSmem::kBytes, stream>>>(maps, P);
         gla::gla_bwd_chunk_kernel<64><<<ctas, gla::kBwdChunkThreads, gla::BwdChunkSmem::kBytes, stream>>>(maps, P);
     } else {
-        gla::gla_bwd_state_kernel<32><<<states, gla::kBwdThreads, gla::BwdStateSmem::kBytes, stream>>>(maps, P);
+        gla::gla_bwd_state_kernel<32><<<states, gla::kComputeThreads, gla::BwdStateSmem::kBytes, stream>>>(maps, P);
         gla::gla_bwd_chunk_kernel<32><<<ctas, gla::kBwdChunkThreads, gla::BwdChunkSmem::kBytes, stream>>>(maps, P);
     }
     e = cudaPeekAtLastError();

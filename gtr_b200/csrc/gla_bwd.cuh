@@ -38,11 +38,10 @@
 #include <cuda_fp16.h>
 #include <cstdint>
 
-#include "gla_kernel.cuh"
+#include "gla_tiles.cuh"
 
 namespace gla {
 
-constexpr int kBwdThreads = 256;
 constexpr float kBwdRefLimit = 8.f;       // log2: qt and kt carry factors up to 2^8, see bwd_scale() for the room they have
 
 struct BwdParams {
@@ -57,144 +56,28 @@ struct BwdParams {
     float* chunk_decay;   // scratch [B*H][NT][64]: log2 decay from the segment's start to the chunk's end
     float* seg_grad;      // scratch [B*H][nseg][4096]: state gradient at a segment's start, from zero at its end
     float* seg_decay;     // scratch [B*H][nseg][64]: log2 decay over the segment
-    float* park;          // scratch [B*H][nseg][2][4096]: what a thread holds (dS; q and k) while a wide chunk has the registers
     uint32_t* ctrl;       // [1] status: a bounded wait expired
+    uint32_t wait_limit_us;
     int B, T, H, NT;
     int nseg, cps;        // segments per sequence, chunks per segment
     int Hc, Wc, rev;      // scan order as in Params
     float scale;
 };
 
-// ------------------------------------------------------------------------------------------ shared pieces
-// One M = 64 accumulator per slot: 64 columns, lanes 0-15 (even slots) or 16-31 (odd) of every quadrant.
-__device__ __forceinline__ uint32_t bwd_slot(uint32_t tmem, int slot) {
-    return tmem + (static_cast<uint32_t>(16 * (slot & 1)) << 16) + 64u * static_cast<uint32_t>(slot >> 1);
-}
-// 16 columns of one accumulator row: lanes 0-15 of warp w columns 32 (w / 4) .. +15 of rows 16 (w % 4) + lane, lanes 16-31
-// columns +16 .. +31 of the same rows.
-__device__ __forceinline__ void bwd_read(uint32_t tmem, int slot, int w, float* x) {
-    const uint32_t a = bwd_slot(tmem, slot) + (static_cast<uint32_t>(32 * (w & 3)) << 16) + 32u * static_cast<uint32_t>(w >> 2);
-    uint32_t* r = reinterpret_cast<uint32_t*>(x);
-    asm volatile(
-        "tcgen05.ld.sync.aligned.16x32bx2.x16.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16], 16;"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(a)
-        : "memory");
-}
-// columns `off` .. +7 of the same piece
-__device__ __forceinline__ void bwd_read8(uint32_t tmem, int slot, int w, uint32_t off, float* x) {
-    const uint32_t a = bwd_slot(tmem, slot) + (static_cast<uint32_t>(32 * (w & 3)) << 16) + 32u * static_cast<uint32_t>(w >> 2) + off;
-    uint32_t* r = reinterpret_cast<uint32_t*>(x);
-    asm volatile("tcgen05.ld.sync.aligned.16x32bx2.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8], 16;"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(a)
-                 : "memory");
-}
-__device__ __forceinline__ void bwd_write(uint32_t tmem, int slot, int w, const float* x) {
-    const uint32_t a = bwd_slot(tmem, slot) + (static_cast<uint32_t>(32 * (w & 3)) << 16) + 32u * static_cast<uint32_t>(w >> 2);
-    const uint32_t* r = reinterpret_cast<const uint32_t*>(x);
-    asm volatile(
-        "tcgen05.st.sync.aligned.16x32bx2.x16.b32 [%0], 16, "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-        ::"r"(a), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
-          "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-        : "memory");
-}
-
-// D (+)= A B over K = 64 from two swizzled tiles; kA / kB: 1 when the tile's rows are the contraction index.
-template <uint32_t kA, uint32_t kB>
-__device__ __forceinline__ void bwd_mma(uint32_t d, uint32_t a, uint32_t b, bool accumulate) {
-    constexpr uint32_t id = umma_idesc(FMT_F16, kA, kB, 64, 64);
-    const uint64_t da = umma_desc_sw128(a, 8192), db = umma_desc_sw128(b, 8192);
-#pragma unroll
-    for (uint32_t ks = 0; ks < 4; ++ks)
-        umma_f16(d, da + ks * (kA ? 128u : 2u), db + ks * (kB ? 128u : 2u), id, (accumulate || ks > 0) ? 1u : 0u);
-}
-
-// Bounded wait for an MMA batch; on expiry the status word is set and the kernel goes on (its result is undefined).
-__device__ __forceinline__ void bwd_wait(uint32_t* ctrl, uint32_t bar, uint32_t parity) {
-    if (mbar_try_wait(bar, parity)) return;
-    const uint64_t t0 = globaltimer_ns();
-    for (uint32_t n = 0;; ++n) {
-        if (mbar_try_wait(bar, parity)) return;
-        if ((n & 63u) == 63u && globaltimer_ns() - t0 > 2000000000ull) {
-            atomicCAS(ctrl + 1, 0u, static_cast<uint32_t>(WHERE_MBAR));
-            return;
-        }
-    }
-}
-
-// token (row of the [B,T,...] tensors) at scan position p, or -1 past the end
-__device__ __forceinline__ int bwd_token(const BwdParams& P, int p) {
-    if (p >= P.T) return -1;
-    const int u = P.rev ? P.T - 1 - p : p;
-    if (P.Wc == 1) return u;
-    const int c = u / P.Hc;
-    return (u - c * P.Hc) * P.Wc + c;
-}
-
-// One chunk of `n` tensors into tiles, in the order the rows lie in memory (a reversed scan's chunk is mirrored: its first
-// token along the scan is row 63).  Rows past the sequence are filled with zeros, channels a K = 32 head does not have too.
-__device__ __forceinline__ void bwd_load(const Maps& maps, const BwdParams& P, int chunk, int b, int h, uint32_t bar, int n,
-                                         const int* tensors, const uint32_t* tiles) {
-    const BoxWalker bw(P, chunk * kChunk);
-    bw.for_each(P, [&](int id, int r, int c, int row) {
-        for (int i = 0; i < n; ++i) tma_load_5d(tiles[i] + 128u * row, &maps.m[tensors[i]][id], bar, 0, h, r, c, b);
-    });
-    bw.for_each_missing(P, [&](int id, int row) {
-        for (int i = 0; i < n; ++i) tma_load_5d(tiles[i] + 128u * row, &maps.m[tensors[i]][id], bar, 0, h, P.Hc, 0, b);
-    });
-}
-__device__ __forceinline__ void bwd_bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
-}
-__device__ __forceinline__ void bwd_bar_arrive(uint32_t id, uint32_t threads) {
-    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
-}
-
-// 16 columns of one row of a swizzled fp16 tile as they lie there
-__device__ __forceinline__ void bwd_row16(uint32_t tile, uint32_t row, uint32_t unit, uint32_t* r) {
-    const uint4 a = ld_shared_v4(sw_unit(tile, row, unit)), b = ld_shared_v4(sw_unit(tile, row, unit + 1));
-    r[0] = a.x; r[1] = a.y; r[2] = a.z; r[3] = a.w; r[4] = b.x; r[5] = b.y; r[6] = b.z; r[7] = b.w;
-}
-__device__ __forceinline__ void bwd_put16(uint32_t tile, uint32_t row, uint32_t unit, const uint32_t* r) {
-    st_shared_v4(sw_unit(tile, row, unit), r[0], r[1], r[2], r[3]);
-    st_shared_v4(sw_unit(tile, row, unit + 1), r[4], r[5], r[6], r[7]);
-}
-// Two fp32 lanes per instruction: these kernels are bound by instruction issue first.
-__device__ __forceinline__ float2 bwd_fma2(float2 a, float2 b, float2 c) {
-    unsigned long long d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d)
-        : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)),
-          "l"(reinterpret_cast<const unsigned long long&>(c)));
-    return reinterpret_cast<const float2&>(d);
-}
-__device__ __forceinline__ float2 bwd_mul2(float2 a, float2 b) {
-    unsigned long long d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d)
-        : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)));
-    return reinterpret_cast<const float2&>(d);
-}
-__device__ __forceinline__ float2 bwd_two(float x) { return make_float2(x, x); }
-__device__ __forceinline__ float2 bwd_pair(const float* x, int e) { return make_float2(x[2 * e], x[2 * e + 1]); }
-__device__ __forceinline__ float2 bwd_ex2(float2 x) { return make_float2(ex2(x.x), ex2(x.y)); }
-
+// ------------------------------------------------------------------------------------------ operands and scales
 // a pair as a high and a low fp16 part
 __device__ __forceinline__ void bwd_split(float2 x, uint32_t& h, uint32_t& l) {
     h = pack_half2(x.x, x.y);
-    const float2 d = bwd_fma2(unpack_half2(h), make_float2(-1.f, -1.f), x);
+    const float2 d = fma2(unpack_half2(h), make_float2(-1.f, -1.f), x);
     l = pack_half2(d.x, d.y);
 }
 // x[0..15] * f as a high and a low fp16 part, one row piece of two tiles
 __device__ __forceinline__ void bwd_put_split(uint32_t hi, uint32_t lo, uint32_t row, uint32_t unit, const float* x, float f = 1.f) {
     uint32_t h[8], l[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) bwd_split(bwd_mul2(bwd_pair(x, i), bwd_two(f)), h[i], l[i]);
-    bwd_put16(hi, row, unit, h);
-    bwd_put16(lo, row, unit, l);
+    for (int i = 0; i < 8; ++i) bwd_split(mul2(pair_of(x, i), two(f)), h[i], l[i]);
+    put16(hi, row, unit, h);
+    put16(lo, row, unit, l);
 }
 // in[0..15] * 2^(x * mul + add) likewise: the gated operands
 __device__ __forceinline__ void bwd_put_gated(uint32_t hi, uint32_t lo, uint32_t row, uint32_t unit, const uint32_t* in, const float* x,
@@ -202,9 +85,9 @@ __device__ __forceinline__ void bwd_put_gated(uint32_t hi, uint32_t lo, uint32_t
     uint32_t h[8], l[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i)
-        bwd_split(bwd_mul2(unpack_half2(in[i]), bwd_ex2(bwd_fma2(bwd_pair(x, i), bwd_two(mul), bwd_two(add)))), h[i], l[i]);
-    bwd_put16(hi, row, unit, h);
-    bwd_put16(lo, row, unit, l);
+        bwd_split(mul2(unpack_half2(in[i]), ex2_2(fma2(pair_of(x, i), two(mul), two(add)))), h[i], l[i]);
+    put16(hi, row, unit, h);
+    put16(lo, row, unit, l);
 }
 
 // largest |x| of 16 packed halves, as the bits of a half2 (both halves)
@@ -218,9 +101,6 @@ __device__ __forceinline__ float bwd_half_max(uint32_t m) {
     const float2 f = unpack_half2(m);
     return fmaxf(f.x, f.y);
 }
-__device__ __forceinline__ float bwd_warp_max(float x) {          // x >= 0: ordered like its bits
-    return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(x)));
-}
 // the power of two that brings m to [2^(to-1), 2^to); 1 for zero and for what is not finite
 __device__ __forceinline__ float bwd_scale(float m, int to) {
     const int e = static_cast<int>(__float_as_uint(m) >> 23);     // biased exponent: m in [2^(e-127), 2^(e-126))
@@ -230,14 +110,6 @@ __device__ __forceinline__ float bwd_scale(float m, int to) {
 __device__ __forceinline__ float bwd_log2(float f) { return static_cast<float>(static_cast<int>(__float_as_uint(f) >> 23) - 127); }  // of a power of two
 __device__ __forceinline__ float bwd_inverse(float f) { return __uint_as_float((254u << 23) - __float_as_uint(f)); }   // of a power of two
 
-// A [64 x 64] constant operand of the gate-sum MMA: out-of-place K-major tile, entry (r, s) = value(r, s)
-template <class F>
-__device__ __forceinline__ void bwd_constant(uint8_t* tile, F value) {
-    for (int e = threadIdx.x; e < 64 * 64; e += blockDim.x) {
-        const uint32_t r = static_cast<uint32_t>(e) >> 6, s = static_cast<uint32_t>(e) & 63u;
-        *reinterpret_cast<__half*>(tile + sw_f16(r, s)) = __float2half(value(r, s));
-    }
-}
 // ------------------------------------------------------------------------------------------ segments' states
 // blockIdx.y 0: S after every chunk of a segment, from zero at its start:     S' = 2^G_L S + (k 2^(G_L-G))^T v
 // blockIdx.y 1: dS at a segment's start, from zero at its end (walked backwards): dS' = 2^G_L dS + scale (q 2^G)^T do
@@ -257,7 +129,7 @@ struct BwdStateMisc {
 static_assert(sizeof(BwdStateMisc) <= 1024, "misc block too large");
 
 template <int K>
-__global__ void __launch_bounds__(kBwdThreads, 3) gla_bwd_state_kernel(const __grid_constant__ Maps maps, const __grid_constant__ BwdParams P) {
+__global__ void __launch_bounds__(kComputeThreads, 3) gla_bwd_state_kernel(const __grid_constant__ Maps maps, const __grid_constant__ BwdParams P) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw), base = (raw + 1023u) & ~1023u;
     uint8_t* base_ptr = smem_raw + (base - raw);
@@ -284,7 +156,7 @@ __global__ void __launch_bounds__(kBwdThreads, 3) gla_bwd_state_kernel(const __g
         tmem_relinquish();
     }
     // log factor of a row: the gates after it (forward), its own and those before it (backward), along the scan
-    bwd_constant(base_ptr + BwdStateSmem::kMat, [&](uint32_t r, uint32_t s) { return (back ? (rev ? s >= r : s <= r) : (rev ? s < r : s > r)) ? 1.f : 0.f; });
+    fill_constant(base + BwdStateSmem::kMat, [&](uint32_t r, uint32_t s) { return (back ? (rev ? s >= r : s <= r) : (rev ? s < r : s > r)) ? 1.f : 0.f; });
     fence_proxy_async_smem();
     tc_fence_before();
     __syncthreads();
@@ -296,7 +168,7 @@ __global__ void __launch_bounds__(kBwdThreads, 3) gla_bwd_state_kernel(const __g
         const int tensors[3] = {TG, back ? TQ : TK, back ? TO : TV};
         const uint32_t tiles[3] = {s + 2 * kTileBytes, s, s + kTileBytes};
         mbar_arrive_expect_tx(bar, 3 * kTileBytes);
-        bwd_load(maps, P, chunk_of(i), b, h, bar, 3, tensors, tiles);
+        load_chunk(maps, Scan{P.T, P.Hc, P.rev}, chunk_of(i), b, h, 0, P.Hc, bar, tensors, tiles, l2_policy_normal());
     };
     if (w == 0 && elect_one()) load(0);
 
@@ -310,23 +182,23 @@ __global__ void __launch_bounds__(kBwdThreads, 3) gla_bwd_state_kernel(const __g
     for (int i = 0; i < n; ++i) {
         const int st = i & 1;
         const uint32_t ta = base + st * BwdStateSmem::kStage, tb = ta + kTileBytes, tg = tb + kTileBytes;
-        bwd_wait(P.ctrl, smem_u32(&M.full[st]), (i >> 1) & 1);
+        wait_bar(P, M.full[st], (i >> 1) & 1);
         if (w == 0 && elect_one()) {
             tc_fence_after();
-            bwd_mma<0, 1>(bwd_slot(tmem, 0), mat, tg, false);
+            tile_mma<0, 1>(acc_slot(tmem, 0), mat, tg, false);
             umma_commit(smem_u32(&M.bar_x));
             if (i + 1 < n) load(i + 1);
         }
         uint32_t a[8];
-        bwd_row16(ta, row, u0, a);
+        row16(ta, row, u0, a);
         {
             const uint32_t m = __reduce_max_sync(0xffffffffu, __float_as_uint(bwd_half_max(bwd_max16(a))));
             if (l == 0) M.top[w] = m;
         }
-        bwd_wait(P.ctrl, smem_u32(&M.bar_x), i & 1);
+        wait_bar(P, M.bar_x, i & 1);
         tc_fence_after();
         float x[16];
-        bwd_read(tmem, 0, w, x);
+        acc_read(tmem, 0, w, x);
         tmem_ld_wait();
         __syncthreads();                                            // every warp's maximum is there
         uint32_t m = M.top[0];
@@ -335,7 +207,7 @@ __global__ void __launch_bounds__(kBwdThreads, 3) gla_bwd_state_kernel(const __g
         const float f = bwd_scale(__uint_as_float(m), 15);
         if (row == ((back != rev) ? 63u : 0u)) {                             // x + own gate (forward), x (backward) = G_L
             uint32_t gr[8];
-            bwd_row16(tg, row, u0, gr);
+            row16(tg, row, u0, gr);
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
                 const float2 gf = unpack_half2(gr[e]);
@@ -349,27 +221,27 @@ __global__ void __launch_bounds__(kBwdThreads, 3) gla_bwd_state_kernel(const __g
         __syncthreads();
         if (w == 0 && elect_one()) {
             tc_fence_after();
-            bwd_mma<1, 1>(bwd_slot(tmem, 1), ta, tb, false);
-            bwd_mma<1, 1>(bwd_slot(tmem, 1), low, tb, true);
+            tile_mma<1, 1>(acc_slot(tmem, 1), ta, tb, false);
+            tile_mma<1, 1>(acc_slot(tmem, 1), low, tb, true);
             umma_commit(smem_u32(&M.bar_inc));
         }
         const float gl = M.gl[row], decay = ex2(gl), c = (back ? P.scale : 1.f) * bwd_inverse(f);
         total += gl;
-        bwd_wait(P.ctrl, smem_u32(&M.bar_inc), i & 1);
+        wait_bar(P, M.bar_inc, i & 1);
         tc_fence_after();
-        bwd_read(tmem, 1, w, x);
+        acc_read(tmem, 1, w, x);
         tmem_ld_wait();
         tc_fence_before();
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-            const float2 s = bwd_fma2(bwd_two(decay), bwd_pair(S, e), bwd_mul2(bwd_two(c), bwd_pair(x, e)));
+            const float2 s = fma2(two(decay), pair_of(S, e), mul2(two(c), pair_of(x, e)));
             S[2 * e] = s.x; S[2 * e + 1] = s.y;
         }
         if (!back) {
             const size_t at = cslot + chunk_of(i);
             float4* dst = reinterpret_cast<float4*>(P.chunk_state + at * 4096) + tid;
 #pragma unroll
-            for (int e = 0; e < 4; ++e) dst[e * kBwdThreads] = make_float4(S[4 * e], S[4 * e + 1], S[4 * e + 2], S[4 * e + 3]);
+            for (int e = 0; e < 4; ++e) dst[e * kComputeThreads] = make_float4(S[4 * e], S[4 * e + 1], S[4 * e + 2], S[4 * e + 3]);
             if (c0 == 0) P.chunk_decay[at * 64 + row] = total;
         }
     }
@@ -377,7 +249,7 @@ __global__ void __launch_bounds__(kBwdThreads, 3) gla_bwd_state_kernel(const __g
         const size_t at = static_cast<size_t>(bh) * P.nseg + seg;
         float4* dst = reinterpret_cast<float4*>(P.seg_grad + at * 4096) + tid;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) dst[e * kBwdThreads] = make_float4(S[4 * e], S[4 * e + 1], S[4 * e + 2], S[4 * e + 3]);
+        for (int e = 0; e < 4; ++e) dst[e * kComputeThreads] = make_float4(S[4 * e], S[4 * e + 1], S[4 * e + 2], S[4 * e + 3]);
         if (c0 == 0) P.seg_decay[at * 64 + row] = total;
     }
     tc_fence_before();
@@ -438,12 +310,12 @@ __device__ __noinline__ void bwd_wide_chunk(uint32_t base, const float* vec, uin
     const uint32_t tg = base + BwdChunkSmem::kG, tq = base + BwdChunkSmem::kQ, tk = base + BwdChunkSmem::kK;
     const uint32_t dp = base + BwdChunkSmem::kR, out = dp + 2 * kTileBytes;
     float x[16];
-    auto sync = [] { named_bar_sync(BWD_BAR_COMPUTE, kBwdThreads); };
+    auto sync = [] { named_bar_sync(BWD_BAR_COMPUTE, kComputeThreads); };
     auto at = [&](int t) { return static_cast<uint32_t>(rev ? 63 - t : t); };     // row of the chunk's t-th token
     uint32_t qr[8], kr[8];
-    bwd_row16(tq, row, u0, qr);
-    bwd_row16(tk, row, u0, kr);
-    bwd_read(tmem, BWD_DP, w, x);
+    row16(tq, row, u0, qr);
+    row16(tk, row, u0, kr);
+    acc_read(tmem, BWD_DP, w, x);
     tmem_ld_wait();
     bwd_f32_put16(dp, row, c0, x);
     sync();
@@ -453,7 +325,7 @@ __device__ __noinline__ void bwd_wide_chunk(uint32_t base, const float* vec, uin
     float acc[16], D[16];
     {
         uint32_t own[8];
-        bwd_row16(tq, at(i), cu, own);
+        row16(tq, at(i), cu, own);
 #pragma unroll
         for (int e = 0; e < 16; ++e) acc[e] = D[e] = 0.f;
         for (int s = 0; s < 64; ++s) {
@@ -461,8 +333,8 @@ __device__ __noinline__ void bwd_wide_chunk(uint32_t base, const float* vec, uin
             float a = 0.f;
             if (j >= 0) {
                 uint32_t kk[8], gg[8];
-                bwd_row16(tk, at(j), cu, kk);
-                bwd_row16(tg, at(j), cu, gg);
+                row16(tk, at(j), cu, kk);
+                row16(tg, at(j), cu, gg);
                 const float d = ld_shared_f(bwd_f32(dp, at(i), at(j)));
 #pragma unroll
                 for (int e = 0; e < 8; ++e) {
@@ -483,20 +355,20 @@ __device__ __noinline__ void bwd_wide_chunk(uint32_t base, const float* vec, uin
     }
     sync();
     bwd_f32_row16(out, row, c0, x);
-    bwd_write(tmem, BWD_P, w, x);
+    acc_write(tmem, BWD_P, w, x);
     sync();
 #pragma unroll
     for (int e = 0; e < 16; ++e) acc[e] *= scale;
     bwd_f32_put16(out, at(i), ch, acc);
     sync();
     bwd_f32_row16(out, row, c0, x);
-    bwd_write(tmem, BWD_DQ_I, w, x);
+    acc_write(tmem, BWD_DQ_I, w, x);
 #pragma unroll
     for (int e = 0; e < 16; ++e) acc[e] = D[e] = 0.f;
     for (int t = i; t < 64; ++t) {
         uint32_t qq[8], gg[8];
         if (t > i) {
-            bwd_row16(tg, at(t), cu, gg);
+            row16(tg, at(t), cu, gg);
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
                 const float2 gf = unpack_half2(gg[e]);
@@ -504,7 +376,7 @@ __device__ __noinline__ void bwd_wide_chunk(uint32_t base, const float* vec, uin
                 D[2 * e + 1] = fmaf(gf.y, kLog2e, D[2 * e + 1]);
             }
         }
-        bwd_row16(tq, at(t), cu, qq);
+        row16(tq, at(t), cu, qq);
         const float d = ld_shared_f(bwd_f32(dp, at(t), at(i))) * scale;
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
@@ -517,9 +389,9 @@ __device__ __noinline__ void bwd_wide_chunk(uint32_t base, const float* vec, uin
     bwd_f32_put16(out, at(i), ch, acc);
     sync();
     bwd_f32_row16(out, row, c0, x);
-    bwd_write(tmem, BWD_DP, w, x);
+    acc_write(tmem, BWD_DP, w, x);
     float gsum[16];
-    bwd_read(tmem, BWD_X, w, gsum);
+    acc_read(tmem, BWD_X, w, gsum);
     tmem_ld_wait();
 #pragma unroll
     for (int e = 0; e < 16; ++e) x[e] = fmaf(gsum[e], kLog2e, vec[c0 + e]);
@@ -530,7 +402,7 @@ __device__ __noinline__ void bwd_wide_chunk(uint32_t base, const float* vec, uin
     tmem_st_wait();
 }
 
-constexpr int kBwdChunkThreads = kBwdThreads + 32;       // eight compute warps, one that issues MMAs and copies
+constexpr int kBwdChunkThreads = kComputeThreads + 32;       // eight compute warps, one that issues MMAs and copies
 
 // Per chunk (walked from the segment's last to its first), compute warps | issuing warp:
 //   tiles landed:  maxima of the tiles and states    | X = G - G_L/2 and dP = do v^T
@@ -572,7 +444,7 @@ __global__ void __launch_bounds__(kBwdChunkThreads, 2) gla_bwd_chunk_kernel(cons
         tmem_alloc(smem_u32(&M.tmem), 256);
         tmem_relinquish();
     }
-    bwd_constant(base_ptr + BwdChunkSmem::kMat, [&](uint32_t r, uint32_t s) { return (rev ? s >= r : s <= r) ? 0.5f : -0.5f; });      // G - G_L / 2
+    fill_constant(base + BwdChunkSmem::kMat, [&](uint32_t r, uint32_t s) { return (rev ? s >= r : s <= r) ? 0.5f : -0.5f; });      // G - G_L / 2
     if (tid < 16) M.top[tid >> 3][tid & 7] = 0u;
     fence_proxy_async_smem();
     tc_fence_before();
@@ -580,77 +452,77 @@ __global__ void __launch_bounds__(kBwdChunkThreads, 2) gla_bwd_chunk_kernel(cons
     tc_fence_after();
     const uint32_t tmem = M.tmem;
 
-    if (w == kBwdThreads / 32) {
+    if (w == kComputeThreads / 32) {
         // ==================================================================== issuing warp
-        const uint32_t sx = bwd_slot(tmem, BWD_X), sp = bwd_slot(tmem, BWD_P), sdp = bwd_slot(tmem, BWD_DP), sdq = bwd_slot(tmem, BWD_DQ_S),
-                       sdk = bwd_slot(tmem, BWD_DK_S), sdv = bwd_slot(tmem, BWD_DV_S), sinc = bwd_slot(tmem, BWD_INC), sdqi = bwd_slot(tmem, BWD_DQ_I);
+        const uint32_t sx = acc_slot(tmem, BWD_X), sp = acc_slot(tmem, BWD_P), sdp = acc_slot(tmem, BWD_DP), sdq = acc_slot(tmem, BWD_DQ_S),
+                       sdk = acc_slot(tmem, BWD_DK_S), sdv = acc_slot(tmem, BWD_DV_S), sinc = acc_slot(tmem, BWD_INC), sdqi = acc_slot(tmem, BWD_DQ_I);
         // chunk i's tiles, and the state after chunk i - 1 (relative to the segment's start) into r2, r3
         auto load = [&](int i) {
             const uint32_t bar = smem_u32(&M.full);
             mbar_arrive_expect_tx(bar, i > 0 ? 7 * kTileBytes + 256 : 5 * kTileBytes);
             const int tensors[5] = {TG, TO, TV, TQ, TK};
             const uint32_t tiles[5] = {tg, tdo, tv, tq, tk};
-            bwd_load(maps, P, first + i, b, h, bar, 5, tensors, tiles);
+            load_chunk(maps, Scan{P.T, P.Hc, P.rev}, first + i, b, h, 0, P.Hc, bar, tensors, tiles, l2_policy_normal());
             if (i > 0) {
-                bwd_bulk_load(r2, P.chunk_state + (cslot + first + i - 1) * 4096, 2 * kTileBytes, bar);
-                bwd_bulk_load(smem_u32(M.decay), P.chunk_decay + (cslot + first + i - 1) * 64, 256, bar);
+                bulk_load(r2, P.chunk_state + (cslot + first + i - 1) * 4096, 2 * kTileBytes, bar);
+                bulk_load(smem_u32(M.decay), P.chunk_decay + (cslot + first + i - 1) * 64, 256, bar);
             }
         };
         if (elect_one()) load(n - 1);
         __syncwarp();
         for (int i = n - 1, it = 0; i >= 0; --i, ++it) {
             const uint32_t ph = it & 1;
-            bwd_wait(P.ctrl, smem_u32(&M.full), ph);
+            wait_bar(P, M.full, ph);
             if (it > 0) named_bar_sync(BWD_BAR_READ, kBwdChunkThreads);            // the previous chunk's accumulators are read
             tc_fence_after();
             if (elect_one()) {
-                bwd_mma<0, 1>(sx, base + BwdChunkSmem::kMat, tg, false);
-                bwd_mma<0, 0>(sdp, tdo, tv, false);
+                tile_mma<0, 1>(sx, base + BwdChunkSmem::kMat, tg, false);
+                tile_mma<0, 0>(sdp, tdo, tv, false);
                 umma_commit(smem_u32(&M.bar_x));
             }
             named_bar_sync(BWD_BAR_STATES, kBwdChunkThreads);
             tc_fence_after();
             const bool wide = M.top[i & 1][6] != 0u;
             if (elect_one()) {
-                bwd_mma<0, 0>(sdq, tdo, r0, false);
-                bwd_mma<0, 0>(sdq, tdo, r1, true);
-                bwd_mma<0, 0>(sdk, tv, r2, false);
-                bwd_mma<0, 0>(sdk, tv, r3, true);
+                tile_mma<0, 0>(sdq, tdo, r0, false);
+                tile_mma<0, 0>(sdq, tdo, r1, true);
+                tile_mma<0, 0>(sdk, tv, r2, false);
+                tile_mma<0, 0>(sdk, tv, r3, true);
             }
             named_bar_sync(BWD_BAR_GATED, kBwdChunkThreads);
             tc_fence_after();
             if (elect_one()) {
                 if (!wide) {
-                    bwd_mma<0, 0>(sp, tq, tk, false);
-                    bwd_mma<0, 0>(sp, tq, kl, true);
-                    bwd_mma<0, 0>(sp, ql, tk, true);
+                    tile_mma<0, 0>(sp, tq, tk, false);
+                    tile_mma<0, 0>(sp, tq, kl, true);
+                    tile_mma<0, 0>(sp, ql, tk, true);
                 }
                 umma_commit(smem_u32(&M.bar_a));
-                bwd_mma<1, 1>(sinc, tq, tdo, false);
-                bwd_mma<1, 1>(sinc, ql, tdo, true);
-                bwd_mma<0, 1>(sdv, tk, r2, false);
-                bwd_mma<0, 1>(sdv, tk, r3, true);
-                bwd_mma<0, 1>(sdv, kl, r2, true);
+                tile_mma<1, 1>(sinc, tq, tdo, false);
+                tile_mma<1, 1>(sinc, ql, tdo, true);
+                tile_mma<0, 1>(sdv, tk, r2, false);
+                tile_mma<0, 1>(sdv, tk, r3, true);
+                tile_mma<0, 1>(sdv, kl, r2, true);
                 umma_commit(smem_u32(&M.bar_s));
             }
             named_bar_sync(BWD_BAR_SCORES, kBwdChunkThreads);
             tc_fence_after();
             if (elect_one()) {
                 const uint32_t dv = wide ? sp : sdp;
-                bwd_mma<1, 1>(dv, r0, tdo, false);
-                bwd_mma<1, 1>(dv, r1, tdo, true);
+                tile_mma<1, 1>(dv, r0, tdo, false);
+                tile_mma<1, 1>(dv, r1, tdo, true);
                 if (!wide) {
-                    bwd_mma<0, 1>(sdqi, r2, tk, false);
-                    bwd_mma<0, 1>(sdqi, r2, kl, true);
-                    bwd_mma<0, 1>(sdqi, r3, tk, true);
-                    bwd_mma<1, 1>(sp, r2, tq, false);
-                    bwd_mma<1, 1>(sp, r2, ql, true);
-                    bwd_mma<1, 1>(sp, r3, tq, true);
+                    tile_mma<0, 1>(sdqi, r2, tk, false);
+                    tile_mma<0, 1>(sdqi, r2, kl, true);
+                    tile_mma<0, 1>(sdqi, r3, tk, true);
+                    tile_mma<1, 1>(sp, r2, tq, false);
+                    tile_mma<1, 1>(sp, r2, ql, true);
+                    tile_mma<1, 1>(sp, r3, tq, true);
                 }
                 umma_commit(smem_u32(&M.bar_o));
             }
             __syncwarp();
-            bwd_wait(P.ctrl, smem_u32(&M.bar_o), ph);
+            wait_bar(P, M.bar_o, ph);
             if (i > 0 && elect_one()) load(i - 1);
             __syncwarp();
         }
@@ -660,18 +532,18 @@ __global__ void __launch_bounds__(kBwdChunkThreads, 2) gla_bwd_chunk_kernel(cons
         // a key channel (states).
         const uint32_t row = 16u * (w & 3) + (l & 15u), c0 = 32u * (w >> 2) + 16u * (static_cast<uint32_t>(l) >> 4), u0 = c0 >> 3;
         const bool real_row = row < K;
-        auto sync = [] { named_bar_sync(BWD_BAR_COMPUTE, kBwdThreads); };
+        auto sync = [] { named_bar_sync(BWD_BAR_COMPUTE, kComputeThreads); };
         auto hand_over = [](uint32_t id) {                   // operands written by this thread may be read by the tensor core
             fence_proxy_async_smem();
             tc_fence_before();
-            bwd_bar_arrive(id, kBwdChunkThreads);
+            named_bar_arrive(id, kBwdChunkThreads);
         };
         float dS[16];                 // the state gradient at the end of the current chunk
         const uint32_t s0_at = base + BwdChunkSmem::kS0 + 16u * tid;           // float4 e of this thread 4096 bytes apart
         auto own = [&](uint32_t at, float* x) {
 #pragma unroll
             for (uint32_t e = 0; e < 4; ++e) {
-                const float4 v = ld_shared_f4(at + 16u * kBwdThreads * e);
+                const float4 v = ld_shared_f4(at + 16u * kComputeThreads * e);
                 x[4 * e] = v.x; x[4 * e + 1] = v.y; x[4 * e + 2] = v.z; x[4 * e + 3] = v.w;
             }
         };
@@ -685,7 +557,7 @@ __global__ void __launch_bounds__(kBwdChunkThreads, 2) gla_bwd_chunk_kernel(cons
         auto chain = [&](float* x, float f, const float* y) {                // x = f x + y
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
-                const float2 z = bwd_fma2(bwd_two(f), bwd_pair(x, e), bwd_pair(y, e));
+                const float2 z = fma2(two(f), pair_of(x, e), pair_of(y, e));
                 x[2 * e] = z.x; x[2 * e + 1] = z.y;
             }
         };
@@ -700,23 +572,23 @@ __global__ void __launch_bounds__(kBwdChunkThreads, 2) gla_bwd_chunk_kernel(cons
             for (int j = 0; j < seg; ++j) {
                 const size_t at = cslot + static_cast<size_t>(j + 1) * P.cps - 1;
                 float y[16];
-                get(P.chunk_state + at * 4096 + 4 * tid, kBwdThreads, y);
+                get(P.chunk_state + at * 4096 + 4 * tid, kComputeThreads, y);
                 chain(S0, ex2(__ldcg(P.chunk_decay + at * 64 + row)), y);
             }
 #pragma unroll 2
             for (int j = P.nseg - 1; j > seg; --j) {
                 const size_t at = static_cast<size_t>(bh) * P.nseg + j;
                 float y[16];
-                get(P.seg_grad + at * 4096 + 4 * tid, kBwdThreads, y);
+                get(P.seg_grad + at * 4096 + 4 * tid, kComputeThreads, y);
                 chain(dS, ex2(__ldcg(P.seg_decay + at * 64 + row)), y);
             }
 #pragma unroll
-            for (uint32_t e = 0; e < 4; ++e) st_shared_f4(s0_at + 16u * kBwdThreads * e, S0[4 * e], S0[4 * e + 1], S0[4 * e + 2], S0[4 * e + 3]);
+            for (uint32_t e = 0; e < 4; ++e) st_shared_f4(s0_at + 16u * kComputeThreads * e, S0[4 * e], S0[4 * e + 1], S0[4 * e + 2], S0[4 * e + 3]);
             float later = 0.f;
             if (P.dht != nullptr || seg + 1 < P.nseg) {                  // dS is not zero at the segment's end
                 float y[16];
                 const size_t at = cslot + first + n - 1;
-                get(P.chunk_state + at * 4096 + 4 * tid, kBwdThreads, y);
+                get(P.chunk_state + at * 4096 + 4 * tid, kComputeThreads, y);
                 chain(S0, ex2(__ldcg(P.chunk_decay + at * 64 + row)), y);          // now the state after the segment
 #pragma unroll
                 for (int e = 0; e < 16; ++e) later = fmaf(S0[e], dS[e], later);
@@ -738,7 +610,7 @@ __global__ void __launch_bounds__(kBwdChunkThreads, 2) gla_bwd_chunk_kernel(cons
         for (int i = n - 1, it = 0; i >= 0; --i, ++it) {
             const int p = i & 1;
             const uint32_t ph = it & 1;
-            bwd_wait(P.ctrl, smem_u32(&M.full), ph);
+            wait_bar(P, M.full, ph);
             uint32_t qr[8], kr[8];
             float S[16], x[16];
             own(s0_at, S);
@@ -746,16 +618,16 @@ __global__ void __launch_bounds__(kBwdChunkThreads, 2) gla_bwd_chunk_kernel(cons
                 own(r2 + 16u * tid, x);
                 chain(S, ex2(ld_shared_f(decay_at + 4u * row)), x);
             }
-            bwd_row16(tq, row, u0, qr);
-            bwd_row16(tk, row, u0, kr);
+            row16(tq, row, u0, qr);
+            row16(tk, row, u0, kr);
             {
                 float m[6];
                 uint32_t t[8];
                 m[0] = bwd_half_max(bwd_max16(qr));
                 m[1] = bwd_half_max(bwd_max16(kr));
-                bwd_row16(tv, row, u0, t);
+                row16(tv, row, u0, t);
                 m[2] = bwd_half_max(bwd_max16(t));
-                bwd_row16(tdo, row, u0, t);
+                row16(tdo, row, u0, t);
                 m[3] = bwd_half_max(bwd_max16(t));
                 m[4] = m[5] = 0.f;
 #pragma unroll
@@ -771,9 +643,9 @@ __global__ void __launch_bounds__(kBwdChunkThreads, 2) gla_bwd_chunk_kernel(cons
                 }
                 if (l < 6) atomicMax(&M.top[p][l], mine);
             }
-            bwd_wait(P.ctrl, smem_u32(&M.bar_x), ph);
+            wait_bar(P, M.bar_x, ph);
             tc_fence_after();
-            bwd_read(tmem, BWD_X, w, x);
+            acc_read(tmem, BWD_X, w, x);
             tmem_ld_wait();
             if (row == last_row) {                                      // X of the last row is half the chunk's decay
                 bool far = false;
@@ -791,30 +663,27 @@ __global__ void __launch_bounds__(kBwdChunkThreads, 2) gla_bwd_chunk_kernel(cons
             const float fS = bwd_scale(__uint_as_float(M.top[p][4]), 15), fdS = bwd_scale(__uint_as_float(M.top[p][5]), 15);
             const bool wide = M.top[p][6] != 0u;
             if (wide) {
-                // out of line, and everything a register holds across the call is fetched again afterwards: the ordinary chunk
-                // must not pay for it with spills (the SM's shared memory leaves no L1 to catch them)
-                float* park = P.park + (static_cast<size_t>(bh) * P.nseg + seg) * 8192 + 4 * tid;
-                uint4* raw = reinterpret_cast<uint4*>(park + 4096);
+                // out of line, and what registers hold across the call waits in accumulators that are not in use yet: the ordinary
+                // chunk must not pay for it with spills (the SM's shared memory leaves no L1 to catch them)
+                acc_write(tmem, BWD_DQ_S, w, dS);
+                acc_write(tmem, BWD_DK_S, w, S);
 #pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    *reinterpret_cast<float4*>(park + 4 * kBwdThreads * e) = make_float4(dS[4 * e], dS[4 * e + 1], dS[4 * e + 2], dS[4 * e + 3]);
-                raw[0] = make_uint4(qr[0], qr[1], qr[2], qr[3]);
-                raw[kBwdThreads] = make_uint4(qr[4], qr[5], qr[6], qr[7]);
-                raw[2 * kBwdThreads] = make_uint4(kr[0], kr[1], kr[2], kr[3]);
-                raw[3 * kBwdThreads] = make_uint4(kr[4], kr[5], kr[6], kr[7]);
+                for (int e = 0; e < 8; ++e) {
+                    x[e] = __uint_as_float(qr[e]);
+                    x[8 + e] = __uint_as_float(kr[e]);
+                }
+                acc_write(tmem, BWD_DV_S, w, x);
+                tmem_st_wait();
                 bwd_wide_chunk(base, M.vec, tmem, fq, fk, P.scale, rev);
                 sync();
-                get(park, kBwdThreads, dS);
+                acc_read(tmem, BWD_DQ_S, w, dS);
+                acc_read(tmem, BWD_DK_S, w, S);
+                acc_read(tmem, BWD_DV_S, w, x);
+                tmem_ld_wait();
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const uint4 v = __ldcg(raw + e * kBwdThreads);
-                    uint32_t* to = e < 2 ? qr + 4 * e : kr + 4 * (e - 2);
-                    to[0] = v.x; to[1] = v.y; to[2] = v.z; to[3] = v.w;
-                }
-                own(s0_at, S);
-                if (i > 0) {
-                    get(P.chunk_state + (cslot + first + i - 1) * 4096 + 4 * tid, kBwdThreads, x);
-                    chain(S, ex2(__ldcg(P.chunk_decay + (cslot + first + i - 1) * 64 + row)), x);
+                for (int e = 0; e < 8; ++e) {
+                    qr[e] = __float_as_uint(x[e]);
+                    kr[e] = __float_as_uint(x[8 + e]);
                 }
             }
             const float half_decay = M.vec[row], eR = ex2(half_decay);
@@ -822,19 +691,19 @@ __global__ void __launch_bounds__(kBwdChunkThreads, 2) gla_bwd_chunk_kernel(cons
             bwd_put_split(r2, r3, row, u0, dS, (wide ? 1.f : eR) * fdS);
             hand_over(BWD_BAR_STATES);
             if (!wide) {
-                bwd_read(tmem, BWD_X, w, x);
+                acc_read(tmem, BWD_X, w, x);
                 tmem_ld_wait();
                 bwd_put_gated(tq, ql, row, u0, qr, x, kLog2e, bwd_log2(fq));
                 bwd_put_gated(tk, kl, row, u0, kr, x, -kLog2e, bwd_log2(fk));
             }
             hand_over(BWD_BAR_GATED);
             // ---- within the chunk: P and dP, causal, as split operands
-            bwd_wait(P.ctrl, smem_u32(&M.bar_a), ph);
+            wait_bar(P, M.bar_a, ph);
             tc_fence_after();
             if (!beyond) {
                 float y[16];
-                bwd_read(tmem, BWD_P, w, x);
-                bwd_read(tmem, BWD_DP, w, y);                           // (of no use in a wide chunk)
+                acc_read(tmem, BWD_P, w, x);
+                acc_read(tmem, BWD_DP, w, y);                           // (of no use in a wide chunk)
                 tmem_ld_wait();
                 if (on_diagonal) {
                     const int lim = static_cast<int>(row) - static_cast<int>(c0);
@@ -846,33 +715,33 @@ __global__ void __launch_bounds__(kBwdChunkThreads, 2) gla_bwd_chunk_kernel(cons
                     }
                 }
                 bwd_put_split(r0, r1, row, u0, x, fp);                  // St has been read since bar_a, dSt will have with bar_s
-                bwd_wait(P.ctrl, smem_u32(&M.bar_s), ph);
+                wait_bar(P, M.bar_s, ph);
                 bwd_put_split(r2, r3, row, u0, y, fd);
             } else {
                 const uint32_t z[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
-                bwd_put16(r0, row, u0, z); bwd_put16(r1, row, u0, z);
-                bwd_wait(P.ctrl, smem_u32(&M.bar_s), ph);
-                bwd_put16(r2, row, u0, z); bwd_put16(r3, row, u0, z);
+                put16(r0, row, u0, z); put16(r1, row, u0, z);
+                wait_bar(P, M.bar_s, ph);
+                put16(r2, row, u0, z); put16(r3, row, u0, z);
             }
             hand_over(BWD_BAR_SCORES);
             // ---- the state gradient moves to the chunk's start
             if (tid < 8) M.top[p ^ 1][tid] = 0u;
-            bwd_read(tmem, BWD_INC, w, x);
+            acc_read(tmem, BWD_INC, w, x);
             tmem_ld_wait();
             {
                 const float keep = eR * eR, c = (wide ? 1.f : eR) * P.scale * bwd_inverse(fq);
 #pragma unroll
                 for (int e = 0; e < 8; ++e) {
-                    const float2 z = bwd_fma2(bwd_two(keep), bwd_pair(dS, e), bwd_mul2(bwd_two(c), bwd_pair(x, e)));
+                    const float2 z = fma2(two(keep), pair_of(dS, e), mul2(two(c), pair_of(x, e)));
                     dS[2 * e] = z.x; dS[2 * e + 1] = z.y;
                 }
             }
-            const int tok = bwd_token(P, (first + i) * kChunk + (rev ? 63 - static_cast<int>(row) : static_cast<int>(row)));
+            const int tok = scan_token(P, P.T, (first + i) * kChunk + (rev ? 63 - static_cast<int>(row) : static_cast<int>(row)));
             const bool live = tok >= 0 && c0 < K;
             if (c0 == 0) st_shared_u32(tok_at + 4u * row, static_cast<uint32_t>(tok));
             const long long at = (static_cast<long long>(b) * P.T + max(tok, 0)) * P.H + h;          // in units of one head's row
             const float iS = bwd_inverse(fS), idS = bwd_inverse(fdS), ifd = bwd_inverse(fd), ifq = bwd_inverse(fq), ifk = bwd_inverse(fk);
-            bwd_wait(P.ctrl, smem_u32(&M.bar_o), ph);
+            wait_bar(P, M.bar_o, ph);
             tc_fence_after();
             // ---- outputs, eight columns at a time
             const int slot_dv = wide ? BWD_P : BWD_DP, slot_dk = wide ? BWD_DP : BWD_P;
@@ -883,24 +752,24 @@ __global__ void __launch_bounds__(kBwdChunkThreads, 2) gla_bwd_chunk_kernel(cons
                 // one of dk, dq: gate factor 2^(sign X) (2^(sign X + R) for the state part alone in a wide chunk) times the sum
                 // of state part and chunk part
                 auto finish = [&](int slot_s, int slot_i, float cs, float ci, float sign, const uint32_t* in, __half* out) {
-                    bwd_read8(tmem, slot_s, w, 8 * hf, a);
-                    bwd_read8(tmem, slot_i, w, 8 * hf, y);
-                    if (sign < 0.f) bwd_read8(tmem, BWD_X, w, 8 * hf, g);
+                    acc_read8(tmem, slot_s, w, 8 * hf, a);
+                    acc_read8(tmem, slot_i, w, 8 * hf, y);
+                    if (sign < 0.f) acc_read8(tmem, BWD_X, w, 8 * hf, g);
                     tmem_ld_wait();
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
                         float2 z;
                         if (!wide) {
-                            z = bwd_fma2(bwd_two(cs), bwd_pair(a, e), bwd_mul2(bwd_two(ci), bwd_pair(y, e)));
-                            z = bwd_mul2(z, bwd_ex2(bwd_mul2(bwd_pair(g, e), bwd_two(sign * kLog2e))));
+                            z = fma2(two(cs), pair_of(a, e), mul2(two(ci), pair_of(y, e)));
+                            z = mul2(z, ex2_2(mul2(pair_of(g, e), two(sign * kLog2e))));
                         } else {
                             const float2 r = make_float2(M.vec[c0 + 8 * hf + 2 * e], M.vec[c0 + 8 * hf + 2 * e + 1]);
-                            z = bwd_mul2(bwd_pair(a, e), bwd_two(cs));
-                            z = bwd_fma2(z, bwd_ex2(bwd_fma2(bwd_pair(g, e), bwd_two(sign * kLog2e), r)), bwd_pair(y, e));
+                            z = mul2(pair_of(a, e), two(cs));
+                            z = fma2(z, ex2_2(fma2(pair_of(g, e), two(sign * kLog2e), r)), pair_of(y, e));
                         }
                         o[e] = pack_half2(z.x, z.y);
                         const float2 f = unpack_half2(sign > 0.f ? in[4 * hf + e] : in[4 * hf + e] ^ 0x80008000u);
-                        z = sign > 0.f ? bwd_fma2(f, z, bwd_pair(D, e)) : bwd_mul2(f, z);
+                        z = sign > 0.f ? fma2(f, z, pair_of(D, e)) : mul2(f, z);
                         D[2 * e] = z.x; D[2 * e + 1] = z.y;
                     }
                     if (live) *reinterpret_cast<uint4*>(out + at * K + c0 + 8 * hf) = make_uint4(o[0], o[1], o[2], o[3]);
@@ -909,19 +778,19 @@ __global__ void __launch_bounds__(kBwdChunkThreads, 2) gla_bwd_chunk_kernel(cons
                 finish(BWD_DQ_S, BWD_DQ_I, P.scale * iS, P.scale * ifd * ifk, 1.f, qr, P.dq);
                 st_shared_f4(bwd_f32(r0, row, c0 + 8 * hf), D[0], D[1], D[2], D[3]);
                 st_shared_f4(bwd_f32(r0, row, c0 + 8 * hf + 4), D[4], D[5], D[6], D[7]);
-                bwd_read8(tmem, BWD_DV_S, w, 8 * hf, a);
-                bwd_read8(tmem, slot_dv, w, 8 * hf, y);
+                acc_read8(tmem, BWD_DV_S, w, 8 * hf, a);
+                acc_read8(tmem, slot_dv, w, 8 * hf, y);
                 tmem_ld_wait();
-                const float2 cs = bwd_two(ifk * idS), ci = bwd_two(P.scale * ifq * ifk * 8.f);      // 8 = 1 / fp
+                const float2 cs = two(ifk * idS), ci = two(P.scale * ifq * ifk * 8.f);      // 8 = 1 / fp
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    const float2 z = bwd_fma2(cs, bwd_pair(a, e), bwd_mul2(ci, bwd_pair(y, e)));
+                    const float2 z = fma2(cs, pair_of(a, e), mul2(ci, pair_of(y, e)));
                     o[e] = pack_half2(z.x, z.y);
                 }
                 if (tok >= 0) *reinterpret_cast<uint4*>(P.dv + at * 64 + c0 + 8 * hf) = make_uint4(o[0], o[1], o[2], o[3]);
             }
             tc_fence_before();
-            if (i > 0) bwd_bar_arrive(BWD_BAR_READ, kBwdChunkThreads);
+            if (i > 0) named_bar_arrive(BWD_BAR_READ, kBwdChunkThreads);
             sync();
             // ---- dg: sums of the terms of the tokens at and after each token, a quarter of the rows per thread and channel,
             // handed back to the rows' owners through the tiles of the low parts

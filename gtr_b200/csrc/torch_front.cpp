@@ -32,6 +32,7 @@ decltype(&gla_b200_backward_workspace_bytes) g_backward_workspace_bytes = nullpt
 decltype(&gla_b200_strerror) g_strerror = nullptr;
 decltype(&gla_b200_forward_packed) g_forward_packed = nullptr;
 decltype(&gla_b200_packed_workspace_bytes) g_packed_workspace_bytes = nullptr;
+decltype(&gla_b200_forward_block) g_forward_block = nullptr;
 
 // The tensor inside a Python object, or null when it is not a plain torch.Tensor / Parameter.
 const at::Tensor* tensor(PyObject* o) {
@@ -100,10 +101,11 @@ bool operands(gla_b200_args& a, const at::Tensor& q, const at::Tensor& k, const 
 }
 
 // run(q, k, v, gk, o, ws, scale, gk_normalizer, direction, grid_hw, initial_state, final_state, out_gate, rms_w, eps,
-//     segments, wait_limit) -> 0, a library error, or kSlow.  The operator on caller-owned output and workspace.
+//     segments, wait_limit, block) -> 0, a library error, or kSlow.  The operator on caller-owned output and workspace;
+// block: on the kernel of the backbone's blocks.
 PyObject* run(PyObject*, PyObject* const* v, Py_ssize_t n) {
     HANDLE_TH_ERRORS
-    if (n != 17) return PyLong_FromLong(kSlow);
+    if (n != 18) return PyLong_FromLong(kSlow);
     const at::Tensor* t[6];
     for (int i = 0; i < 6; ++i)
         if (!(t[i] = tensor(v[i]))) return PyLong_FromLong(kSlow);
@@ -142,7 +144,7 @@ PyObject* run(PyObject*, PyObject* const* v, Py_ssize_t n) {
     a.gk_normalizer = static_cast<float>(norm);
     a.wait_limit = static_cast<uint32_t>(limit);
     const c10::cuda::CUDAGuard guard(q.device());
-    return PyLong_FromLong(g_forward(&a, c10::cuda::getCurrentCUDAStream(q.device().index()).stream()));
+    return PyLong_FromLong((v[17] == Py_True ? g_forward_block : g_forward)(&a, c10::cuda::getCurrentCUDAStream(q.device().index()).stream()));
     END_HANDLE_TH_ERRORS
 }
 
@@ -355,11 +357,11 @@ PyObject* packed(PyObject*, PyObject* const* v, Py_ssize_t n) {
 }
 
 // bind(addresses of gla_b200_forward, _workspace_bytes, _backward_scan, _backward_workspace_bytes, _strerror, _forward_packed,
-//      _packed_workspace_bytes)
+//      _packed_workspace_bytes, _forward_block)
 PyObject* bind(PyObject*, PyObject* const* v, Py_ssize_t n) {
-    if (n != 7) { PyErr_SetString(PyExc_TypeError, "bind takes 7 addresses"); return nullptr; }
-    void* p[7];
-    for (int i = 0; i < 7; ++i)
+    if (n != 8) { PyErr_SetString(PyExc_TypeError, "bind takes 8 addresses"); return nullptr; }
+    void* p[8];
+    for (int i = 0; i < 8; ++i)
         if (!(p[i] = PyLong_AsVoidPtr(v[i]))) {
             if (!PyErr_Occurred()) PyErr_SetString(PyExc_ValueError, "null address");
             return nullptr;
@@ -371,6 +373,7 @@ PyObject* bind(PyObject*, PyObject* const* v, Py_ssize_t n) {
     g_strerror = reinterpret_cast<decltype(g_strerror)>(p[4]);
     g_forward_packed = reinterpret_cast<decltype(g_forward_packed)>(p[5]);
     g_packed_workspace_bytes = reinterpret_cast<decltype(g_packed_workspace_bytes)>(p[6]);
+    g_forward_block = reinterpret_cast<decltype(g_forward_block)>(p[7]);
     Py_RETURN_NONE;
 }
 

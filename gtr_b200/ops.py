@@ -83,7 +83,7 @@ def make_workspace(B: int, T: int, H: int, device) -> torch.Tensor:
 
 
 def _forward(q, k, v, gk, o, ws, scale, gk_normalizer, direction, grid_hw, initial_state, final_state,
-             out_gate=None, rms_w=None, eps=0.0, segments=0, wait_limit=0) -> None:
+             out_gate=None, rms_w=None, eps=0.0, segments=0, wait_limit=0, block=False) -> None:
     K = q.shape[-1] if isinstance(q, torch.Tensor) and q.dim() == 4 else kK
     if K not in SUPPORTED_K:
         raise RuntimeError(f"q: last dim must be one of {SUPPORTED_K}, got {K}")
@@ -126,14 +126,15 @@ def _forward(q, k, v, gk, o, ws, scale, gk_normalizer, direction, grid_hw, initi
     a.wait_limit = int(wait_limit)
     with torch.cuda.device(q.device):
         stream = torch.cuda.current_stream(q.device).cuda_stream
-        _lib.check(_lib.lib().gla_b200_forward(ctypes.byref(a), ctypes.c_void_p(stream)))
+        entry = _lib.lib().gla_b200_forward_block if block else _lib.lib().gla_b200_forward
+        _lib.check(entry(ctypes.byref(a), ctypes.c_void_p(stream)))
 
 
 def chunk_gla_run(q, k, v, gk, scale, ws, o, gk_normalizer: float = 0.0, *, direction=0, grid_hw=None,
                   initial_state=None, final_state=None, segments: int = 0, wait_limit: int = 0) -> None:
     """o <- GLA(q, k, v, gk) on the current stream.  Reference: ext.chunk_gla_run (gla_torch_ext.cu:40-90)."""
     rc = _front().run(q, k, v, gk, o, ws, scale, gk_normalizer, direction, grid_hw, initial_state, final_state, None, None,
-                      0.0, segments, wait_limit)
+                      0.0, segments, wait_limit, False)
     if rc == _SLOW:
         _forward(q, k, v, gk, o, ws, scale, gk_normalizer, direction, grid_hw, initial_state, final_state,
                  segments=segments, wait_limit=wait_limit)
@@ -144,13 +145,24 @@ def chunk_gla_run(q, k, v, gk, scale, ws, o, gk_normalizer: float = 0.0, *, dire
 def chunk_gla_run_gated(q, k, v, gk, g, rms_w, scale, eps, ws, y, gk_normalizer: float = 0.0, *, direction=0,
                         grid_hw=None, initial_state=None, final_state=None, segments: int = 0) -> None:
     """y <- RMSNorm(GLA(q,k,v,gk)) * rms_w * silu(g).  Reference: ext.chunk_gla_run_gated (gla_torch_ext.cu:92-154)."""
+    _run_gated(q, k, v, gk, g, rms_w, scale, eps, ws, y, gk_normalizer, direction, grid_hw, initial_state, final_state, segments, False)
+
+
+def _run_gated(q, k, v, gk, g, rms_w, scale, eps, ws, y, gk_normalizer, direction, grid_hw, initial_state, final_state, segments,
+               block) -> None:
     rc = _front().run(q, k, v, gk, y, ws, scale, gk_normalizer, direction, grid_hw, initial_state, final_state, g, rms_w,
-                      eps, segments, 0)
+                      eps, segments, 0, block)
     if rc == _SLOW:
         _forward(q, k, v, gk, y, ws, scale, gk_normalizer, direction, grid_hw, initial_state, final_state,
-                 out_gate=g, rms_w=rms_w, eps=eps, segments=segments)
+                 out_gate=g, rms_w=rms_w, eps=eps, segments=segments, block=block)
     elif rc:
         _lib.check(rc)
+
+
+def block_gla_gated(q, k, v, gk, g, rms_w, scale, eps, ws, y, gk_normalizer: float = 0.0, *, direction=0, grid_hw=None) -> None:
+    """`chunk_gla_run_gated` on the kernel the backbone's blocks run on (gla_b200_forward_block): the same operator to the same
+    accuracy, with the roundings a backbone's results are known with."""
+    _run_gated(q, k, v, gk, g, rms_w, scale, eps, ws, y, gk_normalizer, direction, grid_hw, None, None, 0, True)
 
 
 def chunk_gla_with_ws(q, k, v, gk, scale, ws, **kw) -> torch.Tensor:

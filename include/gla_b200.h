@@ -90,6 +90,10 @@ typedef struct gla_b200_args {
  * the calling thread has run the same shape once.  Returns 0 or a gla_b200_error. */
 int gla_b200_forward(const gla_b200_args* args, void* stream);
 
+/* The fused operator (out_gate and rms_weight given) on the kernel that the backbone's blocks run on.  Same arguments and
+ * accuracy; its roundings are the ones a backbone's results are known with, see gla_block.cuh. */
+int gla_b200_forward_block(const gla_b200_args* args, void* stream);
+
 /* Same operator, but with nothing allocated and no workspace from the caller (`workspace` and
  * `workspace_bytes` of `args` are ignored): the scratch is a fixed array of
  * GLA_B200_STATIC_SCRATCH_BYTES inside the library, one per GPU, held until the process exits.

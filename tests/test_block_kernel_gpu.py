@@ -1,0 +1,38 @@
+"""The kernel of the backbone's blocks (gla_b200_forward_block) in each of its work decompositions, against the CPU oracle."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("B,H,grid,direction,K,logits", [
+    (1, 3, (40, 40), 1, 32, True),       # few sequences: equal segments with pre-passes
+    (2, 12, (40, 50), 2, 64, True),      # the staggered plan
+    (13, 12, (20, 33), 3, 64, False),    # more sequences than CTAs: relayed segments
+    (1, 1, (1, 1), 0, 64, True),         # one token
+    (1, 2, (5, 13), 1, 32, False),       # a full chunk and a ragged one of one token
+])
+def test_block_kernel(B, H, grid, direction, K, logits):
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    import gtr_b200 as G
+    from gtr_b200 import ops
+    from oracle import c_oracle, gla_ref
+    T = grid[0] * grid[1]
+    q, k, v, g = gla_ref.make_inputs(B, T, H, K=K, seed=T)
+    gen = torch.Generator().manual_seed(1)
+    norm, log_gates = 0.0, g
+    if logits:
+        norm, g = 16.0, torch.randn(B, T, H, K, generator=gen).half()
+        log_gates = gla_ref.gate_from_logits(g.float(), norm).half()
+    gate = torch.randn(B, T, H, 64, generator=gen).half()
+    w = (torch.rand(64, generator=gen) + 0.5).half()
+    o, _ = c_oracle.forward(q, k, v, log_gates, direction=direction, grid_hw=grid)
+    want = gla_ref.rmsnorm_swish_gate(o, gate, w, 1e-5)
+    ws = G.make_workspace(B, T, H, "cuda")
+    y = torch.full((B, T, H, 64), float("nan"), dtype=torch.float16, device="cuda")
+    ops.block_gla_gated(q.cuda(), k.cuda(), v.cuda(), g.cuda(), gate.cuda(), w.cuda(), K ** -0.5, 1e-5, ws, y, norm,
+                        direction=direction, grid_hw=grid)
+    G.check_status(ws)
+    m = gla_ref.error_metrics(want, y.float().cpu())
+    assert m["finite"] and m["rel_l2"] <= 1.5e-3, m      # as for the operator's other fused calls with logits
