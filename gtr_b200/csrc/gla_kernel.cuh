@@ -667,10 +667,18 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
         // ---- outputs
         wait_bar(P, M.bar_o, p);
         tc_fence_after();
-        if (w == 0 && more && elect_one()) {                        // nothing reads the chunk's tiles any more
-            M.sq[p ^ 1u] = last ? sequence_of(table, P, chunk + 1) : M.sq[p];
-            load(chunk + 1, M.sq[p ^ 1u], smem_u32(&M.full));
+        if (more && elect_one()) {                                  // nothing reads the chunk's tiles any more: each warp asks for one
+            const Sequence next = last ? sequence_of(table, P, chunk + 1) : M.sq[p];
+            if (w == 0) {
+                M.sq[p ^ 1u] = next;
+                mbar_arrive_expect_tx(smem_u32(&M.full), 4 * kTileBytes);
+            }
+            const int tensors[1] = {w == 0 ? TG : w == 1 ? TK : w == 2 ? TQ : TV};
+            const uint32_t tiles[1] = {w == 0 ? tg : w == 1 ? tk : w == 2 ? tq : tv};
+            load_chunk(maps, Scan{next.T, P.Hc, P.rev}, chunk + 1 - next.chunk0, next.b, next.h, next.tok0, P.Hc, smem_u32(&M.full), tensors, tiles,
+                       l2_policy_stream());
         }
+        __syncwarp();
         half_row_read(tmem, ACC_P, w, x);
         tmem_ld_wait();
         float mul = P.o_mul;
