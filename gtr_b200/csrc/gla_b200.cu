@@ -8,6 +8,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 #include <utility>
 #include <vector>
 
@@ -382,6 +383,29 @@ int get_maps(const MapKey& key, gla::Maps* out) {
     return GLA_B200_OK;
 }
 
+// A kernel whose blocks may start while its predecessor in the stream drains; it waits (gla::pdl_wait) before it touches memory
+// that anything before it in the stream reads or writes.
+int launch_overlapped(const void* kernel, dim3 ctas, unsigned threads, size_t smem, void** args, cudaStream_t stream) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = ctas;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelExC(&cfg, kernel, args);
+    if (e != cudaSuccess) { note_cuda("cudaLaunchKernelExC", e); return GLA_B200_ERR_CUDA; }
+    return GLA_B200_OK;
+}
+template <class... A>
+int launch_simple(void (*kernel)(A...), dim3 ctas, unsigned threads, size_t smem, cudaStream_t stream, typename std::common_type<A>::type... a) {
+    void* args[] = {const_cast<void*>(static_cast<const void*>(&a))...};
+    return launch_overlapped(reinterpret_cast<const void*>(kernel), ctas, threads, smem, args, stream);
+}
+
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 int resolve_strides(const int64_t in[3], int T, int H, int D, int64_t out[3]) {
@@ -409,6 +433,7 @@ __global__ void __launch_bounds__(256) rmsnorm_gated_kernel(const __half* x, con
     const int64_t row = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 3;
     const int sub = threadIdx.x & 7;
     const bool live = row < rows;
+    gla::pdl_wait();
     float xv[8], gv[8], wv[8];
     uint4 xr = make_uint4(0, 0, 0, 0), gr = xr;
     const uint4 wr = __ldg(reinterpret_cast<const uint4*>(wgt) + sub);
@@ -542,23 +567,6 @@ void fill_params(const gla_b200_args* a, const int64_t* o_stride, uint8_t* ws, c
     P->wait_limit_us = a->wait_limit ? a->wait_limit : 2000000u;
 }
 
-// A kernel whose blocks may start while its predecessor in the stream drains; it waits (gla::pdl_wait) before it touches memory
-// that anything before it in the stream reads or writes.
-int launch_overlapped(const void* kernel, unsigned ctas, unsigned threads, size_t smem, void** args, cudaStream_t stream) {
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(ctas);
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelExC(&cfg, kernel, args);
-    if (e != cudaSuccess) { note_cuda("cudaLaunchKernelExC", e); return GLA_B200_ERR_CUDA; }
-    return GLA_B200_OK;
-}
 
 constexpr int64_t kL2Keep = 120ll << 20;
 // The spans' increments (where spans end inside sequences), then the outputs.
@@ -776,11 +784,7 @@ static int forward(const gla_b200_args* a, bool block, void* stream_v) {
         S.scale = a->scale;
         S.inv_norm = a->gk_normalizer > 0.f ? 1.f / a->gk_normalizer : 0.f;
         cudaStream_t st = static_cast<cudaStream_t>(stream_v);
-        if (a->K == 64) gla::gla_step_kernel<64><<<nseq, gla::kStepThreads, 0, st>>>(S);
-        else gla::gla_step_kernel<32><<<nseq, gla::kStepThreads, 0, st>>>(S);
-        ce = cudaPeekAtLastError();
-        if (ce != cudaSuccess) { note_cuda("step kernel launch", ce); return GLA_B200_ERR_CUDA; }
-        return GLA_B200_OK;
+        return launch_simple(a->K == 64 ? &gla::gla_step_kernel<64> : &gla::gla_step_kernel<32>, nseq, gla::kStepThreads, 0, st, S);
     }
 
     key.ptr[gla::TO] = nullptr;                       // outputs are stored from registers
@@ -1075,16 +1079,12 @@ int gla_b200_backward_scan(const gla_b200_bwd_args* a, const gla_b200_bwd_scan* 
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
     const unsigned ctas = static_cast<unsigned>(nseq * P.nseg);
     const dim3 states(ctas, P.nseg > 1 ? 2 : 1);
-    if (a->K == 64) {
-        gla::gla_bwd_state_kernel<64><<<states, gla::kComputeThreads, gla::BwdStateSmem::kBytes, stream>>>(maps, P);
-        gla::gla_bwd_chunk_kernel<64><<<ctas, gla::kBwdChunkThreads, gla::BwdChunkSmem::kBytes, stream>>>(maps, P);
-    } else {
-        gla::gla_bwd_state_kernel<32><<<states, gla::kComputeThreads, gla::BwdStateSmem::kBytes, stream>>>(maps, P);
-        gla::gla_bwd_chunk_kernel<32><<<ctas, gla::kBwdChunkThreads, gla::BwdChunkSmem::kBytes, stream>>>(maps, P);
-    }
-    e = cudaPeekAtLastError();
-    if (e != cudaSuccess) { note_cuda("backward launch", e); return GLA_B200_ERR_CUDA; }
-    return GLA_B200_OK;
+    const bool wide = a->K == 64;
+    if (int rc = launch_simple(wide ? &gla::gla_bwd_state_kernel<64> : &gla::gla_bwd_state_kernel<32>, states, gla::kComputeThreads,
+                               gla::BwdStateSmem::kBytes, stream, maps, P))
+        return rc;
+    return launch_simple(wide ? &gla::gla_bwd_chunk_kernel<64> : &gla::gla_bwd_chunk_kernel<32>, ctas, gla::kBwdChunkThreads,
+                         gla::BwdChunkSmem::kBytes, stream, maps, P);
 }
 
 int gla_b200_rmsnorm_gated(const void* x, const void* g, const void* w, void* y, int64_t rows, int32_t D, float eps,
@@ -1096,12 +1096,9 @@ int gla_b200_rmsnorm_gated(const void* x, const void* g, const void* w, void* y,
     const int64_t threads = rows * 8;
     const int64_t blocks = (threads + 255) / 256;
     if (blocks > 0x7fffffffLL) return GLA_B200_ERR_SHAPE;
-    rmsnorm_gated_kernel<<<static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __half*>(x), static_cast<const __half*>(g), static_cast<const __half*>(w),
-        static_cast<__half*>(y), rows, eps);
-    cudaError_t e = cudaPeekAtLastError();
-    if (e != cudaSuccess) { note_cuda("rmsnorm launch", e); return GLA_B200_ERR_CUDA; }
-    return GLA_B200_OK;
+    return launch_simple(&rmsnorm_gated_kernel, static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream),
+                         static_cast<const __half*>(x), static_cast<const __half*>(g), static_cast<const __half*>(w),
+                         static_cast<__half*>(y), rows, eps);
 }
 
 int gla_b200_swiglu_dwconv(const void* gate, const void* y, const void* weight, const void* bias, void* out,
@@ -1117,14 +1114,11 @@ int gla_b200_swiglu_dwconv(const void* gate, const void* y, const void* weight, 
                               ((grid_w + gla::kDwTileC - 1) / gla::kDwTileC);
         const int64_t blocks = static_cast<int64_t>(B) * tiles * (((C >> 3) + gla::kDwSlab - 1) / gla::kDwSlab);
         if (blocks > 0x7fffffffLL) return GLA_B200_ERR_SHAPE;
-        gla::swiglu_dwconv_kernel<<<static_cast<unsigned>(blocks), gla::kDwTileThreads, gla::kDwTileSmem,
-                                          static_cast<cudaStream_t>(stream)>>>(
-            static_cast<const __half*>(gate), static_cast<const __half*>(y), static_cast<const __half*>(weight),
-            static_cast<const __half*>(bias), static_cast<__half*>(out), B, grid_h, grid_w, C);
+        return launch_simple(&gla::swiglu_dwconv_kernel, static_cast<unsigned>(blocks), gla::kDwTileThreads, gla::kDwTileSmem,
+                             static_cast<cudaStream_t>(stream), static_cast<const __half*>(gate), static_cast<const __half*>(y),
+                             static_cast<const __half*>(weight), static_cast<const __half*>(bias), static_cast<__half*>(out), B, grid_h,
+                             grid_w, C);
     }
-    cudaError_t e = cudaPeekAtLastError();
-    if (e != cudaSuccess) { note_cuda("swiglu_dwconv launch", e); return GLA_B200_ERR_CUDA; }
-    return GLA_B200_OK;
 }
 
 int gla_b200_layernorm(const void* x, const void* weight, const void* bias, void* y, int64_t rows, int32_t D, float eps,
@@ -1136,19 +1130,13 @@ int gla_b200_layernorm(const void* x, const void* weight, const void* bias, void
     const int64_t blocks = (rows + 7) / 8;               // eight warps, one row each
     if (blocks > 0x7fffffffLL) return GLA_B200_ERR_SHAPE;
     const int per_lane = ((D >> 3) + 31) / 32;            // 16-byte vectors per lane
-#define GLA_LN_LAUNCH(V)                                                                                              \
-    gla::layernorm_rows_kernel<V><<<static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(      \
-        static_cast<const __half*>(x), static_cast<const __half*>(weight), static_cast<const __half*>(bias),          \
-        static_cast<__half*>(y), rows, D, eps)
-    if (per_lane <= 1) GLA_LN_LAUNCH(1);
-    else if (per_lane <= 2) GLA_LN_LAUNCH(2);
-    else if (per_lane <= 3) GLA_LN_LAUNCH(3);
-    else if (per_lane <= 4) GLA_LN_LAUNCH(4);
-    else GLA_LN_LAUNCH(gla::kLnMaxVec);
-#undef GLA_LN_LAUNCH
-    cudaError_t e = cudaPeekAtLastError();
-    if (e != cudaSuccess) { note_cuda("layernorm launch", e); return GLA_B200_ERR_CUDA; }
-    return GLA_B200_OK;
+    void (*const kernel)(const __half*, const __half*, const __half*, __half*, long long, int, float) =
+        per_lane <= 1 ? &gla::layernorm_rows_kernel<1> : per_lane <= 2 ? &gla::layernorm_rows_kernel<2>
+        : per_lane <= 3 ? &gla::layernorm_rows_kernel<3> : per_lane <= 4 ? &gla::layernorm_rows_kernel<4>
+                                                         : &gla::layernorm_rows_kernel<gla::kLnMaxVec>;
+    return launch_simple(kernel, static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream), static_cast<const __half*>(x),
+                         static_cast<const __half*>(weight), static_cast<const __half*>(bias), static_cast<__half*>(y),
+                         static_cast<long long>(rows), D, eps);
 }
 
 int32_t gla_b200_trt_enqueue(const void* const* inputs, int32_t n_inputs, void* const* outputs, const int64_t* q_dims,

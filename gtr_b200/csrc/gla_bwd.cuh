@@ -138,8 +138,10 @@ __global__ void __launch_bounds__(kComputeThreads, 3) gla_bwd_state_kernel(const
     const bool back = blockIdx.y != 0;
     const int bh = blockIdx.x / P.nseg, seg = blockIdx.x - bh * P.nseg;
     const int first = seg * P.cps, n = min(P.cps, P.NT - first);
-    if (back && seg == 0) return;                                  // nothing before it needs its gradient
-    if (blockIdx.x == 0 && tid < 2) P.ctrl[tid] = 0u;
+    if (back && seg == 0) {                                        // nothing before it needs its gradient
+        pdl_wait();
+        return;
+    }
 
     const int b = bh / P.H, h = bh - b * P.H;
     const bool rev = P.rev != 0;
@@ -161,6 +163,8 @@ __global__ void __launch_bounds__(kComputeThreads, 3) gla_bwd_state_kernel(const
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    pdl_wait();
+    if (blockIdx.x == 0 && tid < 2) P.ctrl[tid] = 0u;
     const uint32_t tmem = M.tmem;
     auto chunk_of = [&](int i) { return first + (back ? n - 1 - i : i); };
     auto load = [&](int i) {
@@ -450,6 +454,7 @@ __global__ void __launch_bounds__(kBwdChunkThreads, 2) gla_bwd_chunk_kernel(cons
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    pdl_wait();
     const uint32_t tmem = M.tmem;
 
     if (w == kComputeThreads / 32) {

@@ -39,6 +39,8 @@ __global__ void __launch_bounds__(kStepThreads) gla_step_kernel(const __grid_con
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
     const int b = blockIdx.x / P.H, h = blockIdx.x - b * P.H;
     const int row0 = l >> 1, col = 8 * w + 4 * (l & 1);
+    pdl_release();
+    pdl_wait();
     if (blockIdx.x == 0 && threadIdx.x < 4) P.ctrl[threadIdx.x] = 0u;
 
     const size_t soff = static_cast<size_t>(blockIdx.x) * K * 64 + static_cast<size_t>(row0) * 64 + col;

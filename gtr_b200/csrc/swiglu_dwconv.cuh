@@ -12,6 +12,8 @@
 #include <cuda_fp16.h>
 #include <cstdint>
 
+#include "gla_device.cuh"
+
 namespace gla {
 
 __device__ __forceinline__ void dw_unpack8(const uint4& v, float* x) {
@@ -83,6 +85,7 @@ __global__ void __launch_bounds__(kDwTileThreads, DW_MINB) swiglu_dwconv_kernel(
     const uint4* y4 = reinterpret_cast<const uint4*>(y);
     const long long img = static_cast<long long>(b) * hg * wg;
 
+    pdl_wait();
     // ---- the gate vectors this thread will need (one tile row, 16 columns) are asked into L2 first: they are read
     // straight from global memory during the compute phase, two columns ahead of their use, which covers an L2 hit
     // but not a DRAM access under load.  One request per 128-byte line.
@@ -200,6 +203,7 @@ __global__ void __launch_bounds__(256) layernorm_rows_kernel(const __half* x, co
     const long long row = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (row >= rows) return;
+    pdl_wait();
     const int nvec = D >> 3;
     const uint4* x4 = reinterpret_cast<const uint4*>(x) + row * nvec;
     float v[kVec][8];
