@@ -256,7 +256,7 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_state_kernel(const __grid_
     }
     pdl_wait();
     if (blockIdx.x == 0 && tid < 2) P.ctrl[tid] = 0u;
-    if (n == 0) return;
+    if (n == 0) { pdl_release(); return; }
     if (tid == 0) {                                                  // the first tiles come in while the rest is set up
         load_kg(0);
         load_v(0);
@@ -279,6 +279,7 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_state_kernel(const __grid_
 
     for (int i = 0; i < n; ++i) {
         const int st = i & 1;
+        if (i == n - 1) pdl_release();                              // the output kernel's blocks move in as these leave
         const uint32_t tk = base + StateSmem::kK + st * kTileBytes, tg = base + StateSmem::kG + st * kTileBytes;
         wait_bar(P, M.full[st], (i >> 1) & 1);
         if (kLogits) {
