@@ -117,12 +117,13 @@ int device_info(int dev, DeviceInfo* out) {
                 return GLA_B200_ERR_DEVICE;
             }
         }
-        const std::pair<const void*, int> bwd[] = {
+        const std::pair<const void*, int> others[] = {
+            {reinterpret_cast<const void*>(&gla::swiglu_dwconv_kernel), gla::kDwSmem},
             {reinterpret_cast<const void*>(&gla::gla_bwd_state_kernel<64>), gla::BwdStateSmem::kBytes},
             {reinterpret_cast<const void*>(&gla::gla_bwd_state_kernel<32>), gla::BwdStateSmem::kBytes},
             {reinterpret_cast<const void*>(&gla::gla_bwd_chunk_kernel<64>), gla::BwdChunkSmem::kBytes},
             {reinterpret_cast<const void*>(&gla::gla_bwd_chunk_kernel<32>), gla::BwdChunkSmem::kBytes}};
-        for (const auto& k : bwd)
+        for (const auto& k : others)
             if (e == cudaSuccess) e = cudaFuncSetAttribute(k.first, cudaFuncAttributeMaxDynamicSharedMemorySize, k.second);
         if (e != cudaSuccess) { note_cuda("cudaFuncSetAttribute", e); return GLA_B200_ERR_CUDA; }
         d.ok = true;
@@ -278,7 +279,7 @@ int auto_chunks_per_segment(int NT, int nseq, int slots, size_t workspace_bytes)
 // the fused epilogue (which costs the output pass only).  In units of one chunk's output pass every CTA then works
 // (1 + pre) x the middle segments' length.  Returns that cost (plus one for the look-back), or a negative number when
 // the plan does not apply.
-constexpr double kPlanPrePassPlain = 0.68, kPlanPrePassGated = 0.48;
+constexpr double kPlanPrePassGated = 0.48;
 double staggered_plan(int NT, int nseq, int slots, size_t workspace_bytes, double pre, int* seg_start, int* ns_out) {
     const int r = nseq > 0 ? slots / nseq : 0;
     if (r < 2 || r + 1 > gla::block::kMaxPlanSegments || NT < kMinAutoCps * (r + 1)) return -1.0;
@@ -650,6 +651,25 @@ int forward_block(const gla_b200_args* a, const MapKey& key, int sms, cudaStream
     void* args[2] = {&maps, &P};
     return launch_overlapped(block_kernel((P.inv_norm > 0.f ? 2 : 0) | (P.rev ? 1 : 0)), std::min(P.num_items, slots), gla::block::kThreads,
                              gla::block::kSmemBytes, args, stream);
+}
+
+// An fp16 tensor of `rank` dimensions, channels innermost, and the box of 64 channels x wide x high that a stage of the SwiGLU
+// kernel takes of it; what lies outside the tensor reads as zero.
+int dw_map(const void* ptr, int rank, const cuuint64_t* dim, int wide, int high, CUtensorMap* out) {
+    EncodeTiledFn enc = encode_tiled();
+    if (!enc) {
+        snprintf(g_cuda_err, sizeof(g_cuda_err), "cuTensorMapEncodeTiled is not available from this driver");
+        return GLA_B200_ERR_DEVICE;
+    }
+    cuuint64_t str[3] = {dim[0] * 2, 0, 0};
+    for (int i = 1; i < rank - 1; ++i) str[i] = str[i - 1] * dim[i];
+    const cuuint32_t box[4] = {static_cast<cuuint32_t>(gla::kDwSlab), static_cast<cuuint32_t>(wide), static_cast<cuuint32_t>(high), 1};
+    const cuuint32_t one[4] = {1, 1, 1, 1};
+    CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, static_cast<cuuint32_t>(rank), const_cast<void*>(ptr), dim, str, box, one,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) { note_cu("cuTensorMapEncodeTiled", static_cast<int>(r)); return GLA_B200_ERR_CUDA; }
+    return GLA_B200_OK;
 }
 }  // namespace
 
@@ -1109,16 +1129,33 @@ int gla_b200_swiglu_dwconv(const void* gate, const void* y, const void* weight, 
     if (!aligned16(gate) || !aligned16(y) || !aligned16(weight) || !aligned16(out) || (bias && !aligned16(bias)))
         return GLA_B200_ERR_ALIGN;
     if (out == gate || out == y) return GLA_B200_ERR_ARG;      // neighbours are read after their own output is written
-    {
-        const int64_t tiles = static_cast<int64_t>((grid_h + gla::kDwTileR - 1) / gla::kDwTileR) *
-                              ((grid_w + gla::kDwTileC - 1) / gla::kDwTileC);
-        const int64_t blocks = static_cast<int64_t>(B) * tiles * (((C >> 3) + gla::kDwSlab - 1) / gla::kDwSlab);
-        if (blocks > 0x7fffffffLL) return GLA_B200_ERR_SHAPE;
-        return launch_simple(&gla::swiglu_dwconv_kernel, static_cast<unsigned>(blocks), gla::kDwTileThreads, gla::kDwTileSmem,
-                             static_cast<cudaStream_t>(stream), static_cast<const __half*>(gate), static_cast<const __half*>(y),
-                             static_cast<const __half*>(weight), static_cast<const __half*>(bias), static_cast<__half*>(out), B, grid_h,
-                             grid_w, C);
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) { note_cuda("cudaGetDevice", e); return GLA_B200_ERR_CUDA; }
+    if (dev < 0 || dev >= 64) return GLA_B200_ERR_DEVICE;
+    DeviceInfo di;
+    if (int rc = device_info(dev, &di)) return rc;
+    // The tile that covers the grid with the fewest: a stage's turn costs almost the same however much of its tile lies
+    // inside (33 x 100 cells take 21 tiles of 16 x 16 but 15 of 12 x 20).  Of equals, the one that reads the least halo.
+    int rows = 0, strips = 0;
+    int64_t tiles = 0, cells = 0;
+    for (int n = 1; n <= gla::kDwStrips; ++n) {
+        const int cols = n * gla::kDwRun, r = std::min(gla::kDwStrips / n, gla::kDwCells / (cols + 2) - 2);
+        if (r < 1) break;
+        const int64_t t = static_cast<int64_t>((grid_h + r - 1) / r) * ((grid_w + cols - 1) / cols), c = t * (r + 2) * (cols + 2);
+        if (!rows || t < tiles || (t == tiles && c < cells)) { rows = r; strips = n; tiles = t; cells = c; }
     }
+    const int64_t items = B * tiles * ((C + gla::kDwSlab - 1) / gla::kDwSlab);
+    if (items > 0x7fffffffLL) return GLA_B200_ERR_SHAPE;
+    gla::DwMaps maps;
+    const cuuint64_t grid[4] = {static_cast<cuuint64_t>(C), static_cast<cuuint64_t>(grid_w), static_cast<cuuint64_t>(grid_h), static_cast<cuuint64_t>(B)};
+    const cuuint64_t taps[2] = {static_cast<cuuint64_t>(C), 9}, one[2] = {static_cast<cuuint64_t>(C), 1};
+    if (int rc = dw_map(y, 4, grid, strips * gla::kDwRun + 2, rows + 2, &maps.y)) return rc;
+    if (int rc = dw_map(gate, 4, grid, strips * gla::kDwRun, rows, &maps.gate)) return rc;
+    if (int rc = dw_map(weight, 2, taps, 9, 1, &maps.weight)) return rc;
+    if (int rc = dw_map(bias ? bias : weight, 2, one, 1, 1, &maps.bias)) return rc;
+    return launch_simple(&gla::swiglu_dwconv_kernel, static_cast<unsigned>(items), gla::kDwThreads, gla::kDwSmem,
+                         static_cast<cudaStream_t>(stream), maps, static_cast<__half*>(out), bias != nullptr, rows, strips, grid_h, grid_w, C);
 }
 
 int gla_b200_layernorm(const void* x, const void* weight, const void* bias, void* y, int64_t rows, int32_t D, float eps,

@@ -4,9 +4,7 @@
 // form of the reference's SpatialSwiGLU (engine/gtr/backbone/vit_adapter_spatial_swiglu.py:50-60), the chain
 // view/permute -> cuDNN depthwise 3x3 conv -> permute/reshape -> silu -> multiply and the layout copies around it.
 //
-// HBM-bound: gate and y are read once, out is written once (3 * 2 bytes per element).  What limits a direct form
-// (every thread loading its 3x3 window from global memory: 3.4 loads of y per output, two thirds of them L2 hits)
-// is the L2 -> SM path, which moved about 4 TB/s whatever the instruction mix; hence the shared-memory tile below.
+// HBM-bound: gate and y are read once, out is written once (3 * 2 bytes per element).
 #pragma once
 
 #include <cuda_fp16.h>
@@ -26,161 +24,186 @@ __device__ __forceinline__ void dw_unpack8(const uint4& v, float* x) {
     }
 }
 
-// acc[0..7] += w[0..7] * y[0..7] with the fp16 operands taken as they are: fma.rn.f32.f16 multiplies two fp16 values
+// to[0..7] = w[0..7] * y[0..7] + from[0..7] with the fp16 operands taken as they are: fma.rn.f32.f16 multiplies two fp16 values
 // and accumulates in fp32 in one instruction (exact product, one rounding), so the taps cost no conversions.
-__device__ __forceinline__ void dw_fma2(float& a0, float& a1, uint32_t w, uint32_t y) {
+__device__ __forceinline__ void dw_fma2(float* to, uint32_t w, uint32_t y, const float* from) {
     asm("{\n\t.reg .b16 wl, wh, yl, yh;\n\t"
         "mov.b32 {wl, wh}, %2;\n\tmov.b32 {yl, yh}, %3;\n\t"
-        "fma.rn.f32.f16 %0, wl, yl, %0;\n\tfma.rn.f32.f16 %1, wh, yh, %1;\n\t}"
-        : "+f"(a0), "+f"(a1)
-        : "r"(w), "r"(y));
+        "fma.rn.f32.f16 %0, wl, yl, %4;\n\tfma.rn.f32.f16 %1, wh, yh, %5;\n\t}"
+        : "=f"(to[0]), "=f"(to[1])
+        : "r"(w), "r"(y), "f"(from[0]), "f"(from[1]));
 }
-__device__ __forceinline__ void dw_fma8(float* acc, const uint4& wv, const uint4& yv) {
-    dw_fma2(acc[0], acc[1], wv.x, yv.x);
-    dw_fma2(acc[2], acc[3], wv.y, yv.y);
-    dw_fma2(acc[4], acc[5], wv.z, yv.z);
-    dw_fma2(acc[6], acc[7], wv.w, yv.w);
-}
-
-// gate, y, out: [B, hg, wg, C] fp16 contiguous; wt: [3][3][C] fp16 (tap-major); bias: [C] fp16 or null.
-// A CTA brings the y tile of kDwTileR x kDwTileC outputs plus its one-cell halo, for a slab of kDwSlab channel groups
-// (8 channels each), into shared memory with cp.async -- every y element crosses the L2 -> SM path 1.4 times -- and
-// each thread (one tile row, one channel group) then slides its 3x3 window of 16-byte vectors along the row out of
-// shared memory.  The whole tile is in flight at once (45 KB per CTA, four CTAs per SM); consecutive threads hold
-// consecutive channel groups, so every global access of a half-warp is 256 contiguous bytes.
-#ifndef DW_TR
-#define DW_TR 8
-#endif
-#ifndef DW_MINB
-#define DW_MINB 4
-#endif
-#ifndef DW_TC
-#define DW_TC 16
-#endif
-constexpr int kDwTileR = DW_TR, kDwTileC = DW_TC, kDwSlab = 16;
-constexpr int kDwTileThreads = kDwTileR * kDwSlab;                                   // 128
-constexpr int kDwTilePos = (kDwTileR + 2) * (kDwTileC + 2);                          // 180 positions
-constexpr int kDwTileSmem = kDwTilePos * kDwSlab * 16;                               // 46,080 bytes
-
-__device__ __forceinline__ void dw_cp_async16(uint32_t dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+__device__ __forceinline__ void dw_fma8(float* to, const uint4& wv, const uint4& yv, const float* from) {
+    dw_fma2(to, wv.x, yv.x, from);
+    dw_fma2(to + 2, wv.y, yv.y, from + 2);
+    dw_fma2(to + 4, wv.z, yv.z, from + 4);
+    dw_fma2(to + 6, wv.w, yv.w, from + 6);
 }
 
-__global__ void __launch_bounds__(kDwTileThreads, DW_MINB) swiglu_dwconv_kernel(
-    const __half* __restrict__ gate, const __half* __restrict__ y, const __half* __restrict__ wt,
-    const __half* __restrict__ bias, __half* __restrict__ out, int B, int hg, int wg, int C) {
-    extern __shared__ __align__(16) unsigned char dw_smem[];
-    const int CG = C >> 3;
-    const int nslab = (CG + kDwSlab - 1) / kDwSlab;
-    const int tiles_c = (wg + kDwTileC - 1) / kDwTileC, tiles_r = (hg + kDwTileR - 1) / kDwTileR;
-    // block -> (b, tile row, tile column, slab), slab fastest: neighbouring CTAs read neighbouring bytes
-    long long rest = blockIdx.x;
-    const int slab = static_cast<int>(rest % nslab); rest /= nslab;
-    const int tc = static_cast<int>(rest % tiles_c); rest /= tiles_c;
-    const int tr = static_cast<int>(rest % tiles_r);
-    const int b = static_cast<int>(rest / tiles_r);
-    const int r0 = tr * kDwTileR, c0 = tc * kDwTileC, cg0 = slab * kDwSlab;
+// A CTA per SM with a ring of three stages.  A stage holds, for a slab of 64 channels, a y tile of up to 256 outputs (16 x 16 where
+// the grid is a multiple of that) plus its one-cell halo, the gate tile, and the slab's weights and bias, filled by four
+// TMA copies (cells outside the grid and channels past C read as zero), so that 150 KB per SM are in flight while 16
+// warps work on a stage.  Neighbouring blocks are neighbouring slabs of a tile, so that what is in flight at one time is
+// whole cells.  Memory does not serve all SMs equally: a CTA that is done with its block takes over one that has not been
+// launched (a cluster launch control request, in flight with the copies); with equal ranges SMs were idle for an eighth of
+// the time.  A thread owns 8 channels and a strip of 4 outputs, its 3 x 3 window sliding along the strip out of shared
+// memory; 8 threads cover the 128 bytes a cell has in a slab.  At 8 x 64 x 128 cells of 3072 channels 202 us, 6.0 TB/s
+// (blocks that each loaded a tile and then worked on it: 254 us; this ring with equal ranges: 256 us).
+constexpr int kDwSlab = 64, kDwStages = 3, kDwRun = 4;
+constexpr int kDwStrips = 64, kDwCells = 18 * 18;                                    // at most, of a tile and with its halo
+constexpr int kDwYBytes = kDwCells * kDwSlab * 2, kDwGateBytes = kDwStrips * kDwRun * kDwSlab * 2;
+constexpr int kDwWeights = kDwYBytes + kDwGateBytes, kDwBias = kDwWeights + 9 * kDwSlab * 2;
+constexpr int kDwStageBytes = kDwBias + kDwSlab * 2;                                 // 75,520: a multiple of 128
+constexpr int kDwThreads = kDwStrips * (kDwSlab / 8);                                // 512: 128 registers each
+constexpr int kDwSmem = kDwStages * kDwStageBytes + 128 + 128;                       // control words, alignment
+
+struct DwMaps { CUtensorMap y, gate, weight, bias; };
+
+__device__ __forceinline__ void dw_load4(uint32_t dst, const CUtensorMap* m, uint32_t bar, int c0, int c1, int c2, int c3,
+                                         uint64_t policy) {
+    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], "
+                 "[%1, {%3, %4, %5, %6}], [%2], %7;"
+                 ::"r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "l"(policy) : "memory");
+}
+__device__ __forceinline__ void dw_load2(uint32_t dst, const CUtensorMap* m, uint32_t bar, int c0) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+                 ::"r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(c0), "r"(0) : "memory");
+}
+// Asks for a block of the grid that has not been launched; the 16-byte answer arrives on `bar`.
+__device__ __forceinline__ void dw_ask(uint32_t answer, uint32_t bar) {
+    fence_proxy_async_smem();            // the answer before it has been read
+    mbar_arrive_expect_tx(bar, 16);
+    asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];"
+                 ::"r"(answer), "r"(bar) : "memory");
+}
+__device__ __forceinline__ int dw_answer(uint32_t answer) {       // the block, or -1: none is left
+    uint32_t got, x;
+    asm volatile("{\n\t.reg .pred p;\n\t.reg .b128 h;\n\tld.shared.b128 h, [%2];\n\t"
+                 "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\tselp.u32 %0, 1, 0, p;\n\tmov.u32 %1, 0;\n\t"
+                 "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, h;\n\t}"
+                 : "=r"(got), "=r"(x) : "r"(answer) : "memory");
+    return got ? static_cast<int>(x) : -1;
+}
+// Waits here are for copies and for warps of the same CTA; the limit only bounds what a fault elsewhere could make of them.
+__device__ __forceinline__ bool dw_wait(uint32_t bar, uint32_t parity) {
+    for (int n = 0; n < (1 << 22); ++n)
+        if (mbar_try_wait(bar, parity)) return true;
+    return false;
+}
+
+__global__ void __launch_bounds__(kDwThreads, 1) swiglu_dwconv_kernel(const __grid_constant__ DwMaps maps, __half* __restrict__ out,
+                                                                      bool biased, int rows, int strips, int hg, int wg, int C) {
+    extern __shared__ uint8_t dw_smem[];
+    const uint32_t base = (smem_u32(dw_smem) + 127u) & ~127u, control = base + kDwStages * kDwStageBytes;
     const int tid = threadIdx.x;
-    const uint32_t sbase = static_cast<uint32_t>(__cvta_generic_to_shared(dw_smem));
-    const uint4* y4 = reinterpret_cast<const uint4*>(y);
-    const long long img = static_cast<long long>(b) * hg * wg;
-
-    pdl_wait();
-    // ---- the gate vectors this thread will need (one tile row, 16 columns) are asked into L2 first: they are read
-    // straight from global memory during the compute phase, two columns ahead of their use, which covers an L2 hit
-    // but not a DRAM access under load.  One request per 128-byte line.
-    {
-        const int pci = tid % kDwSlab, prow = r0 + tid / kDwSlab, pcg = cg0 + pci;
-        if ((pci & 7) == 0 && prow < hg && pcg < CG) {
-            const uint4* gp = reinterpret_cast<const uint4*>(gate) + (img + static_cast<long long>(prow) * wg + c0) * CG + pcg;
-            const int n = min(kDwTileC, wg - c0);
-            for (int j = 0; j < n; ++j)
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(gp + static_cast<long long>(j) * CG) : "memory");
+    const int cols = strips * kDwRun, tiles_c = (wg + cols - 1) / cols, tiles_r = (hg + rows - 1) / rows;
+    const int slabs = (C + kDwSlab - 1) / kDwSlab;
+    // control words: the answer, a stage's item (-1: none is left), barriers
+    auto item_of = [&](int s) { return control + 16u + 4u * s; };
+    auto full = [&](int s) { return control + 32u + 8u * s; };
+    auto empty = [&](int s) { return control + 32u + 8u * (kDwStages + s); };
+    const uint32_t answered = control + 32u + 16u * kDwStages;
+    if (tid == 0) {
+        for (int s = 0; s < kDwStages; ++s) {
+            mbar_init(full(s), 1);
+            mbar_init(empty(s), kDwThreads / 32);
         }
+        mbar_init(answered, 1);
+        fence_mbar_init();
     }
-
-    // ---- fill: position (pr, pc) of the halo tile is grid cell (r0 - 1 + pr, c0 - 1 + pc); zeros outside the grid
-    for (int idx = tid; idx < kDwTilePos * kDwSlab; idx += kDwTileThreads) {
-        const int pos = idx / kDwSlab, ci = idx - pos * kDwSlab;
-        const int pr = pos / (kDwTileC + 2), pc = pos - pr * (kDwTileC + 2);
-        const int r = r0 - 1 + pr, c = c0 - 1 + pc, cg = cg0 + ci;
-        const uint32_t dst = sbase + static_cast<uint32_t>(idx) * 16u;
-        if (r >= 0 && r < hg && c >= 0 && c < wg && cg < CG)
-            dw_cp_async16(dst, y4 + (img + static_cast<long long>(r) * wg + c) * CG + cg);
-        else
-            asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(dst), "r"(0u) : "memory");
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-
-    // ---- this thread: tile row trow, channel group cg; weights and bias while the tile is in flight
-    const int ci = tid % kDwSlab, trow = tid / kDwSlab;
-    const int cg = cg0 + ci, r = r0 + trow;
-    const bool active = cg < CG && r < hg;
-    const int cgc = cg < CG ? cg : CG - 1;
-    uint4 wv[9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) wv[k] = __ldg(reinterpret_cast<const uint4*>(wt) + static_cast<long long>(k) * CG + cgc);
-    float bv[8];
-    if (bias != nullptr) dw_unpack8(__ldg(reinterpret_cast<const uint4*>(bias) + cgc), bv);
-    else {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) bv[i] = 0.f;
-    }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
-    if (!active) return;
-
-    auto ld = [&](int pr, int pc) {
-        uint4 v;
-        const uint32_t a = sbase + static_cast<uint32_t>((pr * (kDwTileC + 2) + pc) * kDwSlab + ci) * 16u;
-        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
-        return v;
+    pdl_wait();
+    const uint32_t bytes = ((rows + 2) * (cols + 2) + rows * cols + 9 + (biased ? 1 : 0)) * kDwSlab * 2u;
+    // thread 0 fills the stages in turn, two items ahead of the work, and asks for the item after each
+    int to_fill = 0;
+    uint32_t fill_turn = 0, asked = 0;
+    bool more = true;
+    auto fill = [&](int item) {
+        const int s = to_fill;
+        dw_wait(empty(s), (fill_turn & 1u) ^ 1u);
+        asm volatile("st.shared.b32 [%0], %1;" ::"r"(item_of(s)), "r"(item) : "memory");
+        if (item < 0) {
+            more = false;
+            mbar_arrive(full(s));
+            return;
+        }
+        const int slab = item % slabs, tile = item / slabs;
+        const int tc = tile % tiles_c, rest = tile / tiles_c, tr = rest % tiles_r, b = rest / tiles_r;
+        const uint32_t to = base + s * kDwStageBytes;
+        mbar_arrive_expect_tx(full(s), bytes);
+        dw_load4(to, &maps.y, full(s), slab * kDwSlab, tc * cols - 1, tr * rows - 1, b, l2_policy_normal());
+        dw_load4(to + kDwYBytes, &maps.gate, full(s), slab * kDwSlab, tc * cols, tr * rows, b, l2_policy_stream());
+        dw_load2(to + kDwWeights, &maps.weight, full(s), slab * kDwSlab);
+        if (biased) dw_load2(to + kDwBias, &maps.bias, full(s), slab * kDwSlab);
+        if (++to_fill == kDwStages) { to_fill = 0; ++fill_turn; }
+        dw_ask(control, answered);
     };
-    const long long base = (img + static_cast<long long>(r) * wg) * CG + cg;
-    const uint4* g4 = reinterpret_cast<const uint4*>(gate);
-    uint4* o4 = reinterpret_cast<uint4*>(out);
-    const int ncol = min(kDwTileC, wg - c0);
-    // the 3x3 window slides along the row: three columns of three 16-byte vectors in registers; the column loop is
-    // unrolled so that the columns change roles by renaming, not by moves
-    uint4 win[3][3];                     // win[column slot][row]
+    auto fill_next = [&] {
+        if (!more) return;
+        const int item = dw_wait(answered, asked & 1u) ? dw_answer(control) : -1;
+        ++asked;
+        fill(item);
+    };
+    if (tid == 0) {
+        fill(static_cast<int>(blockIdx.x));
+        fill_next();
+    }
+    const int ci = tid & 7, trow = (tid >> 3) / strips, tcol = (tid >> 3) % strips * kDwRun;
+    const uint32_t line = (cols + 2) * 128u, y_at = trow * line + tcol * 128u + 16u * ci;
+    const uint32_t gate_at = kDwYBytes + (trow * cols + tcol) * 128u + 16u * ci;
+    const int CG = C >> 3;
+    uint32_t turn = 0;
+    for (int s = 0;;) {
+        if (tid == 0) fill_next();
+        __syncwarp();
+        if (!dw_wait(full(s), turn & 1u)) return;
+        int item;
+        asm volatile("ld.shared.b32 %0, [%1];" : "=r"(item) : "r"(item_of(s)) : "memory");
+        if (item < 0) return;
+        const int slab = item % slabs, tile = item / slabs, cg = slab * (kDwSlab / 8) + ci;
+        const int tc = tile % tiles_c, rest = tile / tiles_c, tr = rest % tiles_r, b = rest / tiles_r;
+        const int r = tr * rows + trow, c = tc * cols + tcol;
+        const uint32_t stage = base + s * kDwStageBytes;
+        if (trow < rows && r < hg && c < wg && cg < CG) {
+            uint4 wv[9];
 #pragma unroll
-    for (int rr = 0; rr < 3; ++rr) { win[0][rr] = ld(trow + rr, 0); win[1][rr] = ld(trow + rr, 1); }
-    // the gate vectors come straight from global memory (L2 after the prefetch above), two columns ahead of their use
-    const long long pcol = base + static_cast<long long>(c0) * CG;
-    uint4 gq[3];
-    gq[0] = __ldg(g4 + pcol);
-    gq[1] = ncol > 1 ? __ldg(g4 + pcol + CG) : gq[0];
-#pragma unroll
-    for (int j = 0; j < kDwTileC; ++j) {
-        if (j < ncol) {
-            const int sl = j % 3, sm = (j + 1) % 3, sn = (j + 2) % 3;     // left, middle, new column slots
-#pragma unroll
-            for (int rr = 0; rr < 3; ++rr) win[sn][rr] = ld(trow + rr, j + 2);
-            const long long p = pcol + static_cast<long long>(j) * CG;
-            if (j + 2 < ncol) gq[(j + 2) % 3] = __ldg(g4 + p + 2 * static_cast<long long>(CG));
-            float acc[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) acc[i] = bv[i];
+            for (int k = 0; k < 9; ++k) wv[k] = ld_shared_v4(stage + kDwWeights + 128u * k + 16u * ci);
+            float bv[8] = {};
+            if (biased) dw_unpack8(ld_shared_v4(stage + kDwBias + 16u * ci), bv);
+            uint4 win[3][3];                 // win[column slot][row]; the columns change roles by renaming
 #pragma unroll
             for (int rr = 0; rr < 3; ++rr) {
-                dw_fma8(acc, wv[3 * rr + 0], win[sl][rr]);
-                dw_fma8(acc, wv[3 * rr + 1], win[sm][rr]);
-                dw_fma8(acc, wv[3 * rr + 2], win[sn][rr]);
+                win[0][rr] = ld_shared_v4(stage + y_at + rr * line);
+                win[1][rr] = ld_shared_v4(stage + y_at + rr * line + 128u);
             }
-            float g[8];
-            dw_unpack8(gq[j % 3], g);
-            uint4 o;
-            __half2* oh = reinterpret_cast<__half2*>(&o);
+            uint4* to = reinterpret_cast<uint4*>(out) + ((static_cast<long long>(b) * hg + r) * wg + c) * CG + cg;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float h0 = 0.5f * g[2 * i], h1 = 0.5f * g[2 * i + 1];      // silu(x) = h + h * tanh(h), h = x / 2
-                float t0, t1;
-                asm("tanh.approx.f32 %0, %1;" : "=f"(t0) : "f"(h0));
-                asm("tanh.approx.f32 %0, %1;" : "=f"(t1) : "f"(h1));
-                oh[i] = __floats2half2_rn(fmaf(h0, t0, h0) * acc[2 * i], fmaf(h1, t1, h1) * acc[2 * i + 1]);
+            for (int j = 0; j < kDwRun; ++j) {
+                const int sl = j % 3, sm = (j + 1) % 3, sn = (j + 2) % 3;     // left, middle, new column slots
+#pragma unroll
+                for (int rr = 0; rr < 3; ++rr) win[sn][rr] = ld_shared_v4(stage + y_at + rr * line + (j + 2) * 128u);
+                float g[8], acc[8];
+                dw_unpack8(ld_shared_v4(stage + gate_at + 128u * j), g);
+#pragma unroll
+                for (int rr = 0; rr < 3; ++rr) {
+                    dw_fma8(acc, wv[3 * rr + 0], win[sl][rr], rr == 0 ? bv : acc);
+                    dw_fma8(acc, wv[3 * rr + 1], win[sm][rr], acc);
+                    dw_fma8(acc, wv[3 * rr + 2], win[sn][rr], acc);
+                }
+                uint4 o;
+                __half2* oh = reinterpret_cast<__half2*>(&o);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float2 h = mul2(two(0.5f), pair_of(g, e));       // silu(x) = h + h * tanh(h), h = x / 2
+                    const float2 z = mul2(fma2(h, tanh_2(h), h), pair_of(acc, e));
+                    oh[e] = __floats2half2_rn(z.x, z.y);
+                }
+                if (c + j < wg) __stcs(to + static_cast<long long>(j) * CG, o);
             }
-            o4[p] = o;
         }
+        __syncwarp();
+        if ((tid & 31) == 0) mbar_arrive(empty(s));
+        if (++s == kDwStages) { s = 0; ++turn; }
     }
 }
 
