@@ -1098,9 +1098,8 @@ int gla_b200_backward_scan(const gla_b200_bwd_args* a, const gla_b200_bwd_scan* 
     P.scale = a->scale;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
     const unsigned ctas = static_cast<unsigned>(nseq * P.nseg);
-    const dim3 states(ctas, P.nseg > 1 ? 2 : 1);
     const bool wide = a->K == 64;
-    if (int rc = launch_simple(wide ? &gla::gla_bwd_state_kernel<64> : &gla::gla_bwd_state_kernel<32>, states, gla::kComputeThreads,
+    if (int rc = launch_simple(wide ? &gla::gla_bwd_state_kernel<64> : &gla::gla_bwd_state_kernel<32>, ctas, gla::kComputeThreads,
                                gla::BwdStateSmem::kBytes, stream, maps, P))
         return rc;
     return launch_simple(wide ? &gla::gla_bwd_chunk_kernel<64> : &gla::gla_bwd_chunk_kernel<32>, ctas, gla::kBwdChunkThreads,

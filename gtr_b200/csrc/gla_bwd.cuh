@@ -111,38 +111,37 @@ __device__ __forceinline__ float bwd_log2(float f) { return static_cast<float>(s
 __device__ __forceinline__ float bwd_inverse(float f) { return __uint_as_float((254u << 23) - __float_as_uint(f)); }   // of a power of two
 
 // ------------------------------------------------------------------------------------------ segments' states
-// blockIdx.y 0: S after every chunk of a segment, from zero at its start:     S' = 2^G_L S + (k 2^(G_L-G))^T v
-// blockIdx.y 1: dS at a segment's start, from zero at its end (walked backwards): dS' = 2^G_L dS + scale (q 2^G)^T do
-// Bound by latency (a chunk is two dependent MMA round trips and two block barriers with little between them), then by memory:
-// hence three CTAs per SM (66 KB each) and the next chunk's tiles in flight meanwhile.  3.9 TB/s at B4 H12 T6400.
+//   S after every chunk of a segment, from zero at its start:   S' = 2^G_L S + (k 2^(G_L-G))^T v
+//   dS at a segment's start, from zero at its end, as a sum over the chunks in the same order, D their decay so far:
+//                                                               dS' = dS + 2^D scale (q 2^G)^T do
+// Both in one walk, so that the gates are read once, the two products share a chunk's round trips, and the blocks are as many as
+// the gradient's, two to an SM in one wave (walks of their own, three to an SM, left the SMs idle for a third of the
+// time).  Bound by memory, then by latency: a chunk is two dependent MMA round trips and two block barriers, the next chunk's
+// tiles in flight meanwhile.
 struct BwdStateSmem {
-    static constexpr int kStage = 3 * kTileBytes;                                      // a (k or q), b (v or do), g
-    static constexpr int kLow = 2 * kStage, kMat = kLow + kTileBytes, kMisc = kMat + kTileBytes;
+    static constexpr int kStage = 5 * kTileBytes;                                      // k, v, g, q, do
+    static constexpr int kLowQ = 2 * kStage, kAfter = kLowQ + kTileBytes, kUpTo = kAfter + kTileBytes, kMisc = kUpTo + kTileBytes;
     static constexpr int kBytes = kMisc + 1024 + 1024;                                 // misc, alignment
 };
 struct BwdStateMisc {
     uint64_t full[2], bar_x, bar_inc;
     uint32_t tmem;
-    uint32_t top[8];                  // per warp: largest |a|, as half2 bits
-    alignas(16) float gl[64];         // log2 decay of the chunk per channel
+    uint32_t top[2][8];               // per warp: largest |k|, |q|, as half2 bits
+    alignas(16) float gl[2][64];      // log2 decay of the chunk per channel
 };
 static_assert(sizeof(BwdStateMisc) <= 1024, "misc block too large");
+enum { BWD_AFTER = 0, BWD_UP_TO = 1, BWD_INC_S = 2, BWD_INC_DS = 3 };
 
 template <int K>
-__global__ void __launch_bounds__(kComputeThreads, 3) gla_bwd_state_kernel(const __grid_constant__ Maps maps, const __grid_constant__ BwdParams P) {
+__global__ void __launch_bounds__(kComputeThreads, 2) gla_bwd_state_kernel(const __grid_constant__ Maps maps, const __grid_constant__ BwdParams P) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw), base = (raw + 1023u) & ~1023u;
     uint8_t* base_ptr = smem_raw + (base - raw);
     BwdStateMisc& M = *reinterpret_cast<BwdStateMisc*>(base_ptr + BwdStateSmem::kMisc);
     const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
-    const bool back = blockIdx.y != 0;
     const int bh = blockIdx.x / P.nseg, seg = blockIdx.x - bh * P.nseg;
     const int first = seg * P.cps, n = min(P.cps, P.NT - first);
-    if (back && seg == 0) {                                        // nothing before it needs its gradient
-        pdl_wait();
-        return;
-    }
-
+    const bool grad = seg > 0;                                     // nothing before the first segment needs its gradient
     const int b = bh / P.H, h = bh - b * P.H;
     const bool rev = P.rev != 0;
 
@@ -154,11 +153,13 @@ __global__ void __launch_bounds__(kComputeThreads, 3) gla_bwd_state_kernel(const
         fence_mbar_init();
     }
     if (w == 0) {
-        tmem_alloc(smem_u32(&M.tmem), 64);
+        tmem_alloc(smem_u32(&M.tmem), 128);
         tmem_relinquish();
     }
-    // log factor of a row: the gates after it (forward), its own and those before it (backward), along the scan
-    fill_constant(base + BwdStateSmem::kMat, [&](uint32_t r, uint32_t s) { return (back ? (rev ? s >= r : s <= r) : (rev ? s < r : s > r)) ? 1.f : 0.f; });
+    // log factor of a row: the gates after it (k), its own and those before it (q), along the scan
+    const uint32_t after = base + BwdStateSmem::kAfter, up_to = base + BwdStateSmem::kUpTo, low_q = base + BwdStateSmem::kLowQ;
+    fill_constant(after, [&](uint32_t r, uint32_t s) { return (rev ? s < r : s > r) ? 1.f : 0.f; });
+    fill_constant(up_to, [&](uint32_t r, uint32_t s) { return (rev ? s >= r : s <= r) ? 1.f : 0.f; });
     fence_proxy_async_smem();
     tc_fence_before();
     __syncthreads();
@@ -166,99 +167,128 @@ __global__ void __launch_bounds__(kComputeThreads, 3) gla_bwd_state_kernel(const
     pdl_wait();
     if (blockIdx.x == 0 && tid < 2) P.ctrl[tid] = 0u;
     const uint32_t tmem = M.tmem;
-    auto chunk_of = [&](int i) { return first + (back ? n - 1 - i : i); };
     auto load = [&](int i) {
         const uint32_t s = base + (i & 1) * BwdStateSmem::kStage, bar = smem_u32(&M.full[i & 1]);
-        const int tensors[3] = {TG, back ? TQ : TK, back ? TO : TV};
-        const uint32_t tiles[3] = {s + 2 * kTileBytes, s, s + kTileBytes};
-        mbar_arrive_expect_tx(bar, 3 * kTileBytes);
-        load_chunk(maps, Scan{P.T, P.Hc, P.rev}, chunk_of(i), b, h, 0, P.Hc, bar, tensors, tiles, l2_policy_normal());
+        const Scan order{P.T, P.Hc, P.rev};
+        const int tensors[3] = {TG, TK, TV}, others[2] = {TQ, TO};
+        const uint32_t tiles[3] = {s + 2 * kTileBytes, s, s + kTileBytes}, other_tiles[2] = {s + 3 * kTileBytes, s + 4 * kTileBytes};
+        mbar_arrive_expect_tx(bar, (grad ? 5 : 3) * kTileBytes);
+        load_chunk(maps, order, first + i, b, h, 0, P.Hc, bar, tensors, tiles, l2_policy_normal());
+        if (grad) load_chunk(maps, order, first + i, b, h, 0, P.Hc, bar, others, other_tiles, l2_policy_normal());
     };
-    if (w == 0 && elect_one()) load(0);
+    auto gate_sums = [&](int i) {          // of chunk i, as soon as it has landed
+        const uint32_t tg = base + (i & 1) * BwdStateSmem::kStage + 2 * kTileBytes;
+        wait_bar(P, M.full[i & 1], (i >> 1) & 1);
+        tc_fence_after();
+        tile_mma<0, 1>(acc_slot(tmem, BWD_AFTER), after, tg, false);
+        if (grad) tile_mma<0, 1>(acc_slot(tmem, BWD_UP_TO), up_to, tg, false);
+        umma_commit(smem_u32(&M.bar_x));
+    };
+    if (w == 0 && elect_one()) {
+        load(0);
+        if (n > 1) load(1);
+        gate_sums(0);
+    }
+    __syncwarp();
 
     const uint32_t row = 16u * (w & 3) + (l & 15u), c0 = 32u * (w >> 2) + 16u * (static_cast<uint32_t>(l) >> 4), u0 = c0 >> 3;
-    float S[16], total = 0.f;          // a state row piece: channel `row`, columns c0 .. +15
+    float S[16], dS[16], total = 0.f;          // a state row piece each: channel `row`, columns c0 .. +15
 #pragma unroll
-    for (int e = 0; e < 16; ++e) S[e] = 0.f;
+    for (int e = 0; e < 16; ++e) S[e] = dS[e] = 0.f;
     const size_t cslot = static_cast<size_t>(bh) * P.NT;
-    const uint32_t low = base + BwdStateSmem::kLow, mat = base + BwdStateSmem::kMat;
 
     for (int i = 0; i < n; ++i) {
         const int st = i & 1;
-        const uint32_t ta = base + st * BwdStateSmem::kStage, tb = ta + kTileBytes, tg = tb + kTileBytes;
+        const uint32_t tk = base + st * BwdStateSmem::kStage, tv = tk + kTileBytes, tg = tv + kTileBytes, tq = tg + kTileBytes,
+                       tdo = tq + kTileBytes;
+        if (i == n - 1) pdl_release();
         wait_bar(P, M.full[st], (i >> 1) & 1);
-        if (w == 0 && elect_one()) {
-            tc_fence_after();
-            tile_mma<0, 1>(acc_slot(tmem, 0), mat, tg, false);
-            umma_commit(smem_u32(&M.bar_x));
-            if (i + 1 < n) load(i + 1);
+        uint32_t k[8], q[8];
+        row16(tk, row, u0, k);
+        const uint32_t mk = __reduce_max_sync(0xffffffffu, __float_as_uint(bwd_half_max(bwd_max16(k))));
+        uint32_t mq = 0u;
+        if (grad) {
+            row16(tq, row, u0, q);
+            mq = __reduce_max_sync(0xffffffffu, __float_as_uint(bwd_half_max(bwd_max16(q))));
         }
-        uint32_t a[8];
-        row16(ta, row, u0, a);
-        {
-            const uint32_t m = __reduce_max_sync(0xffffffffu, __float_as_uint(bwd_half_max(bwd_max16(a))));
-            if (l == 0) M.top[w] = m;
-        }
+        if (l == 0) { M.top[0][w] = mk; M.top[1][w] = mq; }
         wait_bar(P, M.bar_x, i & 1);
         tc_fence_after();
-        float x[16];
-        acc_read(tmem, 0, w, x);
+        float x[16], y[16];
+        acc_read(tmem, BWD_AFTER, w, x);
+        if (grad) acc_read(tmem, BWD_UP_TO, w, y);
         tmem_ld_wait();
-        __syncthreads();                                            // every warp's maximum is there
-        uint32_t m = M.top[0];
-#pragma unroll
-        for (int j = 1; j < 8; ++j) m = max(m, M.top[j]);
-        const float f = bwd_scale(__uint_as_float(m), 15);
-        if (row == ((back != rev) ? 63u : 0u)) {                             // x + own gate (forward), x (backward) = G_L
+        if (row == (rev ? 63u : 0u)) {                              // all later gates + its own = the chunk's decay
             uint32_t gr[8];
             row16(tg, row, u0, gr);
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
                 const float2 gf = unpack_half2(gr[e]);
-                M.gl[c0 + 2 * e] = (x[2 * e] + (back ? 0.f : gf.x)) * kLog2e;
-                M.gl[c0 + 2 * e + 1] = (x[2 * e + 1] + (back ? 0.f : gf.y)) * kLog2e;
+                M.gl[st][c0 + 2 * e] = (x[2 * e] + gf.x) * kLog2e;
+                M.gl[st][c0 + 2 * e + 1] = (x[2 * e + 1] + gf.y) * kLog2e;
             }
         }
-        bwd_put_gated(ta, low, row, u0, a, x, kLog2e, bwd_log2(f));
+        __syncthreads();                                            // every warp's maxima are there
+        uint32_t top_k = M.top[0][0], top_q = M.top[1][0];
+#pragma unroll
+        for (int j = 1; j < 8; ++j) { top_k = max(top_k, M.top[0][j]); top_q = max(top_q, M.top[1][j]); }
+        const float fk = bwd_scale(__uint_as_float(top_k), 15), fq = bwd_scale(__uint_as_float(top_q), 15);
+        bwd_put_gated(tk, tg, row, u0, k, x, kLog2e, bwd_log2(fk));            // the gates have been read: the low part's tile
+        if (grad) bwd_put_gated(tq, low_q, row, u0, q, y, kLog2e, bwd_log2(fq));
         fence_proxy_async_smem();
         tc_fence_before();
         __syncthreads();
         if (w == 0 && elect_one()) {
             tc_fence_after();
-            tile_mma<1, 1>(acc_slot(tmem, 1), ta, tb, false);
-            tile_mma<1, 1>(acc_slot(tmem, 1), low, tb, true);
+            tile_mma<1, 1>(acc_slot(tmem, BWD_INC_S), tk, tv, false);
+            tile_mma<1, 1>(acc_slot(tmem, BWD_INC_S), tg, tv, true);
+            if (grad) {
+                tile_mma<1, 1>(acc_slot(tmem, BWD_INC_DS), tq, tdo, false);
+                tile_mma<1, 1>(acc_slot(tmem, BWD_INC_DS), low_q, tdo, true);
+            }
             umma_commit(smem_u32(&M.bar_inc));
         }
-        const float gl = M.gl[row], decay = ex2(gl), c = (back ? P.scale : 1.f) * bwd_inverse(f);
+        const float gl = M.gl[st][row], decay = ex2(gl), ck = bwd_inverse(fk), cq = P.scale * bwd_inverse(fq) * ex2(total);
         total += gl;
         wait_bar(P, M.bar_inc, i & 1);
         tc_fence_after();
-        acc_read(tmem, 1, w, x);
+        if (w == 0 && elect_one()) {                                // this chunk's stage is free, and so are its gate sums
+            if (i + 2 < n) load(i + 2);
+            if (i + 1 < n) gate_sums(i + 1);
+        }
+        __syncwarp();
+        acc_read(tmem, BWD_INC_S, w, x);
+        if (grad) acc_read(tmem, BWD_INC_DS, w, y);
         tmem_ld_wait();
         tc_fence_before();
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-            const float2 s = fma2(two(decay), pair_of(S, e), mul2(two(c), pair_of(x, e)));
+            const float2 s = fma2(two(decay), pair_of(S, e), mul2(two(ck), pair_of(x, e)));
             S[2 * e] = s.x; S[2 * e + 1] = s.y;
         }
-        if (!back) {
-            const size_t at = cslot + chunk_of(i);
-            float4* dst = reinterpret_cast<float4*>(P.chunk_state + at * 4096) + tid;
+        const size_t at = cslot + first + i;
+        float4* dst = reinterpret_cast<float4*>(P.chunk_state + at * 4096) + tid;
 #pragma unroll
-            for (int e = 0; e < 4; ++e) dst[e * kComputeThreads] = make_float4(S[4 * e], S[4 * e + 1], S[4 * e + 2], S[4 * e + 3]);
-            if (c0 == 0) P.chunk_decay[at * 64 + row] = total;
+        for (int e = 0; e < 4; ++e) dst[e * kComputeThreads] = make_float4(S[4 * e], S[4 * e + 1], S[4 * e + 2], S[4 * e + 3]);
+        if (c0 == 0) P.chunk_decay[at * 64 + row] = total;
+        if (grad) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const float2 s = fma2(two(cq), pair_of(y, e), pair_of(dS, e));
+                dS[2 * e] = s.x; dS[2 * e + 1] = s.y;
+            }
         }
     }
-    if (back) {
+    if (grad) {
         const size_t at = static_cast<size_t>(bh) * P.nseg + seg;
         float4* dst = reinterpret_cast<float4*>(P.seg_grad + at * 4096) + tid;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) dst[e * kComputeThreads] = make_float4(S[4 * e], S[4 * e + 1], S[4 * e + 2], S[4 * e + 3]);
+        for (int e = 0; e < 4; ++e) dst[e * kComputeThreads] = make_float4(dS[4 * e], dS[4 * e + 1], dS[4 * e + 2], dS[4 * e + 3]);
         if (c0 == 0) P.seg_decay[at * 64 + row] = total;
     }
     tc_fence_before();
     __syncthreads();
-    if (w == 0) tmem_dealloc(tmem, 64);
+    if (w == 0) tmem_dealloc(tmem, 128);
 }
 
 // ------------------------------------------------------------------------------------------ the gradient
