@@ -1094,6 +1094,8 @@ int gla_b200_backward_scan(const gla_b200_bwd_args* a, const gla_b200_bwd_scan* 
     P.seg_grad = reinterpret_cast<float*>(ws + L.seg_grad); P.seg_decay = reinterpret_cast<float*>(ws + L.seg_decay);
     P.B = a->B; P.T = a->T; P.H = a->H; P.NT = NT;
     P.Hc = key.Hc; P.Wc = key.Wc; P.rev = o ? (o->direction & 1) : 0;
+    P.sectors = ((reinterpret_cast<uintptr_t>(a->dq) | reinterpret_cast<uintptr_t>(a->dk) | reinterpret_cast<uintptr_t>(a->dv) |
+                  reinterpret_cast<uintptr_t>(a->dg)) & 31u) == 0 ? 1 : 0;
     P.wait_limit_us = 2000000u;
     P.scale = a->scale;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);

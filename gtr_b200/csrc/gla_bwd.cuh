@@ -25,9 +25,9 @@
 // A chunk in which some channel decays by more than 2^(2 kBwdRefLimit) has no common reference that keeps both operands in
 // range; its products within the chunk are computed pair by pair in fp32 from gate differences (bwd_wide_chunk).
 //
-// Measured (B200): B4 H12 T6400 K64 238 us (states 74, chunks 164) against 1080 us for three recurrent sweeps in fp32, whose
-// bound was the FMA pipe (500 us); B8 H6 T1600 75 against 285.  HBM alone would take about 115 us at 6.5 TB/s (96 KB per
-// chunk and head in the chunk kernel, 40 KB in the states'); what is left is the latency of the chunk's five dependent
+// Measured (B200): B4 H12 T6400 K64 187 us (states 52, chunks 143) against 1080 us for three recurrent sweeps in fp32, whose
+// bound was the FMA pipe (500 us); B8 H6 T1600 64 against 285.  HBM alone would take about 115 us at 6.5 TB/s (96 KB per
+// chunk and head in the chunk kernel, 56 KB in the states'); what is left is the latency of the chunk's five dependent
 // tensor-core round trips with two CTAs per SM.
 //
 // Two kernels.  gla_bwd_state_kernel walks the segments of every sequence and leaves the local state after every chunk
@@ -61,6 +61,7 @@ struct BwdParams {
     int B, T, H, NT;
     int nseg, cps;        // segments per sequence, chunks per segment
     int Hc, Wc, rev;      // scan order as in Params
+    int sectors;          // dq, dk, dv and dg start on 32-byte boundaries
     float scale;
 };
 
@@ -309,7 +310,6 @@ struct BwdChunkMisc {
     // per chunk: largest |q|, |k|, |v|, |do|, |S|, |dS| as float bits, and whether the chunk needs the pair-by-pair path
     uint32_t top[2][8];
     alignas(16) float vec[64];        // log2: half the chunk's total decay per channel
-    int tok[64];                      // the chunk's tokens by row, -1 past the end
     alignas(16) float decay[64];      // log2 decay from the segment's start to the chunk's start
 };
 static_assert(sizeof(BwdChunkMisc) <= 1024, "misc block too large");
@@ -635,8 +635,14 @@ __global__ void __launch_bounds__(kBwdChunkThreads, 2) gla_bwd_chunk_kernel(cons
         sync();
         float later = ld_shared_f(kl + 4u * (tid & 63)) + ld_shared_f(kl + 256u + 4u * (tid & 63));         // dg's share of all later tokens, channel tid & 63
         const uint32_t decay_at = smem_u32(M.decay);
-        const uint32_t tok_at = smem_u32(M.tok);
-        const long long head_row = (static_cast<long long>(b) * P.T * P.H + h) * K;
+        // 16 halves: 32 bytes, in one store where the caller's tensors allow it (whole sectors: 164 -> 153 us)
+        auto put_row = [&](void* to, const uint32_t* r) {
+            if (P.sectors) st_global_v8(to, r);
+            else {
+                reinterpret_cast<uint4*>(to)[0] = make_uint4(r[0], r[1], r[2], r[3]);
+                reinterpret_cast<uint4*>(to)[1] = make_uint4(r[4], r[5], r[6], r[7]);
+            }
+        };
         const uint32_t last_row = rev ? 0u : 63u;
         const int above = 32 * (w >> 2) - 16 * (w & 3);                  // first column - first row of this warp's piece
         const bool on_diagonal = above == 0 || above == -16;
@@ -773,62 +779,66 @@ __global__ void __launch_bounds__(kBwdChunkThreads, 2) gla_bwd_chunk_kernel(cons
             }
             const int tok = scan_token(P, P.T, (first + i) * kChunk + (rev ? 63 - static_cast<int>(row) : static_cast<int>(row)));
             const bool live = tok >= 0 && c0 < K;
-            if (c0 == 0) st_shared_u32(tok_at + 4u * row, static_cast<uint32_t>(tok));
             const long long at = (static_cast<long long>(b) * P.T + max(tok, 0)) * P.H + h;          // in units of one head's row
             const float iS = bwd_inverse(fS), idS = bwd_inverse(fdS), ifd = bwd_inverse(fd), ifq = bwd_inverse(fq), ifk = bwd_inverse(fk);
             wait_bar(P, M.bar_o, ph);
             tc_fence_after();
-            // ---- outputs, eight columns at a time
+            // ---- outputs, read eight columns at a time, written as whole 32-byte sectors
             const int slot_dv = wide ? BWD_P : BWD_DP, slot_dk = wide ? BWD_DP : BWD_P;
-#pragma unroll
-            for (int hf = 0; hf < 2; ++hf) {
-                float a[8], y[8], g[8], D[8];
-                uint32_t o[4];
+            {
+                float a[8], y[8], g[8], D[16];
+                uint32_t o[8];
                 // one of dk, dq: gate factor 2^(sign X) (2^(sign X + R) for the state part alone in a wide chunk) times the sum
                 // of state part and chunk part
                 auto finish = [&](int slot_s, int slot_i, float cs, float ci, float sign, const uint32_t* in, __half* out) {
-                    acc_read8(tmem, slot_s, w, 8 * hf, a);
-                    acc_read8(tmem, slot_i, w, 8 * hf, y);
-                    if (sign < 0.f) acc_read8(tmem, BWD_X, w, 8 * hf, g);
-                    tmem_ld_wait();
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        float2 z;
-                        if (!wide) {
-                            z = fma2(two(cs), pair_of(a, e), mul2(two(ci), pair_of(y, e)));
-                            z = mul2(z, ex2_2(mul2(pair_of(g, e), two(sign * kLog2e))));
-                        } else {
-                            const float2 r = make_float2(M.vec[c0 + 8 * hf + 2 * e], M.vec[c0 + 8 * hf + 2 * e + 1]);
-                            z = mul2(pair_of(a, e), two(cs));
-                            z = fma2(z, ex2_2(fma2(pair_of(g, e), two(sign * kLog2e), r)), pair_of(y, e));
+                    for (int hf = 0; hf < 2; ++hf) {
+                        acc_read8(tmem, slot_s, w, 8 * hf, a);
+                        acc_read8(tmem, slot_i, w, 8 * hf, y);
+                        acc_read8(tmem, BWD_X, w, 8 * hf, g);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            float2 z;
+                            if (!wide) {
+                                z = fma2(two(cs), pair_of(a, e), mul2(two(ci), pair_of(y, e)));
+                                z = mul2(z, ex2_2(mul2(pair_of(g, e), two(sign * kLog2e))));
+                            } else {
+                                const float2 r = make_float2(M.vec[c0 + 8 * hf + 2 * e], M.vec[c0 + 8 * hf + 2 * e + 1]);
+                                z = mul2(pair_of(a, e), two(cs));
+                                z = fma2(z, ex2_2(fma2(pair_of(g, e), two(sign * kLog2e), r)), pair_of(y, e));
+                            }
+                            const int at2 = 4 * hf + e;
+                            o[at2] = pack_half2(z.x, z.y);
+                            const float2 f = unpack_half2(sign > 0.f ? in[at2] : in[at2] ^ 0x80008000u);
+                            z = sign > 0.f ? fma2(f, z, pair_of(D, at2)) : mul2(f, z);
+                            D[2 * at2] = z.x; D[2 * at2 + 1] = z.y;
                         }
-                        o[e] = pack_half2(z.x, z.y);
-                        const float2 f = unpack_half2(sign > 0.f ? in[4 * hf + e] : in[4 * hf + e] ^ 0x80008000u);
-                        z = sign > 0.f ? fma2(f, z, pair_of(D, e)) : mul2(f, z);
-                        D[2 * e] = z.x; D[2 * e + 1] = z.y;
                     }
-                    if (live) *reinterpret_cast<uint4*>(out + at * K + c0 + 8 * hf) = make_uint4(o[0], o[1], o[2], o[3]);
+                    if (live) put_row(out + at * K + c0, o);
                 };
                 finish(BWD_DK_S, slot_dk, idS, P.scale * ifd * ifq, -1.f, kr, P.dk);
                 finish(BWD_DQ_S, BWD_DQ_I, P.scale * iS, P.scale * ifd * ifk, 1.f, qr, P.dq);
-                st_shared_f4(bwd_f32(r0, row, c0 + 8 * hf), D[0], D[1], D[2], D[3]);
-                st_shared_f4(bwd_f32(r0, row, c0 + 8 * hf + 4), D[4], D[5], D[6], D[7]);
-                acc_read8(tmem, BWD_DV_S, w, 8 * hf, a);
-                acc_read8(tmem, slot_dv, w, 8 * hf, y);
-                tmem_ld_wait();
+                bwd_f32_put16(r0, row, c0, D);
                 const float2 cs = two(ifk * idS), ci = two(P.scale * ifq * ifk * 8.f);      // 8 = 1 / fp
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const float2 z = fma2(cs, pair_of(a, e), mul2(ci, pair_of(y, e)));
-                    o[e] = pack_half2(z.x, z.y);
+                for (int hf = 0; hf < 2; ++hf) {
+                    acc_read8(tmem, BWD_DV_S, w, 8 * hf, a);
+                    acc_read8(tmem, slot_dv, w, 8 * hf, y);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const float2 z = fma2(cs, pair_of(a, e), mul2(ci, pair_of(y, e)));
+                        o[4 * hf + e] = pack_half2(z.x, z.y);
+                    }
                 }
-                if (tok >= 0) *reinterpret_cast<uint4*>(P.dv + at * 64 + c0 + 8 * hf) = make_uint4(o[0], o[1], o[2], o[3]);
+                if (tok >= 0) put_row(P.dv + at * 64 + c0, o);
             }
             tc_fence_before();
             if (i > 0) named_bar_arrive(BWD_BAR_READ, kBwdChunkThreads);
             sync();
-            // ---- dg: sums of the terms of the tokens at and after each token, a quarter of the rows per thread and channel,
-            // handed back to the rows' owners through the tiles of the low parts
+            // ---- dg: sums of the terms of the tokens at and after each token, a quarter of the rows per thread and channel, handed
+            // back to the rows' owners in place
             {
                 const uint32_t c = tid & 63u, q4 = static_cast<uint32_t>(tid) >> 6;
                 float t[16], run = 0.f;
@@ -849,14 +859,24 @@ __global__ void __launch_bounds__(kBwdChunkThreads, 2) gla_bwd_chunk_kernel(cons
                     add += (rev ? j < q4 : j > q4) ? s : 0.f;
                     later += s;
                 }
-                if (c < K) {
 #pragma unroll
-                    for (int r = 0; r < 16; ++r) {
-                        const int o = static_cast<int>(ld_shared_u32(tok_at + 4u * (16u * q4 + r)));
-                        if (o < 0) continue;
-                        const long long at = head_row + static_cast<long long>(o) * (P.H * K) + c;
-                        if (P.dg_half != nullptr) P.dg_half[at] = __float2half_rn(t[r] + add);
-                        else P.dg[at] = t[r] + add;
+                for (int r = 0; r < 16; ++r)
+                    asm volatile("st.shared.f32 [%0], %1;" ::"r"(bwd_f32(r0, 16u * q4 + r, c)), "f"(t[r] + add) : "memory");
+                sync();
+                bwd_f32_row16(r0, row, c0, t);
+                if (live) {
+                    uint32_t o[8];
+                    if (P.dg_half != nullptr) {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) o[e] = pack_half2(t[2 * e], t[2 * e + 1]);
+                        put_row(P.dg_half + at * K + c0, o);
+                    } else {
+#pragma unroll
+                        for (int m = 0; m < 2; ++m) {
+#pragma unroll
+                            for (int e = 0; e < 8; ++e) o[e] = __float_as_uint(t[8 * m + e]);
+                            put_row(P.dg + at * K + c0 + 8 * m, o);
+                        }
                     }
                 }
             }
