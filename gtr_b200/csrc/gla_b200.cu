@@ -334,7 +334,18 @@ struct MapEntry {
 std::vector<MapEntry> g_map_cache;
 constexpr size_t kMapCacheMax = 64;
 
+// Encoding a tensor map needs the device's context current in this thread, which a thread that has called nothing of the runtime
+// that needs one (autograd's, with all its memory from the allocator's cache) does not have yet.
+int make_context_current() {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaSetDevice(dev);
+    if (e != cudaSuccess) { note_cuda("cudaSetDevice", e); return GLA_B200_ERR_CUDA; }
+    return GLA_B200_OK;
+}
+
 int build_maps(const MapKey& key, gla::Maps* out) {
+    if (int rc = make_context_current()) return rc;
     EncodeTiledFn enc = encode_tiled();
     if (!enc) {
         snprintf(g_cuda_err, sizeof(g_cuda_err), "cuTensorMapEncodeTiled is not available from this driver");
@@ -1148,6 +1159,7 @@ int gla_b200_swiglu_dwconv(const void* gate, const void* y, const void* weight, 
     }
     const int64_t items = B * tiles * ((C + gla::kDwSlab - 1) / gla::kDwSlab);
     if (items > 0x7fffffffLL) return GLA_B200_ERR_SHAPE;
+    if (int rc = make_context_current()) return rc;
     gla::DwMaps maps;
     const cuuint64_t grid[4] = {static_cast<cuuint64_t>(C), static_cast<cuuint64_t>(grid_w), static_cast<cuuint64_t>(grid_h), static_cast<cuuint64_t>(B)};
     const cuuint64_t taps[2] = {static_cast<cuuint64_t>(C), 9}, one[2] = {static_cast<cuuint64_t>(C), 1};
