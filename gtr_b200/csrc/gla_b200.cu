@@ -1177,13 +1177,18 @@ int gla_b200_layernorm(const void* x, const void* weight, const void* bias, void
     if (rows == 0) return GLA_B200_OK;
     if (!x || !weight || !y) return GLA_B200_ERR_NULL;
     if (!aligned16(x) || !aligned16(weight) || !aligned16(y) || (bias && !aligned16(bias))) return GLA_B200_ERR_ALIGN;
-    const int64_t blocks = (rows + 7) / 8;               // eight warps, one row each
-    if (blocks > 0x7fffffffLL) return GLA_B200_ERR_SHAPE;
     const int per_lane = ((D >> 3) + 31) / 32;            // 16-byte vectors per lane
-    void (*const kernel)(const __half*, const __half*, const __half*, __half*, long long, int, float) =
-        per_lane <= 1 ? &gla::layernorm_rows_kernel<1> : per_lane <= 2 ? &gla::layernorm_rows_kernel<2>
-        : per_lane <= 3 ? &gla::layernorm_rows_kernel<3> : per_lane <= 4 ? &gla::layernorm_rows_kernel<4>
-                                                         : &gla::layernorm_rows_kernel<gla::kLnMaxVec>;
+    // two rows per warp once every warp the chip holds has one, as long as their registers leave room for that many
+    const int rows_per_warp = rows > 148 * 64 && per_lane <= 4 ? 2 : 1;
+    const int64_t blocks = (rows + 8 * rows_per_warp - 1) / (8 * rows_per_warp);
+    if (blocks > 0x7fffffffLL) return GLA_B200_ERR_SHAPE;
+    using Kernel = void (*)(const __half*, const __half*, const __half*, __half*, long long, int, float);
+    constexpr Kernel kernels[5][2] = {{&gla::layernorm_rows_kernel<1, 1>, &gla::layernorm_rows_kernel<1, 2>},
+                                      {&gla::layernorm_rows_kernel<2, 1>, &gla::layernorm_rows_kernel<2, 2>},
+                                      {&gla::layernorm_rows_kernel<3, 1>, &gla::layernorm_rows_kernel<3, 2>},
+                                      {&gla::layernorm_rows_kernel<4, 1>, &gla::layernorm_rows_kernel<4, 2>},
+                                      {&gla::layernorm_rows_kernel<gla::kLnMaxVec, 1>, nullptr}};
+    const Kernel kernel = kernels[std::min(per_lane, 5) - 1][rows_per_warp - 1];
     return launch_simple(kernel, static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream), static_cast<const __half*>(x),
                          static_cast<const __half*>(weight), static_cast<const __half*>(bias), static_cast<__half*>(y),
                          static_cast<long long>(rows), D, eps);

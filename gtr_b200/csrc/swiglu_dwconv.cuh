@@ -207,56 +207,75 @@ __global__ void __launch_bounds__(kDwThreads, 1) swiglu_dwconv_kernel(const __gr
     }
 }
 
-}  // namespace gla
-
-namespace gla {
-
-// LayerNorm over rows of D fp16 values (D a multiple of 8, D <= 2048), affine, fp32 statistics: one warp per row,
-// the row held in registers between the mean, the variance and the output pass, so that x is read once and y written
-// once (the backbone's norms run at a quarter of that with the framework's kernel).
-// kVec = 16-byte vectors per lane, chosen by the host from D: a narrow row must not pay for the registers of the
-// widest one (occupancy is what keeps enough loads in flight here).
+// LayerNorm over rows of D fp16 values (D a multiple of 8, D <= 2048), affine, fp32 statistics: one warp per kRows rows, held
+// in registers as they came between the mean, the variance and the output pass, so that x is read once and y written
+// once.  HBM-bound: what matters is the bytes in flight, so the rows stay packed (as floats they took the registers of half
+// the warps) and, where there are rows enough, a warp asks for two at once: 32768 rows of 768 27.9 -> 18.5 us, 5.4 TB/s;
+// of 2048 (one row a warp) 68.9 -> 45.3 us.
+// kVec = 16-byte vectors per lane and row, chosen by the host from D: a narrow row must not pay for the registers of the
+// widest one.
 constexpr int kLnMaxVec = 8;
 
 // y may alias x (in-place use): x is read with plain loads and neither pointer is declared restrict.
-template <int kVec>
+template <int kVec, int kRows>
 __global__ void __launch_bounds__(256) layernorm_rows_kernel(const __half* x, const __half* __restrict__ w,
                                                              const __half* __restrict__ b, __half* y,
                                                              long long rows, int D, float eps) {
-    const long long row = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    const long long row = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) / 32 * kRows;
     const int lane = threadIdx.x & 31;
     if (row >= rows) return;
     pdl_wait();
     const int nvec = D >> 3;
     const uint4* x4 = reinterpret_cast<const uint4*>(x) + row * nvec;
-    float v[kVec][8];
-    float sum = 0.f;
+    uint4 in[kRows][kVec];
 #pragma unroll
-    for (int k = 0; k < kVec; ++k) {
-        const int i = lane + 32 * k;
-        if (i < nvec) {
-            dw_unpack8(x4[i], v[k]);
+    for (int r = 0; r < kRows; ++r)
 #pragma unroll
-            for (int e = 0; e < 8; ++e) sum += v[k][e];
-        }
-    }
+        for (int k = 0; k < kVec; ++k)
+            in[r][k] = row + r < rows && lane + 32 * k < nvec ? x4[static_cast<long long>(r) * nvec + lane + 32 * k] : make_uint4(0u, 0u, 0u, 0u);
+    float mean[kRows], rstd[kRows];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    const float mean = sum / static_cast<float>(D);
-    float sq = 0.f;
+    for (int r = 0; r < kRows; ++r) {
+        float sum = 0.f;
 #pragma unroll
-    for (int k = 0; k < kVec; ++k) {
-        if (lane + 32 * k < nvec) {
+        for (int k = 0; k < kVec; ++k) {
+            if (lane + 32 * k < nvec) {
+                float v[8];
+                dw_unpack8(in[r][k], v);
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                const float d = v[k][e] - mean;
-                sq = fmaf(d, d, sq);
+                for (int e = 0; e < 8; ++e) sum += v[e];
             }
         }
+        mean[r] = sum;
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-    const float rstd = rsqrtf(sq / static_cast<float>(D) + eps);
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) mean[r] += __shfl_xor_sync(0xffffffffu, mean[r], o);
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+        mean[r] = mean[r] / static_cast<float>(D);
+        float sq = 0.f;
+#pragma unroll
+        for (int k = 0; k < kVec; ++k) {
+            if (lane + 32 * k < nvec) {
+                float v[8];
+                dw_unpack8(in[r][k], v);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    const float d = v[e] - mean[r];
+                    sq = fmaf(d, d, sq);
+                }
+            }
+        }
+        rstd[r] = sq;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) rstd[r] += __shfl_xor_sync(0xffffffffu, rstd[r], o);
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) rstd[r] = rsqrtf(rstd[r] / static_cast<float>(D) + eps);
     uint4* y4 = reinterpret_cast<uint4*>(y) + row * nvec;
 #pragma unroll
     for (int k = 0; k < kVec; ++k) {
@@ -265,15 +284,20 @@ __global__ void __launch_bounds__(256) layernorm_rows_kernel(const __half* x, co
             float wv[8], bv[8];
             dw_unpack8(__ldg(reinterpret_cast<const uint4*>(w) + i), wv);
             if (b != nullptr) dw_unpack8(__ldg(reinterpret_cast<const uint4*>(b) + i), bv);
-            uint4 o;
-            __half2* oh = reinterpret_cast<__half2*>(&o);
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float a0 = (v[k][2 * e] - mean) * rstd * wv[2 * e] + (b != nullptr ? bv[2 * e] : 0.f);
-                const float a1 = (v[k][2 * e + 1] - mean) * rstd * wv[2 * e + 1] + (b != nullptr ? bv[2 * e + 1] : 0.f);
-                oh[e] = __floats2half2_rn(a0, a1);
+            for (int r = 0; r < kRows; ++r) {
+                float v[8];
+                dw_unpack8(in[r][k], v);
+                uint4 o;
+                __half2* oh = reinterpret_cast<__half2*>(&o);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float a0 = (v[2 * e] - mean[r]) * rstd[r] * wv[2 * e] + (b != nullptr ? bv[2 * e] : 0.f);
+                    const float a1 = (v[2 * e + 1] - mean[r]) * rstd[r] * wv[2 * e + 1] + (b != nullptr ? bv[2 * e + 1] : 0.f);
+                    oh[e] = __floats2half2_rn(a0, a1);
+                }
+                if (row + r < rows) y4[static_cast<long long>(r) * nvec + i] = o;
             }
-            y4[i] = o;
         }
     }
 }
