@@ -61,6 +61,7 @@ EXPORTS = (
     "gla_b200_forward_static", "gla_b200_selftest_wait_timeout", "gla_b200_swiglu_dwconv", "gla_b200_layernorm",
     "gla_b200_stream_probe", "gla_b200_backward", "gla_b200_backward_workspace_bytes",
     "gla_b200_backward_scan", "gla_b200_forward_packed", "gla_b200_packed_workspace_bytes",
+    "gla_b200_forward_packed_device", "gla_b200_packed_device_workspace_bytes",
     "gla_b200_forward_block",
 )
 
@@ -89,6 +90,11 @@ def lib() -> ctypes.CDLL:
     L.gla_b200_forward_packed.restype = ctypes.c_int
     L.gla_b200_packed_workspace_bytes.argtypes = [ctypes.POINTER(ctypes.c_int32), ctypes.c_int32, ctypes.c_int32]
     L.gla_b200_packed_workspace_bytes.restype = ctypes.c_size_t
+    L.gla_b200_forward_packed_device.argtypes = [ctypes.POINTER(Args), ctypes.c_void_p, ctypes.c_int32, ctypes.c_int32, ctypes.c_void_p,
+                                                 ctypes.c_void_p]
+    L.gla_b200_forward_packed_device.restype = ctypes.c_int
+    L.gla_b200_packed_device_workspace_bytes.argtypes = [ctypes.c_int32, ctypes.c_int32, ctypes.c_int32]
+    L.gla_b200_packed_device_workspace_bytes.restype = ctypes.c_size_t
     L.gla_b200_forward_block.argtypes = [ctypes.POINTER(Args), ctypes.c_void_p]
     L.gla_b200_forward_block.restype = ctypes.c_int
     L.gla_b200_forward_static.argtypes = [ctypes.POINTER(Args), ctypes.c_void_p]
@@ -139,7 +145,8 @@ def front():
         address = lambda fn: ctypes.cast(fn, ctypes.c_void_p).value
         F.bind(*(address(fn) for fn in (L.gla_b200_forward, L.gla_b200_workspace_bytes, L.gla_b200_backward_scan,
                                         L.gla_b200_backward_workspace_bytes, L.gla_b200_strerror, L.gla_b200_forward_packed,
-                                        L.gla_b200_packed_workspace_bytes, L.gla_b200_forward_block)))
+                                        L.gla_b200_packed_workspace_bytes, L.gla_b200_forward_block,
+                                        L.gla_b200_forward_packed_device, L.gla_b200_packed_device_workspace_bytes)))
         _front = F
     return _front
 

@@ -45,24 +45,20 @@ EncodeTiledFn encode_tiled() {
 
 // The forward's instantiations: outputs by (fused epilogue, raw-logit gates), span increments by raw-logit gates; packed
 // sequences have no fused epilogue.
-const void* out_kernel(bool gated, bool logits, bool packed) {
+template <class Table>
+const void* out_kernel(bool gated, bool logits) {
     using namespace gla;
-    if (packed)
-        return logits ? reinterpret_cast<const void*>(&gla_out_kernel<false, true, PackedTable>)
-                      : reinterpret_cast<const void*>(&gla_out_kernel<false, false, PackedTable>);
-    if (gated)
+    if (std::is_same<Table, NoTable>::value && gated)
         return logits ? reinterpret_cast<const void*>(&gla_out_kernel<true, true, NoTable>)
                       : reinterpret_cast<const void*>(&gla_out_kernel<true, false, NoTable>);
-    return logits ? reinterpret_cast<const void*>(&gla_out_kernel<false, true, NoTable>)
-                  : reinterpret_cast<const void*>(&gla_out_kernel<false, false, NoTable>);
+    return logits ? reinterpret_cast<const void*>(&gla_out_kernel<false, true, Table>)
+                  : reinterpret_cast<const void*>(&gla_out_kernel<false, false, Table>);
 }
-const void* state_kernel(bool logits, bool packed) {
+template <class Table>
+const void* state_kernel(bool logits) {
     using namespace gla;
-    if (packed)
-        return logits ? reinterpret_cast<const void*>(&gla_state_kernel<true, PackedTable>)
-                      : reinterpret_cast<const void*>(&gla_state_kernel<false, PackedTable>);
-    return logits ? reinterpret_cast<const void*>(&gla_state_kernel<true, NoTable>)
-                  : reinterpret_cast<const void*>(&gla_state_kernel<false, NoTable>);
+    return logits ? reinterpret_cast<const void*>(&gla_state_kernel<true, Table>)
+                  : reinterpret_cast<const void*>(&gla_state_kernel<false, Table>);
 }
 
 // The block kernel's: bit 1 raw-logit gates, bit 0 reversed scan.
@@ -94,12 +90,13 @@ int device_info(int dev, DeviceInfo* out) {
             snprintf(g_cuda_err, sizeof(g_cuda_err), "device %d has compute capability %d.x, need 10.x", dev, major);
             return GLA_B200_ERR_DEVICE;
         }
-        for (int v = 0; v < 8 && e == cudaSuccess; ++v)
-            e = cudaFuncSetAttribute(out_kernel((v & 1) != 0, (v & 2) != 0, (v & 4) != 0), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     gla::OutSmem::kBytes);
-        for (int v = 0; v < 4 && e == cudaSuccess; ++v)
-            e = cudaFuncSetAttribute(state_kernel((v & 1) != 0, (v & 2) != 0), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     gla::StateSmem::kBytes);
+        for (int v = 0; v < 2; ++v) {
+            for (const void* k : {out_kernel<gla::NoTable>(false, v), out_kernel<gla::NoTable>(true, v), out_kernel<gla::PackedTable>(false, v),
+                                  out_kernel<gla::DeviceTable>(false, v)})
+                if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, gla::OutSmem::kBytes);
+            for (const void* k : {state_kernel<gla::NoTable>(v), state_kernel<gla::PackedTable>(v), state_kernel<gla::DeviceTable>(v)})
+                if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, gla::StateSmem::kBytes);
+        }
         if (e != cudaSuccess) { note_cuda("cudaFuncSetAttribute", e); return GLA_B200_ERR_CUDA; }
         for (int v = 0; v < 4 && e == cudaSuccess; ++v)
             e = cudaFuncSetAttribute(block_kernel(v), cudaFuncAttributeMaxDynamicSharedMemorySize, gla::block::kSmemBytes);
@@ -584,15 +581,14 @@ constexpr int64_t kL2Keep = 120ll << 20;
 // The spans' increments (where spans end inside sequences), then the outputs.
 template <class Table>
 int launch_forward(bool gated, const gla::Maps& maps, gla::Params& P, const Table& table, cudaStream_t stream) {
-    constexpr bool packed = std::is_same<Table, gla::PackedTable>::value;
     const bool logits = P.inv_norm > 0.f;
     const int states = P.per > 0 ? P.spans / P.per * (P.per - 1) : P.spans - 1;
     P.alone = states == 0 ? 1 : 0;
     P.keep = static_cast<int64_t>(P.chunks) * (4 * P.K + 128) * gla::kChunk <= kL2Keep ? 1 : 0;
     void* args[3] = {const_cast<gla::Maps*>(&maps), &P, const_cast<Table*>(&table)};
     if (states > 0)
-        if (int rc = launch_overlapped(state_kernel(logits, packed), states, gla::kFwdThreads, gla::StateSmem::kBytes, args, stream)) return rc;
-    return launch_overlapped(out_kernel(gated, logits, packed), P.spans, gla::kFwdThreads, gla::OutSmem::kBytes, args, stream);
+        if (int rc = launch_overlapped(state_kernel<Table>(logits), states, gla::kFwdThreads, gla::StateSmem::kBytes, args, stream)) return rc;
+    return launch_overlapped(out_kernel<Table>(gated, logits), P.spans, gla::kFwdThreads, gla::OutSmem::kBytes, args, stream);
 }
 
 // The fused operator on the block kernel (gla_block.cuh).
@@ -861,26 +857,15 @@ size_t gla_b200_packed_workspace_bytes(const int32_t* offsets, int32_t n, int32_
     return ws_layout(most).total;
 }
 
-int gla_b200_forward_packed(const gla_b200_args* a, const int32_t* offsets, int32_t n, void* stream_v) {
-    if (!a || !offsets) return GLA_B200_ERR_NULL;
+// What packed sequences have in common however their offsets come: arguments, tensor maps, the output's strides.
+static int packed_arguments(const gla_b200_args* a, int32_t n) {
     if ((a->K != 32 && a->K != gla::kD) || a->V != gla::kD || a->B != 1 || a->T < 0 || a->H <= 0 || n < 0) return GLA_B200_ERR_SHAPE;
     if (a->direction != 0 || a->out_gate || a->rms_weight || a->segments != 0) return GLA_B200_ERR_ARG;
     if (a->scale != a->scale || a->gk_normalizer < 0.f) return GLA_B200_ERR_ARG;
-    for (int i = 0; i < n; ++i)
-        if (offsets[i + 1] < offsets[i]) return GLA_B200_ERR_SHAPE;
-    if (n > 0 && (offsets[0] != 0 || offsets[n] != a->T)) return GLA_B200_ERR_SHAPE;
-    cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
-    const size_t state_floats = static_cast<size_t>(a->H) * a->K * gla::kD;
     if ((a->initial_state && !aligned16(a->initial_state)) || (a->final_state && !aligned16(a->final_state))) return GLA_B200_ERR_ALIGN;
-    cudaError_t ce = cudaSuccess;
-    for (int i = 0; i < n && a->final_state; ++i) {                  // an empty sequence leaves the state as it came in
-        if (offsets[i + 1] != offsets[i]) continue;
-        float* to = a->final_state + i * state_floats;
-        ce = a->initial_state ? cudaMemcpyAsync(to, a->initial_state + i * state_floats, state_floats * 4, cudaMemcpyDeviceToDevice, stream)
-                              : cudaMemsetAsync(to, 0, state_floats * 4, stream);
-        if (ce != cudaSuccess) { note_cuda("final state of an empty sequence", ce); return GLA_B200_ERR_CUDA; }
-    }
-    if (a->T == 0 || n == 0) return GLA_B200_OK;
+    return GLA_B200_OK;
+}
+static int packed_maps(const gla_b200_args* a, gla::Maps* maps, int64_t o_stride[3]) {
     if (!a->q || !a->k || !a->v || !a->g || !a->o) return GLA_B200_ERR_NULL;
     MapKey key;
     memset(&key, 0, sizeof(key));
@@ -894,18 +879,38 @@ int gla_b200_forward_packed(const gla_b200_args* a, const int32_t* offsets, int3
         if (int rc = resolve_strides(strides[t], a->T, a->H, key_side ? a->K : gla::kD, key.stride[t])) return rc;
     }
     int dev = 0;
-    ce = cudaGetDevice(&dev);
+    const cudaError_t ce = cudaGetDevice(&dev);
     if (ce != cudaSuccess) { note_cuda("cudaGetDevice", ce); return GLA_B200_ERR_CUDA; }
     if (dev < 0 || dev >= 64) return GLA_B200_ERR_DEVICE;
     DeviceInfo di;
     if (int rc = device_info(dev, &di)) return rc;
     key.B = 1; key.T = a->T; key.H = a->H; key.K = a->K; key.Hc = a->T; key.Wc = 1; key.dev = dev;
-    int64_t o_stride[3];
-    memcpy(o_stride, key.stride[gla::TO], sizeof(o_stride));
+    memcpy(o_stride, key.stride[gla::TO], 3 * sizeof(int64_t));
     key.ptr[gla::TO] = nullptr;                       // outputs are stored from registers
     memset(key.stride[gla::TO], 0, sizeof(key.stride[gla::TO]));
+    return get_maps(key, maps);
+}
+
+int gla_b200_forward_packed(const gla_b200_args* a, const int32_t* offsets, int32_t n, void* stream_v) {
+    if (!a || !offsets) return GLA_B200_ERR_NULL;
+    if (int rc = packed_arguments(a, n)) return rc;
+    for (int i = 0; i < n; ++i)
+        if (offsets[i + 1] < offsets[i]) return GLA_B200_ERR_SHAPE;
+    if (n > 0 && (offsets[0] != 0 || offsets[n] != a->T)) return GLA_B200_ERR_SHAPE;
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
+    const size_t state_floats = static_cast<size_t>(a->H) * a->K * gla::kD;
+    cudaError_t ce = cudaSuccess;
+    for (int i = 0; i < n && a->final_state; ++i) {                  // an empty sequence leaves the state as it came in
+        if (offsets[i + 1] != offsets[i]) continue;
+        float* to = a->final_state + i * state_floats;
+        ce = a->initial_state ? cudaMemcpyAsync(to, a->initial_state + i * state_floats, state_floats * 4, cudaMemcpyDeviceToDevice, stream)
+                              : cudaMemsetAsync(to, 0, state_floats * 4, stream);
+        if (ce != cudaSuccess) { note_cuda("final state of an empty sequence", ce); return GLA_B200_ERR_CUDA; }
+    }
+    if (a->T == 0 || n == 0) return GLA_B200_OK;
     gla::Maps maps;
-    if (int rc = get_maps(key, &maps)) return rc;
+    int64_t o_stride[3];
+    if (int rc = packed_maps(a, &maps, o_stride)) return rc;
     uint8_t* ws = static_cast<uint8_t*>(a->workspace);
     if (!ws || (reinterpret_cast<uintptr_t>(ws) & 255u)) return GLA_B200_ERR_WORKSPACE;
     for (int at = 0; at < n; at += gla::kMaxPacked) {
@@ -926,6 +931,40 @@ int gla_b200_forward_packed(const gla_b200_args* a, const int32_t* offsets, int3
         if (int rc = launch_forward(false, maps, P, tab, stream)) return rc;
     }
     return GLA_B200_OK;
+}
+
+// The split for n packed sequences of T tokens in all: their chunks are at least T / 64 (which bounds the spans: none may be
+// empty) and at most n more per head.
+static Split unread_split(int32_t T, int32_t n, int32_t H) {
+    const int64_t least = static_cast<int64_t>(num_chunks(T)) * H;
+    Split s = packed_split(least + static_cast<int64_t>(n) * H / 2, static_cast<int64_t>(n) * H, 148);
+    s.spans = static_cast<int>(std::min<int64_t>(s.spans, least));
+    return s;
+}
+size_t gla_b200_packed_device_workspace_bytes(int32_t T, int32_t n, int32_t H) {
+    if (T <= 0 || n <= 0 || n > gla::kMaxPacked || H <= 0) return 0;
+    return ws_layout(exchange_spans(unread_split(T, n, H))).total;
+}
+int gla_b200_forward_packed_device(const gla_b200_args* a, const void* offsets, int32_t wide, int32_t n, int32_t* echo, void* stream) {
+    if (!a || !offsets) return GLA_B200_ERR_NULL;
+    if (int rc = packed_arguments(a, n)) return rc;
+    if (a->T == 0 || n == 0 || n > gla::kMaxPacked) return GLA_B200_ERR_SHAPE;
+    gla::Maps maps;
+    int64_t o_stride[3];
+    if (int rc = packed_maps(a, &maps, o_stride)) return rc;
+    uint8_t* ws = static_cast<uint8_t*>(a->workspace);
+    if (!ws || (reinterpret_cast<uintptr_t>(ws) & 255u)) return GLA_B200_ERR_WORKSPACE;
+    const Split split = unread_split(a->T, n, a->H);
+    const WsLayout L = ws_layout(exchange_spans(split));
+    if (a->workspace_bytes < L.total) return GLA_B200_ERR_WORKSPACE;
+    gla::Params P;
+    memset(&P, 0, sizeof(P));
+    P.B = 1; P.T = a->T; P.H = a->H; P.K = a->K; P.Hc = a->T; P.Wc = 1;
+    set_split(split, static_cast<int64_t>(num_chunks(a->T)) * a->H, &P);
+    fill_params(a, o_stride, ws, L, &P);
+    P.s0 = a->initial_state;
+    P.sT = a->final_state;
+    return launch_forward(false, maps, P, gla::DeviceTable{offsets, echo, n, wide != 0}, static_cast<cudaStream_t>(stream));
 }
 
 int gla_b200_stream_probe(const void* buf, int64_t rows, int32_t heads, int32_t ctas, int32_t tiles, int32_t chunks,

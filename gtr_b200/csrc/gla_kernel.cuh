@@ -81,8 +81,79 @@ struct PackedTable {
     PackedSeq seq[kMaxPacked];
 };
 struct NoTable {};
+// The same table from offsets that only the GPU has: every block makes its own, in shared memory, from the n + 1 offsets (a load
+// and two scans, about 1 us), so that the launches need not wait for the host to read them.  Offsets that do not rise
+// from 0 to T leave an empty table, and nothing is computed.  The first kernel's first block writes them to `echo`
+// (pinned host memory: n + 1 offsets, and a one at [kMaxPacked + 1] when they are there), where the host checks them.
+struct DeviceTable {
+    const void* offsets;                  // n + 1 int32, or int64 where `wide`
+    int32_t* echo;
+    int n, wide;
+    // -1, which no table of rising offsets has, for what lies outside the row
+    __device__ __forceinline__ int offset(int i, int T) const {
+        const long long x = wide ? __ldg(static_cast<const long long*>(offsets) + i) : __ldg(static_cast<const int32_t*>(offsets) + i);
+        return x < 0 || x > T ? -1 : static_cast<int>(x);
+    }
+};
+struct SharedTable : PackedTable {
+    int len_, longer;                     // the spans' (see Params)
+};
+__device__ __forceinline__ const NoTable& table_here(const NoTable& t, const Params&, bool) { return t; }
+__device__ __forceinline__ const PackedTable& table_here(const PackedTable& t, const Params&, bool) { return t; }
+__device__ __forceinline__ const SharedTable& table_here(const DeviceTable& t, const Params& P, bool first) {
+    __shared__ SharedTable tab;
+    __shared__ int2 sums[4];              // of each warp: chunks, sequences
+    const int tid = threadIdx.x, l = tid & 31;
+    static_assert(kMaxPacked + 1 <= 128, "one offset per thread");
+    const int a = tid <= t.n ? t.offset(tid, P.T) : 0, b = tid < t.n ? t.offset(tid + 1, P.T) : 0;
+    bool fine = true;
+    if (tid < t.n) fine = b >= a && (tid > 0 || a == 0) && (tid < t.n - 1 || b == P.T);
+    if (first && blockIdx.x == 0 && t.echo != nullptr) {
+        if (tid <= t.n) {
+            *reinterpret_cast<volatile int32_t*>(t.echo + tid) = a;
+            __threadfence_system();
+        }
+        __syncthreads();
+        if (tid == 0) *reinterpret_cast<volatile int32_t*>(t.echo + kMaxPacked + 1) = 1;
+    }
+    fine = __syncthreads_and(fine);
+    const int len = fine && tid < t.n ? b - a : 0;
+    const int2 own = make_int2((len / kChunk + (len % kChunk != 0)) * P.H, len > 0);
+    int2 run = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, run.x, o), y = __shfl_up_sync(0xffffffffu, run.y, o);
+        if (l >= o) { run.x += x; run.y += y; }
+    }
+    if (l == 31) sums[tid >> 5] = run;
+    __syncthreads();
+    int2 all = make_int2(0, 0);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int2 x = sums[j];
+        if (j < (tid >> 5)) { run.x += x.x; run.y += x.y; }
+        all.x += x.x; all.y += x.y;
+    }
+    if (len > 0) tab.seq[run.y - 1] = {run.x - own.x, a, len, tid};
+    if (tid == 0) {
+        tab.n = all.y;
+        tab.len_ = all.x / P.spans;
+        tab.longer = all.x % P.spans;
+    }
+    __syncthreads();
+    return tab;
+}
+template <class Table>
+__device__ __forceinline__ bool nothing_in(const Table&) { return false; }
+__device__ __forceinline__ bool nothing_in(const SharedTable& tab) { return tab.n == 0; }
 
-__device__ __forceinline__ int span_begin(const Params& P, int i) {
+__device__ __forceinline__ int span_begin(const SharedTable& tab, const Params&, int i) { return i * tab.len_ + min(i, tab.longer); }
+__device__ __forceinline__ int span_of(const SharedTable& tab, const Params&, int chunk) {
+    const int head = tab.longer * (tab.len_ + 1);
+    return chunk < head ? chunk / (tab.len_ + 1) : tab.longer + (chunk - head) / tab.len_;
+}
+template <class Table>
+__device__ __forceinline__ int span_begin(const Table&, const Params& P, int i) {
     if (P.per > 0) {
         const int s = i / P.per, j = i - s * P.per;
         return s * P.NT + j * P.NT / P.per;
@@ -90,7 +161,8 @@ __device__ __forceinline__ int span_begin(const Params& P, int i) {
     return i * P.len_ + min(i, P.longer);
 }
 // The span that holds the first chunk of a sequence.
-__device__ __forceinline__ int span_of(const Params& P, int chunk) {
+template <class Table>
+__device__ __forceinline__ int span_of(const Table&, const Params& P, int chunk) {
     if (P.per > 0) return chunk / P.NT * P.per;
     const int head = P.longer * (P.len_ + 1);
     return chunk < head ? chunk / (P.len_ + 1) : P.longer + (chunk - head) / P.len_;
@@ -225,11 +297,14 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_state_kernel(const __grid_
     const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
     // per sequence, the last span needs no increment and gets no CTA; in the flat split it is found here
     const int span = P.per > 0 ? blockIdx.x + blockIdx.x / (P.per - 1) : blockIdx.x;
-    const int end = span_begin(P, span + 1);
+    if (std::is_same<Table, DeviceTable>::value) pdl_wait();
+    const auto& tab = table_here(table, P, true);
+    if (nothing_in(tab)) return;
+    const int end = span_begin(tab, P, span + 1);
     const bool rev = P.rev != 0;
     const uint32_t mat = base + StateSmem::kMat, tv = base + StateSmem::kV;
-    const Sequence sq = sequence_of(table, P, end - 1);
-    const int n = end == sq.chunk0 + sq.nt ? 0 : end - max(span_begin(P, span), sq.chunk0), c_last = end - 1 - sq.chunk0, T = sq.T;
+    const Sequence sq = sequence_of(tab, P, end - 1);
+    const int n = end == sq.chunk0 + sq.nt ? 0 : end - max(span_begin(tab, P, span), sq.chunk0), c_last = end - 1 - sq.chunk0, T = sq.T;
     auto load_kg = [&](int i) {
         const uint32_t bar = smem_u32(&M.full[i & 1]), off = (i & 1) * kTileBytes;
         const int tensors[2] = {TG, TK};
@@ -441,9 +516,13 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
     const bool rev = P.rev != 0;
     const uint32_t tq = base + OutSmem::kQ, tk = base + OutSmem::kK, tg = base + OutSmem::kG, tv = base + OutSmem::kV,
                    s16 = base + OutSmem::kS16, mat = base + OutSmem::kMat;
-    int chunk = span_begin(P, blockIdx.x);                           // of all chunks, the one at hand; the span's end
-    const int end = span_begin(P, blockIdx.x + 1);
-    const Sequence first_sq = sequence_of(table, P, chunk);
+    // (offsets on the GPU: the state kernel has waited for them before it let these blocks start)
+    if (std::is_same<Table, DeviceTable>::value && P.alone) pdl_wait();
+    const auto& tab = table_here(table, P, P.alone != 0);
+    if (nothing_in(tab)) return;
+    int chunk = span_begin(tab, P, blockIdx.x);                      // of all chunks, the one at hand; the span's end
+    const int end = span_begin(tab, P, blockIdx.x + 1);
+    const Sequence first_sq = sequence_of(tab, P, chunk);
     auto load = [&](int c, const Sequence& s, uint32_t bar) {
         const int tensors[4] = {TG, TK, TQ, TV};
         const uint32_t tiles[4] = {tg, tk, tq, tv};
@@ -493,7 +572,7 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
     initial_state(first_sq.state);
     if (chunk > first_sq.chunk0) {                                    // the spans before this one
 #pragma unroll 2
-        for (int j = span_of(P, first_sq.chunk0); j < static_cast<int>(blockIdx.x); ++j) {
+        for (int j = span_of(tab, P, first_sq.chunk0); j < static_cast<int>(blockIdx.x); ++j) {
             const float4* src = reinterpret_cast<const float4*>(P.agg + static_cast<size_t>(j) * 4096) + tid;
             const float f = ex2(__ldcg(P.agg_decay + static_cast<size_t>(j) * 64 + row));
 #pragma unroll
@@ -662,14 +741,14 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
 #pragma unroll
                     for (int e = 0; e < 8; ++e) dst[e] = make_float4(S[4 * e], S[4 * e + 1], S[4 * e + 2], S[4 * e + 3]);
                 }
-                if (more) initial_state(sequence_of(table, P, chunk + 1).state);
+                if (more) initial_state(sequence_of(tab, P, chunk + 1).state);
             }
         }
         // ---- outputs
         wait_bar(P, M.bar_o, p);
         tc_fence_after();
         if (more && elect_one()) {                                  // nothing reads the chunk's tiles any more: each warp asks for one
-            const Sequence next = last ? sequence_of(table, P, chunk + 1) : M.sq[p];
+            const Sequence next = last ? sequence_of(tab, P, chunk + 1) : M.sq[p];
             if (w == 0) {
                 M.sq[p ^ 1u] = next;
                 mbar_arrive_expect_tx(smem_u32(&M.full), 4 * kTileBytes);

@@ -118,6 +118,13 @@ int gla_b200_forward_static(const gla_b200_args* args, void* stream);
 int gla_b200_forward_packed(const gla_b200_args* args, const int32_t* offsets, int32_t n, void* stream);
 size_t gla_b200_packed_workspace_bytes(const int32_t* offsets, int32_t n, int32_t H);
 
+/* The same with the offsets in DEVICE memory (int32, or int64 with `wide` set), so that the launches do not wait for the host to read them: at most 96 sequences,
+ * T > 0.  Offsets that do not rise from 0 to args->T are found on the GPU, which then writes nothing; for the caller to find
+ * them too, `echo` (NULL, or 98 int32 of page-locked host memory with a 0 in the last) receives the n + 1 offsets and then a 1 in
+ * the last as the work starts.  The final states of empty sequences are left as they are. */
+int gla_b200_forward_packed_device(const gla_b200_args* args, const void* offsets, int32_t wide, int32_t n, int32_t* echo, void* stream);
+size_t gla_b200_packed_device_workspace_bytes(int32_t T, int32_t n, int32_t H);
+
 /* Replaces workspace_floats (gla_torch_ext.cu:24-33); bytes, not floats.  0 on bad shape. */
 size_t gla_b200_workspace_bytes(int32_t B, int32_t T, int32_t H, int32_t K, int32_t V);
 
