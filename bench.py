@@ -661,7 +661,7 @@ def run_ours(args, rank, local_rank, world):
             "e2e": {"value": world * B * T * e2e_steps / (e2e_ms * 1e-3), "unit": "tokens/s",
                     "h2d_bytes_per_step": in_bytes, "d2h_bytes_per_step": out_bytes, "steps": e2e_steps,
                     "pipelined": "3 streams, 2 staging sets", "output_checked": e2e_ok},
-            "gpu_launches": args.steps * inner, "clocks": clocks, "timed_region_s": total_ms * 1e-3, "ranks": ranks,
+            "gpu_launches": 2 * args.steps * inner, "clocks": clocks, "timed_region_s": total_ms * 1e-3, "ranks": ranks,
             "gpu": torch.cuda.get_device_name(dev), "host_cores": os.cpu_count(),
             "parity_check": parity, "backbone": backbone, "extra": extra,
         }
