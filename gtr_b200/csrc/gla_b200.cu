@@ -61,13 +61,15 @@ const void* state_kernel(bool logits) {
                   : reinterpret_cast<const void*>(&gla_state_kernel<false, Table>);
 }
 
-// The block kernel's: bit 1 raw-logit gates, bit 0 reversed scan.
+// The block kernel's: bit 2 fused epilogue, bit 1 raw-logit gates, bit 0 reversed scan.
 const void* block_kernel(int variant) {
     using gla::block::gla_block_kernel;
-    static const void* const table[4] = {
-        reinterpret_cast<const void*>(&gla_block_kernel<false, false>), reinterpret_cast<const void*>(&gla_block_kernel<false, true>),
-        reinterpret_cast<const void*>(&gla_block_kernel<true, false>), reinterpret_cast<const void*>(&gla_block_kernel<true, true>)};
-    return table[variant & 3];
+    static const void* const table[8] = {
+        reinterpret_cast<const void*>(&gla_block_kernel<false, false, false>), reinterpret_cast<const void*>(&gla_block_kernel<false, false, true>),
+        reinterpret_cast<const void*>(&gla_block_kernel<false, true, false>), reinterpret_cast<const void*>(&gla_block_kernel<false, true, true>),
+        reinterpret_cast<const void*>(&gla_block_kernel<true, false, false>), reinterpret_cast<const void*>(&gla_block_kernel<true, false, true>),
+        reinterpret_cast<const void*>(&gla_block_kernel<true, true, false>), reinterpret_cast<const void*>(&gla_block_kernel<true, true, true>)};
+    return table[variant & 7];
 }
 
 struct DeviceInfo {
@@ -98,13 +100,13 @@ int device_info(int dev, DeviceInfo* out) {
                 if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, gla::StateSmem::kBytes);
         }
         if (e != cudaSuccess) { note_cuda("cudaFuncSetAttribute", e); return GLA_B200_ERR_CUDA; }
-        for (int v = 0; v < 4 && e == cudaSuccess; ++v)
+        for (int v = 0; v < 8 && e == cudaSuccess; ++v)
             e = cudaFuncSetAttribute(block_kernel(v), cudaFuncAttributeMaxDynamicSharedMemorySize, gla::block::kSmemBytes);
         if (e != cudaSuccess) { note_cuda("cudaFuncSetAttribute", e); return GLA_B200_ERR_CUDA; }
         // The warpgroups of that kernel re-divide the registers the CTA was launched with (setmaxnreg); a group that
         // asks for more than the others release would wait for ever, so the budgets are checked against what this
         // build of the kernel really gets at launch.
-        for (int v = 0; v < 4; ++v) {
+        for (int v = 0; v < 8; ++v) {
             cudaFuncAttributes fa;
             e = cudaFuncGetAttributes(&fa, block_kernel(v));
             if (e != cudaSuccess) { note_cuda("cudaFuncGetAttributes", e); return GLA_B200_ERR_CUDA; }
@@ -276,7 +278,7 @@ int auto_chunks_per_segment(int NT, int nseq, int slots, size_t workspace_bytes)
 // the fused epilogue (which costs the output pass only).  In units of one chunk's output pass every CTA then works
 // (1 + pre) x the middle segments' length.  Returns that cost (plus one for the look-back), or a negative number when
 // the plan does not apply.
-constexpr double kPlanPrePassGated = 0.48;
+constexpr double kPlanPrePassPlain = 0.68, kPlanPrePassGated = 0.48;
 double staggered_plan(int NT, int nseq, int slots, size_t workspace_bytes, double pre, int* seg_start, int* ns_out) {
     const int r = nseq > 0 ? slots / nseq : 0;
     if (r < 2 || r + 1 > gla::block::kMaxPlanSegments || NT < kMinAutoCps * (r + 1)) return -1.0;
@@ -591,11 +593,22 @@ int launch_forward(bool gated, const gla::Maps& maps, gla::Params& P, const Tabl
     return launch_overlapped(out_kernel<Table>(gated, logits), P.spans, gla::kFwdThreads, gla::OutSmem::kBytes, args, stream);
 }
 
-// The fused operator on the block kernel (gla_block.cuh).
+// Which calls the block kernel serves better than the two kernels of gla_kernel.cuh.  Measured (us, block kernel / those two; row
+// scans), plain: 48 sequences x 100 chunks 65 / 71, 96 x 100 125 / 127-135, 192 x 64 118 / 151, 192 x 25 60 / 69, 192 x 128
+// 211 / 296, but 24 x 100 45 / 43 and 48 x 50 39 / 40: from 32 chunks per SM on.  The fused epilogue and raw-logit gates keep the
+// block kernel's teams busy for longer: 96 x 128 298 / 208, 384 x 128 756 / 664; it is ahead only where whole sequences just
+// about fill the SMs once and are long (144 x 128 286 / 299, 192 x 128 369 / 394).
+bool block_pays(bool gated, bool logits, int NT, int64_t nseq, int sms) {
+    if (!gated && !logits) return NT >= 24 && nseq * NT >= 32 * sms;
+    return NT >= 96 && 10 * nseq >= 9 * sms && 10 * nseq <= 14 * sms;
+}
+
+// The operator on the block kernel (gla_block.cuh).
 int forward_block(const gla_b200_args* a, const MapKey& key, int sms, cudaStream_t stream) {
     using namespace block_plan;
     const int NT = num_chunks(a->T), nseq = a->B * a->H;
     const int slots = sms;
+    const bool gated = a->out_gate != nullptr;
     int cps;
     int plan_start[gla::block::kMaxPlanSegments + 1] = {0}, plan_ns = 0;
     bool plan = false, relay = false;
@@ -606,7 +619,7 @@ int forward_block(const gla_b200_args* a, const MapKey& key, int sms, cudaStream
         const int ns_u = (NT + cps - 1) / cps;
         const long rounds = (static_cast<long>(nseq) * ns_u + slots - 1) / slots;
         // what the slowest item of the equal split costs, in the plan's units: every segment but the last pays the pre-pass
-        const double pre = kPlanPrePassGated;
+        const double pre = gated ? kPlanPrePassGated : kPlanPrePassPlain;
         const double uniform_cost = rounds * (cps * (1.0 + (ns_u > 1 ? pre : 0.0)) + (ns_u > 1 ? 1.0 : 0.0));
         const double plan_cost = staggered_plan(NT, nseq, slots, have, pre, plan_start, &plan_ns);
         plan = plan_cost > 0.0 && plan_cost < uniform_cost;
@@ -640,9 +653,11 @@ int forward_block(const gla_b200_args* a, const MapKey& key, int sms, cudaStream
     P.rms_eps = a->rms_eps;
     P.rms_w = static_cast<const __half*>(a->rms_weight);
     P.gate = static_cast<const __half*>(a->out_gate);
-    int64_t gs[3];
-    if (int rc = resolve_strides(a->gate_stride, a->T, a->H, gla::kD, gs)) return rc;
-    P.gate_sb = gs[0]; P.gate_st = gs[1]; P.gate_sh = gs[2];
+    if (gated) {
+        int64_t gs[3];
+        if (int rc = resolve_strides(a->gate_stride, a->T, a->H, gla::kD, gs)) return rc;
+        P.gate_sb = gs[0]; P.gate_st = gs[1]; P.gate_sh = gs[2];
+    }
     P.s0 = a->initial_state;
     P.sT = a->final_state;
     P.ctrl = reinterpret_cast<uint32_t*>(ws + L.ctrl);
@@ -656,7 +671,7 @@ int forward_block(const gla_b200_args* a, const MapKey& key, int sms, cudaStream
     void* clear[3] = {&P.ctrl, &P.flags, &words};
     if (int rc = launch_overlapped(reinterpret_cast<const void*>(&gla::clear_kernel), 1, 256, 0, clear, stream)) return rc;
     void* args[2] = {&maps, &P};
-    return launch_overlapped(block_kernel((P.inv_norm > 0.f ? 2 : 0) | (P.rev ? 1 : 0)), std::min(P.num_items, slots), gla::block::kThreads,
+    return launch_overlapped(block_kernel((gated ? 4 : 0) | (P.inv_norm > 0.f ? 2 : 0) | (P.rev ? 1 : 0)), std::min(P.num_items, slots), gla::block::kThreads,
                              gla::block::kSmemBytes, args, stream);
 }
 
@@ -771,17 +786,20 @@ static int forward(const gla_b200_args* a, bool block, void* stream_v) {
     rc = device_info(dev, &di);
     if (rc != GLA_B200_OK) return rc;
     const bool col = a->direction >= 2;
+    const int nseq = a->B * a->H;
     key.B = a->B; key.T = a->T; key.H = a->H; key.K = a->K;
     key.col = col ? 1 : 0;
     key.Hc = col ? gh : a->T;
     key.Wc = col ? gw : 1;
     key.dev = dev;
-    if (block) return forward_block(a, key, di.sms, static_cast<cudaStream_t>(stream_v));
+    if (block || (a->segments == 0 && block_pays(gated, a->gk_normalizer > 0.f, num_chunks(a->T), nseq, di.sms))) {
+        rc = forward_block(a, key, di.sms, static_cast<cudaStream_t>(stream_v));
+        if (block || rc != GLA_B200_ERR_WORKSPACE) return rc;
+    }
     int64_t o_stride[3];
     memcpy(o_stride, key.stride[gla::TO], sizeof(o_stride));
 
     const int NT = num_chunks(a->T);
-    const int nseq = a->B * a->H;
     const int64_t chunks = static_cast<int64_t>(nseq) * NT;
     if (chunks > 0x3fffffff) return GLA_B200_ERR_SHAPE;
     Split split;

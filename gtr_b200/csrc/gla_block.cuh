@@ -1,6 +1,8 @@
-// The fused operator (RMSNorm * w * silu(gate) epilogue) as one persistent CTA of specialised warpgroups per SM.
+// The operator as one persistent CTA of specialised warpgroups per SM.  It reads a sequence about once and a half where the two kernels of
+// gla_kernel.cuh read k, g and v twice, and needs about as many sequences as SMs, or long ones, for that to pay: the host sends
+// it the calls of that kind (block_pays()), whatever the backbone's blocks call, and nothing else.
 //
-// The backbone's blocks run on this kernel, everything else on gla_kernel.cuh.  The two compute the same sums with fp16 operands
+// The backbone's blocks always run on this kernel.  The two compute the same sums with fp16 operands
 // rounded at different references; outputs differ by 2e-4, as both do from exact arithmetic by 5e-4.  In a chain of blocks every
 // stage rounds to fp16, and a difference of any size at one stage becomes one of half units in the last place at the next:
 // twelve blocks end 0.6 to 1.8 percent apart (measured over 40 models and image sizes with random weights).  A network's results
@@ -545,9 +547,9 @@ template <int N> __device__ __forceinline__ void reg_budget() {
     else if constexpr (N < kLaunchRegs) reg_dealloc<N>();
 }
 
-// One instantiation per combination of raw-logit gates and scan sense: each holds only the code of its
+// One instantiation per combination of fused epilogue, raw-logit gates and scan sense: each holds only the code of its
 // own case, which keeps the instruction working set of the concurrently running roles small.
-template <bool kLogits, bool kRev>
+template <bool kGated, bool kLogits, bool kRev>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm)
 gla_block_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Params P) {
     extern __shared__ uint8_t smem_raw[];
@@ -999,7 +1001,7 @@ gla_block_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Para
                     // ---- scores: TMEM -> causal mask -> fp16 tile over the gate tile
                     // fused epilogue: this thread's half row of the chunk's output gate is asked for now, into L2
                     const uint4* gp = nullptr;
-                    {
+                    if (kGated) {
                         const int p0 = (it.first_chunk + i) * kChunk;
                         const int u = (rev ? (P.T - p0 - kChunk) : p0) + static_cast<int>(rho);   // position along the scan
                         if (u >= 0 && u < P.T) {
@@ -1047,7 +1049,12 @@ gla_block_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Para
                     tc_fence_after();
                     tmem_half_row(tmem, tw, kTmT + 64u * team, x);
                     tc_fence_before();
-                    {
+                    if (!kGated) {
+                        if (P.o_mul != 1.f) {         // scale not folded into q and k (zero, negative or not finite)
+#pragma unroll
+                            for (int e = 0; e < 32; ++e) x[e] *= P.o_mul;
+                        }
+                    } else {
                         // y = o * rsqrt(mean(o^2) + eps) * w * silu(gate): the two lanes of a row share its sum of squares
                         float s4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
