@@ -271,7 +271,7 @@ int auto_chunks_per_segment(int NT, int nseq, int slots, size_t workspace_bytes)
     return best_cps;
 }
 
-// Staggered plan for r = slots / nseq CTAs per sequence, 2 <= r < kMaxPlanSegments (gla::block::Params::plan): segment 0 of
+// Staggered plan for r CTAs per sequence (slots / nseq of them, unless fewer are wanted), 2 <= r < kMaxPlanSegments (gla::block::Params::plan): segment 0 of
 // `pre` x the length of the others, r equal ones after it.  `pre` is what a pre-pass chunk costs next to an output-pass
 // chunk while both kinds run side by side; measured on 100 chunks with three CTAs per sequence, the fastest splits are
 // 18 + 28 + 27 + 27 for the plain operator (and with raw gate logits, which cost both passes) and 14 + 29 + 29 + 28 with
@@ -279,8 +279,7 @@ int auto_chunks_per_segment(int NT, int nseq, int slots, size_t workspace_bytes)
 // (1 + pre) x the middle segments' length.  Returns that cost (plus one for the look-back), or a negative number when
 // the plan does not apply.
 constexpr double kPlanPrePassPlain = 0.68, kPlanPrePassGated = 0.48;
-double staggered_plan(int NT, int nseq, int slots, size_t workspace_bytes, double pre, int* seg_start, int* ns_out) {
-    const int r = nseq > 0 ? slots / nseq : 0;
+double staggered_plan(int NT, int nseq, int r, size_t workspace_bytes, double pre, int* seg_start, int* ns_out) {
     if (r < 2 || r + 1 > gla::block::kMaxPlanSegments || NT < kMinAutoCps * (r + 1)) return -1.0;
     if (ws_layout(static_cast<size_t>(nseq), static_cast<size_t>(r + 1)).total > workspace_bytes) return -1.0;
     const double mid = NT / (r + pre);
@@ -603,25 +602,40 @@ bool block_pays(bool gated, bool logits, int NT, int64_t nseq, int sms) {
     return NT >= 96 && 10 * nseq >= 9 * sms && 10 * nseq <= 14 * sms;
 }
 
-// The operator on the block kernel (gla_block.cuh).
-int forward_block(const gla_b200_args* a, const MapKey& key, int sms, cudaStream_t stream) {
+// Whether a call's final states are written over its initial states.
+bool states_overlap(const gla_b200_args* a, size_t bytes) {
+    const uintptr_t x = reinterpret_cast<uintptr_t>(a->initial_state), y = reinterpret_cast<uintptr_t>(a->final_state);
+    return x && y && x < y + bytes && y < x + bytes;
+}
+
+// The operator on the block kernel (gla_block.cuh).  in_place: the final states replace the initial ones, so that a sequence's last
+// segment must not finish before its first has read its state for good.  In the staggered and relay plans the first
+// segment reads it once, before it publishes what all others wait for; with equal segments and pre-passes it reads it twice.
+int forward_block(const gla_b200_args* a, const MapKey& key, int sms, bool in_place, cudaStream_t stream) {
     using namespace block_plan;
     const int NT = num_chunks(a->T), nseq = a->B * a->H;
     const int slots = sms;
     const bool gated = a->out_gate != nullptr;
+    const size_t have = a->workspace ? a->workspace_bytes : 0;
+    const double pre = gated ? kPlanPrePassGated : kPlanPrePassPlain;
     int cps;
     int plan_start[gla::block::kMaxPlanSegments + 1] = {0}, plan_ns = 0;
     bool plan = false, relay = false;
-    if (a->segments > 0) cps = a->segments;
+    if (in_place) {
+        const int r = std::min({slots / nseq, gla::block::kMaxPlanSegments - 1, NT / kMinAutoCps - 1});
+        plan = staggered_plan(NT, nseq, r, have, pre, plan_start, &plan_ns) > 0.0;
+        double relay_cost = 0.0;
+        const int ns_r = !plan && nseq >= slots ? relay_segments(NT, nseq, slots, have, &relay_cost) : 1;
+        relay = ns_r > 1;
+        cps = (NT + ns_r - 1) / ns_r;
+    } else if (a->segments > 0) cps = a->segments;
     else {
-        const size_t have = a->workspace ? a->workspace_bytes : 0;
         cps = auto_chunks_per_segment(NT, nseq, slots, have);
         const int ns_u = (NT + cps - 1) / cps;
         const long rounds = (static_cast<long>(nseq) * ns_u + slots - 1) / slots;
         // what the slowest item of the equal split costs, in the plan's units: every segment but the last pays the pre-pass
-        const double pre = gated ? kPlanPrePassGated : kPlanPrePassPlain;
         const double uniform_cost = rounds * (cps * (1.0 + (ns_u > 1 ? pre : 0.0)) + (ns_u > 1 ? 1.0 : 0.0));
-        const double plan_cost = staggered_plan(NT, nseq, slots, have, pre, plan_start, &plan_ns);
+        const double plan_cost = staggered_plan(NT, nseq, slots / nseq, have, pre, plan_start, &plan_ns);
         plan = plan_cost > 0.0 && plan_cost < uniform_cost;
         if (!plan && 2 * nseq > slots) {
             double relay_cost = 0.0;
@@ -792,9 +806,12 @@ static int forward(const gla_b200_args* a, bool block, void* stream_v) {
     key.Hc = col ? gh : a->T;
     key.Wc = col ? gw : 1;
     key.dev = dev;
-    if (block || (a->segments == 0 && block_pays(gated, a->gk_normalizer > 0.f, num_chunks(a->T), nseq, di.sms))) {
-        rc = forward_block(a, key, di.sms, static_cast<cudaStream_t>(stream_v));
-        if (block || rc != GLA_B200_ERR_WORKSPACE) return rc;
+    // The output kernel's blocks read their sequences' initial states at different times, some when others have left a final
+    // state behind; the step kernel holds a state from its load to its store.
+    const bool in_place = states_overlap(a, static_cast<size_t>(nseq) * a->K * gla::kD * sizeof(float)) && !step_serves(a->T, gated, a->segments);
+    if (block || in_place || (a->segments == 0 && block_pays(gated, a->gk_normalizer > 0.f, num_chunks(a->T), nseq, di.sms))) {
+        rc = forward_block(a, key, di.sms, in_place, static_cast<cudaStream_t>(stream_v));
+        if (block || in_place || rc != GLA_B200_ERR_WORKSPACE) return rc;
     }
     int64_t o_stride[3];
     memcpy(o_stride, key.stride[gla::TO], sizeof(o_stride));
@@ -880,6 +897,7 @@ static int packed_arguments(const gla_b200_args* a, int32_t n) {
     if ((a->K != 32 && a->K != gla::kD) || a->V != gla::kD || a->B != 1 || a->T < 0 || a->H <= 0 || n < 0) return GLA_B200_ERR_SHAPE;
     if (a->direction != 0 || a->out_gate || a->rms_weight || a->segments != 0) return GLA_B200_ERR_ARG;
     if (a->scale != a->scale || a->gk_normalizer < 0.f) return GLA_B200_ERR_ARG;
+    if (states_overlap(a, static_cast<size_t>(n) * a->H * a->K * gla::kD * sizeof(float))) return GLA_B200_ERR_ARG;
     if ((a->initial_state && !aligned16(a->initial_state)) || (a->final_state && !aligned16(a->final_state))) return GLA_B200_ERR_ALIGN;
     return GLA_B200_OK;
 }

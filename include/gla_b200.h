@@ -67,7 +67,8 @@ typedef struct gla_b200_args {
      * gla_torch_ext.cu:92-154); both NULL for the plain operator */
     const void* out_gate;
     const void* rms_weight;          /* fp16 [V] */
-    /* optional fp32 [B,H,K,V] states (FLA call signature, vit_adapter.py:566-568) */
+    /* optional fp32 [B,H,K,V] states (FLA call signature, vit_adapter.py:566-568); both may be the same array, which is then
+     * updated in place (packed sequences excepted) */
     const float* initial_state;
     float* final_state;
     /* caller-owned scratch, >= gla_b200_workspace_bytes(B,T,H,K,V), 256-byte aligned */
@@ -113,8 +114,8 @@ int gla_b200_forward_static(const gla_b200_args* args, void* stream);
 
 /* The operator on n sequences of different lengths packed back to back in one row (the cu_seqlens convention of the FLA call
  * the reference block makes, vit_adapter.py:448-451,566-568): args->B = 1, args->T their total length, `offsets` their n + 1
- * cumulative offsets in HOST memory, states [n,H,K,V].  Forward row scan, plain operator, automatic decomposition.  One launch
- * for up to 96 sequences. */
+ * cumulative offsets in HOST memory, states [n,H,K,V], the final ones not over the initial ones.  Forward row scan, plain operator,
+ * automatic decomposition.  One launch for up to 96 sequences. */
 int gla_b200_forward_packed(const gla_b200_args* args, const int32_t* offsets, int32_t n, void* stream);
 size_t gla_b200_packed_workspace_bytes(const int32_t* offsets, int32_t n, int32_t H);
 
