@@ -602,9 +602,9 @@ bool block_pays(bool gated, bool logits, int NT, int64_t nseq, int sms) {
     return NT >= 96 && 10 * nseq >= 9 * sms && 10 * nseq <= 14 * sms;
 }
 
-// Whether a call's final states are written over its initial states.
-bool states_overlap(const gla_b200_args* a, size_t bytes) {
-    const uintptr_t x = reinterpret_cast<uintptr_t>(a->initial_state), y = reinterpret_cast<uintptr_t>(a->final_state);
+// Whether states are written over others that the call reads.
+bool overlap(const float* in, const float* out, size_t bytes) {
+    const uintptr_t x = reinterpret_cast<uintptr_t>(in), y = reinterpret_cast<uintptr_t>(out);
     return x && y && x < y + bytes && y < x + bytes;
 }
 
@@ -808,7 +808,7 @@ static int forward(const gla_b200_args* a, bool block, void* stream_v) {
     key.dev = dev;
     // The output kernel's blocks read their sequences' initial states at different times, some when others have left a final
     // state behind; the step kernel holds a state from its load to its store.
-    const bool in_place = states_overlap(a, static_cast<size_t>(nseq) * a->K * gla::kD * sizeof(float)) && !step_serves(a->T, gated, a->segments);
+    const bool in_place = overlap(a->initial_state, a->final_state, static_cast<size_t>(nseq) * a->K * gla::kD * sizeof(float)) && !step_serves(a->T, gated, a->segments);
     if (block || in_place || (a->segments == 0 && block_pays(gated, a->gk_normalizer > 0.f, num_chunks(a->T), nseq, di.sms))) {
         rc = forward_block(a, key, di.sms, in_place, static_cast<cudaStream_t>(stream_v));
         if (block || in_place || rc != GLA_B200_ERR_WORKSPACE) return rc;
@@ -897,7 +897,7 @@ static int packed_arguments(const gla_b200_args* a, int32_t n) {
     if ((a->K != 32 && a->K != gla::kD) || a->V != gla::kD || a->B != 1 || a->T < 0 || a->H <= 0 || n < 0) return GLA_B200_ERR_SHAPE;
     if (a->direction != 0 || a->out_gate || a->rms_weight || a->segments != 0) return GLA_B200_ERR_ARG;
     if (a->scale != a->scale || a->gk_normalizer < 0.f) return GLA_B200_ERR_ARG;
-    if (states_overlap(a, static_cast<size_t>(n) * a->H * a->K * gla::kD * sizeof(float))) return GLA_B200_ERR_ARG;
+    if (overlap(a->initial_state, a->final_state, static_cast<size_t>(n) * a->H * a->K * gla::kD * sizeof(float))) return GLA_B200_ERR_ARG;
     if ((a->initial_state && !aligned16(a->initial_state)) || (a->final_state && !aligned16(a->final_state))) return GLA_B200_ERR_ALIGN;
     return GLA_B200_OK;
 }
@@ -1143,6 +1143,11 @@ int gla_b200_backward_scan(const gla_b200_bwd_args* a, const gla_b200_bwd_scan* 
     const int NT = num_chunks(a->T);
     gla::BwdParams P{};
     P.nseg = bwd_segments(nseq, NT, &P.cps);
+    const size_t state_bytes = static_cast<size_t>(nseq) * a->K * gla::kD * sizeof(float);
+    if (overlap(a->initial_state, a->d_initial_state, state_bytes) || overlap(a->d_final_state, a->d_initial_state, state_bytes)) {
+        P.nseg = 1;                                   // every segment reads those states, the first one replaces them: one block for all
+        P.cps = NT;
+    }
     const BwdLayout L = bwd_layout(nseq, NT, P.nseg);
     if (!a->workspace || a->workspace_bytes < L.total) return GLA_B200_ERR_WORKSPACE;
     if (nseq * P.nseg > 0x7fffffffLL) return GLA_B200_ERR_SHAPE;

@@ -178,7 +178,7 @@ typedef struct gla_b200_bwd_args {
     float* dg;
     const float* initial_state;      /* the forward call's initial state, or NULL */
     const float* d_final_state;      /* gradient flowing into the forward call's final state, or NULL */
-    float* d_initial_state;          /* out, or NULL */
+    float* d_initial_state;          /* out, or NULL; may be either of the arrays above */
     void* workspace;                 /* >= gla_b200_backward_workspace_bytes(B,T,H,K,V), 256-byte aligned */
     size_t workspace_bytes;
     int32_t B, T, H, K, V;

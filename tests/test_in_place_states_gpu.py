@@ -1,5 +1,5 @@
-"""States updated in place: `final_state` over `initial_state`, in every decomposition such a call can take, against the same call
-with arrays of their own."""
+"""States updated in place: `final_state` over `initial_state`, in every decomposition such a call can take, and the gradient's over
+either state it reads, against the same call with arrays of their own."""
 import ctypes
 
 import pytest
@@ -63,3 +63,39 @@ def test_packed_sequences_refuse_it():
     a.B, a.T, a.H, a.K, a.V, a.scale = 1, 64, 1, 64, 64, 0.125
     offsets = (ctypes.c_int32 * 2)(0, 64)
     assert _lib.lib().gla_b200_forward_packed(ctypes.byref(a), offsets, 1, None) == -9
+
+
+def _gradient(q, k, v, g, do, s0, d_final, d_initial):
+    """One gla_b200_backward call on the given state arrays; returns dq and dg."""
+    import gtr_b200 as G
+    from gtr_b200 import _lib, ops
+    B, T, H, K = q.shape
+    dq, dk, dv, dg = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v), torch.empty(q.shape, device="cuda")
+    ws = torch.empty(ops.backward_workspace_bytes(B, T, H, K), dtype=torch.uint8, device="cuda")
+    a = _lib.BwdArgs()
+    a.q, a.k, a.v, a.g, a.d_o = (x.data_ptr() for x in (q, k, v, g, do))
+    a.dq, a.dk, a.dv, a.dg = (x.data_ptr() for x in (dq, dk, dv, dg))
+    a.initial_state, a.d_final_state, a.d_initial_state = s0.data_ptr(), d_final.data_ptr(), d_initial.data_ptr()
+    a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
+    a.B, a.T, a.H, a.K, a.V, a.scale = B, T, H, K, 64, K ** -0.5
+    _lib.check(_lib.lib().gla_b200_backward(ctypes.byref(a), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    G.check_status(ws)
+    return dq.float(), dg
+
+
+@pytest.mark.parametrize("B,H,T,repeats", [(25, 12, 6400, 20), (1, 6, 1600, 5)])     # three segments in four rounds of blocks; many in one
+@pytest.mark.parametrize("over", ["initial_state", "d_final_state"])
+def test_gradient_in_place(B, H, T, repeats, over):
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    draw = lambda *shape: torch.randn(*shape, generator=gen, device="cuda")
+    q, k, v, do = (draw(B, T, H, 64).mul(0.3).half() for _ in range(4))
+    g = torch.nn.functional.logsigmoid(draw(B, T, H, 64)).div(16).half()
+    s0, d_final = draw(B, H, 64, 64) * 10, draw(B, H, 64, 64) * 10
+    d_initial = torch.empty_like(s0)
+    want = _gradient(q, k, v, g, do, s0, d_final, d_initial)
+    for _ in range(repeats):
+        state = (s0 if over == "initial_state" else d_final).clone()
+        got = _gradient(q, k, v, g, do, state if over == "initial_state" else s0, state if over == "d_final_state" else d_final, state)
+        # dq in fp16 (the fp32 sums before it in another order round a few values the other way), the others in fp32
+        for x, y, most in ((want[0], got[0], 5e-5), (want[1], got[1], 1e-5), (d_initial, state, 1e-5)):
+            assert float((x - y).norm() / x.norm()) <= most
