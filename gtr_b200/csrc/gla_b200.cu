@@ -535,8 +535,8 @@ __global__ void __launch_bounds__(kProbeThreads) stream_probe_kernel(const __gri
 // up with cudaGetSymbolAddress, once per device and with that device current.  That happens in the
 // first call on a device: make that call before any stream capture.
 // All calls share the one array per device; it keeps the previous call's contents.  The words that
-// must start at zero (ticket, status, flags) are cleared on the stream at the start of every call;
-// everything else is written before it is read.  Two calls that overlap on the same GPU (different
+// must start at zero (status; the block kernel's ticket and flags) are cleared on the stream before a kernel
+// looks at them; everything else is written before it is read.  Two calls that overlap on the same GPU (different
 // streams, or graph branches) would race on the array: serialise them.
 static __device__ __align__(256) unsigned char g_static_scratch[GLA_B200_STATIC_SCRATCH_BYTES];
 
@@ -579,12 +579,22 @@ void fill_params(const gla_b200_args* a, const int64_t* o_stride, uint8_t* ws, c
 
 
 constexpr int64_t kL2Keep = 120ll << 20;
-// The spans' increments (where spans end inside sequences), then the outputs.
+// Clears the control words, and `words` words of flags, for the launches that follow.
+int launch_clear(uint32_t* ctrl, uint32_t* flags, int words, unsigned threads, cudaStream_t stream) {
+    return launch_simple(&gla::clear_kernel, 1, threads, 0, stream, ctrl, flags, words);
+}
+
+// The spans' increments (where spans end inside sequences), then the outputs.  A kernel whose waits look at the status word must find it
+// cleared: the state kernel, whose waits do not, clears it for the output kernel; an output kernel on its own has it
+// cleared by a launch of its own (a block that cleared it itself could come after another one's report).  `first`: of the call.
 template <class Table>
-int launch_forward(bool gated, const gla::Maps& maps, gla::Params& P, const Table& table, cudaStream_t stream) {
+int launch_forward(bool gated, const gla::Maps& maps, gla::Params& P, const Table& table, bool first, cudaStream_t stream) {
     const bool logits = P.inv_norm > 0.f;
     const int states = P.per > 0 ? P.spans / P.per * (P.per - 1) : P.spans - 1;
     P.alone = states == 0 ? 1 : 0;
+    P.clear = first ? 1 : 0;
+    if (P.alone && first)
+        if (int rc = launch_clear(P.ctrl, nullptr, 0, 32, stream)) return rc;
     P.keep = static_cast<int64_t>(P.chunks) * (4 * P.K + 128) * gla::kChunk <= kL2Keep ? 1 : 0;
     void* args[3] = {const_cast<gla::Maps*>(&maps), &P, const_cast<Table*>(&table)};
     if (states > 0)
@@ -681,9 +691,8 @@ int forward_block(const gla_b200_args* a, const MapKey& key, int sms, bool in_pl
     P.wait_limit_us = a->wait_limit ? a->wait_limit : 2000000u;
 
 
-    int words = static_cast<int>((L.clear_bytes - L.flags) / sizeof(uint32_t));
-    void* clear[3] = {&P.ctrl, &P.flags, &words};
-    if (int rc = launch_overlapped(reinterpret_cast<const void*>(&gla::clear_kernel), 1, 256, 0, clear, stream)) return rc;
+    const int words = static_cast<int>((L.clear_bytes - L.flags) / sizeof(uint32_t));
+    if (int rc = launch_clear(P.ctrl, P.flags, words, 256, stream)) return rc;
     void* args[2] = {&maps, &P};
     return launch_overlapped(block_kernel((gated ? 4 : 0) | (P.inv_norm > 0.f ? 2 : 0) | (P.rev ? 1 : 0)), std::min(P.num_items, slots), gla::block::kThreads,
                              gla::block::kSmemBytes, args, stream);
@@ -871,7 +880,7 @@ static int forward(const gla_b200_args* a, bool block, void* stream_v) {
         if (rc != GLA_B200_OK) return rc;
         for (int i = 0; i < 3; ++i) P.gate_s[i] = gs[i];
     }
-    return launch_forward(gated, maps, P, gla::NoTable{}, static_cast<cudaStream_t>(stream_v));
+    return launch_forward(gated, maps, P, gla::NoTable{}, true, static_cast<cudaStream_t>(stream_v));
 }
 
 int gla_b200_forward(const gla_b200_args* a, void* stream) { return forward(a, false, stream); }
@@ -949,6 +958,7 @@ int gla_b200_forward_packed(const gla_b200_args* a, const int32_t* offsets, int3
     if (int rc = packed_maps(a, &maps, o_stride)) return rc;
     uint8_t* ws = static_cast<uint8_t*>(a->workspace);
     if (!ws || (reinterpret_cast<uintptr_t>(ws) & 255u)) return GLA_B200_ERR_WORKSPACE;
+    bool first = true;
     for (int at = 0; at < n; at += gla::kMaxPacked) {
         gla::PackedTable tab;
         gla::Params P;
@@ -964,7 +974,8 @@ int gla_b200_forward_packed(const gla_b200_args* a, const int32_t* offsets, int3
         fill_params(a, o_stride, ws, L, &P);
         P.s0 = a->initial_state ? a->initial_state + at * state_floats : nullptr;
         P.sT = a->final_state ? a->final_state + at * state_floats : nullptr;
-        if (int rc = launch_forward(false, maps, P, tab, stream)) return rc;
+        if (int rc = launch_forward(false, maps, P, tab, first, stream)) return rc;
+        first = false;
     }
     return GLA_B200_OK;
 }
@@ -1000,7 +1011,7 @@ int gla_b200_forward_packed_device(const gla_b200_args* a, const void* offsets, 
     fill_params(a, o_stride, ws, L, &P);
     P.s0 = a->initial_state;
     P.sT = a->final_state;
-    return launch_forward(false, maps, P, gla::DeviceTable{offsets, echo, n, wide != 0}, static_cast<cudaStream_t>(stream));
+    return launch_forward(false, maps, P, gla::DeviceTable{offsets, echo, n, wide != 0}, true, static_cast<cudaStream_t>(stream));
 }
 
 int gla_b200_stream_probe(const void* buf, int64_t rows, int32_t heads, int32_t ctas, int32_t tiles, int32_t chunks,

@@ -126,7 +126,7 @@ struct BwdStateSmem {
 };
 struct BwdStateMisc {
     uint64_t full[2], bar_x, bar_inc;
-    uint32_t tmem;
+    uint32_t tmem, gave_up;
     uint32_t top[2][8];               // per warp: largest |k|, |q|, as half2 bits
     alignas(16) float gl[2][64];      // log2 decay of the chunk per channel
 };
@@ -151,6 +151,7 @@ __global__ void __launch_bounds__(kComputeThreads, 2) gla_bwd_state_kernel(const
         mbar_init(smem_u32(&M.full[1]), 1);
         mbar_init(smem_u32(&M.bar_x), 1);
         mbar_init(smem_u32(&M.bar_inc), 1);
+        M.gave_up = 0u;
         fence_mbar_init();
     }
     if (w == 0) {
@@ -179,7 +180,7 @@ __global__ void __launch_bounds__(kComputeThreads, 2) gla_bwd_state_kernel(const
     };
     auto gate_sums = [&](int i) {          // of chunk i, as soon as it has landed
         const uint32_t tg = base + (i & 1) * BwdStateSmem::kStage + 2 * kTileBytes;
-        wait_bar(P, M.full[i & 1], (i >> 1) & 1);
+        wait_bar(P, M.full[i & 1], (i >> 1) & 1, M.gave_up);
         tc_fence_after();
         tile_mma<0, 1>(acc_slot(tmem, BWD_AFTER), after, tg, false);
         if (grad) tile_mma<0, 1>(acc_slot(tmem, BWD_UP_TO), up_to, tg, false);
@@ -203,7 +204,7 @@ __global__ void __launch_bounds__(kComputeThreads, 2) gla_bwd_state_kernel(const
         const uint32_t tk = base + st * BwdStateSmem::kStage, tv = tk + kTileBytes, tg = tv + kTileBytes, tq = tg + kTileBytes,
                        tdo = tq + kTileBytes;
         if (i == n - 1) pdl_release();
-        wait_bar(P, M.full[st], (i >> 1) & 1);
+        wait_bar(P, M.full[st], (i >> 1) & 1, M.gave_up);
         uint32_t k[8], q[8];
         row16(tk, row, u0, k);
         const uint32_t mk = __reduce_max_sync(0xffffffffu, __float_as_uint(bwd_half_max(bwd_max16(k))));
@@ -213,7 +214,7 @@ __global__ void __launch_bounds__(kComputeThreads, 2) gla_bwd_state_kernel(const
             mq = __reduce_max_sync(0xffffffffu, __float_as_uint(bwd_half_max(bwd_max16(q))));
         }
         if (l == 0) { M.top[0][w] = mk; M.top[1][w] = mq; }
-        wait_bar(P, M.bar_x, i & 1);
+        wait_bar(P, M.bar_x, i & 1, M.gave_up);
         tc_fence_after();
         float x[16], y[16];
         acc_read(tmem, BWD_AFTER, w, x);
@@ -251,7 +252,7 @@ __global__ void __launch_bounds__(kComputeThreads, 2) gla_bwd_state_kernel(const
         }
         const float gl = M.gl[st][row], decay = ex2(gl), ck = bwd_inverse(fk), cq = P.scale * bwd_inverse(fq) * ex2(total);
         total += gl;
-        wait_bar(P, M.bar_inc, i & 1);
+        wait_bar(P, M.bar_inc, i & 1, M.gave_up);
         tc_fence_after();
         if (w == 0 && elect_one()) {                                // this chunk's stage is free, and so are its gate sums
             if (i + 2 < n) load(i + 2);
@@ -289,6 +290,7 @@ __global__ void __launch_bounds__(kComputeThreads, 2) gla_bwd_state_kernel(const
     }
     tc_fence_before();
     __syncthreads();
+    if (tid == 0 && M.gave_up) P.chunk_decay[(cslot + first + n - 1) * 64] = __uint_as_float(kTimedOut);
     if (w == 0) tmem_dealloc(tmem, 128);
 }
 
@@ -619,6 +621,8 @@ __global__ void __launch_bounds__(kBwdChunkThreads, 2) gla_bwd_chunk_kernel(cons
             }
 #pragma unroll
             for (uint32_t e = 0; e < 4; ++e) st_shared_f4(s0_at + 16u * kComputeThreads * e, S0[4 * e], S0[4 * e + 1], S0[4 * e + 2], S0[4 * e + 3]);
+            // did a wait run out where the segment's states were made?
+            if (c0 == 0 && __float_as_uint(__ldcg(P.chunk_decay + (cslot + first + n - 1) * 64 + row)) == kTimedOut) report_timeout(P);
             float later = 0.f;
             if (P.dht != nullptr || seg + 1 < P.nseg) {                  // dS is not zero at the segment's end
                 float y[16];

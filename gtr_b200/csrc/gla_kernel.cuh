@@ -54,7 +54,8 @@ struct Params {
     // of them one chunk longer
     int chunks, spans, per, len_, longer;
     int keep;            // k, g and v fit the L2: what the state kernel reads is kept there for the output kernel
-    int alone;           // no state kernel runs before the output kernel (which then clears the status)
+    int alone;           // no state kernel runs before the output kernel
+    int clear;           // the state kernel clears the status (the call's first launch)
     // The output scale is folded into the exponents of the gate factors (q_exp = log2(scale) - 4, half of it on q and half
     // on k, o_mul = 16) when it is positive and finite; otherwise the epilogue multiplies (q_exp = -4, o_mul = 16 scale).
     float q_exp, q_mul, o_mul;
@@ -282,7 +283,7 @@ struct StateSmem {
 };
 struct StateMisc {
     uint64_t full[2], full_v, bar_x, bar_inc;
-    uint32_t tmem;
+    uint32_t tmem, gave_up;
     Sequence sq;
     alignas(16) float gl[2][64];      // log2 decay of the chunk per channel
 };
@@ -297,7 +298,13 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_state_kernel(const __grid_
     const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
     // per sequence, the last span needs no increment and gets no CTA; in the flat split it is found here
     const int span = P.per > 0 ? blockIdx.x + blockIdx.x / (P.per - 1) : blockIdx.x;
-    if (std::is_same<Table, DeviceTable>::value) pdl_wait();
+    auto clear_status = [&] {
+        if (P.clear && blockIdx.x == 0 && tid < 2) P.ctrl[tid] = 0u;
+    };
+    if (std::is_same<Table, DeviceTable>::value) {
+        pdl_wait();
+        clear_status();
+    }
     const auto& tab = table_here(table, P, true);
     if (nothing_in(tab)) return;
     const int end = span_begin(tab, P, span + 1);
@@ -328,9 +335,10 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_state_kernel(const __grid_
         fence_mbar_init();
         fence_proxy_async_smem();
         M.sq = sq;
+        M.gave_up = 0u;
     }
     pdl_wait();
-    if (blockIdx.x == 0 && tid < 2) P.ctrl[tid] = 0u;
+    clear_status();
     if (n == 0) { pdl_release(); return; }
     if (tid == 0) {                                                  // the first tiles come in while the rest is set up
         load_kg(0);
@@ -356,7 +364,7 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_state_kernel(const __grid_
         const int st = i & 1;
         if (i == n - 1) pdl_release();                              // the output kernel's blocks move in as these leave
         const uint32_t tk = base + StateSmem::kK + st * kTileBytes, tg = base + StateSmem::kG + st * kTileBytes;
-        wait_bar(P, M.full[st], (i >> 1) & 1);
+        wait_bar(P, M.full[st], (i >> 1) & 1, M.gave_up);
         if (kLogits) {
             const int p = (c_last - i) * kChunk + (rev ? 63 - static_cast<int>(row) : static_cast<int>(row));
             logits_to_log_gates(at, StateSmem::kG + st * kTileBytes, P.inv_norm, p < T);
@@ -370,7 +378,7 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_state_kernel(const __grid_
         }
         uint32_t k[16];
         at.get(StateSmem::kK + st * kTileBytes, k);
-        wait_bar(P, M.bar_x, st);
+        wait_bar(P, M.bar_x, st, M.gave_up);
         tc_fence_after();
         float x[32];
         half_row_read(tmem, 0, w, x);
@@ -395,7 +403,7 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_state_kernel(const __grid_
         tc_fence_before();
         __syncthreads();
         if (w == 0) {
-            wait_bar(P, M.full_v, st);
+            wait_bar(P, M.full_v, st, M.gave_up);
             if (elect_one()) {
                 tc_fence_after();
                 tile_mma<1, 1>(acc_slot(tmem, 1), tk, tv, false);
@@ -405,7 +413,7 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_state_kernel(const __grid_
         }
         const float after = ex2(total);                              // decay of the chunks after this one
         total += M.gl[st][row];
-        wait_bar(P, M.bar_inc, st);
+        wait_bar(P, M.bar_inc, st, M.gave_up);
         tc_fence_after();
         if (w == 0 && i + 1 < n && elect_one()) load_v(i + 1);
         half_row_read(tmem, 1, w, x);
@@ -421,6 +429,7 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_state_kernel(const __grid_
     if (c0 == 0) P.agg_decay[static_cast<size_t>(span) * 64 + row] = total;
     tc_fence_before();
     __syncthreads();
+    if (tid == 0 && M.gave_up) P.agg_decay[static_cast<size_t>(span) * 64] = __uint_as_float(kTimedOut);
     if (w == 1) tmem_dealloc(tmem, 64);
 }
 
@@ -543,7 +552,6 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
     pdl_wait();
     if (!P.alone) pdl_release();
     if (tid == 0) load(chunk, M.sq[0], smem_u32(&M.full));           // the first tiles come in while the rest is set up
-    if (P.alone && blockIdx.x == 0 && tid < 2) P.ctrl[tid] = 0u;
     if (w == 1) {
         tmem_alloc(smem_u32(&M.tmem), 128);
         tmem_relinquish();
@@ -799,7 +807,10 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
         }
         tc_fence_before();
         ++chunk;
-        if (!more) break;
+        if (!more) {                                                // did a wait run out where this span's increment was made?
+            if (!last && tid == 0 && __float_as_uint(__ldcg(P.agg_decay + static_cast<size_t>(blockIdx.x) * 64)) == kTimedOut) report_timeout(P);
+            break;
+        }
     }
     tc_fence_before();
     __syncthreads();

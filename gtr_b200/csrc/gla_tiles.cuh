@@ -30,10 +30,10 @@ struct Maps {
 
 enum { WHERE_MBAR = 1, WHERE_LOOKBACK = 2 };
 
-// Bounded wait.  On expiry, or once any CTA of the launch has given up, the status word ctrl[1] is set and the wait returns, so
-// that all warps keep following the protocol and the kernel drains and exits; its result is then undefined and the status says so.
-template <class P_t>
-__device__ __forceinline__ void wait_bar(const P_t& P, uint64_t& bar, uint32_t parity) {
+// Bounded waits.  On expiry, or once another wait of its group has given up, a wait returns without its barrier, so that all warps keep
+// following the protocol and the kernel drains and exits; its result is then undefined and the status word ctrl[1] says so.
+template <class Gave, class Give>
+__device__ __forceinline__ void bounded_wait(uint64_t& bar, uint32_t parity, uint32_t limit_us, Gave gave_up, Give give_up) {
     const uint32_t b = smem_u32(&bar);
     for (int n = 0; n < 8; ++n)
         if (mbar_try_wait(b, parity)) return;
@@ -41,13 +41,27 @@ __device__ __forceinline__ void wait_bar(const P_t& P, uint64_t& bar, uint32_t p
     for (uint32_t n = 1;; ++n) {
         if (mbar_try_wait(b, parity)) return;
         if ((n & 63u) != 0u) continue;
-        if (*reinterpret_cast<volatile uint32_t*>(P.ctrl + 1) != 0u) return;
-        if (globaltimer_1024ns() - t0 > P.wait_limit_us) {
-            atomicCAS(P.ctrl + 1, 0u, static_cast<uint32_t>(WHERE_MBAR));
-            return;
-        }
+        if (gave_up()) return;
+        if (globaltimer_1024ns() - t0 > limit_us) { give_up(); return; }
     }
 }
+template <class P_t>
+__device__ __forceinline__ void report_timeout(const P_t& P) { atomicCAS(P.ctrl + 1, 0u, static_cast<uint32_t>(WHERE_MBAR)); }
+
+// For a kernel that starts with the status word cleared, by the kernel before it in the stream: its group is the launch.
+template <class P_t>
+__device__ __forceinline__ void wait_bar(const P_t& P, uint64_t& bar, uint32_t parity) {
+    bounded_wait(bar, parity, P.wait_limit_us, [&] { return *reinterpret_cast<volatile uint32_t*>(P.ctrl + 1) != 0u; }, [&] { report_timeout(P); });
+}
+// For the first kernel of a call, whose block 0 clears the word (what lies there is an earlier call's, or never was written): its
+// group is the block, by a flag in shared memory.  Such a kernel leaves kTimedOut in place of a decay, which the second one reports;
+// no arithmetic makes a NaN of these bits.
+template <class P_t>
+__device__ __forceinline__ void wait_bar(const P_t& P, uint64_t& bar, uint32_t parity, uint32_t& flag) {
+    volatile uint32_t* f = &flag;
+    bounded_wait(bar, parity, P.wait_limit_us, [&] { return *f != 0u; }, [&] { *f = 1u; });
+}
+constexpr uint32_t kTimedOut = 0x7fc0deadu;
 
 // Enumerates the TMA boxes that cover one chunk of the scan: f(box_id, r, c, smem_row) with (r, c) the row inside the
 // column and the column where the box starts.

@@ -1,0 +1,91 @@
+"""The status word when a call's scratch holds anything at all: what lies there decides no wait and reaches no report."""
+import ctypes
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+STREAM = lambda: ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+
+def _dirty(nbytes):
+    """0xFF throughout: flags, sums and a time-out of some earlier call."""
+    return torch.full((nbytes,), 0xFF, dtype=torch.uint8, device="cuda")
+
+
+def _inputs(B, T, H, K):
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    draw = lambda d: torch.randn(B, T, H, d, generator=gen, device="cuda")
+    q, k, v, do = (draw(d).mul(0.3).half() for d in (K, K, 64, 64))
+    return q, k, v, torch.nn.functional.logsigmoid(draw(K)).div(16).half(), do
+
+
+@pytest.mark.parametrize("B,H,T,K", [
+    (8, 12, 3200, 64),        # the two kernels, blocks in several waves
+    (3, 3, 1050, 32),
+    (64, 16, 64, 64),         # the output kernel on its own, blocks in two waves
+    (4, 12, 6400, 64),        # the persistent kernel
+    (2, 3, 20, 64),           # token by token
+])
+def test_forward(B, H, T, K):
+    import gtr_b200 as G
+    q, k, v, g, _ = _inputs(B, T, H, K)
+    clean = G.make_workspace(B, T, H, "cuda")
+    dirty = _dirty(clean.numel() * 4)
+    outs = []
+    for ws in (clean, dirty, dirty):
+        o = torch.full((B, T, H, 64), float("nan"), dtype=torch.float16, device="cuda")
+        G.chunk_gla_run(q, k, v, g, K ** -0.5, ws, o)
+        G.check_status(ws)
+        outs.append(o)
+    assert torch.isfinite(outs[0]).all() and torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+
+
+@pytest.mark.parametrize("B,H,T,K", [(8, 6, 1600, 64), (40, 8, 100, 32)])
+def test_gradient(B, H, T, K):
+    from gtr_b200 import _lib, ops
+    q, k, v, g, do = _inputs(B, T, H, K)
+    outs = []
+    for fill in (0, 0xFF, 0xFF):
+        ws = _dirty(ops.backward_workspace_bytes(B, T, H, K)).fill_(fill)
+        out = [torch.full_like(x, float("nan")) for x in (q, k, v)] + [torch.full(q.shape, float("nan"), device="cuda")]
+        a = _lib.BwdArgs()
+        a.q, a.k, a.v, a.g, a.d_o = (x.data_ptr() for x in (q, k, v, g, do))
+        a.dq, a.dk, a.dv, a.dg = (x.data_ptr() for x in out)
+        a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
+        a.B, a.T, a.H, a.K, a.V, a.scale = B, T, H, K, 64, K ** -0.5
+        _lib.check(_lib.lib().gla_b200_backward(ctypes.byref(a), STREAM()))
+        _lib.check(_lib.lib().gla_b200_check_status(ws.data_ptr(), STREAM()))
+        outs.append(out)
+    for x, y, z in zip(*outs):
+        assert torch.isfinite(x).all() and torch.equal(x, y) and torch.equal(x, z)
+
+
+@pytest.mark.parametrize("ends,device", [
+    ([0, 300, 1000], True),
+    ([0, 300, 200, 1000], True),                    # no good: found on the GPU, nothing is computed
+    ([0, 40], True), ([0, 41, 40], True),           # one span: the output kernel on its own
+    (list(range(0, 1010, 10)), False),              # 101 sequences: two groups of launches
+])
+def test_packed(ends, device):
+    from gtr_b200 import _lib
+    L = _lib.lib()
+    T, n = ends[-1], len(ends) - 1
+    good = all(b >= a for a, b in zip(ends, ends[1:]))
+    q, k, v, g, _ = _inputs(1, T, 1, 64)
+    outs = []
+    for fill in (0, 0xFF):
+        ws = _dirty(1 << 22).fill_(fill)
+        o = torch.zeros_like(v)
+        a = _lib.Args()
+        a.q, a.k, a.v, a.g, a.o = (x.data_ptr() for x in (q, k, v, g, o))
+        a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
+        a.B, a.T, a.H, a.K, a.V, a.scale = 1, T, 1, 64, 64, 0.125
+        if device:
+            offsets = torch.tensor(ends, dtype=torch.int32, device="cuda")
+            _lib.check(L.gla_b200_forward_packed_device(ctypes.byref(a), offsets.data_ptr(), 0, n, None, STREAM()))
+        else:
+            _lib.check(L.gla_b200_forward_packed(ctypes.byref(a), (ctypes.c_int32 * (n + 1))(*ends), n, STREAM()))
+        _lib.check(L.gla_b200_check_status(ws.data_ptr(), STREAM()))
+        outs.append(o)
+    assert torch.equal(*outs) and bool(outs[0].any()) == good
