@@ -1067,11 +1067,12 @@ int gla_b200_selftest_wait_timeout(void* workspace, size_t workspace_bytes, uint
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
     cudaError_t e = cudaMemsetAsync(workspace, 0, 512, stream);
     if (e != cudaSuccess) { note_cuda("cudaMemsetAsync", e); return GLA_B200_ERR_CUDA; }
-    gla::Params P;
+    gla::block::Params P;
     memset(&P, 0, sizeof(P));
     P.ctrl = static_cast<uint32_t*>(workspace);
+    P.flags = P.ctrl + 64;
     P.wait_limit_us = limit_us;
-    gla::wait_timeout_selftest_kernel<<<1, 32, 0, stream>>>(P);
+    gla::block::wait_timeout_selftest_kernel<<<1, 32, 0, stream>>>(P);
     e = cudaPeekAtLastError();
     if (e != cudaSuccess) { note_cuda("self-test launch", e); return GLA_B200_ERR_CUDA; }
     return GLA_B200_OK;

@@ -250,6 +250,23 @@ __device__ __forceinline__ void mbar_wait(const Ctx& c, uint64_t* bar, uint32_t 
     mbar_wait_slow(c, b, parity);
 }
 
+// Look-back: the flag of an earlier segment once it is set, or 0 when this or any other CTA has given up.
+__device__ __forceinline__ uint32_t wait_flag(const Ctx& c, const uint32_t* flag, uint64_t t0) {
+    uint32_t f = ld_acquire_gpu(flag);
+    for (uint32_t n = 1; f == 0u; ++n) {
+        if ((n & 15u) == 0u) {
+            if (c.misc->abort || ld_acquire_gpu(c.p->ctrl + 1) != 0u) break;
+            if (globaltimer_ns() - t0 > c.deadline_span_ns) {
+                raise_timeout(c, WHERE_LOOKBACK);
+                break;
+            }
+        }
+        __nanosleep(128);
+        f = ld_acquire_gpu(flag);
+    }
+    return f;
+}
+
 // Wait of a whole warp group: its first warp polls the mbarrier, the others sleep in the hardware barrier
 // `bar_id` (a warp parked in bar.sync issues nothing, a polling warp competes with the working ones).
 __device__ __forceinline__ void group_wait(const Ctx& c, uint64_t* bar, uint32_t parity, int group_warp, uint32_t bar_id,
@@ -708,18 +725,7 @@ gla_block_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Para
                         // their predecessors), the warp barrier of the shuffle passes the acquired view on
                         uint32_t f = 0u;
                         if (l == 0) {
-                            f = ld_acquire_gpu(P.flags + sj);
-                            for (uint32_t n = 1; f == 0u; ++n) {
-                                if ((n & 15u) == 0u) {
-                                    if (M.abort || ld_acquire_gpu(P.ctrl + 1) != 0u) break;
-                                    if (globaltimer_ns() - t0 > ctx.deadline_span_ns) {
-                                        raise_timeout(ctx, WHERE_LOOKBACK);
-                                        break;
-                                    }
-                                }
-                                __nanosleep(128);
-                                f = ld_acquire_gpu(P.flags + sj);
-                            }
+                            f = wait_flag(ctx, P.flags + sj, t0);
                         }
                         f = __shfl_sync(0xffffffffu, f, 0);
                         const bool gave_up = f == 0u;
@@ -1179,6 +1185,50 @@ gla_block_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Para
     tc_fence_before();
     __syncthreads();
     if (w == kWarpProducer) tmem_dealloc(tmem, kTmemCols);
+}
+
+// Self-test of every bounded wait there is: one warp waits for barriers that nobody arrives at and for a flag that nobody sets.  Each
+// wait must give up after the limit and say so; what it said goes to a control word of its own, 1 where it was right.
+//   [2] wait by the status word   [3] wait by the block's flag   [4] this kernel's barrier wait, and the next one at once   [5] look-back
+__global__ void wait_timeout_selftest_kernel(Params P) {
+    __shared__ Misc M;
+    __shared__ uint32_t flag;
+    Ctx ctx;
+    ctx.p = &P;
+    ctx.misc = &M;
+    ctx.base = nullptr;
+    ctx.smem = 0;
+    ctx.deadline_span_ns = static_cast<uint64_t>(P.wait_limit_us) * 1000ull;
+    volatile uint32_t* status = P.ctrl + 1;
+    if (threadIdx.x == 0) {
+        mbar_init(smem_u32(&M.full[0]), 1);
+        M.abort = 0;
+        flag = 0;
+        fence_mbar_init();
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    const uint64_t tick = 2048;                    // the timer of the common waits counts in units of 1024 ns
+    auto long_enough = [&](uint64_t t0) { return globaltimer_ns() - t0 + tick >= ctx.deadline_span_ns; };
+    uint64_t t0 = globaltimer_ns();
+    wait_bar(P, M.full[0], 0);
+    P.ctrl[2] = long_enough(t0) && *status == WHERE_MBAR;
+    *status = 0u;
+    t0 = globaltimer_ns();
+    wait_bar(P, M.full[0], 0, flag);
+    P.ctrl[3] = long_enough(t0) && flag == 1u && *status == 0u;
+    t0 = globaltimer_ns();
+    mbar_wait(ctx, &M.full[0], 0);
+    const bool waited = long_enough(t0) && M.abort == 1u && *status == WHERE_MBAR;
+    t0 = globaltimer_ns();
+    mbar_wait(ctx, &M.full[0], 0);
+    P.ctrl[4] = waited && globaltimer_ns() - t0 < ctx.deadline_span_ns / 2 + 5000000u;       // (its polls before it looks at the flag: 3 ms)
+    *status = 0u;
+    M.abort = 0;
+    __threadfence();
+    t0 = globaltimer_ns();
+    const bool nothing = wait_flag(ctx, P.flags, t0) == 0u;
+    P.ctrl[5] = nothing && long_enough(t0) && M.abort == 1u && *status == WHERE_LOOKBACK;
 }
 
 }  // namespace block

@@ -242,20 +242,6 @@ __device__ __forceinline__ void half_row_store(float* to, const float* x) {
     for (int e = 0; e < 8; ++e) dst[e * kFwdThreads] = make_float4(x[4 * e], x[4 * e + 1], x[4 * e + 2], x[4 * e + 3]);
 }
 
-// Self-test of the bounded waits: one warp waits on an mbarrier nobody arrives at; the wait must give up after the limit, set the
-// status word and return.
-__global__ void wait_timeout_selftest_kernel(Params P) {
-    __shared__ uint64_t bar;
-    if (threadIdx.x == 0) {
-        mbar_init(smem_u32(&bar), 1);
-        fence_mbar_init();
-    }
-    __syncthreads();
-    wait_bar(P, bar, 0);                           // never completes: returns after the limit
-    __syncthreads();
-    if (threadIdx.x == 0) P.ctrl[2] = *reinterpret_cast<volatile uint32_t*>(P.ctrl + 1) != 0u ? 1u : 0u;     // 1: the CTA noticed the time-out
-}
-
 // Raw-logit gates (gk_normalizer > 0): this thread's piece of the gate tile is rewritten in place as fp16 log gates,
 // logsigmoid(x) / normalizer, before the gate-sum MMA reads it; rows the sequence does not have (zero-filled) must not decay.
 __device__ __forceinline__ void logits_to_log_gates(const HalfRow& at, uint32_t tile, float inv_norm, bool real_row) {

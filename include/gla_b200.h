@@ -136,9 +136,11 @@ size_t gla_b200_workspace_bytes(int32_t B, int32_t T, int32_t H, int32_t K, int3
  * The reference has no counterpart (its waits are unbounded, gla_chunk.cuh:1229-1233). */
 int gla_b200_check_status(const void* workspace, void* stream);
 
-/* Exercises the kernel's bounded waits without any real work: one warp waits on a barrier and on a
- * flag that nothing ever completes, with a limit of `limit_us` microseconds (<= 1 s).  Afterwards
- * gla_b200_check_status(workspace) must report GLA_B200_ERR_TIMEOUT and the context stays usable.
+/* Exercises the kernels' bounded waits without any real work: one thread waits, with a limit of `limit_us` microseconds (<= 1 s)
+ * each, in turn on a barrier as the forward's output kernel and the gradient's do, as their first kernels do and as the block
+ * kernel does, and on a flag as that kernel's look-back does; nothing ever completes either.  The words 2 to 5 of the workspace
+ * then hold 1 for each of the four that gave up as it should.  Afterwards gla_b200_check_status(workspace) must report
+ * GLA_B200_ERR_TIMEOUT and the context stays usable.
  * `workspace` == NULL runs the test on the built-in array of gla_b200_forward_static.
  * No counterpart in the reference, whose device-side waits are unbounded. */
 int gla_b200_selftest_wait_timeout(void* workspace, size_t workspace_bytes, uint32_t limit_us, void* stream);

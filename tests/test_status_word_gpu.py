@@ -89,3 +89,11 @@ def test_packed(ends, device):
         _lib.check(L.gla_b200_check_status(ws.data_ptr(), STREAM()))
         outs.append(o)
     assert torch.equal(*outs) and bool(outs[0].any()) == good
+
+
+def test_every_kind_of_wait_gives_up():
+    from gtr_b200 import _lib
+    ws = torch.zeros(256, dtype=torch.int32, device="cuda")
+    _lib.check(_lib.lib().gla_b200_selftest_wait_timeout(ws.data_ptr(), ws.numel() * 4, 20000, STREAM()))     # 20 ms each
+    assert _lib.lib().gla_b200_check_status(ws.data_ptr(), STREAM()) == _lib.ERR_TIMEOUT
+    assert ws[2:6].tolist() == [1, 1, 1, 1]
