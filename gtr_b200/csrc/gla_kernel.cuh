@@ -536,7 +536,6 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
         M.sq[0] = first_sq;
     }
     pdl_wait();
-    if (!P.alone) pdl_release();
     if (tid == 0) load(chunk, M.sq[0], smem_u32(&M.full));           // the first tiles come in while the rest is set up
     if (w == 1) {
         tmem_alloc(smem_u32(&M.tmem), 128);
@@ -584,6 +583,8 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = M.tmem;
+    // Not before this block has its tensor memory: what follows in the stream may take some before it waits for this kernel
+    if (!P.alone) pdl_release();
 
     uint32_t wides = 0;
     for (uint32_t p = 0;; p ^= 1u) {
