@@ -201,7 +201,7 @@ void set_split(const Split& s, int64_t chunks, gla::Params* P) {
     P->spans = s.spans;
     P->per = s.per;
     P->len_ = static_cast<int>(chunks / s.spans);
-    P->longer = static_cast<int>(chunks % s.spans);
+    P->longer = s.per > 0 ? P->NT % s.per : static_cast<int>(chunks % s.spans);
 }
 
 // q and k each carry sqrt(scale) / 4 (head-room for the gate factors in fp16); the 16 comes back in the epilogue
@@ -830,7 +830,7 @@ static int forward(const gla_b200_args* a, bool block, void* stream_v) {
     if (chunks > 0x3fffffff) return GLA_B200_ERR_SHAPE;
     Split split;
     if (a->segments > 0) {
-        split.per = (NT + a->segments - 1) / a->segments;
+        split.per = std::min((NT + a->segments - 1) / a->segments, gla::kMaxParts);
         split.spans = nseq * split.per;
     } else {
         split = choose_split(chunks, NT, nseq, di.sms, a->workspace ? a->workspace_bytes : 0);

@@ -50,8 +50,8 @@ struct Params {
                          // and state rows 32..63 stay zero
     int Hc, Wc;          // column length / number of columns of the scan (row scans: Hc = T, Wc = 1)
     int rev;             // scan runs from the last token to the first
-    // Spans: per > 0: `per` nearly equal ones per sequence; per == 0: all chunks in equal ones of len_ chunks, the first `longer`
-    // of them one chunk longer
+    // Spans: per > 0: `per` nearly equal ones per sequence, NT = per * len_ + longer; per == 0: all chunks in equal ones of len_
+    // chunks, the first `longer` of them one chunk longer
     int chunks, spans, per, len_, longer;
     int keep;            // k, g and v fit the L2: what the state kernel reads is kept there for the output kernel
     int alone;           // no state kernel runs before the output kernel
@@ -157,7 +157,7 @@ template <class Table>
 __device__ __forceinline__ int span_begin(const Table&, const Params& P, int i) {
     if (P.per > 0) {
         const int s = i / P.per, j = i - s * P.per;
-        return s * P.NT + j * P.NT / P.per;
+        return s * P.NT + part_begin(j, P.len_, P.longer, P.per);
     }
     return i * P.len_ + min(i, P.longer);
 }

@@ -24,6 +24,13 @@ constexpr float kLog2e = 1.4426950408889634f;
 enum { TQ = 0, TK = 1, TG = 2, TV = 3, TO = 4, TGATE = 5, kNumTensors = 6 };
 constexpr int kNumBoxes = 4;              // box heights 64, 16, 4, 1 rows
 
+// Where the j-th of `parts` nearly equal parts of n things begins, floor(j n / parts), from n = parts * len + rest: no product
+// leaves 32 bits while there are at most kMaxParts of them.
+constexpr int kMaxParts = 65535;
+__host__ __device__ constexpr int part_begin(int j, int len, int rest, int parts) {
+    return j * len + static_cast<int>(static_cast<uint32_t>(j) * static_cast<uint32_t>(rest) / static_cast<uint32_t>(parts));
+}
+
 struct Maps {
     CUtensorMap m[kNumTensors][kNumBoxes];
 };
