@@ -1263,6 +1263,28 @@ int gla_b200_swiglu_dwconv(const void* gate, const void* y, const void* weight, 
                          static_cast<cudaStream_t>(stream), maps, static_cast<__half*>(out), bias != nullptr, rows, strips, grid_h, grid_w, C);
 }
 
+int gla_b200_swiglu_status(void* stream_v) {
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
+    uint32_t status = 0;
+    cudaError_t e = cudaMemcpyFromSymbolAsync(&status, gla::g_dw_status, sizeof(status), 0, cudaMemcpyDeviceToHost, stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    if (e == cudaSuccess && status != 0) {
+        const uint32_t none = 0;
+        e = cudaMemcpyToSymbolAsync(gla::g_dw_status, &none, sizeof(none), 0, cudaMemcpyHostToDevice, stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    }
+    if (e != cudaSuccess) { note_cuda("status read", e); return GLA_B200_ERR_CUDA; }
+    return status == 0 ? GLA_B200_OK : GLA_B200_ERR_TIMEOUT;
+}
+
+int gla_b200_selftest_swiglu_timeout(uint32_t limit_us, void* stream) {
+    if (limit_us == 0 || limit_us > 1000000u) return GLA_B200_ERR_ARG;      // a self-test never waits longer than 1 s
+    gla::dw_timeout_selftest_kernel<<<1, 1, 0, static_cast<cudaStream_t>(stream)>>>(limit_us);
+    const cudaError_t e = cudaPeekAtLastError();
+    if (e != cudaSuccess) { note_cuda("self-test launch", e); return GLA_B200_ERR_CUDA; }
+    return GLA_B200_OK;
+}
+
 int gla_b200_layernorm(const void* x, const void* weight, const void* bias, void* y, int64_t rows, int32_t D, float eps,
                        void* stream) {
     if (rows < 0 || D <= 0 || (D & 7) || D > 256 * gla::kLnMaxVec) return GLA_B200_ERR_SHAPE;

@@ -84,11 +84,34 @@ __device__ __forceinline__ int dw_answer(uint32_t answer) {       // the block, 
                  : "=r"(got), "=r"(x) : "r"(answer) : "memory");
     return got ? static_cast<int>(x) : -1;
 }
-// Waits here are for copies and for warps of the same CTA; the limit only bounds what a fault elsewhere could make of them.
-__device__ __forceinline__ bool dw_wait(uint32_t bar, uint32_t parity) {
-    for (int n = 0; n < (1 << 22); ++n)
+// Set when a wait of this kernel ran out anywhere on the device, until it is read (gla_b200_swiglu_status): the call has no scratch that
+// could hold a word of its own.
+__device__ uint32_t g_dw_status;
+constexpr uint32_t kDwWaitUs = 2000000;
+// Waits here are for copies, for warps of the same CTA and for the launch control's answers.  False after the limit, or as soon as
+// another wait of this CTA (which sets its shared `flag`) has given up: the CTA then leaves, its outputs are undefined and the status says so.
+__device__ __forceinline__ bool dw_wait(uint32_t bar, uint32_t parity, uint32_t flag, uint32_t limit_us = kDwWaitUs) {
+    for (int n = 0; n < 64; ++n)
         if (mbar_try_wait(bar, parity)) return true;
+    const uint32_t t0 = globaltimer_1024ns();
+    while (ld_shared_u32(flag) == 0u) {
+        for (int n = 0; n < 64; ++n)
+            if (mbar_try_wait(bar, parity)) return true;
+        if (globaltimer_1024ns() - t0 > limit_us) {
+            st_shared_u32(flag, 1u);
+            atomicExch(&g_dw_status, 1u);
+        }
+    }
     return false;
+}
+// One thread waits for a barrier that nobody arrives at.
+__global__ void dw_timeout_selftest_kernel(uint32_t limit_us) {
+    __shared__ uint64_t bar;
+    __shared__ uint32_t flag;
+    mbar_init(smem_u32(&bar), 1);
+    flag = 0u;
+    fence_mbar_init();
+    dw_wait(smem_u32(&bar), 0, smem_u32(&flag), limit_us);
 }
 
 __global__ void __launch_bounds__(kDwThreads, 1) swiglu_dwconv_kernel(const __grid_constant__ DwMaps maps, __half* __restrict__ out,
@@ -98,17 +121,18 @@ __global__ void __launch_bounds__(kDwThreads, 1) swiglu_dwconv_kernel(const __gr
     const int tid = threadIdx.x;
     const int cols = strips * kDwRun, tiles_c = (wg + cols - 1) / cols, tiles_r = (hg + rows - 1) / rows;
     const int slabs = (C + kDwSlab - 1) / kDwSlab;
-    // control words: the answer, a stage's item (-1: none is left), barriers
+    // control words: the answer, a stage's item (-1: none is left), barriers, a flag
     auto item_of = [&](int s) { return control + 16u + 4u * s; };
     auto full = [&](int s) { return control + 32u + 8u * s; };
     auto empty = [&](int s) { return control + 32u + 8u * (kDwStages + s); };
-    const uint32_t answered = control + 32u + 16u * kDwStages;
+    const uint32_t answered = control + 32u + 16u * kDwStages, gave_up = answered + 8u;
     if (tid == 0) {
         for (int s = 0; s < kDwStages; ++s) {
             mbar_init(full(s), 1);
             mbar_init(empty(s), kDwThreads / 32);
         }
         mbar_init(answered, 1);
+        st_shared_u32(gave_up, 0u);
         fence_mbar_init();
     }
     __syncthreads();
@@ -120,7 +144,7 @@ __global__ void __launch_bounds__(kDwThreads, 1) swiglu_dwconv_kernel(const __gr
     bool more = true;
     auto fill = [&](int item) {
         const int s = to_fill;
-        dw_wait(empty(s), (fill_turn & 1u) ^ 1u);
+        if (!dw_wait(empty(s), (fill_turn & 1u) ^ 1u, gave_up)) { more = false; return; }       // the stage may still be read
         asm volatile("st.shared.b32 [%0], %1;" ::"r"(item_of(s)), "r"(item) : "memory");
         if (item < 0) {
             more = false;
@@ -140,9 +164,9 @@ __global__ void __launch_bounds__(kDwThreads, 1) swiglu_dwconv_kernel(const __gr
     };
     auto fill_next = [&] {
         if (!more) return;
-        const int item = dw_wait(answered, asked & 1u) ? dw_answer(control) : -1;
+        if (!dw_wait(answered, asked & 1u, gave_up)) { more = false; return; }
         ++asked;
-        fill(item);
+        fill(dw_answer(control));
     };
     if (tid == 0) {
         fill(static_cast<int>(blockIdx.x));
@@ -156,10 +180,10 @@ __global__ void __launch_bounds__(kDwThreads, 1) swiglu_dwconv_kernel(const __gr
     for (int s = 0;;) {
         if (tid == 0) fill_next();
         __syncwarp();
-        if (!dw_wait(full(s), turn & 1u)) return;
+        if (!dw_wait(full(s), turn & 1u, gave_up)) break;
         int item;
         asm volatile("ld.shared.b32 %0, [%1];" : "=r"(item) : "r"(item_of(s)) : "memory");
-        if (item < 0) return;
+        if (item < 0) break;
         const int slab = item % slabs, tile = item / slabs, cg = slab * (kDwSlab / 8) + ci;
         const int tc = tile % tiles_c, rest = tile / tiles_c, tr = rest % tiles_r, b = rest / tiles_r;
         const int r = tr * rows + trow, c = tc * cols + tcol;
@@ -204,6 +228,15 @@ __global__ void __launch_bounds__(kDwThreads, 1) swiglu_dwconv_kernel(const __gr
         __syncwarp();
         if ((tid & 31) == 0) mbar_arrive(empty(s));
         if (++s == kDwStages) { s = 0; ++turn; }
+    }
+    if (tid == 0 && ld_shared_u32(gave_up) != 0u) {           // what this CTA still has under way must land before its memory is given back
+        st_shared_u32(gave_up, 0u);
+        const uint32_t filled = fill_turn * kDwStages + to_fill;
+        for (uint32_t s = 0; s < kDwStages; ++s) {
+            const uint32_t n = (filled + kDwStages - 1 - s) / kDwStages;
+            if (n > 0 && !dw_wait(full(s), (n - 1) & 1u, gave_up)) return;
+        }
+        if (filled > asked) dw_wait(answered, asked & 1u, gave_up);
     }
 }
 

@@ -449,6 +449,13 @@ def swiglu_dwconv(gate: torch.Tensor, y: torch.Tensor, weight_taps: torch.Tensor
     return out
 
 
+def check_swiglu_status(device) -> None:
+    """Synchronise the current stream and raise if a bounded wait expired in any `swiglu_dwconv` on `device` since the last check."""
+    with torch.cuda.device(device):
+        stream = torch.cuda.current_stream(device).cuda_stream
+        _lib.check(_lib.lib().gla_b200_swiglu_status(ctypes.c_void_p(stream)))
+
+
 def layernorm(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], eps: float,
               out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """LayerNorm over the last dimension of a contiguous float16 CUDA tensor (fp32 statistics); the backbone block's

@@ -213,6 +213,13 @@ int gla_b200_rmsnorm_gated(const void* x, const void* g, const void* w, void* y,
 int gla_b200_swiglu_dwconv(const void* gate, const void* y, const void* weight, const void* bias, void* out,
                            int32_t B, int32_t grid_h, int32_t grid_w, int32_t C, void* stream);
 
+/* The waits of that kernel are bounded too (2 s).  It has no scratch of the caller's to report in; a word on the device notes a wait that
+ * ran out in any call there.  This synchronises `stream`, clears the word and returns 0, or GLA_B200_ERR_TIMEOUT if it was set
+ * since it was last read: the outputs of a call since then are undefined. */
+int gla_b200_swiglu_status(void* stream);
+/* Makes one such wait run out after `limit_us` microseconds (<= 1 s); gla_b200_swiglu_status must report it, once. */
+int gla_b200_selftest_swiglu_timeout(uint32_t limit_us, void* stream);
+
 /* LayerNorm over rows of D fp16 values with fp32 statistics: y = (x - mean) * rsqrt(var + eps) * weight + bias.
  * The norms in front of the backbone block's attention and MLP (engine/gtr/backbone/vit_adapter.py:608-642, nn.LayerNorm
  * with eps 1e-6) in one read and one write of the activations.  D a multiple of 8, at most 2048; bias may be NULL;

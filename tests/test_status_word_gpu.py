@@ -97,3 +97,19 @@ def test_every_kind_of_wait_gives_up():
     _lib.check(_lib.lib().gla_b200_selftest_wait_timeout(ws.data_ptr(), ws.numel() * 4, 20000, STREAM()))     # 20 ms each
     assert _lib.lib().gla_b200_check_status(ws.data_ptr(), STREAM()) == _lib.ERR_TIMEOUT
     assert ws[2:6].tolist() == [1, 1, 1, 1]
+
+
+def test_swiglu_waits_give_up_and_say_so():
+    import gtr_b200 as G
+    from gtr_b200 import _lib, ops
+    L = _lib.lib()
+    assert L.gla_b200_swiglu_status(STREAM()) == 0
+    assert L.gla_b200_selftest_swiglu_timeout(20000, STREAM()) == 0          # 20 ms
+    with pytest.raises(_lib.GlaError) as err:
+        ops.check_swiglu_status("cuda")
+    assert err.value.code == _lib.ERR_TIMEOUT
+    ops.check_swiglu_status("cuda")                                          # reported once
+    gate, y, taps = (torch.randn(*s, device="cuda").half() for s in ((2, 40 * 40, 768), (2, 40 * 40, 768), (3, 3, 768)))
+    out = G.swiglu_dwconv(gate, y, taps, None, (40, 40))
+    ops.check_swiglu_status("cuda")
+    assert torch.isfinite(out).all()
