@@ -307,7 +307,8 @@ PyObject* gla(PyObject*, PyObject* const* v, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
-bool rising(const int32_t* p, int64_t count, int64_t total) {
+template <class Int>
+bool rising(const Int* p, int64_t count, int64_t total) {
     bool fine = p[0] == 0 && p[count] == total;
     for (int64_t i = 0; i < count && fine; ++i) fine = p[i + 1] >= p[i];
     return fine;
@@ -391,10 +392,11 @@ PyObject* packed(PyObject*, PyObject* const* v, Py_ssize_t n) {
     at::Tensor off;
     {
         pybind11::gil_scoped_release release;
-        off = ends->to(at::kCPU, at::kInt).contiguous();
+        off = ends->to(at::kCPU, at::kLong).contiguous();
     }
+    if (!rising(off.const_data_ptr<int64_t>(), count, a.T)) return PyLong_FromLong(kSlow);     // as they came: 2^32 + 5 is not 5
+    off = off.to(at::kInt);
     const int32_t* p = off.const_data_ptr<int32_t>();
-    if (!rising(p, count, a.T)) return PyLong_FromLong(kSlow);
     a.workspace_bytes = g_packed_workspace_bytes(p, static_cast<int32_t>(count), a.H);
     const at::Tensor ws = at::empty({static_cast<int64_t>(a.workspace_bytes)}, opts.dtype(at::kByte));
     a.workspace = ws.data_ptr();

@@ -198,7 +198,11 @@ def _chunk_gla_forward(q, k, v, g, scale: Optional[float] = None, initial_state:
         if direction != 0 or grid_hw is not None:
             raise ValueError("cu_seqlens describes plain forward scans")
         if segments == 0:
-            ends = cu_seqlens if isinstance(cu_seqlens, torch.Tensor) else torch.tensor(cu_seqlens, dtype=torch.int32)
+            if isinstance(cu_seqlens, torch.Tensor):
+                ends = cu_seqlens
+            else:
+                cu_seqlens = _sequence_bounds(cu_seqlens, B, T)
+                ends = torch.tensor(cu_seqlens, dtype=torch.int64)
             done = _front().packed(q, k, v, g, scale, initial_state, output_final_state, ends, gk_normalizer)
             if type(done) is tuple:
                 return done

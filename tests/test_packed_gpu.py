@@ -1,5 +1,6 @@
 """Packed sequences in one launch: lengths around the chunk size, empty ones, one long sequence cut into segments among short
 ones, more sequences than a launch's table holds (96), with log gates and raw logits, states in and out."""
+import numpy as np
 import pytest
 import torch
 
@@ -43,3 +44,25 @@ def test_packed(lens, H, K, logits):
     assert torch.isfinite(o).all() and float((o - want_o).norm() / want_o.norm()) <= 1e-3
     assert float((s - want_s).norm() / want_s.norm()) < 5e-4
     assert float((o - want_o).abs().max()) <= 4e-3 * float(want_o.abs().max())
+
+
+@pytest.mark.parametrize("ends", [
+    torch.tensor([0, 2 ** 32 + 30, 100]), torch.tensor([2 ** 32, 30, 100]), torch.tensor([0, 30, 2 ** 33 + 100]),   # good in their low halves
+    [0, 2 ** 32 + 30, 100], [0, 2 ** 70, 100], [0, 40, 30, 100], [0], [],
+])
+def test_offsets_that_are_no_good_as_they_came(ends):
+    import gtr_b200 as G
+    x = torch.zeros(1, 100, 2, 64, dtype=torch.float16, device="cuda")
+    with pytest.raises(ValueError):
+        G.chunk_gla(x, x, x, x, cu_seqlens=ends)
+
+
+def test_offsets_may_come_as_any_iterable():
+    import gtr_b200 as G
+    gen = torch.Generator().manual_seed(0)
+    x = torch.randn(1, 100, 2, 64, generator=gen).half().cuda()
+    g = -torch.rand(1, 100, 2, 64, generator=gen).half().cuda()
+    want, state = G.chunk_gla(x, x, x, g, output_final_state=True, cu_seqlens=torch.tensor([0, 30, 60, 90, 100]))
+    for ends in ([0, 30, 60, 90, 100], (0, 30, 60, 90, 100), iter([0, 30, 60, 90, 100]), np.array([0, 30, 60, 90, 100]), torch.tensor([0., 30, 60, 90, 100])):
+        got, final = G.chunk_gla(x, x, x, g, output_final_state=True, cu_seqlens=ends)
+        assert torch.equal(want, got) and torch.equal(state, final)
