@@ -255,10 +255,10 @@ constexpr int kMinAutoCps = 4;   // smallest automatic segment length
 int auto_chunks_per_segment(int NT, int nseq, int slots, size_t workspace_bytes) {
     int best_cps = NT;
     double best = 1e300;
-    for (int cps = NT; cps >= 1; --cps) {
-        const int ns = (NT + cps - 1) / cps;
+    for (int ns = 1; ns == 1 || NT >= ns * (kMinAutoCps - 1); ++ns) {
+        const int cps = (NT + ns - 1) / ns;
         if (ns > 1 && cps < kMinAutoCps) break;
-        if (cps != (NT + ns - 1) / ns) continue;               // only the balanced split for each segment count
+        if ((NT + cps - 1) / cps != ns) continue;              // only the balanced split for each segment count
         // a split whose scratch does not fit the caller's workspace is not a candidate: the policy then settles
         // for a coarser one (one segment per sequence needs next to nothing)
         if (ns > 1 && ws_layout(static_cast<size_t>(nseq), static_cast<size_t>(ns)).total > workspace_bytes) continue;
@@ -310,6 +310,75 @@ int relay_segments(int NT, int nseq, int slots, size_t workspace_bytes, double* 
     }
     *cost_out = best_cost;
     return best;
+}
+
+enum { EQUAL = 0, STAGGERED = 1, RELAY = 2 };           // gla::block::Params::plan
+struct Plan {
+    int kind = EQUAL, cps = 0, ns = 0, start[gla::block::kMaxPlanSegments + 1] = {0};
+};
+// `segments` > 0: equal segments of that many chunks.  in_place: the final states replace the initial ones, so that a sequence's last
+// segment must not finish before its first has read its state for good.  In the staggered and relay plans the first
+// segment reads it once, before it publishes what all others wait for; with equal segments and pre-passes it reads it twice.
+Plan make_plan(int NT, int nseq, int slots, size_t have, bool gated, int segments, bool in_place) {
+    Plan p;
+    const double pre = gated ? kPlanPrePassGated : kPlanPrePassPlain;
+    if (in_place) {
+        const int r = std::min({slots / nseq, gla::block::kMaxPlanSegments - 1, NT / kMinAutoCps - 1});
+        double relay_cost = 0.0;
+        if (staggered_plan(NT, nseq, r, have, pre, p.start, &p.ns) > 0.0) { p.kind = STAGGERED; return p; }
+        const int ns = nseq >= slots ? relay_segments(NT, nseq, slots, have, &relay_cost) : 1;
+        if (ns > 1) p.kind = RELAY;
+        p.cps = (NT + ns - 1) / ns;
+    } else if (segments > 0) {
+        p.cps = std::min(segments, NT);
+    } else {
+        p.cps = auto_chunks_per_segment(NT, nseq, slots, have);
+        const int ns = (NT + p.cps - 1) / p.cps;
+        const long rounds = (static_cast<long>(nseq) * ns + slots - 1) / slots;
+        // what the slowest item of the equal split costs, in the plan's units: every segment but the last pays the pre-pass
+        const double uniform_cost = rounds * (p.cps * (1.0 + (ns > 1 ? pre : 0.0)) + (ns > 1 ? 1.0 : 0.0));
+        const double plan_cost = staggered_plan(NT, nseq, slots / nseq, have, pre, p.start, &p.ns);
+        if (plan_cost > 0.0 && plan_cost < uniform_cost) { p.kind = STAGGERED; return p; }
+        if (2 * nseq > slots) {
+            double relay_cost = 0.0;
+            const int ns_r = relay_segments(NT, nseq, slots, have, &relay_cost);
+            if (ns_r > 1 && relay_cost < 0.97 * uniform_cost) { p.kind = RELAY; p.cps = (NT + ns_r - 1) / ns_r; }
+        }
+    }
+    p.ns = (NT + p.cps - 1) / p.cps;
+    return p;
+}
+
+// What a plan takes (us): its chunks, one after another on the busiest CTA, kChunkTime[fused epilogue][raw-logit gates] each and kBox more for
+// every copy past the first that it takes to bring a tensor's tile (one thread asks for them all); kItem for each item that
+// is not its first or exchanges states; kLookBack for each segment that a state is looked for in.
+constexpr double kLaunch = 6.0, kItem = 3.5, kLookBack = 0.55, kBox = 0.1, kChunkTime[2][2] = {{1.18, 1.64}, {1.57, 2.08}};
+double time_of(const Plan& p, int NT, int nseq, int slots, bool gated, bool logits, double boxes) {
+    const double pre = gated ? kPlanPrePassGated : kPlanPrePassPlain;
+    double work = 0.0, items = 0.0;
+    int look = 0;
+    if (p.kind == STAGGERED) {
+        work = std::max((1.0 + pre) * (p.start[2] - p.start[1]), static_cast<double>(p.start[1] + p.start[p.ns] - p.start[p.ns - 1]));
+        items = 1.5;
+        look = p.ns;
+    } else if (p.kind == RELAY) {
+        const int64_t rounds = (static_cast<int64_t>(nseq) * p.ns + slots - 1) / slots;
+        work = static_cast<double>(std::max<int64_t>(rounds * p.cps, NT));          // a sequence's segments run one after another
+        items = static_cast<double>(rounds);
+    } else if (p.ns == 1) {
+        const int64_t rounds = (nseq + slots - 1) / slots;
+        work = static_cast<double>(rounds * NT);
+        items = static_cast<double>(rounds - 1);
+    } else {
+        // all but the last segments come first, each with its pre-pass; the last ones fill up what these leave
+        const double each = p.cps * (1.0 + pre), last = NT - (p.ns - 1) * p.cps;
+        const int64_t first = static_cast<int64_t>(nseq) * (p.ns - 1), rounds = (first + slots - 1) / slots, idle = rounds * slots - first;
+        const int64_t rest = std::max<int64_t>(nseq - idle * std::max<int64_t>(static_cast<int64_t>(each / last), 1), 0), more = (rest + slots - 1) / slots;
+        work = rounds * each + more * last;
+        items = static_cast<double>(rounds + more);
+        look = p.ns;
+    }
+    return kLaunch + (kChunkTime[gated][logits] + kBox * (boxes - 1.0)) * work + kItem * items + kLookBack * std::min(look, 30);
 }
 }  // namespace block_plan
 
@@ -602,14 +671,35 @@ int launch_forward(bool gated, const gla::Maps& maps, gla::Params& P, const Tabl
     return launch_overlapped(out_kernel<Table>(gated, logits), P.spans, gla::kFwdThreads, gla::OutSmem::kBytes, args, stream);
 }
 
-// Which calls the block kernel serves better than the two kernels of gla_kernel.cuh.  Measured (us, block kernel / those two; row
-// scans), plain: 48 sequences x 100 chunks 65 / 71, 96 x 100 125 / 127-135, 192 x 64 118 / 151, 192 x 25 60 / 69, 192 x 128
-// 211 / 296, but 24 x 100 45 / 43 and 48 x 50 39 / 40: from 32 chunks per SM on.  The fused epilogue and raw-logit gates keep the
-// block kernel's teams busy for longer: 96 x 128 298 / 208, 384 x 128 756 / 664; it is ahead only where whole sequences just
-// about fill the SMs once and are long (144 x 128 286 / 299, 192 x 128 369 / 394).
-bool block_pays(bool gated, bool logits, int NT, int64_t nseq, int sms) {
-    if (!gated && !logits) return NT >= 24 && nseq * NT >= 32 * sms;
-    return NT >= 96 && 10 * nseq >= 9 * sms && 10 * nseq <= 14 * sms;
+// Copies that bring a chunk of a scan over columns of `rows` tokens, in boxes of 64, 16, 4 and 1 rows; the mean of the first few chunks.
+double boxes_per_chunk(int rows, int T) {
+    const int end = std::min(T, 8 * gla::kChunk);
+    int64_t boxes = 0;
+    for (int u = 0; u < end;) {
+        const int n = std::min({rows - u % rows, gla::kChunk - u % gla::kChunk, end - u});
+        boxes += n / 64 + n % 64 / 16 + n % 16 / 4 + n % 4;
+        u += n;
+    }
+    return static_cast<double>(boxes) / num_chunks(end);
+}
+
+// Whether the block kernel serves a call better than the two kernels of gla_kernel.cuh: the two models' times (us) are compared.  They were
+// fitted to 525 calls on both (1 to 944 sequences of 1 to 1500 chunks, up to 49 000 in all; plain, fused and raw-logit; row
+// and column scans; K = 64 and 32) and are off by 8 percent of a time (one standard deviation).  Where the two meet (block kernel /
+// the other two): plain 48 x 50 chunks 40 / 39, 48 x 75 51 / 54, 96 x 48 68 / 64, 192 x 24 60 / 62, 592 x 7 53 / 37; fused with
+// logits 96 x 128 291 / 208, 120 x 128 288 / 264, 144 x 128 288 / 309, 220 x 128 415 / 528, 384 x 128 726 / 670;
+// 48 x 100 on columns of 64, 40, 8 and 3 rows 67 / 73, 87 / 75, 139 / 87 and 402 / 166.
+// It has to be ahead by kMargin (us): with none of it small calls lose up to 20 percent to the models' error, and no call that it serves by
+// more than 3 percent better is lost.  (On gates that send every chunk down the exact path, which the host cannot foresee, the small kernels are four times as fast at any
+// size; GTR's never do.)  A caller's own segments make few long items or many short ones, which the models know less well: the block kernel's, whose
+// unit they are, unless the others are well ahead (12 x 256 chunks by segments of 1, 4, 8, 16, 32: 332 / 425, 115 / 84, 84 / 61, 80 / 88, 75 / 149).
+constexpr double kSplitLaunch = 2.4, kLongChain = 0.03, kSplitBox = 0.055, kSplitUnit[2][2] = {{2.6, 3.1}, {2.95, 3.4}}, kMargin = 3.0, kOwnSegments = 1.2;
+bool block_pays(const block_plan::Plan& plan, const Split& split, int NT, int nseq, int sms, bool gated, bool logits, double boxes, bool own_segments) {
+    const int64_t chunks = static_cast<int64_t>(nseq) * NT;
+    const double chain = std::max((split.per > 0 ? split.per : static_cast<double>(split.spans) / nseq) - 1.0, 0.0);
+    const double small = kSplitLaunch + (kSplitUnit[gated][logits] + kSplitBox * (boxes - 1.0)) * (split_cost(chunks, nseq, split.per, split.spans, sms) + kLongChain * chain);
+    const double block = block_plan::time_of(plan, NT, nseq, sms, gated, logits, boxes);
+    return own_segments ? block < kOwnSegments * small : block + kMargin < small;
 }
 
 // Whether states are written over others that the call reads.
@@ -618,43 +708,11 @@ bool overlap(const float* in, const float* out, size_t bytes) {
     return x && y && x < y + bytes && y < x + bytes;
 }
 
-// The operator on the block kernel (gla_block.cuh).  in_place: the final states replace the initial ones, so that a sequence's last
-// segment must not finish before its first has read its state for good.  In the staggered and relay plans the first
-// segment reads it once, before it publishes what all others wait for; with equal segments and pre-passes it reads it twice.
-int forward_block(const gla_b200_args* a, const MapKey& key, int sms, bool in_place, cudaStream_t stream) {
+// The operator on the block kernel (gla_block.cuh).
+int forward_block(const gla_b200_args* a, const MapKey& key, const block_plan::Plan& plan, int slots, cudaStream_t stream) {
     using namespace block_plan;
-    const int NT = num_chunks(a->T), nseq = a->B * a->H;
-    const int slots = sms;
+    const int NT = num_chunks(a->T), nseq = a->B * a->H, NS = plan.ns;
     const bool gated = a->out_gate != nullptr;
-    const size_t have = a->workspace ? a->workspace_bytes : 0;
-    const double pre = gated ? kPlanPrePassGated : kPlanPrePassPlain;
-    int cps;
-    int plan_start[gla::block::kMaxPlanSegments + 1] = {0}, plan_ns = 0;
-    bool plan = false, relay = false;
-    if (in_place) {
-        const int r = std::min({slots / nseq, gla::block::kMaxPlanSegments - 1, NT / kMinAutoCps - 1});
-        plan = staggered_plan(NT, nseq, r, have, pre, plan_start, &plan_ns) > 0.0;
-        double relay_cost = 0.0;
-        const int ns_r = !plan && nseq >= slots ? relay_segments(NT, nseq, slots, have, &relay_cost) : 1;
-        relay = ns_r > 1;
-        cps = (NT + ns_r - 1) / ns_r;
-    } else if (a->segments > 0) cps = a->segments;
-    else {
-        cps = auto_chunks_per_segment(NT, nseq, slots, have);
-        const int ns_u = (NT + cps - 1) / cps;
-        const long rounds = (static_cast<long>(nseq) * ns_u + slots - 1) / slots;
-        // what the slowest item of the equal split costs, in the plan's units: every segment but the last pays the pre-pass
-        const double uniform_cost = rounds * (cps * (1.0 + (ns_u > 1 ? pre : 0.0)) + (ns_u > 1 ? 1.0 : 0.0));
-        const double plan_cost = staggered_plan(NT, nseq, slots / nseq, have, pre, plan_start, &plan_ns);
-        plan = plan_cost > 0.0 && plan_cost < uniform_cost;
-        if (!plan && 2 * nseq > slots) {
-            double relay_cost = 0.0;
-            const int ns_r = relay_segments(NT, nseq, slots, have, &relay_cost);
-            if (ns_r > 1 && relay_cost < 0.97 * uniform_cost) { relay = true; cps = (NT + ns_r - 1) / ns_r; }
-        }
-    }
-    if (cps > NT) cps = NT;
-    const int NS = plan ? plan_ns : (NT + cps - 1) / cps;
     const block_plan::WsLayout L = block_plan::ws_layout(static_cast<size_t>(nseq), static_cast<size_t>(NS));
     if (!a->workspace || (reinterpret_cast<uintptr_t>(a->workspace) & 255u) || a->workspace_bytes < L.total)
         return GLA_B200_ERR_WORKSPACE;
@@ -668,9 +726,9 @@ int forward_block(const gla_b200_args* a, const MapKey& key, int sms, bool in_pl
     P.B = a->B; P.T = a->T; P.H = a->H; P.NT = NT; P.K = a->K;
     P.Hc = key.Hc; P.Wc = key.Wc;
     P.rev = a->direction & 1;
-    P.NS = NS; P.cps = cps;
-    P.plan = plan ? 1 : relay ? 2 : 0;
-    for (int i = 0; i <= gla::block::kMaxPlanSegments; ++i) P.seg_start[i] = plan_start[i];
+    P.NS = NS; P.cps = plan.cps;
+    P.plan = plan.kind;
+    for (int i = 0; i <= gla::block::kMaxPlanSegments; ++i) P.seg_start[i] = plan.start[i];
     P.num_items = nseq * NS;
     fold_scale(a->scale, &P);
     P.inv_norm = a->gk_normalizer > 0.f ? 1.f / a->gk_normalizer : 0.f;
@@ -815,32 +873,37 @@ static int forward(const gla_b200_args* a, bool block, void* stream_v) {
     key.Hc = col ? gh : a->T;
     key.Wc = col ? gw : 1;
     key.dev = dev;
-    // The output kernel's blocks read their sequences' initial states at different times, some when others have left a final
-    // state behind; the step kernel holds a state from its load to its store.
-    const bool in_place = overlap(a->initial_state, a->final_state, static_cast<size_t>(nseq) * a->K * gla::kD * sizeof(float)) && !step_serves(a->T, gated, a->segments);
-    if (block || in_place || (a->segments == 0 && block_pays(gated, a->gk_normalizer > 0.f, num_chunks(a->T), nseq, di.sms))) {
-        rc = forward_block(a, key, di.sms, in_place, static_cast<cudaStream_t>(stream_v));
-        if (block || in_place || rc != GLA_B200_ERR_WORKSPACE) return rc;
-    }
     int64_t o_stride[3];
     memcpy(o_stride, key.stride[gla::TO], sizeof(o_stride));
 
     const int NT = num_chunks(a->T);
     const int64_t chunks = static_cast<int64_t>(nseq) * NT;
     if (chunks > 0x3fffffff) return GLA_B200_ERR_SHAPE;
+    const size_t have = a->workspace ? a->workspace_bytes : 0;
+    const bool step = step_serves(a->T, gated, a->segments);
     Split split;
     if (a->segments > 0) {
         split.per = std::min((NT + a->segments - 1) / a->segments, gla::kMaxParts);
         split.spans = nseq * split.per;
     } else {
-        split = choose_split(chunks, NT, nseq, di.sms, a->workspace ? a->workspace_bytes : 0);
+        split = choose_split(chunks, NT, nseq, di.sms, have);
+    }
+    // The output kernel's blocks read their sequences' initial states at different times, some when others have left a final
+    // state behind; the step kernel holds a state from its load to its store.
+    const bool in_place = overlap(a->initial_state, a->final_state, static_cast<size_t>(nseq) * a->K * gla::kD * sizeof(float));
+    if (block || !step) {
+        const block_plan::Plan plan = block_plan::make_plan(NT, nseq, di.sms, have, gated, a->segments, in_place);
+        if (block || in_place || block_pays(plan, split, NT, nseq, di.sms, gated, a->gk_normalizer > 0.f, col ? boxes_per_chunk(gh, a->T) : 1.0, a->segments > 0)) {
+            rc = forward_block(a, key, plan, di.sms, static_cast<cudaStream_t>(stream_v));
+            if (block || in_place || rc != GLA_B200_ERR_WORKSPACE) return rc;
+        }
     }
     const WsLayout L = ws_layout(exchange_spans(split));
     if (!a->workspace || (reinterpret_cast<uintptr_t>(a->workspace) & 255u) || a->workspace_bytes < L.total)
         return GLA_B200_ERR_WORKSPACE;
 
     uint8_t* ws = static_cast<uint8_t*>(a->workspace);
-    if (step_serves(a->T, gated, a->segments)) {
+    if (step) {
         gla::StepParams S;
         S.q = static_cast<const __half*>(a->q); S.k = static_cast<const __half*>(a->k);
         S.v = static_cast<const __half*>(a->v); S.g = static_cast<const __half*>(a->g);
