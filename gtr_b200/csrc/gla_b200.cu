@@ -4,6 +4,7 @@
 #include "gla_b200.h"
 
 #include <algorithm>
+#include <atomic>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -648,22 +649,14 @@ void fill_params(const gla_b200_args* a, const int64_t* o_stride, uint8_t* ws, c
 
 
 constexpr int64_t kL2Keep = 120ll << 20;
-// Clears the control words, and `words` words of flags, for the launches that follow.
-int launch_clear(uint32_t* ctrl, uint32_t* flags, int words, unsigned threads, cudaStream_t stream) {
-    return launch_simple(&gla::clear_kernel, 1, threads, 0, stream, ctrl, flags, words);
-}
-
-// The spans' increments (where spans end inside sequences), then the outputs.  A kernel whose waits look at the status word must find it
-// cleared: the state kernel, whose waits do not, clears it for the output kernel; an output kernel on its own has it
-// cleared by a launch of its own (a block that cleared it itself could come after another one's report).  `first`: of the call.
+std::atomic<uint32_t> g_launches{0};
+// The spans' increments (where spans end inside sequences), then the outputs.  `first`: of the call, which clears the status.
 template <class Table>
 int launch_forward(bool gated, const gla::Maps& maps, gla::Params& P, const Table& table, bool first, cudaStream_t stream) {
     const bool logits = P.inv_norm > 0.f;
     const int states = P.per > 0 ? P.spans / P.per * (P.per - 1) : P.spans - 1;
     P.alone = states == 0 ? 1 : 0;
-    P.clear = first ? 1 : 0;
-    if (P.alone && first)
-        if (int rc = launch_clear(P.ctrl, nullptr, 0, 32, stream)) return rc;
+    P.clear = first ? g_launches.fetch_add(1, std::memory_order_relaxed) % 0xfffffffeu + 1u : 0u;
     P.keep = static_cast<int64_t>(P.chunks) * (4 * P.K + 128) * gla::kChunk <= kL2Keep ? 1 : 0;
     void* args[3] = {const_cast<gla::Maps*>(&maps), &P, const_cast<Table*>(&table)};
     if (states > 0)
@@ -750,7 +743,7 @@ int forward_block(const gla_b200_args* a, const MapKey& key, const block_plan::P
 
 
     const int words = static_cast<int>((L.clear_bytes - L.flags) / sizeof(uint32_t));
-    if (int rc = launch_clear(P.ctrl, P.flags, words, 256, stream)) return rc;
+    if (int rc = launch_simple(&gla::clear_kernel, 1, 256, 0, stream, P.ctrl, P.flags, words)) return rc;
     void* args[2] = {&maps, &P};
     return launch_overlapped(block_kernel((gated ? 4 : 0) | (P.inv_norm > 0.f ? 2 : 0) | (P.rev ? 1 : 0)), std::min(P.num_items, slots), gla::block::kThreads,
                              gla::block::kSmemBytes, args, stream);

@@ -55,7 +55,7 @@ struct Params {
     int chunks, spans, per, len_, longer;
     int keep;            // k, g and v fit the L2: what the state kernel reads is kept there for the output kernel
     int alone;           // no state kernel runs before the output kernel
-    int clear;           // the state kernel clears the status (the call's first launch)
+    uint32_t clear;      // the call's first kernel clears the status: not 0, and another for each launch
     // The output scale is folded into the exponents of the gate factors (q_exp = log2(scale) - 4, half of it on q and half
     // on k, o_mul = 16) when it is positive and finite; otherwise the epilogue multiplies (q_exp = -4, o_mul = 16 scale).
     float q_exp, q_mul, o_mul;
@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_state_kernel(const __grid_
     // per sequence, the last span needs no increment and gets no CTA; in the flat split it is found here
     const int span = P.per > 0 ? blockIdx.x + blockIdx.x / (P.per - 1) : blockIdx.x;
     auto clear_status = [&] {
-        if (P.clear && blockIdx.x == 0 && tid < 2) P.ctrl[tid] = 0u;
+        if (P.clear != 0u && blockIdx.x == 0 && tid < 2) P.ctrl[tid] = 0u;
     };
     if (std::is_same<Table, DeviceTable>::value) {
         pdl_wait();
@@ -427,7 +427,7 @@ struct OutSmem {
 };
 struct OutMisc {
     uint64_t full, raw, bar_x, bar_p, bar_inc, bar_o;
-    uint32_t tmem;
+    uint32_t tmem, gave_up;
     uint32_t wide[2];                 // per chunk parity: some channel decays too much for the common reference
     alignas(16) float vec[2][64];     // log2: half the chunk's total decay per channel
     Sequence sq[2];                   // per chunk parity; written by the thread that asks for the chunk's tiles, before it does
@@ -512,9 +512,18 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
     const uint32_t tq = base + OutSmem::kQ, tk = base + OutSmem::kK, tg = base + OutSmem::kG, tv = base + OutSmem::kV,
                    s16 = base + OutSmem::kS16, mat = base + OutSmem::kMat;
     // (offsets on the GPU: the state kernel has waited for them before it let these blocks start)
+    const bool clears = P.alone && P.clear != 0u;
     if (std::is_same<Table, DeviceTable>::value && P.alone) pdl_wait();
     const auto& tab = table_here(table, P, P.alone != 0);
-    if (nothing_in(tab)) return;
+    if (nothing_in(tab)) {
+        if (clears && blockIdx.x == 0 && tid < 2) P.ctrl[tid] = 0u;
+        return;
+    }
+    auto wait = [&](uint64_t& bar, uint32_t parity) {
+        volatile uint32_t *f = &M.gave_up, *status = P.ctrl + 1;
+        bounded_wait(bar, parity, P.wait_limit_us, [&] { return *f != 0u || (!clears && *status != 0u); },
+                     [&] { *f = 1u; if (!clears) report_timeout(P); });
+    };
     int chunk = span_begin(tab, P, blockIdx.x);                      // of all chunks, the one at hand; the span's end
     const int end = span_begin(tab, P, blockIdx.x + 1);
     const Sequence first_sq = sequence_of(tab, P, chunk);
@@ -534,8 +543,10 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
         fence_mbar_init();
         fence_proxy_async_smem();
         M.sq[0] = first_sq;
+        M.gave_up = 0u;
     }
     pdl_wait();
+    if (clears && blockIdx.x == 0 && tid == 0) clear_alone(P.ctrl, P.clear);
     if (tid == 0) load(chunk, M.sq[0], smem_u32(&M.full));           // the first tiles come in while the rest is set up
     if (w == 1) {
         tmem_alloc(smem_u32(&M.tmem), 128);
@@ -588,7 +599,7 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
 
     uint32_t wides = 0;
     for (uint32_t p = 0;; p ^= 1u) {
-        wait_bar(P, M.full, p);
+        wait(M.full, p);
         const int tok = scan_token(P, M.sq[p].T, (chunk - M.sq[p].chunk0) * kChunk + (rev ? 63 - static_cast<int>(row) : static_cast<int>(row)));
         if (kLogits) {
             logits_to_log_gates(at, OutSmem::kG, P.inv_norm, tok >= 0);
@@ -602,7 +613,7 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
         float x[32];
         uint32_t r[16];
         at.get(OutSmem::kQ, r);
-        wait_bar(P, M.bar_x, p);
+        wait(M.bar_x, p);
         tc_fence_after();
         half_row_read(tmem, ACC_X, w, x);
         tmem_ld_wait();
@@ -643,7 +654,7 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
                 load_chunk(maps, Scan{s.T, P.Hc, P.rev}, chunk - s.chunk0, s.b, s.h, s.tok0, P.Hc, smem_u32(&M.raw), tensors, tiles, l2_policy_stream());
                 mbar_arrive(smem_u32(&M.bar_p));                    // no score MMA in this chunk
             }
-            wait_bar(P, M.raw, wides & 1u);
+            wait(M.raw, wides & 1u);
             ++wides;
             half_row_write(tmem, ACC_S, w, S);                      // out of the registers' way
             tmem_st_wait();
@@ -674,7 +685,7 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
             at.put(OutSmem::kS16, r);
         }
         // ---- scores: causal, as the fp16 tile over the gates
-        wait_bar(P, M.bar_p, p);
+        wait(M.bar_p, p);
         tc_fence_after();
         if (!wide) {
             half_row_read(tmem, ACC_P, w, x);
@@ -718,7 +729,7 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
             for (int m = 0; m < 4; ++m) gate[m] = __ldg(gp + m);
         }
         // ---- the state after the chunk
-        wait_bar(P, M.bar_inc, p);
+        wait(M.bar_inc, p);
         tc_fence_after();
         const bool more = chunk + 1 < end, last = chunk + 1 == M.sq[p].chunk0 + M.sq[p].nt;
         {
@@ -740,7 +751,7 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
             }
         }
         // ---- outputs
-        wait_bar(P, M.bar_o, p);
+        wait(M.bar_o, p);
         tc_fence_after();
         if (more && elect_one()) {                                  // nothing reads the chunk's tiles any more: each warp asks for one
             const Sequence next = last ? sequence_of(tab, P, chunk + 1) : M.sq[p];
@@ -801,6 +812,10 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
     }
     tc_fence_before();
     __syncthreads();
+    if (clears && tid == 0) {
+        if (M.gave_up) report_alone(P, P.clear);
+        if (blockIdx.x == 0) P.ctrl[0] = 0u;
+    }
     if (w == 1) tmem_dealloc(tmem, 128);
 }
 

@@ -61,14 +61,31 @@ __device__ __forceinline__ void wait_bar(const P_t& P, uint64_t& bar, uint32_t p
     bounded_wait(bar, parity, P.wait_limit_us, [&] { return *reinterpret_cast<volatile uint32_t*>(P.ctrl + 1) != 0u; }, [&] { report_timeout(P); });
 }
 // For the first kernel of a call, whose block 0 clears the word (what lies there is an earlier call's, or never was written): its
-// group is the block, by a flag in shared memory.  Such a kernel leaves kTimedOut in place of a decay, which the second one reports;
-// no arithmetic makes a NaN of these bits.
+// group is the block, by a flag in shared memory.  Where a second kernel follows, this one leaves kTimedOut in place of a decay, which
+// the second one reports; no arithmetic makes a NaN of these bits.
 template <class P_t>
 __device__ __forceinline__ void wait_bar(const P_t& P, uint64_t& bar, uint32_t parity, uint32_t& flag) {
     volatile uint32_t* f = &flag;
     bounded_wait(bar, parity, P.wait_limit_us, [&] { return *f != 0u; }, [&] { *f = 1u; });
 }
 constexpr uint32_t kTimedOut = 0x7fc0deadu;
+// A kernel that is first and last: block 0 clears the word when it starts and says so with a number of the launch in ctrl[0], which it
+// takes back when it leaves (the launch may be replayed); a block that has given up reports when it has seen that number.  Not
+// seeing it for as long as a wait may take means that block 0 has long left.
+__device__ __forceinline__ void clear_alone(uint32_t* ctrl, uint32_t launch) {
+    volatile uint32_t* c = ctrl;
+    c[1] = 0u;
+    __threadfence();
+    c[0] = launch;
+}
+template <class P_t>
+__device__ __forceinline__ void report_alone(const P_t& P, uint32_t launch) {
+    volatile uint32_t* c = P.ctrl;
+    const uint32_t t0 = globaltimer_1024ns();
+    while (c[0] != launch && globaltimer_1024ns() - t0 <= max(P.wait_limit_us, 10000u)) {}
+    __threadfence();
+    report_timeout(P);
+}
 
 // Enumerates the TMA boxes that cover one chunk of the scan: f(box_id, r, c, smem_row) with (r, c) the row inside the
 // column and the column where the box starts.
