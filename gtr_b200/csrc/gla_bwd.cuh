@@ -335,106 +335,173 @@ __device__ __forceinline__ void bwd_f32_row16(uint32_t tile, uint32_t row, uint3
     }
 }
 
+// e^gate of 8 channels (unit u) of a row, fp32: their halves lie 128 bytes apart, so that the eight lanes of a row read without conflicts
+__device__ __forceinline__ uint32_t bwd_decay(uint32_t tile, uint32_t row, uint32_t u, uint32_t half) {
+    return tile + row * 256u + 128u * half + 16u * u;
+}
+
 // A chunk with a strong decay, pair by pair in fp32: P (scaled by fq fk, into its accumulator), and the part of dq and dk that
 // comes from within the chunk (into BWD_DQ_I and BWD_DP, complete); q and k are then rewritten with the references 0 and G_L,
-// whose exponents are never positive.  Out of line; about 30 k cycles a chunk, so a sequence of nothing but such chunks takes
-// some five times the usual time.
+// whose exponents are never positive.
+// A pair's factors are the running product of the decays between its tokens, which are taken once per token and channel: with an
+// exponential per pair and channel the special-function unit alone was busy for 17 thousand cycles a chunk.  Eight neighbouring
+// lanes, 8 channels each, share tokens r and 63 - r, so that all of them have 65 pairs to walk; what bounds it now is the shared memory
+// they read.  A sequence of nothing but such chunks, with an exponential per pair / now: B4 H12 T6400 976 / 640 us, B8 H6 T1600 300 / 198,
+// B32 H12 T2048 2490 / 1600, B8 H3 T1600 K = 32 185 / 126 (ordinary ones 189, 64, 475, 43).
+// Out of line.  Its loads ahead are as many as registers allow: with fewer in use the compiler spilt some of the ordinary chunk's around
+// the call (3 to 6 percent there).
 __device__ __noinline__ void bwd_wide_chunk(uint32_t base, const float* vec, uint32_t tmem, float fq, float fk, float scale,
                                             bool rev) {
     const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
     const uint32_t row = 16u * (w & 3) + (l & 15u), c0 = 32u * (w >> 2) + 16u * (static_cast<uint32_t>(l) >> 4), u0 = c0 >> 3;
     const uint32_t tg = base + BwdChunkSmem::kG, tq = base + BwdChunkSmem::kQ, tk = base + BwdChunkSmem::kK;
     const uint32_t dp = base + BwdChunkSmem::kR, out = dp + 2 * kTileBytes;
-    float x[16];
+    const uint32_t decays = base + BwdChunkSmem::kQl;      // until the low parts of q and k go there
+    static_assert(BwdChunkSmem::kKl == BwdChunkSmem::kQl + kTileBytes, "the decays take both tiles");
     auto sync = [] { named_bar_sync(BWD_BAR_COMPUTE, kComputeThreads); };
     auto at = [&](int t) { return static_cast<uint32_t>(rev ? 63 - t : t); };     // row of the chunk's t-th token
-    uint32_t qr[8], kr[8];
-    row16(tq, row, u0, qr);
-    row16(tk, row, u0, kr);
-    acc_read(tmem, BWD_DP, w, x);
-    tmem_ld_wait();
-    bwd_f32_put16(dp, row, c0, x);
-    sync();
-    // four neighbouring lanes share a row, 16 channels each
-    const int i = tid >> 2;                                // the i-th token
-    const uint32_t ch = 16u * (tid & 3), cu = ch >> 3;
-    float acc[16], D[16];
     {
-        uint32_t own[8];
-        row16(tq, at(i), cu, own);
+        uint32_t g[8];
+        row16(tg, row, u0, g);
 #pragma unroll
-        for (int e = 0; e < 16; ++e) acc[e] = D[e] = 0.f;
-        for (int s = 0; s < 64; ++s) {
-            const int j = i - s;
-            float a = 0.f;
-            if (j >= 0) {
-                uint32_t kk[8], gg[8];
-                row16(tk, at(j), cu, kk);
-                row16(tg, at(j), cu, gg);
-                const float d = ld_shared_f(bwd_f32(dp, at(i), at(j)));
+        for (uint32_t e = 0; e < 4; ++e) {
+            const float2 a = ex2_2(mul2(unpack_half2(g[2 * e]), two(kLog2e))), b = ex2_2(mul2(unpack_half2(g[2 * e + 1]), two(kLog2e)));
+            st_shared_f4(bwd_decay(decays, row, u0 + (e >> 1), e & 1u), a.x, a.y, b.x, b.y);
+        }
+        float x[16];
+        acc_read(tmem, BWD_DP, w, x);
+        tmem_ld_wait();
+        bwd_f32_put16(dp, row, c0, x);
+    }
+    sync();
+    const int r = tid >> 3;
+    const uint32_t u = tid & 7u;
+    float2 acc[4], F[4];
+    auto start = [&] {
 #pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                    const float2 kf = unpack_half2(kk[e]), qf = unpack_half2(own[e]), gf = unpack_half2(gg[e]);
-                    const float k0 = kf.x * ex2(D[2 * e]), k1 = kf.y * ex2(D[2 * e + 1]);
-                    a = fmaf(qf.x, k0, fmaf(qf.y, k1, a));
-                    acc[2 * e] = fmaf(d, k0, acc[2 * e]);
-                    acc[2 * e + 1] = fmaf(d, k1, acc[2 * e + 1]);
-                    D[2 * e] = fmaf(gf.x, kLog2e, D[2 * e]);
-                    D[2 * e + 1] = fmaf(gf.y, kLog2e, D[2 * e + 1]);
+        for (int e = 0; e < 4; ++e) { acc[e] = two(0.f); F[e] = two(1.f); }
+    };
+    auto decay = [&](uint32_t row_t) {                     // F times the decays of a token
+        const float4 a = ld_shared_f4(bwd_decay(decays, row_t, u, 0)), b = ld_shared_f4(bwd_decay(decays, row_t, u, 1));
+        F[0] = mul2(F[0], make_float2(a.x, a.y)); F[1] = mul2(F[1], make_float2(a.z, a.w));
+        F[2] = mul2(F[2], make_float2(b.x, b.y)); F[3] = mul2(F[3], make_float2(b.z, b.w));
+    };
+    auto unit = [&](uint32_t tile, uint32_t row_t, float2* v) {
+        const uint4 h = ld_shared_v4(sw_unit(tile, row_t, u));
+        v[0] = unpack_half2(h.x); v[1] = unpack_half2(h.y); v[2] = unpack_half2(h.z); v[3] = unpack_half2(h.w);
+    };
+    auto put = [&](int t) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[e] = mul2(acc[e], two(scale));
+        st_shared_f4(bwd_f32(out, at(t), 8u * u), acc[0].x, acc[0].y, acc[1].x, acc[1].y);
+        st_shared_f4(bwd_f32(out, at(t), 8u * u + 4u), acc[2].x, acc[2].y, acc[3].x, acc[3].y);
+    };
+    auto take = [&](uint32_t tile, int slot) {             // a whole array into an accumulator
+        float x[16];
+        bwd_f32_row16(tile, row, c0, x);
+        acc_write(tmem, slot, w, x);
+    };
+    // dk: the queries from each key onwards.  A warp's four pairs of tokens go as far as the longest of them.
+#pragma unroll 1
+    for (int second = 0; second < 2; ++second) {
+        const int j = second ? 63 - r : r, steps = second ? r | 3 : 63 - (r & ~3);
+        start();
+#pragma unroll 4
+        for (int s = 0; s <= steps; ++s) {
+            const int t = min(j + s, 63);
+            if (s > 0) decay(at(t));
+            float2 v[4];
+            unit(tq, at(t), v);
+            const float d = j + s <= 63 ? ld_shared_f(bwd_f32(dp, at(t), at(j))) : 0.f;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[e] = fma2(two(d), mul2(v[e], F[e]), acc[e]);
+        }
+        put(j);
+    }
+    sync();
+    take(out, BWD_DP);
+    sync();
+    // dq, and P in the place of dP: the keys from each query backwards, eight at a time, whose sums over the eight lanes end with one lane
+    // each
+#pragma unroll 1
+    for (int second = 0; second < 2; ++second) {
+        const int i = second ? 63 - r : r, steps = second ? 63 - (r & ~3) : r | 3;
+        float2 q[4];
+        unit(tq, at(i), q);
+        start();
+#pragma unroll 1
+        for (int s0 = 0; s0 <= steps; s0 += 8) {
+            float sum[8];
+            uint4 h[8];
+            float d[8];
+            float4 f[2][2];
+#pragma unroll
+            for (int s = 0; s < 8; ++s) {
+                const int j = max(i - s0 - s, 0);
+                h[s] = ld_shared_v4(sw_unit(tk, at(j), u));
+                d[s] = s0 + s <= i ? ld_shared_f(bwd_f32(dp, at(i), at(j))) : 0.f;
+            }
+#pragma unroll
+            for (int s = 0; s < 8; ++s) {
+                if (s % 2 == 0) {
+#pragma unroll
+                    for (int t = 0; t < 2; ++t) {
+                        const uint32_t row_t = at(max(i - s0 - s - t, 0));
+                        f[t][0] = ld_shared_f4(bwd_decay(decays, row_t, u, 0));
+                        f[t][1] = ld_shared_f4(bwd_decay(decays, row_t, u, 1));
+                    }
+                }
+                float2 v[4] = {unpack_half2(h[s].x), unpack_half2(h[s].y), unpack_half2(h[s].z), unpack_half2(h[s].w)};
+                float2 dot = two(0.f);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    v[e] = mul2(v[e], F[e]);
+                    dot = fma2(q[e], v[e], dot);
+                    acc[e] = fma2(two(d[s]), v[e], acc[e]);
+                }
+                sum[s] = dot.x + dot.y;
+                const float4 fa = f[s % 2][0], fb = f[s % 2][1];
+                F[0] = mul2(F[0], make_float2(fa.x, fa.y)); F[1] = mul2(F[1], make_float2(fa.z, fa.w));
+                F[2] = mul2(F[2], make_float2(fb.x, fb.y)); F[3] = mul2(F[3], make_float2(fb.z, fb.w));
+            }
+#pragma unroll
+            for (int m = 4; m > 0; m >>= 1) {
+                const bool upper = (u & m) != 0;
+#pragma unroll
+                for (int e = 0; e < m; ++e) {
+                    const float give = upper ? sum[e] : sum[e + m], keep = upper ? sum[e + m] : sum[e];
+                    sum[e] = keep + __shfl_xor_sync(0xffffffffu, give, m);
                 }
             }
-            a += __shfl_xor_sync(0xffffffffu, a, 1);
-            a += __shfl_xor_sync(0xffffffffu, a, 2);
-            if ((tid & 3) == 0)
-                asm volatile("st.shared.f32 [%0], %1;" ::"r"(bwd_f32(out, at(i), at(j >= 0 ? j : s))), "f"(a * fq * fk) : "memory");
+            const int j = i - s0 - static_cast<int>(u);    // keys after the query are masked later
+            if (j >= 0) st_shared_f(bwd_f32(dp, at(i), at(j)), sum[0] * fq * fk);
         }
+        put(i);
     }
     sync();
-    bwd_f32_row16(out, row, c0, x);
-    acc_write(tmem, BWD_P, w, x);
-    sync();
+    take(dp, BWD_P);
+    take(out, BWD_DQ_I);
+#pragma unroll 1
+    for (uint32_t hf = 0; hf < 2; ++hf) {
+        float x[8];
+        acc_read8(tmem, BWD_X, w, 8 * hf, x);
+        tmem_ld_wait();
+#pragma unroll 1
+        for (int side = 0; side < 2; ++side) {
+            const uint32_t hi = side ? tk : tq, lo = base + (side ? BwdChunkSmem::kKl : BwdChunkSmem::kQl);
+            const float sign = side ? -kLog2e : kLog2e, add = bwd_log2(side ? fk : fq);
+            const uint4 in = ld_shared_v4(sw_unit(hi, row, u0 + hf));
+            const uint32_t i[4] = {in.x, in.y, in.z, in.w};
+            uint32_t h[4], lw[4];
 #pragma unroll
-    for (int e = 0; e < 16; ++e) acc[e] *= scale;
-    bwd_f32_put16(out, at(i), ch, acc);
-    sync();
-    bwd_f32_row16(out, row, c0, x);
-    acc_write(tmem, BWD_DQ_I, w, x);
-#pragma unroll
-    for (int e = 0; e < 16; ++e) acc[e] = D[e] = 0.f;
-    for (int t = i; t < 64; ++t) {
-        uint32_t qq[8], gg[8];
-        if (t > i) {
-            row16(tg, at(t), cu, gg);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                const float2 gf = unpack_half2(gg[e]);
-                D[2 * e] = fmaf(gf.x, kLog2e, D[2 * e]);
-                D[2 * e + 1] = fmaf(gf.y, kLog2e, D[2 * e + 1]);
+            for (int e = 0; e < 4; ++e) {
+                const float2 f = make_float2(vec[c0 + 8 * hf + 2 * e] + add, vec[c0 + 8 * hf + 2 * e + 1] + add);
+                bwd_split(mul2(unpack_half2(i[e]), ex2_2(fma2(pair_of(x, e), two(sign), f))), h[e], lw[e]);
             }
-        }
-        row16(tq, at(t), cu, qq);
-        const float d = ld_shared_f(bwd_f32(dp, at(t), at(i))) * scale;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            const float2 qf = unpack_half2(qq[e]);
-            acc[2 * e] = fmaf(d, qf.x * ex2(D[2 * e]), acc[2 * e]);
-            acc[2 * e + 1] = fmaf(d, qf.y * ex2(D[2 * e + 1]), acc[2 * e + 1]);
+            st_shared_v4(sw_unit(hi, row, u0 + hf), h[0], h[1], h[2], h[3]);
+            st_shared_v4(sw_unit(lo, row, u0 + hf), lw[0], lw[1], lw[2], lw[3]);
         }
     }
-    sync();
-    bwd_f32_put16(out, at(i), ch, acc);
-    sync();
-    bwd_f32_row16(out, row, c0, x);
-    acc_write(tmem, BWD_DP, w, x);
-    float gsum[16];
-    acc_read(tmem, BWD_X, w, gsum);
-    tmem_ld_wait();
-#pragma unroll
-    for (int e = 0; e < 16; ++e) x[e] = fmaf(gsum[e], kLog2e, vec[c0 + e]);
-    bwd_put_gated(tq, base + BwdChunkSmem::kQl, row, u0, qr, x, 1.f, bwd_log2(fq));
-#pragma unroll
-    for (int e = 0; e < 16; ++e) x[e] = fmaf(gsum[e], -kLog2e, vec[c0 + e]);
-    bwd_put_gated(tk, base + BwdChunkSmem::kKl, row, u0, kr, x, 1.f, bwd_log2(fk));
     tmem_st_wait();
 }
 

@@ -279,6 +279,9 @@ __device__ __forceinline__ float4 ld_shared_f4(uint32_t a) {
 __device__ __forceinline__ void st_shared_f4(uint32_t a, float x, float y, float z, float w) {
     asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
 }
+__device__ __forceinline__ void st_shared_f(uint32_t a, float v) {
+    asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
 __device__ __forceinline__ void st_shared_u16(uint32_t a, uint16_t v) {
     asm volatile("st.shared.b16 [%0], %1;" ::"r"(a), "h"(v) : "memory");
 }

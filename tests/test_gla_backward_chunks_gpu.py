@@ -76,3 +76,11 @@ def test_gradient_sizes(G, do_scale):
     if do_scale > 1:
         assert max(_rel(want[i], got[i]) for i in range(3)) <= 1e-3
     assert _rel(want[3], got[3]) <= 1e-4 and _rel(want[4], got[4]) <= 1e-4
+
+
+@pytest.mark.parametrize("K", [64, 32])
+@pytest.mark.parametrize("grid,direction", [((1, 64), 1), ((7, 13), 2), ((1, 300), 0), ((20, 33), 3)])
+def test_nothing_but_strong_chunks(G, K, grid, direction):
+    q, k, v, _, do, s0, dht = _case(2, grid[0] * grid[1], 3, K, seed=11)
+    x = torch.randn(q.shape, generator=torch.Generator().manual_seed(12))
+    _check(G, q, k, v, torch.nn.functional.logsigmoid(x - 2).half(), do, s0, dht, direction, grid)
