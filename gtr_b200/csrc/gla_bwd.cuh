@@ -42,6 +42,7 @@
 
 namespace gla {
 
+constexpr float kBwdFar = 1e30f;          // log2: stands for the decay by a gate of -inf, finite so that differences are too
 constexpr float kBwdRefLimit = 8.f;       // log2: qt and kt carry factors up to 2^8, see bwd_scale() for the room they have
 
 struct BwdParams {
@@ -125,8 +126,9 @@ struct BwdStateSmem {
     static constexpr int kBytes = kMisc + 1024 + 1024;                                 // misc, alignment
 };
 struct BwdStateMisc {
-    uint64_t full[2], bar_x, bar_inc;
+    uint64_t full[2], bar_x, bar_inc, bar_fix;
     uint32_t tmem, gave_up;
+    uint32_t reset;                   // the chunk has a gate of -inf
     uint32_t top[2][8];               // per warp: largest |k|, |q|, as half2 bits
     alignas(16) float gl[2][64];      // log2 decay of the chunk per channel
 };
@@ -151,7 +153,8 @@ __global__ void __launch_bounds__(kComputeThreads, 2) gla_bwd_state_kernel(const
         mbar_init(smem_u32(&M.full[1]), 1);
         mbar_init(smem_u32(&M.bar_x), 1);
         mbar_init(smem_u32(&M.bar_inc), 1);
-        M.gave_up = 0u;
+        mbar_init(smem_u32(&M.bar_fix), 1);
+        M.gave_up = M.reset = 0u;
         fence_mbar_init();
     }
     if (w == 0) {
@@ -195,6 +198,7 @@ __global__ void __launch_bounds__(kComputeThreads, 2) gla_bwd_state_kernel(const
 
     const uint32_t row = 16u * (w & 3) + (l & 15u), c0 = 32u * (w >> 2) + 16u * (static_cast<uint32_t>(l) >> 4), u0 = c0 >> 3;
     float S[16], dS[16], total = 0.f;          // a state row piece each: channel `row`, columns c0 .. +15
+    uint32_t fixes = 0;
 #pragma unroll
     for (int e = 0; e < 16; ++e) S[e] = dS[e] = 0.f;
     const size_t cslot = static_cast<size_t>(bh) * P.NT;
@@ -220,17 +224,48 @@ __global__ void __launch_bounds__(kComputeThreads, 2) gla_bwd_state_kernel(const
         acc_read(tmem, BWD_AFTER, w, x);
         if (grad) acc_read(tmem, BWD_UP_TO, w, y);
         tmem_ld_wait();
-        if (row == (rev ? 63u : 0u)) {                              // all later gates + its own = the chunk's decay
+        auto chunk_decay = [&] {                                    // all gates after the first row + its own
             uint32_t gr[8];
             row16(tg, row, u0, gr);
+            bool lost = false;
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
                 const float2 gf = unpack_half2(gr[e]);
-                M.gl[st][c0 + 2 * e] = (x[2 * e] + gf.x) * kLog2e;
-                M.gl[st][c0 + 2 * e + 1] = (x[2 * e + 1] + gf.y) * kLog2e;
+                const float2 s = mul2(make_float2(x[2 * e] + gf.x, x[2 * e + 1] + gf.y), two(kLog2e));
+                M.gl[st][c0 + 2 * e] = s.x;
+                M.gl[st][c0 + 2 * e + 1] = s.y;
+                lost = lost || !(s.x > -3e38f) || !(s.y > -3e38f);
             }
-        }
+            return lost;
+        };
+        const bool first_row = row == (rev ? 63u : 0u);
+        if (first_row && chunk_decay()) M.reset = 1u;
         __syncthreads();                                            // every warp's maxima are there
+        if (M.reset != 0u) {                                        // 0 x -inf is no sum: once more from the lowest finite gate
+            uint32_t gr[8];
+            row16(tg, row, u0, gr);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) gr[e] = hmax2_lowest(gr[e]);
+            put16(tg, row, u0, gr);
+            fence_proxy_async_smem();
+            tc_fence_before();
+            __syncthreads();
+            if (tid == 0) M.reset = 0u;
+            if (w == 0 && elect_one()) {
+                tc_fence_after();
+                tile_mma<0, 1>(acc_slot(tmem, BWD_AFTER), after, tg, false);
+                if (grad) tile_mma<0, 1>(acc_slot(tmem, BWD_UP_TO), up_to, tg, false);
+                umma_commit(smem_u32(&M.bar_fix));
+            }
+            __syncwarp();
+            wait_bar(P, M.bar_fix, fixes & 1u, M.gave_up);
+            ++fixes;
+            tc_fence_after();
+            acc_read(tmem, BWD_AFTER, w, x);
+            if (grad) acc_read(tmem, BWD_UP_TO, w, y);
+            tmem_ld_wait();
+            if (first_row) chunk_decay();
+        }
         uint32_t top_k = M.top[0][0], top_q = M.top[1][0];
 #pragma unroll
         for (int j = 1; j < 8; ++j) { top_k = max(top_k, M.top[0][j]); top_q = max(top_q, M.top[1][j]); }
@@ -350,7 +385,7 @@ __device__ __forceinline__ uint32_t bwd_decay(uint32_t tile, uint32_t row, uint3
 // B32 H12 T2048 2490 / 1600, B8 H3 T1600 K = 32 185 / 126 (ordinary ones 189, 64, 475, 43).
 // Out of line.  Its loads ahead are as many as registers allow: with fewer in use the compiler spilt some of the ordinary chunk's around
 // the call (3 to 6 percent there).
-__device__ __noinline__ void bwd_wide_chunk(uint32_t base, const float* vec, uint32_t tmem, float fq, float fk, float scale,
+__device__ __noinline__ void bwd_wide_chunk(uint32_t base, float* vec, uint32_t tmem, float fq, float fk, float scale,
                                             bool rev) {
     const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
     const uint32_t row = 16u * (w & 3) + (l & 15u), c0 = 32u * (w >> 2) + 16u * (static_cast<uint32_t>(l) >> 4), u0 = c0 >> 3;
@@ -481,27 +516,66 @@ __device__ __noinline__ void bwd_wide_chunk(uint32_t base, const float* vec, uin
     sync();
     take(dp, BWD_P);
     take(out, BWD_DQ_I);
-#pragma unroll 1
-    for (uint32_t hf = 0; hf < 2; ++hf) {
-        float x[8];
-        acc_read8(tmem, BWD_X, w, 8 * hf, x);
-        tmem_ld_wait();
-#pragma unroll 1
-        for (int side = 0; side < 2; ++side) {
-            const uint32_t hi = side ? tk : tq, lo = base + (side ? BwdChunkSmem::kKl : BwdChunkSmem::kQl);
-            const float sign = side ? -kLog2e : kLog2e, add = bwd_log2(side ? fk : fq);
-            const uint4 in = ld_shared_v4(sw_unit(hi, row, u0 + hf));
-            const uint32_t i[4] = {in.x, in.y, in.z, in.w};
-            uint32_t h[4], lw[4];
+    // The factors of what lies outside the chunk, e^G for q and e^(G_L-G) for k, from sums that run one way each.  X and the chunk's middle
+    // would lose what a hard reset leaves of them (at gates of -1000 the fourth digit, at -60000 all), and a gate of -inf has no X.
+    sync();
+    const uint32_t sums = decays;                          // [4][64]: of 16 tokens each
+    {
+        const uint32_t c = tid & 63u;
+        const int first = 16 * (tid >> 6);
+        float g[16], run = 0.f;
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float2 f = make_float2(vec[c0 + 8 * hf + 2 * e] + add, vec[c0 + 8 * hf + 2 * e + 1] + add);
-                bwd_split(mul2(unpack_half2(i[e]), ex2_2(fma2(pair_of(x, e), two(sign), f))), h[e], lw[e]);
-            }
-            st_shared_v4(sw_unit(hi, row, u0 + hf), h[0], h[1], h[2], h[3]);
-            st_shared_v4(sw_unit(lo, row, u0 + hf), lw[0], lw[1], lw[2], lw[3]);
+        for (int t = 0; t < 16; ++t) g[t] = __half2float(__ushort_as_half(ld_shared_u16(tg + sw_f16(at(first + t), c))));
+#pragma unroll
+        for (int t = 0; t < 16; ++t) st_shared_f(bwd_f32(dp, at(first + t), c), run += g[t]);
+        st_shared_f(sums + 256u * (tid >> 6) + 4u * c, run);
+        run = 0.f;
+#pragma unroll
+        for (int t = 15; t >= 0; --t) {
+            st_shared_f(bwd_f32(out, at(first + t), c), run);
+            run += g[t];
         }
     }
+    sync();
+    float x[16], y[16];
+    bwd_f32_row16(dp, row, c0, x);
+    bwd_f32_row16(out, row, c0, y);
+    const uint32_t quarter = (rev ? 63u - row : row) >> 4;
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j) {
+#pragma unroll
+        for (uint32_t e = 0; e < 4; ++e) {
+            const float4 v = ld_shared_f4(sums + 256u * j + 4u * c0 + 16u * e);
+            const float z[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                if (j < quarter) x[4 * e + i] += z[i];
+                if (j > quarter) y[4 * e + i] += z[i];
+            }
+        }
+    }
+    if (tid < 64) {
+        float half = 0.f;
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) half += ld_shared_f(sums + 256u * j + 4u * tid);
+        half *= 0.5f * kLog2e;
+        vec[tid] = half < -2.f * kBwdFar ? -2.f * kBwdFar : half;
+    }
+    sync();
+    uint32_t in[8];
+    row16(tq, row, u0, in);
+    bwd_put_gated(tq, base + BwdChunkSmem::kQl, row, u0, in, x, kLog2e, bwd_log2(fq));
+    row16(tk, row, u0, in);
+    bwd_put_gated(tk, base + BwdChunkSmem::kKl, row, u0, in, y, kLog2e, bwd_log2(fk));
+    // for the outputs: the smaller of the two, which one it is in its last bit; the other is G_L less this one
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+        const bool after = fabsf(y[e]) < fabsf(x[e]);
+        float v = kLog2e * (after ? y[e] : x[e]);
+        v = v < -kBwdFar ? -kBwdFar : v;
+        x[e] = __uint_as_float((__float_as_uint(v) & ~1u) | (after ? 1u : 0u));
+    }
+    acc_write(tmem, BWD_X, w, x);
     tmem_st_wait();
 }
 
@@ -851,7 +925,6 @@ __global__ void __launch_bounds__(kBwdChunkThreads, 2) gla_bwd_chunk_kernel(cons
             const int tok = scan_token(P, P.T, (first + i) * kChunk + (rev ? 63 - static_cast<int>(row) : static_cast<int>(row)));
             const bool live = tok >= 0 && c0 < K;
             const long long at = (static_cast<long long>(b) * P.T + max(tok, 0)) * P.H + h;          // in units of one head's row
-            const float iS = bwd_inverse(fS), idS = bwd_inverse(fdS), ifd = bwd_inverse(fd), ifq = bwd_inverse(fq), ifk = bwd_inverse(fk);
             wait_bar(P, M.bar_o, ph);
             tc_fence_after();
             // ---- outputs, read eight columns at a time, written as whole 32-byte sectors
@@ -859,8 +932,8 @@ __global__ void __launch_bounds__(kBwdChunkThreads, 2) gla_bwd_chunk_kernel(cons
             {
                 float a[8], y[8], g[8], D[16];
                 uint32_t o[8];
-                // one of dk, dq: gate factor 2^(sign X) (2^(sign X + R) for the state part alone in a wide chunk) times the sum
-                // of state part and chunk part
+                // one of dk, dq: gate factor 2^(sign X) (in a wide chunk e^(G_L-G) or e^G, for the state part alone) times the sum of
+                // state part and chunk part
                 auto finish = [&](int slot_s, int slot_i, float cs, float ci, float sign, const uint32_t* in, __half* out) {
 #pragma unroll
                     for (int hf = 0; hf < 2; ++hf) {
@@ -875,9 +948,11 @@ __global__ void __launch_bounds__(kBwdChunkThreads, 2) gla_bwd_chunk_kernel(cons
                                 z = fma2(two(cs), pair_of(a, e), mul2(two(ci), pair_of(y, e)));
                                 z = mul2(z, ex2_2(mul2(pair_of(g, e), two(sign * kLog2e))));
                             } else {
-                                const float2 r = make_float2(M.vec[c0 + 8 * hf + 2 * e], M.vec[c0 + 8 * hf + 2 * e + 1]);
-                                z = mul2(pair_of(a, e), two(cs));
-                                z = fma2(z, ex2_2(fma2(pair_of(g, e), two(sign * kLog2e), r)), pair_of(y, e));
+                                auto factor = [&](int i) {                    // see the end of bwd_wide_chunk
+                                    const bool after = (__float_as_uint(g[i]) & 1u) != 0u;
+                                    return ex2(after == (sign < 0.f) ? g[i] : 2.f * M.vec[c0 + 8 * hf + i] - g[i]);
+                                };
+                                z = fma2(mul2(pair_of(a, e), two(cs)), make_float2(factor(2 * e), factor(2 * e + 1)), pair_of(y, e));
                             }
                             const int at2 = 4 * hf + e;
                             o[at2] = pack_half2(z.x, z.y);
@@ -888,10 +963,10 @@ __global__ void __launch_bounds__(kBwdChunkThreads, 2) gla_bwd_chunk_kernel(cons
                     }
                     if (live) put_row(out + at * K + c0, o);
                 };
-                finish(BWD_DK_S, slot_dk, idS, P.scale * ifd * ifq, -1.f, kr, P.dk);
-                finish(BWD_DQ_S, BWD_DQ_I, P.scale * iS, P.scale * ifd * ifk, 1.f, qr, P.dq);
+                finish(BWD_DK_S, slot_dk, bwd_inverse(fdS), P.scale * bwd_inverse(fd) * bwd_inverse(fq), -1.f, kr, P.dk);
+                finish(BWD_DQ_S, BWD_DQ_I, P.scale * bwd_inverse(fS), P.scale * bwd_inverse(fd) * bwd_inverse(fk), 1.f, qr, P.dq);
                 bwd_f32_put16(r0, row, c0, D);
-                const float2 cs = two(ifk * idS), ci = two(P.scale * ifq * ifk * 8.f);      // 8 = 1 / fp
+                const float2 cs = two(bwd_inverse(fk) * bwd_inverse(fdS)), ci = two(P.scale * bwd_inverse(fq) * bwd_inverse(fk) * 8.f);      // 8 = 1 / fp
 #pragma unroll
                 for (int hf = 0; hf < 2; ++hf) {
                     acc_read8(tmem, BWD_DV_S, w, 8 * hf, a);

@@ -282,6 +282,11 @@ __device__ __forceinline__ void st_shared_f4(uint32_t a, float x, float y, float
 __device__ __forceinline__ void st_shared_f(uint32_t a, float v) {
     asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
 }
+__device__ __forceinline__ uint16_t ld_shared_u16(uint32_t a) {
+    uint16_t v;
+    asm volatile("ld.shared.b16 %0, [%1];" : "=h"(v) : "r"(a));
+    return v;
+}
 __device__ __forceinline__ void st_shared_u16(uint32_t a, uint16_t v) {
     asm volatile("st.shared.b16 [%0], %1;" ::"r"(a), "h"(v) : "memory");
 }

@@ -151,6 +151,12 @@ __device__ __forceinline__ uint32_t hmin2_zero(uint32_t a) {
     return *reinterpret_cast<uint32_t*>(&r);
 }
 
+// -inf becomes the lowest finite value; NaN stays
+__device__ __forceinline__ uint32_t hmax2_lowest(uint32_t a) {
+    __half2 r = __hmax2_nan(*reinterpret_cast<__half2*>(&a), __half2half2(__ushort_as_half(0xfbffu)));
+    return *reinterpret_cast<uint32_t*>(&r);
+}
+
 // One M = 64 accumulator per slot: 64 columns, lanes 0-15 (even slots) or 16-31 (odd) of every quadrant.
 __device__ __forceinline__ uint32_t acc_slot(uint32_t tmem, int slot) {
     return tmem + (static_cast<uint32_t>(16 * (slot & 1)) << 16) + 64u * static_cast<uint32_t>(slot >> 1);
