@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(kComputeThreads, 2) gla_bwd_state_kernel(const
             uint32_t gr[8];
             row16(tg, row, u0, gr);
 #pragma unroll
-            for (int e = 0; e < 8; ++e) gr[e] = hmax2_lowest(gr[e]);
+            for (int e = 0; e < 8; ++e) gr[e] = hmax2_nan(gr[e], 0xfbfffbffu);      // -65504
             put16(tg, row, u0, gr);
             fence_proxy_async_smem();
             tc_fence_before();

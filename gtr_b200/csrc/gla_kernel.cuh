@@ -41,6 +41,10 @@ namespace gla {
 // every channel) is handled that way.  The host folds sqrt(scale) / 4 into each of q and k (the factor 16 comes back
 // in the output epilogue), so fp16 holds inputs of magnitude up to about 2^(18 - kRefLimit) / sqrt(scale).
 constexpr float kRefLimit = 14.f;
+// Beyond a decay of 2^(2 kExtreme) the exact path's sums of gates would lose what matters of them (a hard reset of -60000 leaves two
+// digits, -inf nothing): gates below kHardest, whose decay of 1e-21 no rounding sees, are then taken as kHardest.
+constexpr float kExtreme = 512.f;
+constexpr uint32_t kHardest = 0xd200d200u;               // -48, as a half2
 
 struct Params {
     int B, T, H, NT;
@@ -426,8 +430,8 @@ struct OutSmem {
     static constexpr int kBytes = kMisc + 2048 + 1024;                                 // misc, alignment
 };
 struct OutMisc {
-    uint64_t full, raw, bar_x, bar_p, bar_inc, bar_o;
-    uint32_t tmem, gave_up;
+    uint64_t full, raw, again, bar_x, bar_p, bar_inc, bar_o;
+    uint32_t tmem, gave_up, agains;
     uint32_t wide[2];                 // per chunk parity: some channel decays too much for the common reference
     alignas(16) float vec[2][64];     // log2: half the chunk's total decay per channel
     Sequence sq[2];                   // per chunk parity; written by the thread that asks for the chunk's tiles, before it does
@@ -536,6 +540,7 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
     if (tid == 0) {
         mbar_init(smem_u32(&M.full), 1);
         mbar_init(smem_u32(&M.raw), 1);
+        mbar_init(smem_u32(&M.again), 1);
         mbar_init(smem_u32(&M.bar_x), 1);
         mbar_init(smem_u32(&M.bar_p), 1);
         mbar_init(smem_u32(&M.bar_inc), 1);
@@ -543,7 +548,7 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
         fence_mbar_init();
         fence_proxy_async_smem();
         M.sq[0] = first_sq;
-        M.gave_up = 0u;
+        M.gave_up = M.agains = 0u;
     }
     pdl_wait();
     if (clears && blockIdx.x == 0 && tid == 0) clear_alone(P.ctrl, P.clear);
@@ -658,6 +663,31 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
             ++wides;
             half_row_write(tmem, ACC_S, w, S);                      // out of the registers' way
             tmem_st_wait();
+            if (__syncthreads_or(!(M.vec[p][tid & 63] > -kExtreme))) {
+                at.get(OutSmem::kG, r);
+#pragma unroll
+                for (int e = 0; e < 16; ++e) r[e] = hmax2_nan(r[e], kHardest);
+                at.put(OutSmem::kG, r);
+                fence_proxy_async_smem();
+                tc_fence_before();
+                __syncthreads();
+                if (w == 0 && elect_one()) {
+                    tc_fence_after();
+                    tile_mma<0, 1>(acc_slot(tmem, ACC_X), mat, tg, false);
+                    umma_commit(smem_u32(&M.again));
+                }
+                __syncwarp();
+                wait(M.again, M.agains & 1u);
+                tc_fence_after();
+                half_row_read(tmem, ACC_X, w, x);
+                tmem_ld_wait();
+                if (row == last_row) {
+#pragma unroll
+                    for (int e = 0; e < 32; ++e) M.vec[p][c0 + e] = x[e] * kLog2e;
+                }
+                __syncthreads();
+                if (tid == 0) ++M.agains;
+            }
             gate_wide_chunk(base, M.vec[p], tmem, rev, P.q_exp, P.q_mul);
             half_row_read(tmem, ACC_S, w, S);
             tmem_ld_wait();

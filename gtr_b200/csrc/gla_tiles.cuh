@@ -151,9 +151,9 @@ __device__ __forceinline__ uint32_t hmin2_zero(uint32_t a) {
     return *reinterpret_cast<uint32_t*>(&r);
 }
 
-// -inf becomes the lowest finite value; NaN stays
-__device__ __forceinline__ uint32_t hmax2_lowest(uint32_t a) {
-    __half2 r = __hmax2_nan(*reinterpret_cast<__half2*>(&a), __half2half2(__ushort_as_half(0xfbffu)));
+// the larger of each; NaN stays
+__device__ __forceinline__ uint32_t hmax2_nan(uint32_t a, uint32_t b) {
+    __half2 r = __hmax2_nan(*reinterpret_cast<__half2*>(&a), *reinterpret_cast<__half2*>(&b));
     return *reinterpret_cast<uint32_t*>(&r);
 }
 

@@ -1,0 +1,34 @@
+"""The forward where gates cut the state off among weak ones, several to a chunk, against float64; -inf within a chunk."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("value,T,K,direction,share", [
+    *[(value, *shape) for value in (-30.0, -1000.0, -60000.0)
+      for shape in ((25, 64, 0, 0.05), (64, 32, 1, 0.3), (130, 64, 1, 0.02), (500, 64, 2, 0.03), (1500, 32, 3, 0.3))],
+    (-float("inf"), 20, 64, 1, 0.1), (-float("inf"), 25, 64, 0, 0.05), (-float("inf"), 60, 32, 3, 0.3), (-float("inf"), 64, 64, 2, 0.02),
+])
+@pytest.mark.parametrize("states", [False, True])
+def test_resets(value, T, K, direction, share, states):
+    import gtr_b200 as G
+    from oracle import gla_ref
+    B, H = 2, 3
+    grid = (5, T // 5) if T % 5 == 0 else (4, T // 4) if T % 4 == 0 else (1, T)
+    gen = torch.Generator().manual_seed(T)
+    q, k, v = (torch.randn(B, T, H, d, generator=gen).mul(0.125).half() for d in (K, K, 64))
+    g = torch.nn.functional.logsigmoid(torch.randn(B, T, H, K, generator=gen)).div(16).half()
+    g[torch.rand(B, T, H, K, generator=gen) < share] = value
+    s0 = torch.randn(B, H, K, 64, generator=gen) * 0.25 if states else None
+    want, want_s = gla_ref.gla_scan(*(x.double() for x in (q, k, v, g)), direction=direction, grid_hw=grid, initial_state=s0,
+                                    output_final_state=True, dtype=torch.float64)
+    ws = G.make_workspace(B, T, H, "cuda")
+    y = torch.full((B, T, H, 64), float("nan"), dtype=torch.float16, device="cuda")
+    final = torch.empty(B, H, K, 64, device="cuda")
+    G.chunk_gla_run(*(x.cuda() for x in (q, k, v, g)), K ** -0.5, ws, y, direction=direction, grid_hw=grid,
+                    initial_state=None if s0 is None else s0.cuda(), final_state=final)
+    G.check_status(ws)
+    for w, x, most in ((want, y, 1e-3), (want_s, final, 5e-4)):            # the operator's own bounds
+        x, w = x.cpu().double(), w.double()
+        assert torch.isfinite(x).all() and float((x - w).norm() / w.norm()) <= most
