@@ -749,9 +749,9 @@ int forward_block(const gla_b200_args* a, const MapKey& key, const block_plan::P
                              gla::block::kSmemBytes, args, stream);
 }
 
-// An fp16 tensor of `rank` dimensions, channels innermost, and the box of 64 channels x wide x high that a stage of the SwiGLU
+// An fp16 tensor of `rank` dimensions, channels innermost, and the box of 64 channels x wide x high x images that a stage of the SwiGLU
 // kernel takes of it; what lies outside the tensor reads as zero.
-int dw_map(const void* ptr, int rank, const cuuint64_t* dim, int wide, int high, CUtensorMap* out) {
+int dw_map(const void* ptr, int rank, const cuuint64_t* dim, int wide, int high, int images, CUtensorMap* out) {
     EncodeTiledFn enc = encode_tiled();
     if (!enc) {
         snprintf(g_cuda_err, sizeof(g_cuda_err), "cuTensorMapEncodeTiled is not available from this driver");
@@ -759,7 +759,7 @@ int dw_map(const void* ptr, int rank, const cuuint64_t* dim, int wide, int high,
     }
     cuuint64_t str[3] = {dim[0] * 2, 0, 0};
     for (int i = 1; i < rank - 1; ++i) str[i] = str[i - 1] * dim[i];
-    const cuuint32_t box[4] = {static_cast<cuuint32_t>(gla::kDwSlab), static_cast<cuuint32_t>(wide), static_cast<cuuint32_t>(high), 1};
+    const cuuint32_t box[4] = {static_cast<cuuint32_t>(gla::kDwSlab), static_cast<cuuint32_t>(wide), static_cast<cuuint32_t>(high), static_cast<cuuint32_t>(images)};
     const cuuint32_t one[4] = {1, 1, 1, 1};
     CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, static_cast<cuuint32_t>(rank), const_cast<void*>(ptr), dim, str, box, one,
                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -1300,23 +1300,31 @@ int gla_b200_swiglu_dwconv(const void* gate, const void* y, const void* weight, 
     int rows = 0, strips = 0;
     int64_t tiles = 0, cells = 0;
     for (int n = 1; n <= gla::kDwStrips; ++n) {
-        const int cols = n * gla::kDwRun, r = std::min(gla::kDwStrips / n, gla::kDwCells / (cols + 2) - 2);
+        const int cols = n * gla::kDwRun, r = std::min({gla::kDwStrips / n, gla::kDwCells / (cols + 2) - 2, grid_h});
         if (r < 1) break;
         const int64_t t = static_cast<int64_t>((grid_h + r - 1) / r) * ((grid_w + cols - 1) / cols), c = t * (r + 2) * (cols + 2);
         if (!rows || t < tiles || (t == tiles && c < cells)) { rows = r; strips = n; tiles = t; cells = c; }
     }
-    const int64_t items = B * tiles * ((C + gla::kDwSlab - 1) / gla::kDwSlab);
+    // Where one tile takes a whole grid, as many images as fit, while every SM still gets a block: a stage's turn would otherwise be
+    // spent on a few cells (256 x 8 x 8 x 768: 30 us with one image a stage, 16.5 with three; 256 x 2 x 2 x 1024: 39 and 12 with ten).
+    const int64_t slabs = (C + gla::kDwSlab - 1) / gla::kDwSlab;
+    int images = 1;
+    if (tiles == 1) {
+        const int64_t fit = std::min(gla::kDwStrips / (rows * strips), gla::kDwCells / ((rows + 2) * (strips * gla::kDwRun + 2)));
+        images = static_cast<int>(std::max<int64_t>(std::min(fit, B * slabs / di.sms), 1));
+    }
+    const int64_t items = (B + images - 1) / images * tiles * slabs;
     if (items > 0x7fffffffLL) return GLA_B200_ERR_SHAPE;
     if (int rc = make_context_current()) return rc;
     gla::DwMaps maps;
     const cuuint64_t grid[4] = {static_cast<cuuint64_t>(C), static_cast<cuuint64_t>(grid_w), static_cast<cuuint64_t>(grid_h), static_cast<cuuint64_t>(B)};
     const cuuint64_t taps[2] = {static_cast<cuuint64_t>(C), 9}, one[2] = {static_cast<cuuint64_t>(C), 1};
-    if (int rc = dw_map(y, 4, grid, strips * gla::kDwRun + 2, rows + 2, &maps.y)) return rc;
-    if (int rc = dw_map(gate, 4, grid, strips * gla::kDwRun, rows, &maps.gate)) return rc;
-    if (int rc = dw_map(weight, 2, taps, 9, 1, &maps.weight)) return rc;
-    if (int rc = dw_map(bias ? bias : weight, 2, one, 1, 1, &maps.bias)) return rc;
+    if (int rc = dw_map(y, 4, grid, strips * gla::kDwRun + 2, rows + 2, images, &maps.y)) return rc;
+    if (int rc = dw_map(gate, 4, grid, strips * gla::kDwRun, rows, images, &maps.gate)) return rc;
+    if (int rc = dw_map(weight, 2, taps, 9, 1, 1, &maps.weight)) return rc;
+    if (int rc = dw_map(bias ? bias : weight, 2, one, 1, 1, 1, &maps.bias)) return rc;
     return launch_simple(&gla::swiglu_dwconv_kernel, static_cast<unsigned>(items), gla::kDwThreads, gla::kDwSmem,
-                         static_cast<cudaStream_t>(stream), maps, static_cast<__half*>(out), bias != nullptr, rows, strips, grid_h, grid_w, C);
+                         static_cast<cudaStream_t>(stream), maps, static_cast<__half*>(out), bias != nullptr, images, rows, strips, B, grid_h, grid_w, C);
 }
 
 int gla_b200_swiglu_status(void* stream_v) {

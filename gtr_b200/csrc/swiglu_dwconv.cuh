@@ -41,7 +41,7 @@ __device__ __forceinline__ void dw_fma8(float* to, const uint4& wv, const uint4&
 }
 
 // A CTA per SM with a ring of three stages.  A stage holds, for a slab of 64 channels, a y tile of up to 256 outputs (16 x 16 where
-// the grid is a multiple of that) plus its one-cell halo, the gate tile, and the slab's weights and bias, filled by four
+// the grid is a multiple of that; of several images where one tile takes a whole grid) plus its one-cell halo, the gate tile, and the slab's weights and bias, filled by four
 // TMA copies (cells outside the grid and channels past C read as zero), so that 150 KB per SM are in flight while 16
 // warps work on a stage.  Neighbouring blocks are neighbouring slabs of a tile, so that what is in flight at one time is
 // whole cells.  Memory does not serve all SMs equally: a CTA that is done with its block takes over one that has not been
@@ -115,7 +115,7 @@ __global__ void dw_timeout_selftest_kernel(uint32_t limit_us) {
 }
 
 __global__ void __launch_bounds__(kDwThreads, 1) swiglu_dwconv_kernel(const __grid_constant__ DwMaps maps, __half* __restrict__ out,
-                                                                      bool biased, int rows, int strips, int hg, int wg, int C) {
+                                                                      bool biased, int images, int rows, int strips, int B, int hg, int wg, int C) {
     extern __shared__ uint8_t dw_smem[];
     const uint32_t base = (smem_u32(dw_smem) + 127u) & ~127u, control = base + kDwStages * kDwStageBytes;
     const int tid = threadIdx.x;
@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(kDwThreads, 1) swiglu_dwconv_kernel(const __gr
     }
     __syncthreads();
     pdl_wait();
-    const uint32_t bytes = ((rows + 2) * (cols + 2) + rows * cols + 9 + (biased ? 1 : 0)) * kDwSlab * 2u;
+    const uint32_t bytes = (images * ((rows + 2) * (cols + 2) + rows * cols) + 9 + (biased ? 1 : 0)) * kDwSlab * 2u;
     // thread 0 fills the stages in turn, two items ahead of the work, and asks for the item after each
     int to_fill = 0;
     uint32_t fill_turn = 0, asked = 0;
@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(kDwThreads, 1) swiglu_dwconv_kernel(const __gr
             return;
         }
         const int slab = item % slabs, tile = item / slabs;
-        const int tc = tile % tiles_c, rest = tile / tiles_c, tr = rest % tiles_r, b = rest / tiles_r;
+        const int tc = tile % tiles_c, rest = tile / tiles_c, tr = rest % tiles_r, b = rest / tiles_r * images;
         const uint32_t to = base + s * kDwStageBytes;
         mbar_arrive_expect_tx(full(s), bytes);
         dw_load4(to, &maps.y, full(s), slab * kDwSlab, tc * cols - 1, tr * rows - 1, b, l2_policy_normal());
@@ -172,9 +172,9 @@ __global__ void __launch_bounds__(kDwThreads, 1) swiglu_dwconv_kernel(const __gr
         fill(static_cast<int>(blockIdx.x));
         fill_next();
     }
-    const int ci = tid & 7, trow = (tid >> 3) / strips, tcol = (tid >> 3) % strips * kDwRun;
-    const uint32_t line = (cols + 2) * 128u, y_at = trow * line + tcol * 128u + 16u * ci;
-    const uint32_t gate_at = kDwYBytes + (trow * cols + tcol) * 128u + 16u * ci;
+    const int ci = tid & 7, tall = (tid >> 3) / strips, image = tall / rows, trow = tall - image * rows, tcol = (tid >> 3) % strips * kDwRun;
+    const uint32_t line = (cols + 2) * 128u, y_at = (tall + 2 * image) * line + tcol * 128u + 16u * ci;
+    const uint32_t gate_at = kDwYBytes + (tall * cols + tcol) * 128u + 16u * ci;
     const int CG = C >> 3;
     uint32_t turn = 0;
     for (int s = 0;;) {
@@ -185,10 +185,10 @@ __global__ void __launch_bounds__(kDwThreads, 1) swiglu_dwconv_kernel(const __gr
         asm volatile("ld.shared.b32 %0, [%1];" : "=r"(item) : "r"(item_of(s)) : "memory");
         if (item < 0) break;
         const int slab = item % slabs, tile = item / slabs, cg = slab * (kDwSlab / 8) + ci;
-        const int tc = tile % tiles_c, rest = tile / tiles_c, tr = rest % tiles_r, b = rest / tiles_r;
+        const int tc = tile % tiles_c, rest = tile / tiles_c, tr = rest % tiles_r, b = rest / tiles_r * images + image;
         const int r = tr * rows + trow, c = tc * cols + tcol;
         const uint32_t stage = base + s * kDwStageBytes;
-        if (trow < rows && r < hg && c < wg && cg < CG) {
+        if (image < images && b < B && r < hg && c < wg && cg < CG) {
             uint4 wv[9];
 #pragma unroll
             for (int k = 0; k < 9; ++k) wv[k] = ld_shared_v4(stage + kDwWeights + 128u * k + 16u * ci);
