@@ -840,9 +840,8 @@ static int forward(const gla_b200_args* a, bool block, void* stream_v) {
 
     MapKey key;
     memset(&key, 0, sizeof(key));
-    const void* ptrs[gla::kNumTensors] = {a->q, a->k, a->g, a->v, a->o, nullptr};
-    const int64_t* strides[gla::kNumTensors] = {a->q_stride, a->k_stride, a->g_stride, a->v_stride, a->o_stride,
-                                                a->gate_stride};
+    const void* ptrs[gla::kNumTensors] = {a->q, a->k, a->g, a->v, a->o};
+    const int64_t* strides[gla::kNumTensors] = {a->q_stride, a->k_stride, a->g_stride, a->v_stride, a->o_stride};
     int rc = GLA_B200_OK;
     for (int t = 0; t < gla::kNumTensors; ++t) {
         key.ptr[t] = ptrs[t];
@@ -970,8 +969,8 @@ static int packed_maps(const gla_b200_args* a, gla::Maps* maps, int64_t o_stride
     if (!a->q || !a->k || !a->v || !a->g || !a->o) return GLA_B200_ERR_NULL;
     MapKey key;
     memset(&key, 0, sizeof(key));
-    const void* ptrs[gla::kNumTensors] = {a->q, a->k, a->g, a->v, a->o, nullptr};
-    const int64_t* strides[gla::kNumTensors] = {a->q_stride, a->k_stride, a->g_stride, a->v_stride, a->o_stride, a->gate_stride};
+    const void* ptrs[gla::kNumTensors] = {a->q, a->k, a->g, a->v, a->o};
+    const int64_t* strides[gla::kNumTensors] = {a->q_stride, a->k_stride, a->g_stride, a->v_stride, a->o_stride};
     for (int t = 0; t < gla::kNumTensors; ++t) {
         key.ptr[t] = ptrs[t];
         if (!ptrs[t]) continue;
@@ -1306,7 +1305,7 @@ int gla_b200_swiglu_dwconv(const void* gate, const void* y, const void* weight, 
         if (!rows || t < tiles || (t == tiles && c < cells)) { rows = r; strips = n; tiles = t; cells = c; }
     }
     // Where one tile takes a whole grid, as many images as fit, while every SM still gets a block: a stage's turn would otherwise be
-    // spent on a few cells (256 x 8 x 8 x 768: 30 us with one image a stage, 16.5 with three; 256 x 2 x 2 x 1024: 39 and 12 with ten).
+    // spent on a few cells (256 x 8 x 8 x 768: 30 us with one image a stage, 16.5 with three; 256 x 2 x 2 x 1024: 39 and 12 with thirteen).
     const int64_t slabs = (C + gla::kDwSlab - 1) / gla::kDwSlab;
     int images = 1;
     if (tiles == 1) {

@@ -188,9 +188,7 @@ static_assert(kSmemBytes <= 227 * 1024, "shared memory budget");
 struct ItemInfo {
     int seq, seg, b, h, first_chunk, nchunks, state_pass;
     int publish_end;     // the state after the segment's output pass is what its successors start from
-    int ns;              // segments of the sequence; segment j keeps its states in slot slot0 + j
-    int T, tok0;         // tokens of the sequence, and its first one in the row (0 unless sequences are packed)
-    size_t slot0;
+    size_t slot0;        // segment j of the sequence keeps its states in slot slot0 + j
 };
 
 struct Misc {
@@ -511,9 +509,6 @@ __device__ __forceinline__ void mask_and_store_scores(bool rev, uint32_t a16, ui
 
 __device__ __forceinline__ ItemInfo decode_item(const Params& P, int item) {
     ItemInfo it;
-    it.ns = P.NS;
-    it.T = P.T;
-    it.tok0 = 0;
     const int nseq = P.B * P.H;
     it.seg = item / nseq;
     it.seq = item - it.seg * nseq;
@@ -628,7 +623,7 @@ gla_block_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Para
         tmem_relinquish();
     }
     if (w == kWarpX && l == 0) {
-        for (int t = 0; t < TGATE; ++t) tma_prefetch_desc(&maps.m[t][0]);
+        for (int t = 0; t < kNumTensors; ++t) tma_prefetch_desc(&maps.m[t][0]);
     }
     tc_fence_before();
     __syncthreads();
@@ -844,7 +839,7 @@ gla_block_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Para
                 }
             }
             if (it.publish_end) publish(P.incl + slot * (kD * kD) + hoff, 2u);
-            if (it.seg == it.ns - 1 && P.sT != nullptr && real_row) {
+            if (it.seg == P.NS - 1 && P.sT != nullptr && real_row) {
                 float4* dst = reinterpret_cast<float4*>(P.sT + srow);
 #pragma unroll
                 for (int x4 = 0; x4 < 8; ++x4)
@@ -886,7 +881,7 @@ gla_block_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Para
                     mbar_wait(ctx, &M.full[s], (ctr / kNumStages) & 1u);
                     if (logits) {
                         const int ci = it.first_chunk + ((state_only && kBackwardPrePass) ? it.nchunks - 1 - i : i);
-                        logits_to_log_gates(tg, P.inv_norm, rev, chunk_valid(ci * kChunk, it.T), tw, l);
+                        logits_to_log_gates(tg, P.inv_norm, rev, chunk_valid(ci * kChunk, P.T), tw, l);
                         warp_arrive(&M.g_ready[s], l);
                     }
                     // ---- gate sums of this thread's row and channel half
@@ -1087,7 +1082,7 @@ gla_block_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Para
                     fence_proxy_async_smem();
                     named_bar_sync(bar_id, kTeamThreads);
                     if (storer && elect_one()) {
-                        const Scan scan = {it.T, P.Hc, P.rev};
+                        const Scan scan = {P.T, P.Hc, P.rev};
                         const BoxWalker bw(scan, (it.first_chunk + i) * kChunk);
                         bw.for_each(scan, [&](int id, int r, int c, int row) {
                             tma_store_5d_hint(&maps.m[TO][id], out_tile + static_cast<uint32_t>(row) * 128u, 0, it.h, r, c, it.b, pol_stream);
@@ -1117,7 +1112,7 @@ gla_block_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Para
                 for (int pass = 0; pass < npass; ++pass) {
                     const bool state_only = it.state_pass && pass == 0;
                     const bool back = state_only && kBackwardPrePass;
-                    const Scan scan = {it.T, P.Hc, P.rev};
+                    const Scan scan = {P.T, P.Hc, P.rev};
                     BoxWalker bw(scan, (it.first_chunk + (back ? it.nchunks - 1 : 0)) * kChunk);
                     // tiles of a pre-pass are read again by the output pass; everything else is read once
                     const uint64_t pol = state_only ? pol_keep : pol_stream;

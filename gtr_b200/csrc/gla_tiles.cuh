@@ -21,7 +21,7 @@ constexpr int kComputeThreads = 256;
 constexpr float kLog2e = 1.4426950408889634f;
 
 // tensor ids inside Maps
-enum { TQ = 0, TK = 1, TG = 2, TV = 3, TO = 4, TGATE = 5, kNumTensors = 6 };
+enum { TQ = 0, TK = 1, TG = 2, TV = 3, TO = 4, kNumTensors = 5 };
 constexpr int kNumBoxes = 4;              // box heights 64, 16, 4, 1 rows
 
 // Where the j-th of `parts` nearly equal parts of n things begins, floor(j n / parts), from n = parts * len + rest: no product
