@@ -648,7 +648,6 @@ void fill_params(const gla_b200_args* a, const int64_t* o_stride, uint8_t* ws, c
 }
 
 
-constexpr int64_t kL2Keep = 120ll << 20;
 std::atomic<uint32_t> g_launches{0};
 // The spans' increments (where spans end inside sequences), then the outputs.  `first`: of the call, which clears the status.
 template <class Table>
@@ -657,7 +656,6 @@ int launch_forward(bool gated, const gla::Maps& maps, gla::Params& P, const Tabl
     const int states = P.per > 0 ? P.spans / P.per * (P.per - 1) : P.spans - 1;
     P.alone = states == 0 ? 1 : 0;
     P.clear = first ? g_launches.fetch_add(1, std::memory_order_relaxed) % 0xfffffffeu + 1u : 0u;
-    P.keep = static_cast<int64_t>(P.chunks) * (4 * P.K + 128) * gla::kChunk <= kL2Keep ? 1 : 0;
     void* args[3] = {const_cast<gla::Maps*>(&maps), &P, const_cast<Table*>(&table)};
     if (states > 0)
         if (int rc = launch_overlapped(state_kernel<Table>(logits), states, gla::kFwdThreads, gla::StateSmem::kBytes, args, stream)) return rc;

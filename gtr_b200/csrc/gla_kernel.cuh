@@ -57,7 +57,6 @@ struct Params {
     // Spans: per > 0: `per` nearly equal ones per sequence, NT = per * len_ + longer; per == 0: all chunks in equal ones of len_
     // chunks, the first `longer` of them one chunk longer
     int chunks, spans, per, len_, longer;
-    int keep;            // k, g and v fit the L2: what the state kernel reads is kept there for the output kernel
     int alone;           // no state kernel runs before the output kernel
     uint32_t clear;      // the call's first kernel clears the status: not 0, and another for each launch
     // The output scale is folded into the exponents of the gate factors (q_exp = log2(scale) - 4, half of it on q and half
@@ -307,14 +306,14 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_state_kernel(const __grid_
         const int tensors[2] = {TG, TK};
         const uint32_t tiles[2] = {base + StateSmem::kG + off, base + StateSmem::kK + off};
         mbar_arrive_expect_tx(bar, 2 * kTileBytes);
-        load_chunk(maps, Scan{M.sq.T, P.Hc, P.rev}, c_last - i, M.sq.b, M.sq.h, M.sq.tok0, P.Hc, bar, tensors, tiles, P.keep ? l2_policy_keep() : l2_policy_normal());
+        load_chunk(maps, Scan{M.sq.T, P.Hc, P.rev}, c_last - i, M.sq.b, M.sq.h, M.sq.tok0, P.Hc, bar, tensors, tiles, l2_policy_normal());
     };
     auto load_v = [&](int i) {
         const int tensors[1] = {TV};
         const uint32_t tiles[1] = {tv};
         mbar_arrive_expect_tx(smem_u32(&M.full_v), kTileBytes);
         load_chunk(maps, Scan{M.sq.T, P.Hc, P.rev}, c_last - i, M.sq.b, M.sq.h, M.sq.tok0, P.Hc, smem_u32(&M.full_v), tensors, tiles,
-                   P.keep ? l2_policy_keep() : l2_policy_normal());
+                   l2_policy_normal());
     };
     if (n > 0 && tid == 0) {
         mbar_init(smem_u32(&M.full[0]), 1);
