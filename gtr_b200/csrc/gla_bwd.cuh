@@ -23,9 +23,10 @@
 // puts it where fp16 has both parts normal, so neither tiny nor huge gradients lose bits.  Measured against the float64
 // recurrence: dg 1e-6 relative, the same as the token-by-token kernels these replace.
 // A chunk in which some channel decays by more than 2^(2 kBwdRefLimit) has no common reference that keeps both operands in
-// range; its products within the chunk are computed pair by pair in fp32 from gate differences (bwd_wide_chunk).
+// range; its products within the chunk are computed pair by pair in fp32 from gate differences, and the factors of what lies outside
+// it from sums of gates that run one way each (bwd_wide_chunk).
 //
-// Measured (B200): B4 H12 T6400 K64 187 us (states 52, chunks 143) against 1080 us for three recurrent sweeps in fp32, whose
+// Measured (B200): B4 H12 T6400 K64 191 us (states 54, chunks 143) against 1080 us for three recurrent sweeps in fp32, whose
 // bound was the FMA pipe (500 us); B8 H6 T1600 64 against 285.  HBM alone would take about 115 us at 6.5 TB/s (96 KB per
 // chunk and head in the chunk kernel, 56 KB in the states'); what is left is the latency of the chunk's five dependent
 // tensor-core round trips with two CTAs per SM.

@@ -27,7 +27,8 @@
 // hardware's warp schedulers do the interleaving.  At four, an SM finishes an output chunk every 2.1 thousand cycles and an increment
 // every 1.4 (5 TB/s in both); the L1's data path, which carries shared memory for threads, copies and tensor cores alike, is
 // then two thirds busy.  Measured (us; the one persistent CTA of five specialised warpgroups per SM this replaced in brackets):
-// B1 H6 T1600 16.0 (26.9), B4 H12 T6400 71 (72), B2 H8 T8192 42 (45), B8 H12 T8192 with logits and epilogue 206 (285).  Tried on the
+// B1 H6 T1600 15.6 (26.9), B4 H12 T6400 74 (72, so it has that kernel still), B2 H8 T8192 41 (45), B8 H12 T8192 with logits and epilogue
+// 207, 226 on inputs that no cache holds (285).  Tried on the
 // way: one fused kernel with flags between increments and outputs (79 us at B4 H12 T6400: the wait for the slowest of the
 // predecessors costs more than the second launch), eight warps of 64 registers per CTA (75), the state in tensor memory (82).
 #pragma once

@@ -7,8 +7,8 @@
 // in fp32.  Warp w owns value columns 8 w .. 8 w + 7 of all key rows -- two lanes share the 32-byte sector of a row, so that
 // every load and store moves whole sectors, and no warp waits for another -- and completes the read-out's sum over the
 // rows with a 5-shuffle butterfly.
-// Measured at B32 H12 K64, one token, state in and out: 4.9 us of kernel against 20.4 us for a chunk of which 63 rows are
-// padding (25 MB of state: 3.9 us at the copy rate).
+// Measured at B32 H12 K64, one token, state in and out: 5.7 us a call in a graph of 24 calls whose states no cache holds (12.6 MB each:
+// 1.9 us at the copy rate), against 20.4 us of kernel for a chunk of which 63 rows are padding.
 #pragma once
 
 #include "gla_device.cuh"

@@ -357,9 +357,8 @@ def chunk_gla(q, k, v, g, scale: Optional[float] = None, initial_state: Optional
 def fused_recurrent_gla(q, k, v, gk, scale: Optional[float] = None, initial_state: Optional[torch.Tensor] = None,
                         output_final_state: bool = False, cu_seqlens=None):
     """The call the reference block makes for sequences of at most 64 tokens and for decoding with a cached state
-    (FLA's fused_recurrent_gla, vit_adapter.py:441,560-562).  The chunkwise kernel serves any length from one token
-    up -- a short sequence is one ragged chunk -- and carries the state in fp32 from call to call, so this is the same
-    operator under the name the block expects."""
+    (FLA's fused_recurrent_gla, vit_adapter.py:441,560-562): the same operator under the name the block expects.  Up to 24
+    tokens go token by token through a state in registers, longer sequences chunk by chunk; the state is fp32 either way."""
     return chunk_gla(q, k, v, gk, scale, initial_state, output_final_state, cu_seqlens)
 
 
