@@ -351,9 +351,9 @@ Plan make_plan(int NT, int nseq, int slots, size_t have, bool gated, int segment
 }
 
 // What a plan takes (us): its chunks, one after another on the busiest CTA, kChunkTime[fused epilogue][raw-logit gates] each and kBox more for
-// every copy past the first that it takes to bring a tensor's tile (one thread asks for them all); kItem for each item that
+// every copy past the fourth that it takes to bring a tensor's tile (one thread asks for them all); kItem for each item that
 // is not its first or exchanges states; kLookBack for each segment that a state is looked for in.
-constexpr double kLaunch = 6.0, kItem = 3.5, kLookBack = 0.55, kBox = 0.1, kChunkTime[2][2] = {{1.18, 1.64}, {1.57, 2.08}};
+constexpr double kLaunch = 6.0, kItem = 3.5, kLookBack = 0.55, kBox = 0.09, kChunkTime[2][2] = {{1.18, 1.64}, {1.57, 2.08}};
 double time_of(const Plan& p, int NT, int nseq, int slots, bool gated, bool logits, double boxes) {
     const double pre = gated ? kPlanPrePassGated : kPlanPrePassPlain;
     double work = 0.0, items = 0.0;
@@ -379,7 +379,7 @@ double time_of(const Plan& p, int NT, int nseq, int slots, bool gated, bool logi
         items = static_cast<double>(rounds + more);
         look = p.ns;
     }
-    return kLaunch + (kChunkTime[gated][logits] + kBox * (boxes - 1.0)) * work + kItem * items + kLookBack * std::min(look, 30);
+    return kLaunch + (kChunkTime[gated][logits] + kBox * std::max(boxes - 4.0, 0.0)) * work + kItem * items + kLookBack * std::min(look, 30);
 }
 }  // namespace block_plan
 
@@ -679,18 +679,21 @@ double boxes_per_chunk(int rows, int T) {
 // and column scans; K = 64 and 32) and are off by 8 percent of a time (one standard deviation).  Where the two meet (block kernel /
 // the other two): plain 48 x 50 chunks 40 / 39, 48 x 75 51 / 54, 96 x 48 68 / 64, 192 x 24 60 / 62, 592 x 7 53 / 37; fused with
 // logits 96 x 128 291 / 208, 120 x 128 288 / 264, 144 x 128 288 / 309, 220 x 128 415 / 528, 384 x 128 726 / 670;
-// 48 x 100 on columns of 64, 40, 8 and 3 rows 67 / 73, 87 / 75, 139 / 87 and 402 / 166.
-// It has to be ahead by kMargin (us): with none of it small calls lose up to 20 percent to the models' error, and no call that it serves by
-// more than 3 percent better is lost.  (On gates that send every chunk down the exact path, which the host cannot foresee, the small kernels are four times as fast at any
-// size; GTR's never do.)  A caller's own segments make few long items or many short ones, which the models know less well: the block kernel's, whose
-// unit they are, unless the others are well ahead (12 x 256 chunks by segments of 1, 4, 8, 16, 32: 332 / 425, 115 / 84, 84 / 61, 80 / 88, 75 / 149).
-constexpr double kSplitLaunch = 2.4, kLongChain = 0.03, kSplitBox = 0.055, kSplitUnit[2][2] = {{2.6, 3.1}, {2.95, 3.4}}, kMargin = 3.0, kOwnSegments = 1.2;
+// 48 x 100 on columns of 160, 80, 100, 40, 8 and 3 rows 68 / 73, 71 / 72, 78 / 74, 87 / 75, 139 / 87 and 402 / 166.
+// In calls of less than kSmall (us) it has to be ahead by kMargin: they would lose up to 20 percent to the models' error.  (On gates that
+// send every chunk down the exact path, which the host cannot foresee, the small kernels are four times as fast at any size;
+// GTR's never do.)  A caller's own segments make few long items or many short ones, which the models know less well: the block kernel's,
+// whose unit they are, unless the others are well ahead (12 x 256 chunks by segments of 1, 4, 8, 16, 32: 332 / 425, 115 / 84,
+// 84 / 61, 80 / 88, 75 / 149).  Over 160 other calls of 3 to 160 chunks a sequence this choice is 0 to 60 percent faster than
+// the block kernel alone; in one of fifty the other kernel would be more than 3 percent better (16 at worst).
+constexpr double kSplitLaunch = 2.4, kLongChain = 0.03, kSplitBox = 0.055, kSplitUnit[2][2] = {{2.6, 3.1}, {2.95, 3.4}}, kMargin = 3.0,
+                 kSmall = 40.0, kOwnSegments = 1.2;
 bool block_pays(const block_plan::Plan& plan, const Split& split, int NT, int nseq, int sms, bool gated, bool logits, double boxes, bool own_segments) {
     const int64_t chunks = static_cast<int64_t>(nseq) * NT;
     const double chain = std::max((split.per > 0 ? split.per : static_cast<double>(split.spans) / nseq) - 1.0, 0.0);
-    const double small = kSplitLaunch + (kSplitUnit[gated][logits] + kSplitBox * (boxes - 1.0)) * (split_cost(chunks, nseq, split.per, split.spans, sms) + kLongChain * chain);
+    const double small = kSplitLaunch + (kSplitUnit[gated][logits] + kSplitBox * std::max(boxes - 4.0, 0.0)) * (split_cost(chunks, nseq, split.per, split.spans, sms) + kLongChain * chain);
     const double block = block_plan::time_of(plan, NT, nseq, sms, gated, logits, boxes);
-    return own_segments ? block < kOwnSegments * small : block + kMargin < small;
+    return own_segments ? block < kOwnSegments * small : block + (small < kSmall ? kMargin : 0.0) < small;
 }
 
 // Whether states are written over others that the call reads.
