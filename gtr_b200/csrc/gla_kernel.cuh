@@ -25,10 +25,9 @@
 // 6 thousand cycles with little work in each, so what counts is how many chunks an SM has under way: four CTAs share one
 // (52 KB of shared memory, 128 TMEM columns, four warps of 128 registers), each working on one chunk with two block barriers, and the
 // hardware's warp schedulers do the interleaving.  At four, an SM finishes an output chunk every 2.1 thousand cycles and an increment
-// every 1.4 (5 TB/s in both); the L1's data path, which carries shared memory for threads, copies and tensor cores alike, is
-// then two thirds busy.  Measured (us; the one persistent CTA of five specialised warpgroups per SM this replaced in brackets):
-// B1 H6 T1600 15.6 (26.9), B4 H12 T6400 74 (72, so it has that kernel still), B2 H8 T8192 41 (45), B8 H12 T8192 with logits and epilogue
-// 207, 226 on inputs that no cache holds (285).  Tried on the
+// every 1.3 (5.9 and 5.25 TB/s at B8 H12 T8192, of 6.5); in shorter calls it is the chain's instructions that count, a warp's straight line
+// of them taking some eight cycles each.  Measured (us; the one persistent CTA of five specialised warpgroups per SM this replaced in brackets):
+// B1 H6 T1600 15.5 (26.9), B4 H12 T6400 70 to 72 (72), B2 H8 T8192 42 (45), B8 H12 T8192 with logits and epilogue 203 (285).  Tried on the
 // way: one fused kernel with flags between increments and outputs (79 us at B4 H12 T6400: the wait for the slowest of the
 // predecessors costs more than the second launch), eight warps of 64 registers per CTA (75), the state in tensor memory (82).
 #pragma once
@@ -434,6 +433,10 @@ struct OutMisc {
     uint32_t tmem, gave_up, agains;
     uint32_t wide[2];                 // per chunk parity: some channel decays too much for the common reference
     alignas(16) float vec[2][64];     // log2: half the chunk's total decay per channel
+    // masks of 16 scores, as fp16 pairs: on the diagonal by the row within its group of 16; all kept; none kept.  (Comparing rows and columns
+    // pair by pair was 870 cycles of a chunk's chain on an SM of its own, this is 250.)
+    alignas(16) uint32_t causal[18][8];
+    alignas(16) uint32_t weight[32];  // fused epilogue: w, as fp16 pairs
     Sequence sq[2];                   // per chunk parity; written by the thread that asks for the chunk's tiles, before it does
 };
 static_assert(sizeof(OutMisc) <= 2048, "misc block too large");
@@ -523,6 +526,11 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
         if (clears && blockIdx.x == 0 && tid < 2) P.ctrl[tid] = 0u;
         return;
     }
+    for (int e = tid; e < 18 * 8; e += kFwdThreads) {
+        const int t = e >> 3, c = 2 * (e & 7);
+        const bool lo = t == 16 || (t < 16 && (rev ? c >= t : c <= t)), hi = t == 16 || (t < 16 && (rev ? c + 1 >= t : c + 1 <= t));
+        M.causal[t][e & 7] = (lo ? 0xffffu : 0u) | (hi ? 0xffff0000u : 0u);
+    }
     auto wait = [&](uint64_t& bar, uint32_t parity) {
         volatile uint32_t *f = &M.gave_up, *status = P.ctrl + 1;
         bounded_wait(bar, parity, P.wait_limit_us, [&] { return *f != 0u || (!clears && *status != 0u); },
@@ -553,6 +561,7 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
     pdl_wait();
     if (clears && blockIdx.x == 0 && tid == 0) clear_alone(P.ctrl, P.clear);
     if (tid == 0) load(chunk, M.sq[0], smem_u32(&M.full));           // the first tiles come in while the rest is set up
+    if (kGated && tid < 32) M.weight[tid] = __ldg(reinterpret_cast<const uint32_t*>(P.rms_w) + tid);
     if (w == 1) {
         tmem_alloc(smem_u32(&M.tmem), 128);
         tmem_relinquish();
@@ -564,6 +573,11 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
     const uint32_t last_row = rev ? 0u : 63u;
     const float hk = 0.5f * P.q_exp, hq = P.q_exp - hk;              // k's and q's share of the output scale (log2)
     const bool real_row = row < static_cast<uint32_t>(P.K);
+    // The masks of this thread's two groups of 16 scores: the group of the warp's parity is the one on the diagonal where its half row is
+    const int side = static_cast<int>(half) - (w >> 1);              // 0: the half row crosses the diagonal; otherwise on which side it lies
+    const bool near = rev ? side > 0 : side < 0;
+    const uint32_t causal = smem_u32(M.causal[side == 0 ? l & 15 : near ? 16 : 17]);
+    const uint32_t beside = near || (side == 0 && ((w & 1) != 0) != rev) ? 0xffffffffu : 0u;
     float S[32];                                                     // the state at the chunk's start
     auto initial_state = [&](int at) {
         if (P.s0 != nullptr && real_row) {
@@ -615,6 +629,11 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
             tile_mma<0, 1>(acc_slot(tmem, ACC_X), mat, tg, false);
             umma_commit(smem_u32(&M.bar_x));
         }
+        const __half* gate_row_at = nullptr;
+        if (kGated && tok >= 0) {                                   // this half row of the output gate: into L2 for now
+            gate_row_at = P.gate + M.sq[p].b * P.gate_s[0] + tok * P.gate_s[1] + M.sq[p].h * P.gate_s[2] + c0;
+            prefetch_l2(gate_row_at);
+        }
         float x[32];
         uint32_t r[16];
         at.get(OutSmem::kQ, r);
@@ -625,12 +644,14 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
         if (w == (rev ? 0 : 3)) {                                   // the warp that holds the last row: X there is G_L / 2
             bool far = false;
             if (row == last_row) {
+                float least = 0.f;
 #pragma unroll
-                for (int e = 0; e < 32; ++e) {
-                    const float half_decay = x[e] * kLog2e;
-                    M.vec[p][c0 + e] = half_decay;
-                    far = far || (-half_decay > kRefLimit);
+                for (int e = 0; e < 8; ++e) {
+                    const float2 a = mul2(pair_of(x, 2 * e), two(kLog2e)), b = mul2(pair_of(x, 2 * e + 1), two(kLog2e));
+                    *reinterpret_cast<float4*>(&M.vec[p][c0 + 4 * e]) = make_float4(a.x, a.y, b.x, b.y);
+                    least = fminf(least, fminf(fminf(a.x, a.y), fminf(b.x, b.y)));
                 }
+                far = least < -kRefLimit;
             }
             far = __any_sync(0xffffffffu, far);
             if (l == 0) M.wide[p] = far ? 1u : 0u;
@@ -720,27 +741,17 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
         if (!wide) {
             half_row_read(tmem, ACC_P, w, x);
             tmem_ld_wait();
-            // of a row's four groups of 16 keys, one lies on the diagonal -- the first or the second of a half row, by the warp --
-            // and those on its far side are dropped whole
-            const int lim = static_cast<int>(row) - static_cast<int>(c0);              // of this half row: keep columns <= lim (>= lim reversed)
+            // of a row's four groups of 16 keys, one lies on the diagonal (the first or the second of a half row, by the warp); those on its
+            // near side are kept whole, the others dropped
+            uint32_t m[8];
+            *reinterpret_cast<uint4*>(m) = ld_shared_v4(causal);
+            *reinterpret_cast<uint4*>(m + 4) = ld_shared_v4(causal + 16u);
+            auto group = [&](int first, bool diagonal) {
 #pragma unroll
-            for (int e = 0; e < 16; ++e) r[e] = pack_half2(x[2 * e], x[2 * e + 1]);
-            auto diagonal = [&](int first) {
-#pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                    const int c = first + 2 * e;
-                    const uint32_t both = r[(first >> 1) + e];
-                    r[(first >> 1) + e] = rev ? (c >= lim ? both : c + 1 >= lim ? both & 0xffff0000u : 0u)
-                                              : (c + 1 <= lim ? both : c <= lim ? both & 0xffffu : 0u);
-                }
+                for (int e = 0; e < 8; ++e) r[(first >> 1) + e] = pack_half2(x[first + 2 * e], x[first + 2 * e + 1]) & (diagonal ? m[e] : beside);
             };
-            auto whole = [&](int first) {
-                const uint32_t keep = (rev ? first >= lim : first + 15 <= lim) ? 0xffffffffu : 0u;
-#pragma unroll
-                for (int e = 0; e < 8; ++e) r[(first >> 1) + e] &= keep;
-            };
-            if (w & 1) { whole(0); diagonal(16); }
-            else { diagonal(0); whole(16); }
+            if (w & 1) { group(0, false); group(16, true); }
+            else { group(0, true); group(16, false); }
             at.put(OutSmem::kG, r);
         }
         fence_proxy_async_smem();
@@ -754,7 +765,7 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
         }
         uint4 gate[4];
         if (kGated && tok >= 0) {
-            const uint4* gp = reinterpret_cast<const uint4*>(P.gate + M.sq[p].b * P.gate_s[0] + tok * P.gate_s[1] + M.sq[p].h * P.gate_s[2] + c0);
+            const uint4* gp = reinterpret_cast<const uint4*>(gate_row_at);
 #pragma unroll
             for (int m = 0; m < 4; ++m) gate[m] = __ldg(gp + m);
         }
@@ -783,6 +794,7 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
         // ---- outputs
         wait(M.bar_o, p);
         tc_fence_after();
+        half_row_read(tmem, ACC_P, w, x);
         if (more && elect_one()) {                                  // nothing reads the chunk's tiles any more: each warp asks for one
             const Sequence next = last ? sequence_of(tab, P, chunk + 1) : M.sq[p];
             if (w == 0) {
@@ -795,7 +807,6 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
                        l2_policy_stream());
         }
         __syncwarp();
-        half_row_read(tmem, ACC_P, w, x);
         tmem_ld_wait();
         float mul = P.o_mul;
         if (kGated) {
@@ -808,12 +819,11 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
             mul *= rsqrtf(ss * (P.o_mul * P.o_mul) * (1.f / kD) + P.rms_eps);
         }
         if (tok >= 0) {
-            const uint4* wp = reinterpret_cast<const uint4*>(P.rms_w + c0);
             __half* op = P.o + M.sq[p].b * P.o_s[0] + (M.sq[p].tok0 + tok) * P.o_s[1] + M.sq[p].h * P.o_s[2] + c0;
 #pragma unroll
             for (int m = 0; m < 4; ++m) {
                 uint4 wv = make_uint4(0u, 0u, 0u, 0u);
-                if (kGated) wv = __ldg(wp + m);
+                if (kGated) wv = ld_shared_v4(smem_u32(M.weight) + 2u * c0 + 16u * m);
                 const uint32_t gu[4] = {gate[m].x, gate[m].y, gate[m].z, gate[m].w}, wu[4] = {wv.x, wv.y, wv.z, wv.w};
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
