@@ -508,20 +508,6 @@ __device__ __forceinline__ void gate_wide_chunk(uint32_t base, const float* vec,
     }
 }
 
-// Tensor memory and the matrix of the gate sums, G - G_L / 2.  (As a lambda that captures by reference the same code made the fused kernel 3 percent
-// slower: its loop's registers come out differently.)
-__device__ __forceinline__ void out_set_up(OutMisc& M, uint32_t mat, bool rev, int w) {
-    if (w == 1) {
-        tmem_alloc(smem_u32(&M.tmem), 128);
-        tmem_relinquish();
-    }
-    fill_constant(mat, [&](uint32_t r, uint32_t s) { return (rev ? s >= r : s <= r) ? 0.5f : -0.5f; });
-    fence_proxy_async_smem();
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-}
-
 template <bool kGated, bool kLogits, class Table>
 __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Params P,
                                                                      const __grid_constant__ Table table) {
@@ -572,6 +558,19 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
         M.sq[0] = first_sq;
         M.gave_up = M.agains = 0u;
     }
+    // Tensor memory and the matrix of the gate sums, G - G_L / 2.  (With captures by reference the same code made the fused kernel 3 percent
+    // slower: its loop's registers come out differently.)
+    const auto set_up = [](OutMisc& M, uint32_t mat, bool rev, int w) {
+        if (w == 1) {
+            tmem_alloc(smem_u32(&M.tmem), 128);
+            tmem_relinquish();
+        }
+        fill_constant(mat, [&](uint32_t r, uint32_t s) { return (rev ? s >= r : s <= r) ? 0.5f : -0.5f; });
+        fence_proxy_async_smem();
+        tc_fence_before();
+        __syncthreads();
+        tc_fence_after();
+    };
     // What takes a microsecond to set up is done while the state kernel ends: B1 H6 40x40 15.5 -> 14.9 us, 48 sequences of 25 chunks 27.1 -> 25.7,
     // B2 H8 T8192 42.4 -> 41.5.  Not where no state kernel has run, whose blocks all have their tensor memory when these start: another
     // kernel's may not have theirs yet and would wait for this one's, which waits for them.  And not with the fused epilogue, which
@@ -579,12 +578,12 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
     // What takes a microsecond to set up is done while the state kernel ends (B1 H6 40x40 15.5 -> 15.2 us, B3 H3 25x42 with K = 32 and states 17.7 ->
     // 16.5, 48 sequences of 25 chunks 27.1 -> 25.8, B2 H8 T8192 42.2 -> 41.6).  Not where no state kernel has run, whose blocks all have their
     // tensor memory when these start: another kernel's may not have theirs yet and would wait for this one's, which waits for them.
-    if (!P.alone) out_set_up(M, mat, rev, w);
+    if (!P.alone) set_up(M, mat, rev, w);
     pdl_wait();
     if (clears && blockIdx.x == 0 && tid == 0) clear_alone(P.ctrl, P.clear);
     if (tid == 0) load(chunk, M.sq[0], smem_u32(&M.full));           // the first tiles come in while the rest is set up
     if (kGated && tid < 32) M.weight[tid] = __ldg(reinterpret_cast<const uint32_t*>(P.rms_w) + tid);
-    if (P.alone) out_set_up(M, mat, rev, w);
+    if (P.alone) set_up(M, mat, rev, w);
 
     // This thread's piece of every 64 x 64 array: row `row` (a token, or a key channel of the state), columns c0 .. c0 + 31
     const uint32_t half = static_cast<uint32_t>(l) >> 4, row = 16u * w + (l & 15u), c0 = 32u * half;
