@@ -205,6 +205,8 @@ struct Misc {
     uint32_t wide[kSlots];
     // per chunk and key channel, log2 units: half the chunk's total decay G_L / 2 (output pass) or G_L itself (pre-pass)
     alignas(16) float vec[kSlots][kD];
+    CausalMasks causal;
+    alignas(16) uint32_t weight[32];      // fused epilogue: w, as fp16 pairs (out of global memory it costs every chunk an L2 round trip)
 };
 static_assert(sizeof(Misc) <= kMiscBytes, "misc block too large");
 
@@ -493,14 +495,19 @@ __device__ __noinline__ void logits_to_log_gates(uint32_t tg, float inv_norm, bo
     fence_proxy_async_smem();
 }
 
-// Causal mask along the scan on the 32 score columns j0.. of query row rho (keep key j0 + j at or before the query;
-// at or after it for reversed scans), then the fp16 tile.  Branch-free selects: the two half-warps sit on different
-// sides of the diagonal.
-__device__ __forceinline__ void mask_and_store_scores(bool rev, uint32_t a16, uint32_t rho, uint32_t j0, float* x) {
+// The 32 score columns j0.. of query row rho, causal along the scan, as the fp16 tile.  By selects in the fused variants, whose registers
+// the masks' would not fit into; by masks in the others (B4 H12 80x80 on columns 71.3 -> 68.2 us).
+__device__ __forceinline__ void select_and_store_scores(bool rev, uint32_t a16, uint32_t rho, uint32_t j0, float* x) {
     const int lim = static_cast<int>(rho) - static_cast<int>(j0);
 #pragma unroll
     for (int j = 0; j < 32; ++j) x[j] = (rev ? (j >= lim) : (j <= lim)) ? x[j] : 0.f;
     store_row_f16<4>(a16, rho, j0 >> 3, x);
+}
+__device__ __forceinline__ void mask_and_store_scores(const CausalRow& causal, uint32_t a16, uint32_t rho, uint32_t j0, int tw, const float* x) {
+    uint32_t r[16];
+    causal.mask(tw, x, r);
+#pragma unroll
+    for (uint32_t m = 0; m < 4; ++m) st_shared_v4(sw_unit(a16, rho, (j0 >> 3) + m), r[4 * m], r[4 * m + 1], r[4 * m + 2], r[4 * m + 3]);
 }
 
 __device__ __forceinline__ ItemInfo decode_item(const Params& P, int item) {
@@ -613,6 +620,7 @@ gla_block_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Para
         *reinterpret_cast<__half*>(base_ptr + kOffLmat + o) = __float2half(at_or_before ? 0.5f : -0.5f);
         *reinterpret_cast<__half*>(base_ptr + kOffLmat + kTileBytes + o) = __float2half(at_or_before ? 0.f : -1.f);
     }
+    if (!kGated) M.causal.fill(kRev);
     fence_proxy_async_smem();
     if (w == kWarpProducer) {
         tmem_alloc(smem_u32(&M.tmem_base), kTmemCols);
@@ -626,6 +634,7 @@ gla_block_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Para
     tc_fence_after();
     const uint32_t tmem = __shfl_sync(0xffffffffu, M.tmem_base, 0);
     pdl_wait();
+    if (kGated && tid < 32) M.weight[tid] = __ldg(reinterpret_cast<const uint32_t*>(P.rms_w) + tid);      // (the first item's barrier follows)
     constexpr bool logits = kLogits;
     constexpr bool rev = kRev;
     const float hk = 0.5f * P.q_exp, hq = P.q_exp - hk;       // k's and q's share of the output scale (log2)
@@ -1015,7 +1024,8 @@ gla_block_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Para
                     group_wait(ctx, &M.a_done[team], oturn & 1u, tw, bar_id, kTeamThreads);
                     tc_fence_after();
                     tmem_half_row(tmem, tw, kTmT + 64u * team, x);
-                    mask_and_store_scores(rev, tg, rho, j0, x);
+                    if constexpr (kGated) select_and_store_scores(rev, tg, rho, j0, x);
+                    else mask_and_store_scores(CausalRow(M.causal, tw, l, rev), tg, rho, j0, tw, x);
                     fence_proxy_async_smem();
                     tc_fence_before();
                     if (storer && elect_one()) tma_store_wait_read();   // the team's output tile: its last store has read it
@@ -1060,10 +1070,9 @@ gla_block_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Para
                         ss += __shfl_xor_sync(0xffffffffu, ss, 16);
                         const float rinv = P.o_mul * rsqrtf(ss * (P.o_mul * P.o_mul) * (1.f / kD) + P.rms_eps);
                         if (gp != nullptr) {       // rows past the end of the sequence are never sent out
-                            const uint4* wp = reinterpret_cast<const uint4*>(P.rms_w + j0);
 #pragma unroll
                             for (uint32_t m = 0; m < 4; ++m) {
-                                const uint4 g4 = __ldg(gp + m), w4 = __ldg(wp + m);
+                                const uint4 g4 = __ldg(gp + m), w4 = ld_shared_v4(smem_u32(M.weight) + 2u * j0 + 16u * m);
                                 const uint32_t gu[4] = {g4.x, g4.y, g4.z, g4.w}, wu[4] = {w4.x, w4.y, w4.z, w4.w};
 #pragma unroll
                                 for (int q2 = 0; q2 < 4; ++q2) {

@@ -24,7 +24,7 @@
 // Why this shape.  A chunk is a chain of dependent steps -- tiles, gate sums, gate factors, scores, mask, outputs -- of some
 // 6 thousand cycles with little work in each, so what counts is how many chunks an SM has under way: four CTAs share one
 // (52 KB of shared memory, 128 TMEM columns, four warps of 128 registers), each working on one chunk with two block barriers, and the
-// hardware's warp schedulers do the interleaving.  At four, an SM finishes an output chunk every 2.1 thousand cycles and an increment
+// hardware's warp schedulers do the interleaving.  At four, an SM finishes an output chunk every 1.9 thousand cycles and an increment
 // every 1.3 (5.9 and 5.25 TB/s at B8 H12 T8192, of 6.5); in shorter calls it is the chain's instructions that count, a warp's straight line
 // of them taking some eight cycles each.  Measured (us; the one persistent CTA of five specialised warpgroups per SM this replaced in brackets):
 // B1 H6 T1600 15.5 (26.9), B4 H12 T6400 70 to 72 (72), B2 H8 T8192 42 (45), B8 H12 T8192 with logits and epilogue 203 (285).  Tried on the
@@ -433,9 +433,7 @@ struct OutMisc {
     uint32_t tmem, gave_up, agains;
     uint32_t wide[2];                 // per chunk parity: some channel decays too much for the common reference
     alignas(16) float vec[2][64];     // log2: half the chunk's total decay per channel
-    // masks of 16 scores, as fp16 pairs: on the diagonal by the row within its group of 16; all kept; none kept.  (Comparing rows and columns
-    // pair by pair was 870 cycles of a chunk's chain on an SM of its own, this is 250.)
-    alignas(16) uint32_t causal[18][8];
+    CausalMasks causal;
     alignas(16) uint32_t weight[32];  // fused epilogue: w, as fp16 pairs
     Sequence sq[2];                   // per chunk parity; written by the thread that asks for the chunk's tiles, before it does
 };
@@ -526,11 +524,7 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
         if (clears && blockIdx.x == 0 && tid < 2) P.ctrl[tid] = 0u;
         return;
     }
-    for (int e = tid; e < 18 * 8; e += kFwdThreads) {
-        const int t = e >> 3, c = 2 * (e & 7);
-        const bool lo = t == 16 || (t < 16 && (rev ? c >= t : c <= t)), hi = t == 16 || (t < 16 && (rev ? c + 1 >= t : c + 1 <= t));
-        M.causal[t][e & 7] = (lo ? 0xffffu : 0u) | (hi ? 0xffff0000u : 0u);
-    }
+    M.causal.fill(rev);
     auto wait = [&](uint64_t& bar, uint32_t parity) {
         volatile uint32_t *f = &M.gave_up, *status = P.ctrl + 1;
         bounded_wait(bar, parity, P.wait_limit_us, [&] { return *f != 0u || (!clears && *status != 0u); },
@@ -591,11 +585,7 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
     const uint32_t last_row = rev ? 0u : 63u;
     const float hk = 0.5f * P.q_exp, hq = P.q_exp - hk;              // k's and q's share of the output scale (log2)
     const bool real_row = row < static_cast<uint32_t>(P.K);
-    // The masks of this thread's two groups of 16 scores: the group of the warp's parity is the one on the diagonal where its half row is
-    const int side = static_cast<int>(half) - (w >> 1);              // 0: the half row crosses the diagonal; otherwise on which side it lies
-    const bool near = rev ? side > 0 : side < 0;
-    const uint32_t causal = smem_u32(M.causal[side == 0 ? l & 15 : near ? 16 : 17]);
-    const uint32_t beside = near || (side == 0 && ((w & 1) != 0) != rev) ? 0xffffffffu : 0u;
+    const CausalRow causal(M.causal, w, l, rev);
     float S[32];                                                     // the state at the chunk's start
     auto initial_state = [&](int at) {
         if (P.s0 != nullptr && real_row) {
@@ -754,17 +744,7 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
         if (!wide) {
             half_row_read(tmem, ACC_P, w, x);
             tmem_ld_wait();
-            // of a row's four groups of 16 keys, one lies on the diagonal (the first or the second of a half row, by the warp); those on its
-            // near side are kept whole, the others dropped
-            uint32_t m[8];
-            *reinterpret_cast<uint4*>(m) = ld_shared_v4(causal);
-            *reinterpret_cast<uint4*>(m + 4) = ld_shared_v4(causal + 16u);
-            auto group = [&](int first, bool diagonal) {
-#pragma unroll
-                for (int e = 0; e < 8; ++e) r[(first >> 1) + e] = pack_half2(x[first + 2 * e], x[first + 2 * e + 1]) & (diagonal ? m[e] : beside);
-            };
-            if (w & 1) { group(0, false); group(16, true); }
-            else { group(0, true); group(16, false); }
+            causal.mask(w, x, r);
             at.put(OutSmem::kG, r);
         }
         fence_proxy_async_smem();

@@ -225,6 +225,40 @@ __device__ __forceinline__ void fill_constant(uint32_t tile, F value) {
     }
 }
 
+// Masks of 16 scores, as fp16 pairs: on the diagonal by the row within its group of 16; all kept; none kept.  (Comparing rows and columns
+// pair by pair was 870 cycles of a chunk's chain on an SM of its own, this is 250.)
+struct CausalMasks {
+    alignas(16) uint32_t m[18][8];
+    __device__ __forceinline__ void fill(bool rev) {
+        for (uint32_t e = threadIdx.x; e < 18u * 8u; e += blockDim.x) {
+            const int t = static_cast<int>(e >> 3), c = 2 * static_cast<int>(e & 7u);
+            const bool lo = t == 16 || (t < 16 && (rev ? c >= t : c <= t)), hi = t == 16 || (t < 16 && (rev ? c + 1 >= t : c + 1 <= t));
+            m[t][e & 7u] = (lo ? 0xffffu : 0u) | (hi ? 0xffff0000u : 0u);
+        }
+    }
+};
+// Those of the half row of scores that lane l of the w-th warp of four holds: of its two groups of 16 keys, the one of the warp's parity lies on
+// the diagonal where the half row crosses it; what lies on the near side is kept whole, the rest dropped.
+struct CausalRow {
+    uint32_t at, beside;
+    __device__ __forceinline__ CausalRow(const CausalMasks& masks, int w, int l, bool rev) {
+        const int side = (l >> 4) - (w >> 1);              // 0: the half row crosses the diagonal; otherwise on which side it lies
+        const bool near = rev ? side > 0 : side < 0;
+        at = smem_u32(masks.m[side == 0 ? l & 15 : near ? 16 : 17]);
+        beside = near || (side == 0 && ((w & 1) != 0) != rev) ? 0xffffffffu : 0u;
+    }
+    __device__ __forceinline__ void mask(int w, const float* x, uint32_t* r) const {
+        const uint4 a = ld_shared_v4(at), b = ld_shared_v4(at + 16u);
+        const uint32_t m[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        auto group = [&](int first, bool diagonal) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) r[(first >> 1) + e] = pack_half2(x[first + 2 * e], x[first + 2 * e + 1]) & (diagonal ? m[e] : beside);
+        };
+        if (w & 1) { group(0, false); group(16, true); }
+        else { group(0, true); group(16, false); }
+    }
+};
+
 struct Scan { int T, Hc, rev; };          // what the walk over the boxes needs to know; `T` is the sequence's own length
 
 // One chunk of kN tensors into tiles.  Rows past the sequence are filled with zeros, channels a K = 32 head does not have too.
