@@ -31,4 +31,4 @@ def test_counts(grid, direction, in_place):
     gtr_b200.chunk_gla_run(q, q.clone(), v, g, 1.0, gtr_b200.make_workspace(1, T, H, "cuda"), out, direction=direction, grid_hw=grid,
                            initial_state=state, final_state=final)
     assert torch.equal(out, want)
-    assert torch.equal(final[0, :, 5], v[0].float().sum(0))
+    torch.testing.assert_close(final[0, :, 5], v[0].float().sum(0), rtol=1e-6, atol=0)     # exponentials of whole numbers, a few units of 2^-23
