@@ -206,7 +206,6 @@ struct Misc {
     // per chunk and key channel, log2 units: half the chunk's total decay G_L / 2 (output pass) or G_L itself (pre-pass)
     alignas(16) float vec[kSlots][kD];
     CausalMasks causal;
-    alignas(16) uint32_t weight[32];      // fused epilogue: w, as fp16 pairs (out of global memory it costs every chunk an L2 round trip)
 };
 static_assert(sizeof(Misc) <= kMiscBytes, "misc block too large");
 
@@ -634,7 +633,6 @@ gla_block_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Para
     tc_fence_after();
     const uint32_t tmem = __shfl_sync(0xffffffffu, M.tmem_base, 0);
     pdl_wait();
-    if (kGated && tid < 32) M.weight[tid] = __ldg(reinterpret_cast<const uint32_t*>(P.rms_w) + tid);      // (the first item's barrier follows)
     constexpr bool logits = kLogits;
     constexpr bool rev = kRev;
     const float hk = 0.5f * P.q_exp, hq = P.q_exp - hk;       // k's and q's share of the output scale (log2)
@@ -1070,9 +1068,10 @@ gla_block_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Para
                         ss += __shfl_xor_sync(0xffffffffu, ss, 16);
                         const float rinv = P.o_mul * rsqrtf(ss * (P.o_mul * P.o_mul) * (1.f / kD) + P.rms_eps);
                         if (gp != nullptr) {       // rows past the end of the sequence are never sent out
+                            const uint4* wp = reinterpret_cast<const uint4*>(P.rms_w + j0);
 #pragma unroll
                             for (uint32_t m = 0; m < 4; ++m) {
-                                const uint4 g4 = __ldg(gp + m), w4 = ld_shared_v4(smem_u32(M.weight) + 2u * j0 + 16u * m);
+                                const uint4 g4 = __ldg(gp + m), w4 = __ldg(wp + m);
                                 const uint32_t gu[4] = {g4.x, g4.y, g4.z, g4.w}, wu[4] = {w4.x, w4.y, w4.z, w4.w};
 #pragma unroll
                                 for (int q2 = 0; q2 < 4; ++q2) {
