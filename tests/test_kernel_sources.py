@@ -10,22 +10,63 @@ import pytest
 SRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "gtr_b200", "csrc")
 
 
+def _block(text, i):
+    """End of the block that opens at text[i]."""
+    depth = 0
+    while True:
+        depth += {"{": 1, "}": -1}.get(text[i], 0)
+        i += 1
+        if depth == 0:
+            return i
+
+
+def _text(name):
+    return re.sub(r"//[^\n]*", "", open(os.path.join(SRC, name)).read())
+
+
+def _bodies(text):
+    """(head, body) of every __global__ function."""
+    for m in re.finditer(r"__global__", text):
+        i = text.index("{", text.index(")", text.index("__launch_bounds__", m.start()) if "__launch_bounds__" in text[m.start():m.start() + 80] else m.start()))
+        yield text[m.start():i].strip()[:100], text[i:_block(text, i)]
+
+
 def _kernels():
     """(name, body) of every __global__ function."""
     for name in sorted(os.listdir(SRC)):
-        if not name.endswith((".cu", ".cuh")):
-            continue
-        text = open(os.path.join(SRC, name)).read()
-        text = re.sub(r"//[^\n]*", "", text)
-        for m in re.finditer(r"__global__", text):
-            i = text.index("{", text.index(")", text.index("__launch_bounds__", m.start()) if "__launch_bounds__" in text[m.start():m.start() + 80] else m.start()))
-            depth, j = 0, i
-            while True:
-                depth += {"{": 1, "}": -1}.get(text[j], 0)
-                j += 1
-                if depth == 0:
-                    break
-            yield f"{name}: {text[m.start():i].strip()[:100]}", text[i:j]
+        if name.endswith((".cu", ".cuh")):
+            for head, body in _bodies(_text(name)):
+                yield f"{name}: {head}", body
+
+
+def _body(text, kernel):
+    (body,) = (b for head, b in _bodies(text) if kernel in head)
+    return body
+
+
+def _as_run(body):
+    """The body with every local lambda that allocates tensor memory in the place of its calls: where it is defined says nothing."""
+    while True:
+        for m in re.finditer(r"\bauto\s+(\w+)\s*=\s*\[[^\]]*\]\s*\([^)]*\)\s*\{", body):
+            end = _block(body, m.end() - 1)
+            inner = body[m.end() - 1:end]
+            if "tmem_alloc" in inner:
+                body = body[:m.start()] + re.sub(rf"\b{m.group(1)}\([^;]*\);", lambda _: inner, body[end:])
+                break
+        else:
+            return body
+
+
+def _released_too_early(body):
+    """Whether dependents are released anywhere before every thread knows that the block has its tensor memory."""
+    body = _as_run(body)
+    have = body.index("__syncthreads()", body.rindex("tmem_alloc"))
+    return any(not m.group(1) and m.start() < have for m in re.finditer(r"pdl_release\(\);(\s*return)?", body))
+
+
+def _order(body):
+    """The unconditional and the `P.alone` steps of a body that matter to its neighbours in the stream, in order."""
+    return re.findall(r"(?:if \((!?P\.alone)\) (?:\{\s*if \(w == \d+\) \{\s*)?|(?<=[;}])\s*)(tmem_alloc|pdl_wait|pdl_release)\(", _as_run(body))
 
 
 def test_dependents_are_released_after_the_block_has_its_tensor_memory():
@@ -36,10 +77,42 @@ def test_dependents_are_released_after_the_block_has_its_tensor_memory():
         if "tmem_alloc" not in body:
             continue
         seen += 1
-        have = body.index("__syncthreads()", body.index("tmem_alloc"))       # every thread knows then that the allocation is done
-        for m in re.finditer(r"pdl_release\(\);(\s*return)?", body):
-            assert m.group(1) or m.start() > have, name
+        assert "tmem_alloc" in _as_run(body), name
+        assert not _released_too_early(body), name
     assert seen >= 5
+
+
+OUT_ORDER = [("!P.alone", "tmem_alloc"), ("", "pdl_wait"), ("P.alone", "tmem_alloc"), ("!P.alone", "pdl_release")]
+
+
+def test_the_output_kernel_takes_tensor_memory_early_behind_the_state_kernel_only():
+    """The state kernel's blocks have theirs when they let the output kernel's start; and they wait for what is before them in the stream
+    first, so that none of them holds any while something there still needs it.  An output kernel with another in front of it waits."""
+    text = _text("gla_kernel.cuh")
+    assert _order(_body(text, "gla_out_kernel")) == OUT_ORDER
+    state = _as_run(_body(text, "gla_state_kernel"))
+    assert state.rindex("pdl_wait();") < state.index("tmem_alloc")
+
+
+FIRST, SECOND, RELEASE = "if (!P.alone) set_up(M, mat, rev, w);", "if (P.alone) set_up(M, mat, rev, w);", "if (!P.alone) pdl_release();"
+
+
+@pytest.mark.parametrize("early,old,new", [
+    (True, FIRST, RELEASE + FIRST),
+    (True, RELEASE, RELEASE + FIRST),
+    (True, RELEASE, RELEASE + SECOND),
+    (False, FIRST, "set_up(M, mat, rev, w);"),
+    (False, FIRST, FIRST + SECOND),
+], ids=("release before both", "first below it", "second below it", "unguarded", "second before the wait"))
+def test_sources_that_break_these_rules_are_found(early, old, new):
+    text = _text("gla_kernel.cuh")
+    assert all(text.count(x) == 1 for x in (FIRST, SECOND, RELEASE))
+    moved = [x for x in (FIRST, SECOND, RELEASE) if x in new and x != old]
+    for x in moved:
+        text = text.replace(x, "")
+    body = _body(text.replace(old, new), "gla_out_kernel")
+    assert _released_too_early(body) == early
+    assert _order(body) != OUT_ORDER
 
 
 @pytest.mark.skipif(shutil.which("nvcc") is None and not os.path.exists("/usr/local/cuda/bin/nvcc"), reason="needs nvcc")
