@@ -268,7 +268,10 @@ __device__ __forceinline__ void logits_to_log_gates(const HalfRow& at, uint32_t 
 struct StateSmem {
     // k and g two deep, v (needed last) one
     static constexpr int kK = 0, kG = 2 * kTileBytes, kV = 4 * kTileBytes, kMat = 5 * kTileBytes, kMisc = 6 * kTileBytes;
-    static constexpr int kBytes = kMisc + 1024 + 1024;                                 // misc, alignment
+    // misc, alignment: as much as an output block takes, which moves into the place of one of these while its neighbours still run.  A kilobyte less
+    // and the places of two neighbours had to be free: some SMs were left with three output blocks, and the last of all began when
+    // others had ended (48 x 100 chunks on columns of 4, 8, 12 and 20 rows 121, 111, 108 and 81 us; 92, 83, 81 and 74 with places that fit).
+    static constexpr int kBytes = kMisc + 2048 + 1024;
 };
 struct StateMisc {
     uint64_t full[2], full_v, bar_x, bar_inc;
@@ -428,6 +431,7 @@ struct OutSmem {
     static constexpr int kS16 = 4 * kTileBytes, kMat = 5 * kTileBytes, kMisc = 6 * kTileBytes;
     static constexpr int kBytes = kMisc + 2048 + 1024;                                 // misc, alignment
 };
+static_assert(OutSmem::kBytes == StateSmem::kBytes, "output blocks have to fit where state blocks were");
 struct OutMisc {
     uint64_t full, raw, again, bar_x, bar_p, bar_inc, bar_o;
     uint32_t tmem, gave_up, agains;

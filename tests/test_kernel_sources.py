@@ -115,6 +115,22 @@ def test_sources_that_break_these_rules_are_found(early, old, new):
     assert _order(body) != OUT_ORDER
 
 
+def _compiles(tmp_path, header, lines):
+    source = tmp_path / "check.cu"
+    source.write_text(f'#include "{header}"\n' + "\n".join(lines))
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    run = subprocess.run([nvcc, "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-I", SRC, "-I", os.path.join(SRC, "..", "..", "include"), "-c",
+                          str(source), "-o", str(tmp_path / "check.o")], capture_output=True, text=True)
+    assert run.returncode == 0, run.stderr[-2000:]
+
+
+@pytest.mark.skipif(shutil.which("nvcc") is None and not os.path.exists("/usr/local/cuda/bin/nvcc"), reason="needs nvcc")
+def test_output_blocks_fit_where_state_blocks_were(tmp_path):
+    """Output blocks move in one by one as state blocks leave; four of either fill an SM (1 KB of each block's share is the system's)."""
+    _compiles(tmp_path, "gla_kernel.cuh", ["static_assert(gla::StateSmem::kBytes == gla::OutSmem::kBytes);",
+                                           "static_assert(4 * (gla::OutSmem::kBytes + 1024) <= 228 * 1024);"])
+
+
 @pytest.mark.skipif(shutil.which("nvcc") is None and not os.path.exists("/usr/local/cuda/bin/nvcc"), reason="needs nvcc")
 def test_spans_begin_where_they_should_in_the_longest_sequences(tmp_path):
     """floor(j * chunks / parts) up to 2^30 chunks, at the compiler's evaluation of the kernels' own expression."""
@@ -126,11 +142,6 @@ def test_spans_begin_where_they_should_in_the_longest_sequences(tmp_path):
         parts = rng.randint(1, min(n, 65535))
         cases.append((n, parts, rng.randint(0, parts)))
     lines = [f"static_assert(gla::part_begin({j}, {n} / {parts}, {n} % {parts}, {parts}) == {j * n // parts});" for n, parts, j in cases]
-    source = tmp_path / "parts.cu"
-    source.write_text('#include "gla_tiles.cuh"\n' + "\n".join(lines))
-    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
-    run = subprocess.run([nvcc, "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-I", SRC, "-c", str(source), "-o", str(tmp_path / "parts.o")],
-                         capture_output=True, text=True)
-    assert run.returncode == 0, run.stderr[-2000:]
+    _compiles(tmp_path, "gla_tiles.cuh", lines)
     kernel = open(os.path.join(SRC, "gla_kernel.cuh")).read()
     assert "part_begin(j, P.len_, P.longer, P.per)" in kernel
