@@ -528,7 +528,6 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
         if (clears && blockIdx.x == 0 && tid < 2) P.ctrl[tid] = 0u;
         return;
     }
-    M.causal.fill(rev);
     auto wait = [&](uint64_t& bar, uint32_t parity) {
         volatile uint32_t *f = &M.gave_up, *status = P.ctrl + 1;
         bounded_wait(bar, parity, P.wait_limit_us, [&] { return *f != 0u || (!clears && *status != 0u); },
@@ -556,13 +555,14 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
         M.sq[0] = first_sq;
         M.gave_up = M.agains = 0u;
     }
-    // Tensor memory and the matrix of the gate sums, G - G_L / 2.  (With captures by reference the same code made the fused kernel 3 percent
+    // Tensor memory, the masks and the matrix of the gate sums, G - G_L / 2.  (With captures by reference the same code made the fused kernel 3 percent
     // slower: its loop's registers come out differently.)
     const auto set_up = [](OutMisc& M, uint32_t mat, bool rev, int w) {
         if (w == 1) {
             tmem_alloc(smem_u32(&M.tmem), 128);
             tmem_relinquish();
         }
+        M.causal.fill(rev);
         fill_constant(mat, [&](uint32_t r, uint32_t s) { return (rev ? s >= r : s <= r) ? 0.5f : -0.5f; });
         fence_proxy_async_smem();
         tc_fence_before();
