@@ -388,6 +388,12 @@ __device__ __forceinline__ void store_row_f16(uint32_t tile, uint32_t row, uint3
 //    the stage, written as fp32 into the team's accumulator in TMEM (the score step then treats the chunk like any other);
 //  * q and k rewritten in place with the references R_q = 0 and R_k = G_L (every exponent <= 0).
 // Gate sums are rebuilt from the gate tile with running sums; nothing of this weighs on the common path.
+// kOnePass: the two threads of a query sum a channel half each over all its keys and add up; otherwise each walks them twice, once per channel
+// half, and sums those of its own key half.  The same sums in the same order.  One pass is half the instructions and needs fewer registers (16 sequences
+// of 128 chunks, forward and reversed: 462 and 484 us against 824 and 731, or 985 and 823 where the caller's masks make it spill; fused 389 and 428
+// against 728 and 686), but it is for the plain variants only: next to it the loops of the fused ones, which fetch their instructions
+// from elsewhere then, lose 1 to 4 percent on ordinary gates (B8 H12 T8192 with logits 280 -> 284 to 293, by four ways to write it).
+template <bool kOnePass>
 __device__ __noinline__ void gate_wide_chunk(bool rev, float q_exp, float q_mul, uint32_t stage, uint32_t tmem_a, int w, int l,
                                              uint32_t bar_id) {
     const uint32_t tq = stage, tk = stage + kTileBytes, tg = stage + 2 * kTileBytes;
@@ -396,38 +402,70 @@ __device__ __noinline__ void gate_wide_chunk(bool rev, float q_exp, float q_mul,
     float sres[32];
 #pragma unroll
     for (int x = 0; x < 32; ++x) sres[x] = 0.f;
-    // two passes over the channel halves keep the registers bounded
-#pragma unroll 1
-    for (uint32_t ch = 0; ch < 2; ++ch) {
+    if constexpr (kOnePass) {
         float qv[32], D[32];
 #pragma unroll
         for (uint32_t m = 0; m < 4; ++m) {
-            unpack8(ld_shared_v4(sw_unit(tq, rho, 4u * ch + m)), qv + 8 * m);
+            unpack8(ld_shared_v4(sw_unit(tq, rho, 4u * hf + m)), qv + 8 * m);
 #pragma unroll
             for (int e = 0; e < 8; ++e) D[8 * m + e] = 0.f;
         }
         // walk the keys from the query backwards along the scan: D = G[i] - G[j]
 #pragma unroll 1
-        for (int j = i; j >= 0; --j) {
+        for (int n = 0; n < 64; ++n) {
+            const int j = i - n;
             const uint32_t pj = rev ? 63u - j : static_cast<uint32_t>(j);            // physical key row / column
-            if ((pj >> 5) == hf) {
-                float s = 0.f;
+            float s = 0.f;
+            if (j >= 0) {
 #pragma unroll
                 for (uint32_t m = 0; m < 4; ++m) {
-                    float kv[8];
-                    unpack8(ld_shared_v4(sw_unit(tk, pj, 4u * ch + m)), kv);
+                    float kv[8], gv[8];
+                    unpack8(ld_shared_v4(sw_unit(tk, pj, 4u * hf + m)), kv);
+                    unpack8(ld_shared_v4(sw_unit(tg, pj, 4u * hf + m)), gv);
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) s = fmaf(qv[8 * m + e] * kv[e], ex2(D[8 * m + e]), s);
+                    for (int e = 0; e < 8; ++e) {
+                        s = fmaf(qv[8 * m + e] * kv[e], ex2(D[8 * m + e]), s);
+                        D[8 * m + e] = fmaf(gv[e], kLog2e, D[8 * m + e]);   // the next key's gap to the query grows by this key's own gate
+                    }
                 }
-                sres[pj & 31u] += s;
             }
-            // next key is one step earlier: its gap to the query grows by this key's own gate
+            s += __shfl_xor_sync(0xffffffffu, s, 16);
+            if (j >= 0 && (pj >> 5) == hf) sres[pj & 31u] = s;
+        }
+    } else {
+        // two passes over the channel halves keep the registers bounded
+#pragma unroll 1
+        for (uint32_t ch = 0; ch < 2; ++ch) {
+            float qv[32], D[32];
 #pragma unroll
             for (uint32_t m = 0; m < 4; ++m) {
-                float gv[8];
-                unpack8(ld_shared_v4(sw_unit(tg, pj, 4u * ch + m)), gv);
+                unpack8(ld_shared_v4(sw_unit(tq, rho, 4u * ch + m)), qv + 8 * m);
 #pragma unroll
-                for (int e = 0; e < 8; ++e) D[8 * m + e] = fmaf(gv[e], kLog2e, D[8 * m + e]);
+                for (int e = 0; e < 8; ++e) D[8 * m + e] = 0.f;
+            }
+            // walk the keys from the query backwards along the scan: D = G[i] - G[j]
+#pragma unroll 1
+            for (int j = i; j >= 0; --j) {
+                const uint32_t pj = rev ? 63u - j : static_cast<uint32_t>(j);            // physical key row / column
+                if ((pj >> 5) == hf) {
+                    float s = 0.f;
+#pragma unroll
+                    for (uint32_t m = 0; m < 4; ++m) {
+                        float kv[8];
+                        unpack8(ld_shared_v4(sw_unit(tk, pj, 4u * ch + m)), kv);
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) s = fmaf(qv[8 * m + e] * kv[e], ex2(D[8 * m + e]), s);
+                    }
+                    sres[pj & 31u] += s;
+                }
+                // next key is one step earlier: its gap to the query grows by this key's own gate
+#pragma unroll
+                for (uint32_t m = 0; m < 4; ++m) {
+                    float gv[8];
+                    unpack8(ld_shared_v4(sw_unit(tg, pj, 4u * ch + m)), gv);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) D[8 * m + e] = fmaf(gv[e], kLog2e, D[8 * m + e]);
+                }
             }
         }
     }
@@ -968,7 +1006,7 @@ gla_block_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Para
                     named_bar_sync(bar_id, kTeamThreads);             // the exact-path flag is known to the whole team
                     const bool wide = M.wide[slot] != 0u;
                     if (wide) {
-                        gate_wide_chunk(rev, P.q_exp, P.q_mul, stage, tmT, tw, l, bar_id);
+                        gate_wide_chunk<!kGated>(rev, P.q_exp, P.q_mul, stage, tmT, tw, l, bar_id);
                     } else {
 #pragma unroll
                         for (uint32_t m = 0; m < 4; ++m) {

@@ -1,0 +1,45 @@
+"""The persistent kernel on chunks that decay too strongly for a common reference, weak ones between them, in each of its variants, against
+the CPU oracle."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("fused,logits", ((False, False), (False, True), (True, False), (True, True)))
+@pytest.mark.parametrize("T,K,direction,grid", [
+    (26, 64, 1, None),                           # part of a chunk
+    (65, 32, 0, None),                           # a chunk and a token of another
+    (130, 64, 3, (10, 13)),
+    (130, 64, 2, (13, 10)),
+    (700, 64, 1, None),                          # several chunks to a segment
+    (700, 32, 0, None),
+])
+def test_strong_and_weak_chunks(T, K, direction, grid, fused, logits):
+    import gtr_b200 as G
+    from oracle import c_oracle, gla_ref
+    B, H = 2, 3
+    gen = torch.Generator().manual_seed(T + K)
+    draw = lambda *shape: torch.randn(*shape, generator=gen)
+    q, k, v = (draw(B, T, H, d).mul(0.5).half() for d in (K, K, 64))
+    strong = (torch.arange(T) // 50 % 2 == 0).float().view(1, T, 1, 1)        # runs of 50 tokens, out of step with the chunks of 64
+    x = (draw(B, T, H, K) + 3 - 5 * strong).half()                            # strong: some 2 natural units a token
+    gates = torch.nn.functional.logsigmoid(x.float()).half()
+    s0 = draw(B, H, K, 64)
+    want, want_s = c_oracle.forward(q, k, v, gates, initial_state=s0, output_final_state=True, direction=direction, grid_hw=grid)
+    state = s0.cuda()                                                         # states in place go to this kernel
+    ws = G.make_workspace(B, T, H, "cuda")
+    y = torch.full((B, T, H, 64), float("nan"), dtype=torch.float16, device="cuda")
+    g, norm = (x, 1.0) if logits else (gates, 0.0)
+    inputs = [t.cuda() for t in (q, k, v, g)]
+    kw = dict(direction=direction, grid_hw=grid, initial_state=state, final_state=state)
+    if fused:
+        gate, w = draw(B, T, H, 64).half(), (torch.rand(64, generator=gen) + 0.5).half()
+        want = gla_ref.rmsnorm_swish_gate(want, gate, w, 1e-5)
+        G.chunk_gla_run_gated(*inputs, gate.cuda(), w.cuda(), K ** -0.5, 1e-5, ws, y, norm, **kw)
+    else:
+        G.chunk_gla_run(*inputs, K ** -0.5, ws, y, norm, **kw)
+    G.check_status(ws)
+    m = gla_ref.error_metrics(want, y.float().cpu())
+    assert m["finite"] and m["rel_l2"] <= (1.5e-3 if logits else 1e-3), m    # the operator's own bounds
+    assert float((state.cpu() - want_s).norm() / want_s.norm()) < 5e-4
