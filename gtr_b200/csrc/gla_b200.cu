@@ -162,7 +162,9 @@ size_t exchange_spans(const Split& s) { return s.per == 1 ? 0 : static_cast<size
 // What a split costs, in units of the time one output chunk takes a CTA that has its SM to itself (3.2 us).  Up to four CTAs share
 // an SM and slow one another down: a chunk takes kOut[m] with m of them, kState[m] in the state kernel (measured at 4800 chunks
 // of 48 sequences; the sums below then rank the splits of 150 to 12288 chunks as they were timed, to within a few percent).  A span
-// costs its chunks, kStart once, and kChain for each span of its sequence before it.
+// costs its chunks, kStart once, and kChain for each span of its sequence before it.  (Both are of the time before the output kernel set itself up
+// beside the state kernel's end, which took the most of kStart off the path, and a block's timestamps have since shown up to 0.12 units for
+// one earlier span where L2 is busy.  They have not been fitted again.)
 constexpr double kStart = 0.6, kChain = 0.05, kOut[5] = {0.0, 1.0, 1.29, 1.63, 1.95}, kState[5] = {0.0, 0.375, 0.53, 0.75, 1.05};
 double split_cost(int64_t chunks, int64_t nseq, int per, int64_t spans, int sms) {
     auto run = [&](int64_t ctas, const double* each, double mean, double most) {
@@ -676,16 +678,17 @@ double boxes_per_chunk(int rows, int T) {
 
 // Whether the block kernel serves a call better than the two kernels of gla_kernel.cuh: the two models' times (us) are compared.  They were
 // fitted to 525 calls on both (1 to 944 sequences of 1 to 1500 chunks, up to 49 000 in all; plain, fused and raw-logit; row
-// and column scans; K = 64 and 32) and are off by 8 percent of a time (one standard deviation).  Where the two meet (block kernel /
-// the other two): plain 48 x 50 chunks 40 / 39, 48 x 75 51 / 54, 96 x 48 68 / 64, 192 x 24 60 / 62, 592 x 7 53 / 37; fused with
-// logits 96 x 128 291 / 208, 120 x 128 288 / 264, 144 x 128 288 / 309, 220 x 128 415 / 528, 384 x 128 726 / 670;
-// 48 x 100 on columns of 160, 80, 100, 40, 8 and 3 rows 68 / 73, 71 / 72, 78 / 74, 87 / 75, 139 / 87 and 402 / 166.
+// and column scans; K = 64 and 32) and are off by 8 percent of a time (one standard deviation).  Both kernels have become 0 to 6 percent faster
+// since, the constants are as they were; of the calls below 48 x 50 and the one with segments of 4 go to the slower one.  Where the two meet (block kernel /
+// the other two): plain 48 x 50 chunks 41 / 40, 48 x 75 52 / 54, 96 x 48 66 / 63, 192 x 24 59 / 61, 592 x 7 51 / 38; fused with
+// logits 96 x 128 280 / 202, 120 x 128 285 / 252, 144 x 128 274 / 289, 220 x 128 408 / 480, 384 x 128 717 / 643;
+// 48 x 100 on columns of 160, 80, 100, 40, 8 and 3 rows 66 / 70, 68 / 70, 71 / 71, 81 / 71, 137 / 83 and 398 / 162.
 // In calls of less than kSmall (us) it has to be ahead by kMargin: they would lose up to 20 percent to the models' error.  (On gates that
-// send every chunk down the exact path, which the host cannot foresee, the small kernels are four times as fast at any size;
+// send every chunk down the exact path, which the host cannot foresee, the small kernels are 2.6 times (fused 3.6) as fast at any size;
 // GTR's never do.)  A caller's own segments make few long items or many short ones, which the models know less well: the block kernel's,
-// whose unit they are, unless the others are well ahead (12 x 256 chunks by segments of 1, 4, 8, 16, 32: 332 / 425, 115 / 84,
-// 84 / 61, 80 / 88, 75 / 149).  Over 160 other calls of 3 to 160 chunks a sequence this choice is 0 to 60 percent faster than
-// the block kernel alone; in one of fifty the other kernel would be more than 3 percent better (16 at worst).
+// whose unit they are, unless the others are well ahead (12 x 256 chunks by segments of 1, 4, 8, 16, 32: 325 / 427, 111 / 83,
+// 81 / 61, 76 / 85, 70 / 141).  Over 160 other calls of 3 to 160 chunks a sequence this choice was, when it was fitted, 0 to 60 percent faster
+// than the block kernel alone; in one of fifty the other kernel would have been more than 3 percent better (16 at worst).
 constexpr double kSplitLaunch = 2.4, kLongChain = 0.03, kSplitBox = 0.055, kSplitUnit[2][2] = {{2.6, 3.1}, {2.95, 3.4}}, kMargin = 3.0,
                  kSmall = 40.0, kOwnSegments = 1.2;
 bool block_pays(const block_plan::Plan& plan, const Split& split, int NT, int nseq, int sms, bool gated, bool logits, double boxes, bool own_segments) {

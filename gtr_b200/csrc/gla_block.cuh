@@ -390,7 +390,7 @@ __device__ __forceinline__ void store_row_f16(uint32_t tile, uint32_t row, uint3
 // Gate sums are rebuilt from the gate tile with running sums; nothing of this weighs on the common path.
 // kOnePass: the two threads of a query sum a channel half each over all its keys and add up; otherwise each walks them twice, once per channel
 // half, and sums those of its own key half.  The same sums in the same order.  One pass is half the instructions and needs fewer registers (16 sequences
-// of 128 chunks, forward and reversed: 462 and 484 us against 824 and 731, or 985 and 823 where the caller's masks make it spill; fused 389 and 428
+// of 128 chunks, forward and reversed: 463 and 476 us against 824 and 731, or 985 and 823 where the caller's masks make it spill; fused 389 and 428
 // against 728 and 686), but it is for the plain variants only: next to it the loops of the fused ones, which fetch their instructions
 // from elsewhere then, lose 1 to 4 percent on ordinary gates (B8 H12 T8192 with logits 280 -> 284 to 293, by four ways to write it).
 template <bool kOnePass>
@@ -533,7 +533,8 @@ __device__ __noinline__ void logits_to_log_gates(uint32_t tg, float inv_norm, bo
 }
 
 // The 32 score columns j0.. of query row rho, causal along the scan, as the fp16 tile.  By selects in the fused variants, whose registers
-// the masks' would not fit into; by masks in the others (B4 H12 80x80 on columns 71.3 -> 68.2 us).
+// the masks' would not fit into; by masks in the others, three of whose four spill 4 to 8 bytes a thread with them: 48 x 100 chunks on columns of 80 rows
+// 71.0 -> 67.9 us, on rows 65.2 -> 62.8; raw logits 91.5 -> 91.9, reversed 91.5 -> 89.6, 96 x 48 chunks of them 93.7 -> 92.1 and 94.0 -> 90.8.
 __device__ __forceinline__ void select_and_store_scores(bool rev, uint32_t a16, uint32_t rho, uint32_t j0, float* x) {
     const int lim = static_cast<int>(rho) - static_cast<int>(j0);
 #pragma unroll

@@ -26,8 +26,9 @@
 // (52 KB of shared memory, 128 TMEM columns, four warps of 128 registers), each working on one chunk with two block barriers, and the
 // hardware's warp schedulers do the interleaving.  At four, an SM finishes an output chunk every 1.9 thousand cycles and an increment
 // every 1.3 (5.9 and 5.25 TB/s at B8 H12 T8192, of 6.5); in shorter calls it is the chain's instructions that count, a warp's straight line
-// of them taking some eight cycles each.  Measured (us; the one persistent CTA of five specialised warpgroups per SM this replaced in brackets):
-// B1 H6 T1600 15.5 (26.9), B4 H12 T6400 70 to 72 (72), B2 H8 T8192 42 (45), B8 H12 T8192 with logits and epilogue 203 (285).  Tried on the
+// of them taking some eight cycles each.  Measured (us; gla_block.cuh's persistent CTA of five specialised warpgroups per SM in brackets; inputs of
+// two to six sets in turn, contiguous): B1 H6 T1600 14.9 (23.6), B2 H8 T8192 41.0 (44.5), B8 H12 T8192 with logits and epilogue 202 (280), B4 H12 T6400 68.6 on
+// rows and 70.2 on columns (62.8 and 67.9, so it has that kernel).  Tried on the
 // way: one fused kernel with flags between increments and outputs (79 us at B4 H12 T6400: the wait for the slowest of the
 // predecessors costs more than the second launch), eight warps of 64 registers per CTA (75), the state in tensor memory (82).
 #pragma once
@@ -86,9 +87,10 @@ struct PackedTable {
 };
 struct NoTable {};
 // The same table from offsets that only the GPU has: every block makes its own, in shared memory, from the n + 1 offsets (a load
-// and two scans, about 1 us), so that the launches need not wait for the host to read them.  Offsets that do not rise
+// and two scans), so that the launches need not wait for the host to read them.  Offsets that do not rise
 // from 0 to T leave an empty table, and nothing is computed.  The first kernel's first block writes them to `echo`
 // (pinned host memory: n + 1 offsets, and a one at [kMaxPacked + 1] when they are there), where the host checks them.
+// (16 sequences, 12 heads, 2808 chunks with states: 54.1 us; with a table from the host, which has the offsets, 47.7.)
 struct DeviceTable {
     const void* offsets;                  // n + 1 int32, or int64 where `wide`
     int32_t* echo;
@@ -569,17 +571,14 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
         __syncthreads();
         tc_fence_after();
     };
-    // What takes a microsecond to set up is done while the state kernel ends: B1 H6 40x40 15.5 -> 14.9 us, 48 sequences of 25 chunks 27.1 -> 25.7,
-    // B2 H8 T8192 42.4 -> 41.5.  Not where no state kernel has run, whose blocks all have their tensor memory when these start: another
-    // kernel's may not have theirs yet and would wait for this one's, which waits for them.  And not with the fused epilogue, which
-    // became slower by it (B8 H12 T8192 204 -> 209, B1 47.9 -> 50: its loop is compiled differently).
     // What takes a microsecond to set up is done while the state kernel ends (B1 H6 40x40 15.5 -> 15.2 us, B3 H3 25x42 with K = 32 and states 17.7 ->
-    // 16.5, 48 sequences of 25 chunks 27.1 -> 25.8, B2 H8 T8192 42.2 -> 41.6).  Not where no state kernel has run, whose blocks all have their
-    // tensor memory when these start: another kernel's may not have theirs yet and would wait for this one's, which waits for them.
+    // 16.5, 48 sequences of 25 chunks 27.1 -> 25.8, B2 H8 T8192 42.2 -> 41.6).  It is the allocation that counts: with it after the wait, the blocks that share an
+    // SM began over 8 us instead of 4, as if each came in when the one before had its tensor memory.  Not where no state kernel has run, whose blocks all have
+    // theirs when these start: another kernel's may not have it yet and would wait for this one's, which waits for them.
     if (!P.alone) set_up(M, mat, rev, w);
     pdl_wait();
     if (clears && blockIdx.x == 0 && tid == 0) clear_alone(P.ctrl, P.clear);
-    if (tid == 0) load(chunk, M.sq[0], smem_u32(&M.full));           // the first tiles come in while the rest is set up
+    if (tid == 0) load(chunk, M.sq[0], smem_u32(&M.full));           // (alone: the first tiles come in while the rest is set up)
     if (kGated && tid < 32) M.weight[tid] = __ldg(reinterpret_cast<const uint32_t*>(P.rms_w) + tid);
     if (P.alone) set_up(M, mat, rev, w);
 
