@@ -15,7 +15,7 @@ SRC_DIR = os.path.join(PKG, "csrc")
 INCLUDE = os.path.join(ROOT, "include")
 SOURCES = [os.path.join(SRC_DIR, "gla_b200.cu")]
 HEADERS = [os.path.join(SRC_DIR, name) for name in
-           ("gla_kernel.cuh", "gla_block.cuh", "gla_tiles.cuh", "gla_device.cuh", "gla_step.cuh", "swiglu_dwconv.cuh", "gla_bwd.cuh")]
+           ("gla_kernel.cuh", "gla_block.cuh", "gla_tiles.cuh", "gla_device.cuh", "gla_cluster.cuh", "gla_step.cuh", "swiglu_dwconv.cuh", "gla_bwd.cuh")]
 HEADERS.append(os.path.join(INCLUDE, "gla_b200.h"))
 OUT = os.path.join(PKG, "libgla_b200.so")
 FRONT_SOURCES = [os.path.join(SRC_DIR, "torch_front.cpp")]

@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "gla_kernel.cuh"
+#include "gla_cluster.cuh"
 #include "gla_step.cuh"
 #include "gla_block.cuh"
 #include "swiglu_dwconv.cuh"
@@ -62,6 +63,16 @@ const void* state_kernel(bool logits) {
                   : reinterpret_cast<const void*>(&gla_state_kernel<false, Table>);
 }
 
+// The cluster kernel's; the block kernel's arithmetic only with the fused epilogue.
+const void* cluster_kernel(bool gated, bool logits, bool block) {
+    using gla::gla_cluster_kernel;
+    if (block)
+        return logits ? reinterpret_cast<const void*>(&gla_cluster_kernel<true, true, true>) : reinterpret_cast<const void*>(&gla_cluster_kernel<true, false, true>);
+    if (gated)
+        return logits ? reinterpret_cast<const void*>(&gla_cluster_kernel<true, true, false>) : reinterpret_cast<const void*>(&gla_cluster_kernel<true, false, false>);
+    return logits ? reinterpret_cast<const void*>(&gla_cluster_kernel<false, true, false>) : reinterpret_cast<const void*>(&gla_cluster_kernel<false, false, false>);
+}
+
 // The block kernel's: bit 2 fused epilogue, bit 1 raw-logit gates, bit 0 reversed scan.
 const void* block_kernel(int variant) {
     using gla::block::gla_block_kernel;
@@ -73,9 +84,11 @@ const void* block_kernel(int variant) {
     return table[variant & 7];
 }
 
+constexpr int kClusterSmemMax = 227 * 1024;
 struct DeviceInfo {
     bool ok = false;
     int sms = 0;
+    int clusters[2][gla::kClusterGroups + 1][gla::kClusterMax + 1] = {};       // cluster kernel: how many run at a time, plus 1; 0: not known yet
     bool attr_set = false;
 };
 std::mutex g_mu;
@@ -116,6 +129,11 @@ int device_info(int dev, DeviceInfo* out) {
                          fa.numRegs, (gla::block::kRegBudgetTotal + gla::block::kThreads - 1) / gla::block::kThreads);
                 return GLA_B200_ERR_DEVICE;
             }
+        }
+        for (int v = 0; v < 6; ++v) {
+            const void* k = cluster_kernel(v >= 2, v & 1, v >= 4);
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kClusterSmemMax);
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         }
         const std::pair<const void*, int> others[] = {
             {reinterpret_cast<const void*>(&gla::swiglu_dwconv_kernel), gla::kDwSmem},
@@ -467,17 +485,20 @@ int get_maps(const MapKey& key, gla::Maps* out) {
 
 // A kernel whose blocks may start while its predecessor in the stream drains; it waits (gla::pdl_wait) before it touches memory
 // that anything before it in the stream reads or writes.
-int launch_overlapped(const void* kernel, dim3 ctas, unsigned threads, size_t smem, void** args, cudaStream_t stream) {
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
+int launch_overlapped(const void* kernel, dim3 ctas, unsigned threads, size_t smem, void** args, cudaStream_t stream, int cluster = 1) {
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = ctas;
     cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
     const cudaError_t e = cudaLaunchKernelExC(&cfg, kernel, args);
     if (e != cudaSuccess) { note_cuda("cudaLaunchKernelExC", e); return GLA_B200_ERR_CUDA; }
     return GLA_B200_OK;
@@ -651,13 +672,14 @@ void fill_params(const gla_b200_args* a, const int64_t* o_stride, uint8_t* ws, c
 
 
 std::atomic<uint32_t> g_launches{0};
+uint32_t next_launch() { return g_launches.fetch_add(1, std::memory_order_relaxed) % 0xfffffffeu + 1u; }       // not 0
 // The spans' increments (where spans end inside sequences), then the outputs.  `first`: of the call, which clears the status.
 template <class Table>
 int launch_forward(bool gated, const gla::Maps& maps, gla::Params& P, const Table& table, bool first, cudaStream_t stream) {
     const bool logits = P.inv_norm > 0.f;
     const int states = P.per > 0 ? P.spans / P.per * (P.per - 1) : P.spans - 1;
     P.alone = states == 0 ? 1 : 0;
-    P.clear = first ? g_launches.fetch_add(1, std::memory_order_relaxed) % 0xfffffffeu + 1u : 0u;
+    P.clear = first ? next_launch() : 0u;
     void* args[3] = {const_cast<gla::Maps*>(&maps), &P, const_cast<Table*>(&table)};
     if (states > 0)
         if (int rc = launch_overlapped(state_kernel<Table>(logits), states, gla::kFwdThreads, gla::StateSmem::kBytes, args, stream)) return rc;
@@ -699,10 +721,95 @@ bool block_pays(const block_plan::Plan& plan, const Split& split, int NT, int ns
     return own_segments ? block < kOwnSegments * small : block + (small < kSmall ? kMargin : 0.0) < small;
 }
 
+// The cluster kernel's shape for a call: CTAs per sequence and chunks per CTA; groups = 0: not for it.
+struct ClusterShape {
+    int size = 0, groups = 0, rows = 0, smem = 0;
+};
+// How many clusters of that shape the device runs at a time.
+int clusters_at_a_time(const ClusterShape& s, bool block, int dev) {
+    std::lock_guard<std::mutex> lock(g_mu);
+    int& known = g_dev[dev].clusters[block][s.groups][s.size];
+    if (known == 0) {
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = s.size;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(s.size);
+        cfg.blockDim = dim3(gla::kFwdThreads * s.groups);
+        cfg.dynamicSmemBytes = std::min(gla::ClusterSmem(block, s.groups, s.size * s.groups, s.rows).bytes, kClusterSmemMax);      // of the longest sequence
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, cluster_kernel(true, true, block), &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
+        known = n + 1;
+    }
+    return known - 1;
+}
+// The fewest chunks to a CTA with which all sequences run at once: a chunk more costs 1.5 to 2 us, where a second wave of clusters begins when the first has
+// ended.  One wave is 1.2 to 2.9 times as fast as the kernels it takes calls from, over 1 to 45 sequences of 4 to 48 chunks (us, before / now; plain, fused, with
+// the block kernel's arithmetic): 3 x 4 8.7 / 5.7, 10.3 / 6.6, 14.9 / 7.2; 6 x 16 11.8 / 6.3, 13.5 / 7.4, 25.8 / 9.8; 6 x 25 14.7 / 8.0, 17.7 / 9.2, 28.6 / 13.0;
+// 14 x 25 19.4 / 9.7, 22.9 / 11.2; 7 x 48 19.4 / 10.8, 23.8 / 12.4; 45 x 8 15.6 / 11.5, 17.6 / 12.1.  A second wave pays against the block kernel from ten
+// chunks on (12 x 25 29.6 / 25.8, 30 x 10 24.5 / 23.6; 36 x 8 21.0 / 22.0), against the two small kernels hardly ever (12 x 28 19.4 / 16.3, 18 x 22 16.1 / 17.3).
+// Sequences of up to three chunks stay where they were: two spans or a short walk, 0.5 to 2.5 us more (3 x 3 8.7 / 5.9).
+constexpr int kClusterChunks = 4;
+static_assert(kClusterChunks > gla::kClusterGroups, "clusters of two or more");
+ClusterShape cluster_shape(int NT, int64_t nseq, bool block, int dev) {
+    if (NT < kClusterChunks) return ClusterShape();
+    for (int waves = 1; waves <= (block && NT >= 10 ? 2 : 1); ++waves)
+        for (int m = 1; m <= gla::kClusterGroups; ++m)
+            for (int size = (NT + m - 1) / m; size <= gla::kClusterMax; ++size) {       // (never 1: a CTA by itself is no cluster, it has nobody to copy to)
+                ClusterShape s;
+                s.size = size; s.groups = m; s.rows = (64 + size - 1) / size;
+                s.smem = gla::ClusterSmem(block, m, NT, s.rows).bytes;
+                if (s.smem > kClusterSmemMax) continue;                // more owners have less to keep each
+                if (static_cast<int64_t>(waves) * clusters_at_a_time(s, block, dev) >= nseq) return s;
+                break;
+            }
+    return ClusterShape();
+}
+
 // Whether states are written over others that the call reads.
 bool overlap(const float* in, const float* out, size_t bytes) {
     const uintptr_t x = reinterpret_cast<uintptr_t>(in), y = reinterpret_cast<uintptr_t>(out);
     return x && y && x < y + bytes && y < x + bytes;
+}
+
+int output_gate(const gla_b200_args* a, gla::Params* P) {
+    P->rms_eps = a->rms_eps;
+    P->rms_w = static_cast<const __half*>(a->rms_weight);
+    P->gate = static_cast<const __half*>(a->out_gate);
+    int64_t gs[3];
+    if (int rc = resolve_strides(a->gate_stride, a->T, a->H, gla::kD, gs)) return rc;
+    for (int i = 0; i < 3; ++i) P->gate_s[i] = gs[i];
+    return GLA_B200_OK;
+}
+
+// The operator on the cluster kernel (gla_cluster.cuh); `plan`: with the block kernel's arithmetic.  Of the workspace it needs the status word alone.
+int forward_cluster(const gla_b200_args* a, MapKey key, const int64_t* o_stride, const ClusterShape& shape, const block_plan::Plan* plan, cudaStream_t stream) {
+    key.ptr[gla::TO] = nullptr;                       // outputs are stored from registers
+    memset(key.stride[gla::TO], 0, sizeof(key.stride[gla::TO]));
+    gla::Maps maps;
+    if (int rc = get_maps(key, &maps)) return rc;
+    gla::Params P;
+    memset(&P, 0, sizeof(P));
+    P.B = a->B; P.T = a->T; P.H = a->H; P.NT = num_chunks(a->T); P.K = a->K;
+    P.Hc = key.Hc; P.Wc = key.Wc;
+    P.rev = a->direction & 1;
+    fill_params(a, o_stride, static_cast<uint8_t*>(a->workspace), ws_layout(0), &P);
+    if (a->out_gate)
+        if (int rc = output_gate(a, &P)) return rc;
+    P.alone = 1;
+    P.clear = next_launch();
+    gla::ClusterPlan C;
+    memset(&C, 0, sizeof(C));
+    C.size = shape.size; C.groups = shape.groups; C.rows = shape.rows;
+    if (plan) {
+        C.ns = plan->ns; C.cps = plan->cps;
+    }
+    void* args[3] = {&maps, &P, &C};
+    return launch_overlapped(cluster_kernel(a->out_gate != nullptr, P.inv_norm > 0.f, plan != nullptr), a->B * a->H * shape.size,
+                             gla::kFwdThreads * shape.groups, shape.smem, args, stream, shape.size);
 }
 
 // The operator on the block kernel (gla_block.cuh).
@@ -889,6 +996,13 @@ static int forward(const gla_b200_args* a, bool block, void* stream_v) {
     const bool in_place = overlap(a->initial_state, a->final_state, static_cast<size_t>(nseq) * a->K * gla::kD * sizeof(float));
     if (block || !step) {
         const block_plan::Plan plan = block_plan::make_plan(NT, nseq, di.sms, have, gated, a->segments, in_place);
+        const ClusterShape shape = a->segments == 0 && !(block && (in_place || plan.kind != block_plan::EQUAL)) ? cluster_shape(NT, nseq, block, dev) : ClusterShape();
+        if (shape.groups > 0) {
+            const size_t need = block || in_place ? block_plan::ws_layout(static_cast<size_t>(nseq), static_cast<size_t>(plan.ns)).total
+                                                  : ws_layout(exchange_spans(split)).total;       // what the other kernels would refuse stays refused
+            if (!a->workspace || (reinterpret_cast<uintptr_t>(a->workspace) & 255u) || have < need) return GLA_B200_ERR_WORKSPACE;
+            return forward_cluster(a, key, o_stride, shape, block ? &plan : nullptr, static_cast<cudaStream_t>(stream_v));
+        }
         if (block || in_place || block_pays(plan, split, NT, nseq, di.sms, gated, a->gk_normalizer > 0.f, col ? boxes_per_chunk(gh, a->T) : 1.0, a->segments > 0)) {
             rc = forward_block(a, key, plan, di.sms, static_cast<cudaStream_t>(stream_v));
             if (block || in_place || rc != GLA_B200_ERR_WORKSPACE) return rc;
@@ -930,15 +1044,7 @@ static int forward(const gla_b200_args* a, bool block, void* stream_v) {
     P.rev = a->direction & 1;
     set_split(split, chunks, &P);
     fill_params(a, o_stride, ws, L, &P);
-    if (gated) {
-        P.rms_eps = a->rms_eps;
-        P.rms_w = static_cast<const __half*>(a->rms_weight);
-        P.gate = static_cast<const __half*>(a->out_gate);
-        int64_t gs[3];
-        rc = resolve_strides(a->gate_stride, a->T, a->H, gla::kD, gs);
-        if (rc != GLA_B200_OK) return rc;
-        for (int i = 0; i < 3; ++i) P.gate_s[i] = gs[i];
-    }
+    if (gated && (rc = output_gate(a, &P)) != GLA_B200_OK) return rc;
     return launch_forward(gated, maps, P, gla::NoTable{}, true, static_cast<cudaStream_t>(stream_v));
 }
 

@@ -71,6 +71,15 @@ __device__ __forceinline__ void named_bar_sync(uint32_t id, uint32_t nthreads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
+template <uint32_t kId>
+__device__ __forceinline__ bool named_bar_or(uint32_t nthreads, bool x) {
+    uint32_t any;
+    __syncwarp();
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, %2, %3, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                 : "=r"(any) : "r"(static_cast<uint32_t>(x)), "n"(kId), "r"(nthreads) : "memory");
+    return any != 0;
+}
+
 // ------------------------------------------------------------------ programmatic dependent launch
 // Kernels launched with the programmatic-serialization attribute start while their predecessor drains; wait() returns once
 // everything before this kernel in the stream is complete and visible, release() lets the next such kernel's blocks start.

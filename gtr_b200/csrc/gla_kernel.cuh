@@ -450,9 +450,10 @@ enum { ACC_X = 0, ACC_P = 1, ACC_INC = 2, ACC_S = 3 };          // gate sums; sc
 // values.  The scores A[i][j] = scale / 16 sum_c q[i][c] k[j][c] 2^(G[i][c] - G[j][c]) of the keys at or before each query are
 // computed pair by pair -- two neighbouring lanes share a query, 32 channels each -- and replace the gate tile as the masked fp16
 // tile that the output MMA reads; q and k are then rewritten in place with the references 0 and G_L.  Inlined: a call would make
-// every ordinary chunk save what its registers hold.
-__device__ __forceinline__ void gate_wide_chunk(uint32_t base, const float* vec, uint32_t tmem, bool rev, float q_exp, float q_mul) {
-    const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
+// every ordinary chunk save what its registers hold.  `scores`: the tile for them; `tid`, `sync`: of the four warps that do it.
+template <class Sync>
+__device__ __forceinline__ void gate_wide_chunk(uint32_t base, uint32_t scores, const float* vec, uint32_t tmem, bool rev, float q_exp, float q_mul, int tid, Sync sync) {
+    const int w = tid >> 5, l = tid & 31;
     const uint32_t tq = base + OutSmem::kQ, tk = base + OutSmem::kK, tg = base + OutSmem::kG, scratch = base + OutSmem::kS16;
     auto at = [&](int t) { return static_cast<uint32_t>(rev ? 63 - t : t); };            // row of the chunk's t-th token
     const int i = tid >> 1;
@@ -488,12 +489,12 @@ __device__ __forceinline__ void gate_wide_chunk(uint32_t base, const float* vec,
             if ((tid & 1) == 0) st_shared_u16(scratch + sw_f16(at(i), at(j >= 0 ? j : s)), __half_as_ushort(__float2half_rn(a * q_mul)));
         }
     }
-    __syncthreads();
+    sync();
     const uint32_t half = static_cast<uint32_t>(l) >> 4, row = 16u * w + (l & 15u), c0 = 32u * half;
     const HalfRow mine(base, row, half);
     uint32_t r[16];
     mine.get(OutSmem::kS16, r);
-    mine.put(OutSmem::kG, r);
+    mine.put(scores, r);
     float x[32];
     half_row_read(tmem, ACC_X, w, x);
     tmem_ld_wait();
@@ -715,7 +716,7 @@ __global__ void __launch_bounds__(kFwdThreads, 4) gla_out_kernel(const __grid_co
                 __syncthreads();
                 if (tid == 0) ++M.agains;
             }
-            gate_wide_chunk(base, M.vec[p], tmem, rev, P.q_exp, P.q_mul);
+            gate_wide_chunk(base, OutSmem::kG, M.vec[p], tmem, rev, P.q_exp, P.q_mul, tid, [] { __syncthreads(); });
             half_row_read(tmem, ACC_S, w, S);
             tmem_ld_wait();
             fence_proxy_async_smem();

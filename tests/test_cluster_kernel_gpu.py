@@ -1,0 +1,116 @@
+"""The cluster kernel at the edges of what it serves -- clusters of two to sixteen, one to three chunks a CTA, ragged ends, owners of uneven and of no rows --
+against the CPU oracle, and its block arithmetic against the persistent kernel, to the bit."""
+import ctypes
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+EDGES = [  # B, H, T, K, direction, states, fused, logits, gates
+    (1, 1, 193, 64, 0, True, False, False, "weak"),        # four chunks, the last of one token
+    (1, 3, 256, 32, 1, False, True, True, "weak"),
+    (1, 2, 192, 64, 0, True, False, False, "weak"),        # one too few
+    (2, 3, 11 * 64 - 5, 64, 3, True, True, False, "weak"),   # eleven owners, the last of four rows
+    (1, 2, 15 * 64, 64, 1, True, False, True, "weak"),       # thirteen owners of five, two of none
+    (1, 7, 16 * 64, 64, 2, True, False, False, "weak"),      # sixteen CTAs, as many clusters as fit
+    (1, 8, 16 * 64, 64, 0, False, True, True, "weak"),       # one more: two chunks a CTA
+    (1, 2, 17 * 64 - 63, 32, 3, True, False, True, "weak"),  # a group without a chunk
+    (2, 3, 32 * 64, 64, 1, True, False, False, "weak"),
+    (1, 1, 33 * 64 - 8, 64, 0, True, True, True, "weak"),    # three chunks a CTA
+    (1, 12, 25 * 64, 64, 2, False, False, False, "weak"),    # clusters of nine, of which eight own rows
+    (1, 2, 36 * 64, 64, 3, True, False, False, "weak"),      # sixteen CTAs for memory's sake, four of them without chunks
+    (1, 2, 48 * 64, 64, 1, True, False, True, "weak"),       # the longest
+    (1, 2, 49 * 64, 64, 1, True, False, False, "weak"),      # and one that is too long
+    (15, 3, 6 * 64 - 1, 64, 0, True, False, False, "weak"),  # the most sequences
+    (1, 2, 20 * 64 + 7, 64, 0, True, False, False, "strong"),    # every chunk pair by pair
+    (1, 2, 40 * 64 + 7, 32, 3, True, True, False, "strong"),
+    (1, 1, 7 * 64, 64, 1, True, False, False, "hard"),       # resets beyond 2^1024
+]
+
+
+def _grid(T, direction):
+    return next((h, T // h) for h in range(40, 0, -1) if T % h == 0) if direction >= 2 else None
+
+
+def _gates(kind, shape, gen):
+    if kind == "hard":
+        g = torch.full(shape, -0.05)
+        g[:, 10::40] = -900.0
+        return g.half()
+    return (torch.nn.functional.logsigmoid(torch.randn(shape, generator=gen)) * (2.0 if kind == "strong" else 1 / 16)).half()
+
+
+@pytest.mark.parametrize("block", [False, True], ids=("own arithmetic", "block arithmetic"))
+@pytest.mark.parametrize("B,H,T,K,direction,states,fused,logits,gates", EDGES)
+def test_against_the_oracle(B, H, T, K, direction, states, fused, logits, gates, block):
+    import gtr_b200 as G
+    from gtr_b200 import ops
+    from oracle import c_oracle, gla_ref
+    if block and (not fused or gates == "hard"):
+        pytest.skip("the block arithmetic is the fused operator's")
+    q, k, v, _ = gla_ref.make_inputs(B, T, H, K=K, seed=T)
+    gen = torch.Generator().manual_seed(T)
+    g = log_gates = _gates(gates, (B, T, H, K), gen)
+    norm = 0.0
+    if logits:
+        norm = 16.0
+        g = torch.randn(B, T, H, K, generator=gen).half()
+        log_gates = (torch.nn.functional.logsigmoid(g.float()) / norm).half()
+    states = states and not block
+    s0 = torch.randn(B, H, K, 64, generator=gen) * 0.25 if states else None
+    grid = _grid(T, direction)
+    want, want_s = c_oracle.forward(q, k, v, log_gates, initial_state=s0, output_final_state=True, direction=direction, grid_hw=grid)
+    ws = G.make_workspace(B, T, H, "cuda")
+    ws.fill_(float("nan"))
+    y = torch.full((B, T, H, 64), float("nan"), dtype=torch.float16, device="cuda")
+    x = [t.cuda() for t in (q, k, v, g)]
+    final = torch.full((B, H, K, 64), float("nan"), device="cuda") if states else None
+    kw = dict(direction=direction, grid_hw=grid)
+    if not block:
+        kw.update(initial_state=None if s0 is None else s0.cuda(), final_state=final)
+    if fused:
+        gate, w = torch.randn(B, T, H, 64, generator=gen).half(), (torch.rand(64, generator=gen) + 0.5).half()
+        want = gla_ref.rmsnorm_swish_gate(want, gate, w, 1e-5)
+        (ops.block_gla_gated if block else G.chunk_gla_run_gated)(*x, gate.cuda(), w.cuda(), K ** -0.5, 1e-5, ws, y, norm, **kw)
+    else:
+        G.chunk_gla_run(*x, K ** -0.5, ws, y, norm, **kw)
+    G.check_status(ws)
+    m = gla_ref.error_metrics(want, y.float().cpu())
+    assert m["finite"] and m["rel_l2"] <= 1e-3, m           # the operator's own bounds
+    if states:
+        assert float((final.cpu() - want_s).norm() / want_s.norm()) < 5e-4
+
+
+@pytest.mark.parametrize("B,H,hg,wg,K,direction,cps", [
+    (1, 3, 40, 40, 32, 1, 4), (1, 6, 47, 26, 64, 1, 4), (2, 3, 30, 45, 64, 2, 4), (1, 3, 24, 24, 32, 3, 5), (1, 6, 64, 32, 64, 0, 4), (1, 12, 32, 40, 64, 3, 4),
+    (1, 2, 19, 11, 64, 0, 4),
+])
+def test_block_arithmetic_is_the_persistent_kernels_to_the_bit(B, H, hg, wg, K, direction, cps):
+    """A caller's own segments stay on the persistent kernel: with the length that it would have chosen by itself both have the same plan.  The gates are a
+    backbone's, whose decay over a segment leaves no trace of the order in which that kernel adds up what lies further back."""
+    from gtr_b200 import _lib, ops
+    T = hg * wg
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    widths = (H * K, H * K, H * 64, H * 64, H * K)
+    packed = torch.randn(B, T, sum(widths), generator=gen, device="cuda", dtype=torch.float16)
+    packed[..., :2 * H * K] *= 0.3
+    packed[..., -H * K:] *= 0.05
+    q, k, v, gate, logits = (t.unflatten(-1, (H, -1)) for t in packed.split(widths, dim=-1))
+    w = (torch.rand(64, generator=gen, device="cuda") + 0.5).half()
+    ws = ops.make_workspace(B, T, H, "cuda")
+    outs = []
+    for segments in (0, cps):
+        y = torch.full((B, T, H, 64), float("nan"), dtype=torch.float16, device="cuda")
+        a = _lib.Args()
+        a.q, a.k, a.v, a.g, a.o, a.out_gate, a.rms_weight = (t.data_ptr() for t in (q, k, v, logits, y, gate, w))
+        for name, t in (("q", q), ("k", k), ("v", v), ("g", logits), ("gate", gate)):
+            setattr(a, f"{name}_stride", (ctypes.c_int64 * 3)(*t.stride()[:3]))
+        a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel() * 4
+        a.B, a.T, a.H, a.K, a.V, a.scale, a.gk_normalizer, a.rms_eps = B, T, H, K, 64, K ** -0.5, 16.0, 1e-5
+        a.direction, a.grid_h, a.grid_w, a.segments = direction, hg, wg, segments
+        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        _lib.check(_lib.lib().gla_b200_forward_block(ctypes.byref(a), stream))
+        _lib.check(_lib.lib().gla_b200_check_status(ws.data_ptr(), stream))
+        outs.append(y)
+    assert torch.isfinite(outs[0]).all() and torch.equal(*outs)
