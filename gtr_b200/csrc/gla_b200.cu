@@ -701,12 +701,13 @@ double boxes_per_chunk(int rows, int T) {
 // Whether the block kernel serves a call better than the two kernels of gla_kernel.cuh: the two models' times (us) are compared.  They were
 // fitted to 525 calls on both (1 to 944 sequences of 1 to 1500 chunks, up to 49 000 in all; plain, fused and raw-logit; row
 // and column scans; K = 64 and 32) and are off by 8 percent of a time (one standard deviation).  Both kernels have become 0 to 6 percent faster
-// since, the constants are as they were; of the calls below 48 x 50 and the one with segments of 4 go to the slower one.  Where the two meet (block kernel /
+// since, the block kernel's fused variants 4 to 13 percent; the constants are as they were, and over 92 fused calls of 12 to 384 sequences of 16 to 128 chunks the
+// choice they make is at most 9 percent off the better kernel, 1 on the mean; of the calls below 48 x 50 and the one with segments of 4 go to the slower one.  Where the two meet (block kernel /
 // the other two): plain 48 x 50 chunks 41 / 40, 48 x 75 52 / 54, 96 x 48 66 / 63, 192 x 24 59 / 61, 592 x 7 51 / 38; fused with
-// logits 96 x 128 280 / 202, 120 x 128 285 / 252, 144 x 128 274 / 289, 220 x 128 408 / 480, 384 x 128 717 / 643;
+// logits 96 x 128 248 / 203, 120 x 128 263 / 256, 144 x 128 244 / 290, 220 x 128 403 / 511, 384 x 128 685 / 664;
 // 48 x 100 on columns of 160, 80, 100, 40, 8 and 3 rows 66 / 70, 68 / 70, 71 / 71, 81 / 71, 137 / 83 and 398 / 162.
 // In calls of less than kSmall (us) it has to be ahead by kMargin: they would lose up to 20 percent to the models' error.  (On gates that
-// send every chunk down the exact path, which the host cannot foresee, the small kernels are 2.6 times (fused 3.6) as fast at any size;
+// send every chunk down the exact path, which the host cannot foresee, the small kernels are twice as fast at any size;
 // GTR's never do.)  A caller's own segments make few long items or many short ones, which the models know less well: the block kernel's,
 // whose unit they are, unless the others are well ahead (12 x 256 chunks by segments of 1, 4, 8, 16, 32: 325 / 427, 111 / 83,
 // 81 / 61, 76 / 85, 70 / 141).  Over 160 other calls of 3 to 160 chunks a sequence this choice was, when it was fitted, 0 to 60 percent faster

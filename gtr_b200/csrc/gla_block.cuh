@@ -91,12 +91,6 @@ __device__ __forceinline__ void tma_store_wait_read() {
     asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
 }
 __device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-__device__ __forceinline__ float silu_f(float x) {
-    const float h = 0.5f * x;
-    float t;
-    asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(h));
-    return fmaf(h, t, h);
-}
 __device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* p) {
     uint32_t v;
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -206,6 +200,7 @@ struct Misc {
     // per chunk and key channel, log2 units: half the chunk's total decay G_L / 2 (output pass) or G_L itself (pre-pass)
     alignas(16) float vec[kSlots][kD];
     CausalMasks causal;
+    alignas(16) uint32_t weight[32];         // fused epilogue: w, as fp16 pairs
 };
 static_assert(sizeof(Misc) <= kMiscBytes, "misc block too large");
 
@@ -388,12 +383,8 @@ __device__ __forceinline__ void store_row_f16(uint32_t tile, uint32_t row, uint3
 //    the stage, written as fp32 into the team's accumulator in TMEM (the score step then treats the chunk like any other);
 //  * q and k rewritten in place with the references R_q = 0 and R_k = G_L (every exponent <= 0).
 // Gate sums are rebuilt from the gate tile with running sums; nothing of this weighs on the common path.
-// kOnePass: the two threads of a query sum a channel half each over all its keys and add up; otherwise each walks them twice, once per channel
-// half, and sums those of its own key half.  The same sums in the same order.  One pass is half the instructions and needs fewer registers (16 sequences
-// of 128 chunks, forward and reversed: 463 and 476 us against 824 and 731, or 985 and 823 where the caller's masks make it spill; fused 389 and 428
-// against 728 and 686), but it is for the plain variants only: next to it the loops of the fused ones, which fetch their instructions
-// from elsewhere then, lose 1 to 4 percent on ordinary gates (B8 H12 T8192 with logits 280 -> 284 to 293, by four ways to write it).
-template <bool kOnePass>
+// The two threads of a query sum a channel half each over all its keys and add up (16 sequences of 128 chunks, forward and reversed: 463 and 476 us, where each walked
+// the keys twice, once per channel half, for its own key half alone 824 and 731; fused 389 and 428, 728 and 686).
 __device__ __noinline__ void gate_wide_chunk(bool rev, float q_exp, float q_mul, uint32_t stage, uint32_t tmem_a, int w, int l,
                                              uint32_t bar_id) {
     const uint32_t tq = stage, tk = stage + kTileBytes, tg = stage + 2 * kTileBytes;
@@ -402,72 +393,34 @@ __device__ __noinline__ void gate_wide_chunk(bool rev, float q_exp, float q_mul,
     float sres[32];
 #pragma unroll
     for (int x = 0; x < 32; ++x) sres[x] = 0.f;
-    if constexpr (kOnePass) {
-        float qv[32], D[32];
+    float qv[32], D[32];
 #pragma unroll
-        for (uint32_t m = 0; m < 4; ++m) {
-            unpack8(ld_shared_v4(sw_unit(tq, rho, 4u * hf + m)), qv + 8 * m);
+    for (uint32_t m = 0; m < 4; ++m) {
+        unpack8(ld_shared_v4(sw_unit(tq, rho, 4u * hf + m)), qv + 8 * m);
 #pragma unroll
-            for (int e = 0; e < 8; ++e) D[8 * m + e] = 0.f;
-        }
-        // walk the keys from the query backwards along the scan: D = G[i] - G[j]
+        for (int e = 0; e < 8; ++e) D[8 * m + e] = 0.f;
+    }
+    // walk the keys from the query backwards along the scan: D = G[i] - G[j]
 #pragma unroll 1
-        for (int n = 0; n < 64; ++n) {
-            const int j = i - n;
-            const uint32_t pj = rev ? 63u - j : static_cast<uint32_t>(j);            // physical key row / column
-            float s = 0.f;
-            if (j >= 0) {
-#pragma unroll
-                for (uint32_t m = 0; m < 4; ++m) {
-                    float kv[8], gv[8];
-                    unpack8(ld_shared_v4(sw_unit(tk, pj, 4u * hf + m)), kv);
-                    unpack8(ld_shared_v4(sw_unit(tg, pj, 4u * hf + m)), gv);
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) {
-                        s = fmaf(qv[8 * m + e] * kv[e], ex2(D[8 * m + e]), s);
-                        D[8 * m + e] = fmaf(gv[e], kLog2e, D[8 * m + e]);   // the next key's gap to the query grows by this key's own gate
-                    }
-                }
-            }
-            s += __shfl_xor_sync(0xffffffffu, s, 16);
-            if (j >= 0 && (pj >> 5) == hf) sres[pj & 31u] = s;
-        }
-    } else {
-        // two passes over the channel halves keep the registers bounded
-#pragma unroll 1
-        for (uint32_t ch = 0; ch < 2; ++ch) {
-            float qv[32], D[32];
+    for (int n = 0; n < 64; ++n) {
+        const int j = i - n;
+        const uint32_t pj = rev ? 63u - j : static_cast<uint32_t>(j);            // physical key row / column
+        float s = 0.f;
+        if (j >= 0) {
 #pragma unroll
             for (uint32_t m = 0; m < 4; ++m) {
-                unpack8(ld_shared_v4(sw_unit(tq, rho, 4u * ch + m)), qv + 8 * m);
+                float kv[8], gv[8];
+                unpack8(ld_shared_v4(sw_unit(tk, pj, 4u * hf + m)), kv);
+                unpack8(ld_shared_v4(sw_unit(tg, pj, 4u * hf + m)), gv);
 #pragma unroll
-                for (int e = 0; e < 8; ++e) D[8 * m + e] = 0.f;
-            }
-            // walk the keys from the query backwards along the scan: D = G[i] - G[j]
-#pragma unroll 1
-            for (int j = i; j >= 0; --j) {
-                const uint32_t pj = rev ? 63u - j : static_cast<uint32_t>(j);            // physical key row / column
-                if ((pj >> 5) == hf) {
-                    float s = 0.f;
-#pragma unroll
-                    for (uint32_t m = 0; m < 4; ++m) {
-                        float kv[8];
-                        unpack8(ld_shared_v4(sw_unit(tk, pj, 4u * ch + m)), kv);
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) s = fmaf(qv[8 * m + e] * kv[e], ex2(D[8 * m + e]), s);
-                    }
-                    sres[pj & 31u] += s;
-                }
-                // next key is one step earlier: its gap to the query grows by this key's own gate
-#pragma unroll
-                for (uint32_t m = 0; m < 4; ++m) {
-                    float gv[8];
-                    unpack8(ld_shared_v4(sw_unit(tg, pj, 4u * ch + m)), gv);
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) D[8 * m + e] = fmaf(gv[e], kLog2e, D[8 * m + e]);
+                for (int e = 0; e < 8; ++e) {
+                    s = fmaf(qv[8 * m + e] * kv[e], ex2(D[8 * m + e]), s);
+                    D[8 * m + e] = fmaf(gv[e], kLog2e, D[8 * m + e]);   // the next key's gap to the query grows by this key's own gate
                 }
             }
         }
+        s += __shfl_xor_sync(0xffffffffu, s, 16);
+        if (j >= 0 && (pj >> 5) == hf) sres[pj & 31u] = s;
     }
 #pragma unroll
     for (int x = 0; x < 32; ++x) sres[x] *= q_mul;
@@ -521,26 +474,23 @@ __device__ __noinline__ void logits_to_log_gates(uint32_t tg, float inv_norm, bo
 #pragma unroll
     for (uint32_t m = 0; m < 4; ++m) {
         const uint32_t a = sw_unit(tg, rho, 4u * hf + m);
-        float gv[8];
-        unpack8(ld_shared_v4(a), gv);
+        const uint4 g4 = ld_shared_v4(a);
+        const uint32_t g[4] = {g4.x, g4.y, g4.z, g4.w};
         uint32_t h[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
-            h[e] = t < valid ? pack_half2_sat(logsigmoid_f(gv[2 * e]) * inv_norm, logsigmoid_f(gv[2 * e + 1]) * inv_norm) : 0u;
+        for (int e = 0; e < 4; ++e) {                 // min(x, 0) - ln 2 log2(1 + 2^(-|x| log2 e)), times 1 / normaliser
+            const float2 n = mul2(unpack_half2(g[e] & 0x7fff7fffu), two(-kLog2e));
+            const float2 lg = make_float2(lg2(1.f + ex2(n.x)), lg2(1.f + ex2(n.y)));
+            const float2 v = mul2(fma2(lg, two(-0.6931471805599453f), unpack_half2(hmin2_zero(g[e]))), two(inv_norm));
+            h[e] = t < valid ? pack_half2_sat(v.x, v.y) : 0u;
+        }
         st_shared_v4(a, h[0], h[1], h[2], h[3]);
     }
     fence_proxy_async_smem();
 }
 
-// The 32 score columns j0.. of query row rho, causal along the scan, as the fp16 tile.  By selects in the fused variants, whose registers
-// the masks' would not fit into; by masks in the others, three of whose four spill 4 to 8 bytes a thread with them: 48 x 100 chunks on columns of 80 rows
-// 71.0 -> 67.9 us, on rows 65.2 -> 62.8; raw logits 91.5 -> 91.9, reversed 91.5 -> 89.6, 96 x 48 chunks of them 93.7 -> 92.1 and 94.0 -> 90.8.
-__device__ __forceinline__ void select_and_store_scores(bool rev, uint32_t a16, uint32_t rho, uint32_t j0, float* x) {
-    const int lim = static_cast<int>(rho) - static_cast<int>(j0);
-#pragma unroll
-    for (int j = 0; j < 32; ++j) x[j] = (rev ? (j >= lim) : (j <= lim)) ? x[j] : 0.f;
-    store_row_f16<4>(a16, rho, j0 >> 3, x);
-}
+// The 32 score columns j0.. of query row rho, causal along the scan, as the fp16 tile (by masks; by selects 48 x 100 chunks on columns of 80 rows took 71.0 us, 67.9,
+// and 96 x 128 fused ones 255, 248).
 __device__ __forceinline__ void mask_and_store_scores(const CausalRow& causal, uint32_t a16, uint32_t rho, uint32_t j0, int tw, const float* x) {
     uint32_t r[16];
     causal.mask(tw, x, r);
@@ -658,7 +608,7 @@ gla_block_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Para
         *reinterpret_cast<__half*>(base_ptr + kOffLmat + o) = __float2half(at_or_before ? 0.5f : -0.5f);
         *reinterpret_cast<__half*>(base_ptr + kOffLmat + kTileBytes + o) = __float2half(at_or_before ? 0.f : -1.f);
     }
-    if (!kGated) M.causal.fill(kRev);
+    M.causal.fill(kRev);
     fence_proxy_async_smem();
     if (w == kWarpProducer) {
         tmem_alloc(smem_u32(&M.tmem_base), kTmemCols);
@@ -672,6 +622,7 @@ gla_block_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Para
     tc_fence_after();
     const uint32_t tmem = __shfl_sync(0xffffffffu, M.tmem_base, 0);
     pdl_wait();
+    if (kGated && tid < 32) M.weight[tid] = __ldg(reinterpret_cast<const uint32_t*>(P.rms_w) + tid);         // (the first item's barriers lie between)
     constexpr bool logits = kLogits;
     constexpr bool rev = kRev;
     const float hk = 0.5f * P.q_exp, hq = P.q_exp - hk;       // k's and q's share of the output scale (log2)
@@ -845,7 +796,10 @@ gla_block_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Para
                         float x[32];
                         tmem_half_row(tmem, quad, kTmInc + 64u * p, x);
 #pragma unroll
-                        for (int e = 0; e < 32; ++e) S[e] = fmaf(ha, S[e], hb * x[e]);
+                        for (int e = 0; e < 16; ++e) {
+                            const float2 s = fma2(two(ha), pair_of(S, e), mul2(two(hb), pair_of(x, e)));
+                            S[2 * e] = s.x; S[2 * e + 1] = s.y;
+                        }
                     }
                     tc_fence_before();
                     warp_arrive(&M.inc_free[ctr & 3u], l);
@@ -954,8 +908,10 @@ gla_block_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Para
                             const uint4 kr = ld_shared_v4(ak);
                             uint32_t f[4];
 #pragma unroll
-                            for (int e = 0; e < 4; ++e)
-                                f[e] = pack_half2(ex2(-kLog2e * x[8 * m + 2 * e]), ex2(-kLog2e * x[8 * m + 2 * e + 1]));
+                            for (int e = 0; e < 4; ++e) {
+                                const float2 p2 = ex2_2(mul2(pair_of(x + 8 * m, e), two(-kLog2e)));
+                                f[e] = pack_half2(p2.x, p2.y);
+                            }
                             st_shared_v4(ak, hmul2_u32(kr.x, f[0]), hmul2_u32(kr.y, f[1]), hmul2_u32(kr.z, f[2]), hmul2_u32(kr.w, f[3]));
                         }
                         fence_proxy_async_smem();
@@ -992,27 +948,27 @@ gla_block_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Para
                         const bool wide = __any_sync(0xffffffffu, far);
                         if (l == 0) M.wide[slot] = wide ? 1u : 0u;
                     }
-                    uint32_t qo[16], ko[16];
-#pragma unroll
-                    for (uint32_t m = 0; m < 4; ++m) {
-                        const uint4 qr = ld_shared_v4(sw_unit(tq, rho, 4u * hf + m)), kr = ld_shared_v4(sw_unit(tk, rho, 4u * hf + m));
-                        const uint32_t qu[4] = {qr.x, qr.y, qr.z, qr.w}, ku[4] = {kr.x, kr.y, kr.z, kr.w};
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const float a0 = x[8 * m + 2 * e], a1 = x[8 * m + 2 * e + 1];
-                            qo[4 * m + e] = hmul2_u32(qu[e], pack_half2(ex2(fmaf(a0, kLog2e, hq)), ex2(fmaf(a1, kLog2e, hq))));
-                            ko[4 * m + e] = hmul2_u32(ku[e], pack_half2(ex2(fmaf(a0, -kLog2e, hk)), ex2(fmaf(a1, -kLog2e, hk))));
-                        }
-                    }
+                    // The flag first, then the factors, whose products go straight back to their tiles: held in registers until the flag was there they
+                    // took 32, and with a chunk's arithmetic in pairs besides, the masks from a table and w in shared memory everything spilled (any spill
+                    // in here costs 5 to 10 percent).  Fused with logits 96 x 128 chunks 280 -> 248 us, 48 x 128 133 -> 119; of that pairs alone 277 and 128.
                     named_bar_sync(bar_id, kTeamThreads);             // the exact-path flag is known to the whole team
                     const bool wide = M.wide[slot] != 0u;
                     if (wide) {
-                        gate_wide_chunk<!kGated>(rev, P.q_exp, P.q_mul, stage, tmT, tw, l, bar_id);
+                        gate_wide_chunk(rev, P.q_exp, P.q_mul, stage, tmT, tw, l, bar_id);
                     } else {
 #pragma unroll
                         for (uint32_t m = 0; m < 4; ++m) {
-                            st_shared_v4(sw_unit(tq, rho, 4u * hf + m), qo[4 * m], qo[4 * m + 1], qo[4 * m + 2], qo[4 * m + 3]);
-                            st_shared_v4(sw_unit(tk, rho, 4u * hf + m), ko[4 * m], ko[4 * m + 1], ko[4 * m + 2], ko[4 * m + 3]);
+                            const uint32_t aq = sw_unit(tq, rho, 4u * hf + m), ak = sw_unit(tk, rho, 4u * hf + m);
+                            const uint4 qr = ld_shared_v4(aq), kr = ld_shared_v4(ak);
+                            uint32_t qu[4] = {qr.x, qr.y, qr.z, qr.w}, ku[4] = {kr.x, kr.y, kr.z, kr.w};
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                const float2 a = pair_of(x + 8 * m, e), fq = ex2_2(fma2(a, two(kLog2e), two(hq))), fk = ex2_2(fma2(a, two(-kLog2e), two(hk)));
+                                qu[e] = hmul2_u32(qu[e], pack_half2(fq.x, fq.y));
+                                ku[e] = hmul2_u32(ku[e], pack_half2(fk.x, fk.y));
+                            }
+                            st_shared_v4(aq, qu[0], qu[1], qu[2], qu[3]);
+                            st_shared_v4(ak, ku[0], ku[1], ku[2], ku[3]);
                         }
                     }
                     fence_proxy_async_smem();
@@ -1061,8 +1017,7 @@ gla_block_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Para
                     group_wait(ctx, &M.a_done[team], oturn & 1u, tw, bar_id, kTeamThreads);
                     tc_fence_after();
                     tmem_half_row(tmem, tw, kTmT + 64u * team, x);
-                    if constexpr (kGated) select_and_store_scores(rev, tg, rho, j0, x);
-                    else mask_and_store_scores(CausalRow(M.causal, tw, l, rev), tg, rho, j0, tw, x);
+                    mask_and_store_scores(CausalRow(M.causal, tw, l, rev), tg, rho, j0, tw, x);
                     fence_proxy_async_smem();
                     tc_fence_before();
                     if (storer && elect_one()) tma_store_wait_read();   // the team's output tile: its last store has read it
@@ -1100,23 +1055,22 @@ gla_block_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Para
                         }
                     } else {
                         // y = o * rsqrt(mean(o^2) + eps) * w * silu(gate): the two lanes of a row share its sum of squares
-                        float s4[4] = {0.f, 0.f, 0.f, 0.f};
+                        float2 s2[2] = {two(0.f), two(0.f)};
 #pragma unroll
-                        for (int e = 0; e < 32; ++e) s4[e & 3] = fmaf(x[e], x[e], s4[e & 3]);
-                        float ss = (s4[0] + s4[1]) + (s4[2] + s4[3]);
+                        for (int e = 0; e < 16; ++e) s2[e & 1] = fma2(pair_of(x, e), pair_of(x, e), s2[e & 1]);
+                        float ss = (s2[0].x + s2[0].y) + (s2[1].x + s2[1].y);
                         ss += __shfl_xor_sync(0xffffffffu, ss, 16);
                         const float rinv = P.o_mul * rsqrtf(ss * (P.o_mul * P.o_mul) * (1.f / kD) + P.rms_eps);
                         if (gp != nullptr) {       // rows past the end of the sequence are never sent out
-                            const uint4* wp = reinterpret_cast<const uint4*>(P.rms_w + j0);
 #pragma unroll
                             for (uint32_t m = 0; m < 4; ++m) {
-                                const uint4 g4 = __ldg(gp + m), w4 = __ldg(wp + m);
+                                const uint4 g4 = __ldg(gp + m), w4 = ld_shared_v4(smem_u32(M.weight) + 2u * j0 + 16u * m);
                                 const uint32_t gu[4] = {g4.x, g4.y, g4.z, g4.w}, wu[4] = {w4.x, w4.y, w4.z, w4.w};
 #pragma unroll
                                 for (int q2 = 0; q2 < 4; ++q2) {
-                                    const float2 gf = unpack_half2(gu[q2]), wf = unpack_half2(wu[q2]);
-                                    x[8 * m + 2 * q2] *= rinv * wf.x * silu_f(gf.x);
-                                    x[8 * m + 2 * q2 + 1] *= rinv * wf.y * silu_f(gf.y);
+                                    const float2 hg = mul2(unpack_half2(gu[q2]), two(0.5f)), silu = fma2(hg, tanh_2(hg), hg);      // h + h tanh h
+                                    const float2 y = mul2(pair_of(x + 8 * m, q2), mul2(mul2(two(rinv), unpack_half2(wu[q2])), silu));
+                                    x[8 * m + 2 * q2] = y.x; x[8 * m + 2 * q2 + 1] = y.y;
                                 }
                             }
                         }
