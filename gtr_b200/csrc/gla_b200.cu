@@ -88,11 +88,11 @@ constexpr int kClusterSmemMax = 227 * 1024;
 struct DeviceInfo {
     bool ok = false;
     int sms = 0;
-    int clusters[2][gla::kClusterGroups + 1][gla::kClusterMax + 1] = {};       // cluster kernel: how many run at a time, plus 1; 0: not known yet
     bool attr_set = false;
 };
 std::mutex g_mu;
 DeviceInfo g_dev[64];
+int g_clusters[64][2][gla::kClusterGroups + 1][gla::kClusterMax + 1];       // cluster kernel: how many run at a time, plus 1; 0: not known yet
 
 int device_info(int dev, DeviceInfo* out) {
     std::lock_guard<std::mutex> lock(g_mu);
@@ -729,7 +729,7 @@ struct ClusterShape {
 // How many clusters of that shape the device runs at a time.
 int clusters_at_a_time(const ClusterShape& s, bool block, int dev) {
     std::lock_guard<std::mutex> lock(g_mu);
-    int& known = g_dev[dev].clusters[block][s.groups][s.size];
+    int& known = g_clusters[dev][block][s.groups][s.size];
     if (known == 0) {
         cudaLaunchAttribute attr;
         attr.id = cudaLaunchAttributeClusterDimension;
