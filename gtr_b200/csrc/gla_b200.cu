@@ -725,6 +725,8 @@ bool block_pays(const block_plan::Plan& plan, const Split& split, int NT, int ns
 // The cluster kernel's shape for a call: CTAs per sequence and chunks per CTA; groups = 0: not for it.
 struct ClusterShape {
     int size = 0, groups = 0, rows = 0, smem = 0;
+    // The block arithmetic's walk, segments times rows, is shared out over the most warps that a CTA can have
+    int threads(bool block) const { return block ? gla::kClusterThreads : gla::kFwdThreads * groups; }
 };
 // How many clusters of that shape the device runs at a time.
 int clusters_at_a_time(const ClusterShape& s, bool block, int dev) {
@@ -737,7 +739,7 @@ int clusters_at_a_time(const ClusterShape& s, bool block, int dev) {
         attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(s.size);
-        cfg.blockDim = dim3(gla::kFwdThreads * s.groups);
+        cfg.blockDim = dim3(s.threads(block));
         cfg.dynamicSmemBytes = std::min(gla::ClusterSmem(block, s.groups, s.size * s.groups, s.rows).bytes, kClusterSmemMax);      // of the longest sequence
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
@@ -810,7 +812,7 @@ int forward_cluster(const gla_b200_args* a, MapKey key, const int64_t* o_stride,
     }
     void* args[3] = {&maps, &P, &C};
     return launch_overlapped(cluster_kernel(a->out_gate != nullptr, P.inv_norm > 0.f, plan != nullptr), a->B * a->H * shape.size,
-                             gla::kFwdThreads * shape.groups, shape.smem, args, stream, shape.size);
+                             shape.threads(plan != nullptr), shape.smem, args, stream, shape.size);
 }
 
 // The operator on the block kernel (gla_block.cuh).

@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(kClusterThreads) gla_cluster_kernel(const __gr
     const int tid = threadIdx.x, grp = __shfl_sync(0xffffffffu, tid >> 7, 0), w = __shfl_sync(0xffffffffu, (tid >> 5) & 3, 0), l = tid & 31;
     const int seq = blockIdx.x / C.size, rank = blockIdx.x - seq * C.size, b = seq / P.H, h = seq - b * P.H;
     const int chunk = rank * C.groups + grp;
-    const bool live = chunk < P.NT, rev = P.rev != 0;
+    const bool live = grp < C.groups && chunk < P.NT, rev = P.rev != 0;        // (warps beyond the groups help with the walk)
     const uint32_t own = base + grp * lay.group, tq = own + OutSmem::kQ, tk = own + OutSmem::kK, tg = own + OutSmem::kG, tv = own + OutSmem::kV,
                    s16 = own + OutSmem::kS16, ta = own + ClusterSmem::kA, mat = base + lay.mat;
     const int first = rank * C.rows, owned = max(min(C.rows, 64 - first), 0);       // rows of the state
