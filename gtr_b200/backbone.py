@@ -330,8 +330,8 @@ class GTRBackbone(nn.Module):
 
 class GraphedBackbone:
     """Replays one captured CUDA graph per input shape (the reference benchmarks its model the same
-    way, tools/benchmark/torch_speed_fullgraph.py:134-158).  The operator's launches (a clear and one
-    kernel per block) are captured like any other stream work."""
+    way, tools/benchmark/torch_speed_fullgraph.py:134-158).  The operator's launches (one kernel per block,
+    or a clear and one) are captured like any other stream work."""
 
     def __init__(self, model: GTRBackbone):
         self.model = model.eval()

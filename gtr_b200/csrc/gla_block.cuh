@@ -1,8 +1,8 @@
 // The operator as one persistent CTA of specialised warpgroups per SM.  It reads a sequence about once and a half where the two kernels of
 // gla_kernel.cuh read k, g and v twice, and needs about as many sequences as SMs, or long ones, for that to pay: the host sends
-// it the calls of that kind (block_pays()), whatever the backbone's blocks call, and nothing else.
+// it the calls of that kind (block_pays()), what the backbone's blocks call beyond a few short sequences, and nothing else.
 //
-// The backbone's blocks always run on this kernel.  The two compute the same sums with fp16 operands
+// The backbone's blocks always run with this kernel's arithmetic (a few short sequences on gla_cluster.cuh, which keeps it).  The two compute the same sums with fp16 operands
 // rounded at different references; outputs differ by 2e-4, as both do from exact arithmetic by 5e-4.  In a chain of blocks every
 // stage rounds to fp16, and a difference of any size at one stage becomes one of half units in the last place at the next:
 // twelve blocks end 0.6 to 1.8 percent apart (measured over 40 models and image sizes with random weights).  A network's results

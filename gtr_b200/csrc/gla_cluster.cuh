@@ -6,21 +6,23 @@
 // CTAs are a cluster that exchanges states through its shared memories:
 //   1. every chunk by itself: gate sums, gated operands, its state increment k~^T v (as in gla_kernel.cuh)
 //   2. each CTA owns some rows of the 64 x 64 state: increments and decays are sent to the owners of their rows
-//   3. an owner walks its rows through all chunks in registers and sends every chunk its rows of the fp16 start state; meanwhile the
-//      chunks' scores are made
+//   3. an owner walks its rows through all chunks in registers and sends every chunk its rows of the fp16 start state; before that the
+//      chunks' scores are made, while increments are on their way
 //   4. outputs
-// B1 H6 T1600 13.9 -> 7.9 us, B3 H3 T1050 K = 32 with states 15.9 -> 8.9, the block's call at B1 H3 T1600 28 -> 12 (and no launch that clears flags).  Of some 11
+// What is sent goes by bulk copies (factors by st.async) whose bytes the receiver's barriers count; a cluster barrier opens and one closes the exchange.
+//
+// B1 H6 T1600 14.1 -> 7.9 us, B3 H3 T1050 K = 32 with states 15.9 -> 8.9, the block's call at B1 H3 T1600 28 -> 11.4 (and no launch that clears flags).  Of some 11
 // thousand cycles after the predecessor has ended (one image) 1.4 pass until the tiles are there, 0.5 for gate sums, 0.6 for k~, 2.0 until the increment
 // is there (q~ meanwhile), 2.4 until all have arrived (scores meanwhile), 1.5 for the walk, 1.5 until the start state is there, 1.4 for the outputs.
 // Tried on the way: increments and start states by plain stores to the other CTAs (16 bytes a lane, rows apart: 10 bytes a cycle; 8.6 us), start states by
-// st.async (a barrier update for every lane's 8 bytes: 8.0) or by stores and a releasing arrival (8.8), copies sent by one warp (8.9).
-// Asynchronous copies that the receiver's barriers count lie between these, and a walk of NT steps over a few elements a thread takes the place of the chain
-// through memory.
+// st.async (a barrier update for every lane's 8 bytes: 8.0) or by stores and a releasing arrival (8.8), copies sent by one warp (8.9), increments staged
+// apart from k so that they leave before q~ and the scores (7.4 against 7.3, row order), tiles asked for by four warps (columns 0.1 better, rows 0.1 worse).
 //
 // kBlock: the arithmetic of the persistent kernel, to the bit, for the backbone's blocks (gla_block.cuh has the reason).  A sequence has the
 // equal segments of that kernel's plan: increments in the form of its pre-pass (k 2^(G_L-G)) are summed to a segment's aggregate, its start state is chained
-// from those before it, and within it the state goes on in the scale of the next chunk's reference.  That kernel adds up aggregates down to the first segment
-// whose inclusive state happens to be there; here always down to the first segment.
+// from those before it, and within it the state goes on in the scale of the next chunk's reference; segments times rows are walked side by side, by twelve
+// warps whatever the chunks (with four to a chunk B2 H3 T1024 took 9.8 us, 9.2).  That kernel adds up aggregates down to the first segment whose
+// inclusive state happens to be there; here always down to the first segment.
 #pragma once
 
 #include "gla_kernel.cuh"

@@ -92,7 +92,8 @@ typedef struct gla_b200_args {
 int gla_b200_forward(const gla_b200_args* args, void* stream);
 
 /* The fused operator (out_gate and rms_weight given) on the kernel that the backbone's blocks run on.  Same arguments and
- * accuracy; its roundings are the ones a backbone's results are known with, see gla_block.cuh. */
+ * accuracy; its roundings are the ones a backbone's results are known with, see gla_block.cuh (and gla_cluster.cuh, which computes a
+ * few short sequences with the same ones). */
 int gla_b200_forward_block(const gla_b200_args* args, void* stream);
 
 /* Same operator, but with nothing allocated and no workspace from the caller (`workspace` and
