@@ -63,14 +63,19 @@ const void* state_kernel(bool logits) {
                   : reinterpret_cast<const void*>(&gla_state_kernel<false, Table>);
 }
 
-// The cluster kernel's; the block kernel's arithmetic only with the fused epilogue.
-const void* cluster_kernel(bool gated, bool logits, bool block) {
+// The cluster kernel's; the block kernel's arithmetic only with the fused epilogue and in one round.
+template <bool kRounds>
+const void* cluster_kernel_of(bool gated, bool logits) {
+    using gla::gla_cluster_kernel;
+    if (gated)
+        return logits ? reinterpret_cast<const void*>(&gla_cluster_kernel<true, true, false, kRounds>) : reinterpret_cast<const void*>(&gla_cluster_kernel<true, false, false, kRounds>);
+    return logits ? reinterpret_cast<const void*>(&gla_cluster_kernel<false, true, false, kRounds>) : reinterpret_cast<const void*>(&gla_cluster_kernel<false, false, false, kRounds>);
+}
+const void* cluster_kernel(bool gated, bool logits, bool block, bool rounds) {
     using gla::gla_cluster_kernel;
     if (block)
-        return logits ? reinterpret_cast<const void*>(&gla_cluster_kernel<true, true, true>) : reinterpret_cast<const void*>(&gla_cluster_kernel<true, false, true>);
-    if (gated)
-        return logits ? reinterpret_cast<const void*>(&gla_cluster_kernel<true, true, false>) : reinterpret_cast<const void*>(&gla_cluster_kernel<true, false, false>);
-    return logits ? reinterpret_cast<const void*>(&gla_cluster_kernel<false, true, false>) : reinterpret_cast<const void*>(&gla_cluster_kernel<false, false, false>);
+        return logits ? reinterpret_cast<const void*>(&gla_cluster_kernel<true, true, true, false>) : reinterpret_cast<const void*>(&gla_cluster_kernel<true, false, true, false>);
+    return rounds ? cluster_kernel_of<true>(gated, logits) : cluster_kernel_of<false>(gated, logits);
 }
 
 // The block kernel's: bit 2 fused epilogue, bit 1 raw-logit gates, bit 0 reversed scan.
@@ -130,8 +135,8 @@ int device_info(int dev, DeviceInfo* out) {
                 return GLA_B200_ERR_DEVICE;
             }
         }
-        for (int v = 0; v < 6; ++v) {
-            const void* k = cluster_kernel(v >= 2, v & 1, v >= 4);
+        for (int v = 0; v < 10; ++v) {
+            const void* k = cluster_kernel(v & 2, v & 1, v >= 8, v & 4);
             if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kClusterSmemMax);
             if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         }
@@ -724,7 +729,7 @@ bool block_pays(const block_plan::Plan& plan, const Split& split, int NT, int ns
 
 // The cluster kernel's shape for a call: CTAs per sequence and chunks per CTA; groups = 0: not for it.
 struct ClusterShape {
-    int size = 0, groups = 0, rows = 0, smem = 0;
+    int size = 0, groups = 0, rows = 0, smem = 0, round = 0;      // round: chunks of a sequence at a time
     // The block arithmetic's walk, segments times rows, is shared out over the most warps that a CTA can have
     int threads(bool block) const { return block ? gla::kClusterThreads : gla::kFwdThreads * groups; }
 };
@@ -744,7 +749,7 @@ int clusters_at_a_time(const ClusterShape& s, bool block, int dev) {
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
         int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, cluster_kernel(true, true, block), &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
+        if (cudaOccupancyMaxActiveClusters(&n, cluster_kernel(true, true, block, !block), &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
         known = n + 1;
     }
     return known - 1;
@@ -763,12 +768,24 @@ ClusterShape cluster_shape(int NT, int64_t nseq, bool block, int dev) {
         for (int m = 1; m <= gla::kClusterGroups; ++m)
             for (int size = (NT + m - 1) / m; size <= gla::kClusterMax; ++size) {       // (never 1: a CTA by itself is no cluster, it has nobody to copy to)
                 ClusterShape s;
-                s.size = size; s.groups = m; s.rows = (64 + size - 1) / size;
+                s.size = size; s.groups = m; s.rows = (64 + size - 1) / size; s.round = NT;
                 s.smem = gla::ClusterSmem(block, m, NT, s.rows).bytes;
                 if (s.smem > kClusterSmemMax) continue;                // more owners have less to keep each
                 if (static_cast<int64_t>(waves) * clusters_at_a_time(s, block, dev) >= nseq) return s;
                 break;
             }
+    // Longer sequences in two rounds, with the fewest chunks to a CTA that do.  A round more costs as much as a call, 7 us (fused 9): 6 x 50 19.7 / 16.3, 24.3 / 19.5;
+    // 6 x 70 22.0 / 19.1, 26.5 / 23.5; 3 x 50 16.2 / 15.7, 19.4 / 18.8; 12 x 32 18.6 / 15.7, 23.2 / 18.8; 24 x 20 17.0 / 15.7, 21.1 / 18.6.  Not for one or two sequences
+    // of more than 64 chunks (1 x 70 18.9 / 18.3, 22.2 / 22.6), and three rounds are slower as often as not (6 x 100 28.5 / 26.9, 3 x 100 23.7 / 26.1).
+    if (block || (nseq < 3 && NT > 64)) return ClusterShape();
+    for (int m = 1; m <= gla::kClusterGroups; ++m)
+        for (int size = std::max((NT + 2 * m - 1) / (2 * m), 4); size <= gla::kClusterMax; ++size) {
+            ClusterShape s;
+            s.size = size; s.groups = m; s.rows = (64 + size - 1) / size; s.round = size * m;
+            s.smem = gla::ClusterSmem(false, m, s.round, s.rows).bytes;
+            if (s.smem > kClusterSmemMax || s.rows * 16 > gla::kFwdThreads * m) continue;          // (an owner's thread keeps one piece of the state from round to round)
+            if (clusters_at_a_time(s, false, dev) >= nseq) return s;
+        }
     return ClusterShape();
 }
 
@@ -806,12 +823,12 @@ int forward_cluster(const gla_b200_args* a, MapKey key, const int64_t* o_stride,
     P.clear = next_launch();
     gla::ClusterPlan C;
     memset(&C, 0, sizeof(C));
-    C.size = shape.size; C.groups = shape.groups; C.rows = shape.rows;
+    C.size = shape.size; C.groups = shape.groups; C.rows = shape.rows; C.round = shape.round;
     if (plan) {
         C.ns = plan->ns; C.cps = plan->cps;
     }
     void* args[3] = {&maps, &P, &C};
-    return launch_overlapped(cluster_kernel(a->out_gate != nullptr, P.inv_norm > 0.f, plan != nullptr), a->B * a->H * shape.size,
+    return launch_overlapped(cluster_kernel(a->out_gate != nullptr, P.inv_norm > 0.f, plan != nullptr, shape.round < P.NT), a->B * a->H * shape.size,
                              shape.threads(plan != nullptr), shape.smem, args, stream, shape.size);
 }
 

@@ -36,6 +36,7 @@ constexpr int kClusterMax = 16;                            // CTAs per cluster, 
 struct ClusterPlan {
     int size, groups;    // CTAs per sequence, chunks per CTA
     int rows;            // rows of the state that a CTA owns
+    int round;           // chunks at a time: all, or as many as the cluster holds
     int ns, cps;         // kBlock: segments, chunks per segment
 };
 
@@ -130,17 +131,17 @@ __device__ __forceinline__ bool group_or(int grp, bool x) {
     return grp == 0 ? named_bar_or<1>(kFwdThreads, x) : grp == 1 ? named_bar_or<2>(kFwdThreads, x) : named_bar_or<3>(kFwdThreads, x);
 }
 
-template <bool kGated, bool kLogits, bool kBlock>
+template <bool kGated, bool kLogits, bool kBlock, bool kRounds>
 __global__ void __launch_bounds__(kClusterThreads) gla_cluster_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Params P,
                                                                       const __grid_constant__ ClusterPlan C) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw), base = (raw + 1023u) & ~1023u;
-    const ClusterSmem lay(kBlock, C.groups, P.NT, C.rows);
+    const ClusterSmem lay(kBlock, C.groups, kRounds ? C.round : P.NT, C.rows);
     ClusterMisc& M = *reinterpret_cast<ClusterMisc*>(smem_raw + (base - raw) + lay.misc);
     const int tid = threadIdx.x, grp = __shfl_sync(0xffffffffu, tid >> 7, 0), w = __shfl_sync(0xffffffffu, (tid >> 5) & 3, 0), l = tid & 31;
     const int seq = blockIdx.x / C.size, rank = blockIdx.x - seq * C.size, b = seq / P.H, h = seq - b * P.H;
-    const int chunk = rank * C.groups + grp;
-    const bool live = grp < C.groups && chunk < P.NT, rev = P.rev != 0;        // (warps beyond the groups help with the walk)
+    const int place = rank * C.groups + grp;               // the group's chunk in every round
+    const bool mine_first = grp < C.groups && place < P.NT, rev = P.rev != 0;      // (warps beyond the groups help with the walk)
     const uint32_t own = base + grp * lay.group, tq = own + OutSmem::kQ, tk = own + OutSmem::kK, tg = own + OutSmem::kG, tv = own + OutSmem::kV,
                    s16 = own + OutSmem::kS16, ta = own + ClusterSmem::kA, mat = base + lay.mat;
     const int first = rank * C.rows, owned = max(min(C.rows, 64 - first), 0);       // rows of the state
@@ -153,7 +154,7 @@ __global__ void __launch_bounds__(kClusterThreads) gla_cluster_kernel(const __gr
         mbar_init(smem_u32(&M.inbox), 1);
         fence_mbar_init();
         for (int i = 0; i < kClusterGroups; ++i) mbar_arrive_expect_tx(smem_u32(&M.start[i]), kTileBytes);
-        mbar_arrive_expect_tx(smem_u32(&M.inbox), owned * (P.NT * 272 + (kBlock ? (C.ns - 1) * C.cps * 256 : 0)));
+        mbar_arrive_expect_tx(smem_u32(&M.inbox), owned * ((kRounds ? C.round : P.NT) * 272 + (kBlock ? (C.ns - 1) * C.cps * 256 : 0)));
         M.gave_up = 0u;
     }
     fill_constant(mat, [&](uint32_t r, uint32_t s) { return (rev ? s >= r : s <= r) ? 0.5f : -0.5f; });        // G - G_L / 2
@@ -164,12 +165,13 @@ __global__ void __launch_bounds__(kClusterThreads) gla_cluster_kernel(const __gr
     cluster_arrive();                                       // nothing is sent to a CTA that has not begun
     pdl_wait();
     if (blockIdx.x == 0 && tid == 0) clear_alone(P.ctrl, P.clear);
-    if (live && w == 0 && elect_one()) {
+    auto load = [&](int chunk) {
         const int tensors[4] = {TG, TK, TQ, TV};
         const uint32_t tiles[4] = {tg, tk, tq, tv};
         mbar_arrive_expect_tx(smem_u32(&M.full[grp]), 4 * kTileBytes);
         load_chunk(maps, Scan{P.T, P.Hc, P.rev}, chunk, b, h, 0, P.Hc, smem_u32(&M.full[grp]), tensors, tiles, l2_policy_stream());
-    }
+    };
+    if (mine_first && w == 0 && elect_one()) load(place);
     // (another kernel's blocks may not have their tensor memory before this one waits for them)
     const uint32_t columns = C.groups == 3 ? 512u : 128u * C.groups;
     if (tid >= 32 && tid < 64) {
@@ -185,11 +187,19 @@ __global__ void __launch_bounds__(kClusterThreads) gla_cluster_kernel(const __gr
     const uint32_t half = static_cast<uint32_t>(l) >> 4, row = 16u * w + (l & 15u), c0 = 32u * half;
     const HalfRow at(own, row, half);
     const float hk = 0.5f * P.q_exp, hq = P.q_exp - hk;     // k's and q's share of the output scale (log2)
+    // kRounds: a sequence longer than the cluster holds goes in rounds.  The owners keep their rows of the state, a chunk's tiles come in when its place is done
+    // with the last ones, a cluster barrier lies between, and each barrier is used once a round.
+    uint32_t raws = 0, agains = 0, ps = 0;                  // how often their barriers have been used
+    float4 carry = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int at0 = 0, turn = 0;; at0 += C.round, ++turn) {
+    const uint32_t ph = kRounds ? turn & 1 : 0;
+    const int NT = kRounds ? min(C.round, P.NT - at0) : P.NT, chunk = kRounds ? at0 + place : place, left = kRounds ? P.NT - at0 - NT : 0;      // left: for later rounds
+    const bool live = grp < C.groups && place < NT, opening = !kRounds || turn == 0;
     const int tok = live ? scan_token(P, P.T, chunk * kChunk + (rev ? 63 - static_cast<int>(row) : static_cast<int>(row))) : -1;
     const __half* gate_row_at = P.gate;
     __half* const op = P.o + b * P.o_s[0] + max(tok, 0) * P.o_s[1] + h * P.o_s[2] + c0;
     uint32_t weight = 0u;
-    if (kGated && w == 0) weight = __ldg(reinterpret_cast<const uint32_t*>(P.rms_w) + l);
+    if (kGated && w == 0 && opening) weight = __ldg(reinterpret_cast<const uint32_t*>(P.rms_w) + l);
     uint32_t r[16];
     float x[32];
     if (live) {
@@ -199,7 +209,7 @@ __global__ void __launch_bounds__(kClusterThreads) gla_cluster_kernel(const __gr
         }
         const bool pre = kBlock && chunk < (C.ns - 1) * C.cps;       // the chunk's segment has an aggregate
         // ---- gate sums, gated operands
-        wait(M.full[grp], 0);
+        wait(M.full[grp], ph);
         if (kLogits) {
             if (kBlock) block_log_gates(at, OutSmem::kG, P.inv_norm, tok >= 0);
             else logits_to_log_gates(at, OutSmem::kG, P.inv_norm, tok >= 0);
@@ -214,8 +224,8 @@ __global__ void __launch_bounds__(kClusterThreads) gla_cluster_kernel(const __gr
         __syncwarp();
         uint32_t k[16];
         at.get(OutSmem::kK, k);
-        if (kGated && w == 0) M.weight[grp][l] = weight;
-        wait(M.bar_x[grp], 0);
+        if (kGated && w == 0 && opening) M.weight[grp][l] = weight;
+        wait(M.bar_x[grp], ph);
         tc_fence_after();
         if (kBlock && pre) {
             half_row_read(tmem, ACC_S, w, x);
@@ -280,7 +290,7 @@ __global__ void __launch_bounds__(kClusterThreads) gla_cluster_kernel(const __gr
                 load_chunk(maps, Scan{P.T, P.Hc, P.rev}, chunk, b, h, 0, P.Hc, smem_u32(&M.raw[grp]), tensors, tiles, l2_policy_stream());
             }
             __syncwarp();
-            wait(M.raw[grp], 0);
+            wait(M.raw[grp], raws++ & 1u);
             if (group_or(grp, !(M.vec[grp][tid & 63] > -kExtreme))) {
                 at.get(OutSmem::kG, r);
 #pragma unroll
@@ -295,7 +305,7 @@ __global__ void __launch_bounds__(kClusterThreads) gla_cluster_kernel(const __gr
                     umma_commit(smem_u32(&M.again[grp]));
                 }
                 __syncwarp();
-                wait(M.again[grp], 0);
+                wait(M.again[grp], agains++ & 1u);
                 tc_fence_after();
                 half_row_read(tmem, ACC_X, w, x);
                 tmem_ld_wait();
@@ -334,15 +344,15 @@ __global__ void __launch_bounds__(kClusterThreads) gla_cluster_kernel(const __gr
             for (uint32_t e = 0; e < 8; ++e)
                 st_shared_f4(own + to + row * 256u + half * 128u + ((e ^ (row & 7u)) << 4), x[4 * e], x[4 * e + 1], x[4 * e + 2], x[4 * e + 3]);
         };
-        cluster_wait();                                     // every CTA has begun
+        if (opening) cluster_wait();                        // every CTA has begun
         auto copy = [&](uint32_t from, int inbox) {         // a lane has an owner, a warp every fourth (a lane's copy goes out after another's)
             const int who = w + 4 * l, at_row = who * C.rows, n = min(C.rows, 64 - at_row);
             if (who < C.size && n > 0)
-                cluster_copy(cluster_address(base + inbox + chunk * C.rows * 256, who), own + from + at_row * 256, n * 256, cluster_address(smem_u32(&M.inbox), who));
+                cluster_copy(cluster_address(base + inbox + place * C.rows * 256, who), own + from + at_row * 256, n * 256, cluster_address(smem_u32(&M.inbox), who));
             __syncwarp();
         };
         if (half == 0u) {
-            const uint32_t who = row / static_cast<uint32_t>(C.rows), to = cluster_address(base + lay.in_f + (chunk * C.rows + row - who * C.rows) * 16u, who),
+            const uint32_t who = row / static_cast<uint32_t>(C.rows), to = cluster_address(base + lay.in_f + (place * C.rows + row - who * C.rows) * 16u, who),
                            bar = cluster_address(smem_u32(&M.inbox), who);
             if (kBlock) cluster_send(to, v, pre ? M.gl[grp][row] : 0.f, wide ? 1.f : 0.f, 0.f, bar);
             else cluster_send(to, ex2(2.f * v), ex2(wide ? hk : v + hk), 0.f, 0.f, bar);
@@ -358,7 +368,7 @@ __global__ void __launch_bounds__(kClusterThreads) gla_cluster_kernel(const __gr
             sync();
             copy(ClusterSmem::kIncA, lay.in_a);
         }
-        wait(M.bar_inc[grp], 0);
+        wait(M.bar_inc[grp], ph);
         tc_fence_after();
         half_row_read(tmem, ACC_INC, w, x);
         tmem_ld_wait();
@@ -370,7 +380,7 @@ __global__ void __launch_bounds__(kClusterThreads) gla_cluster_kernel(const __gr
                 x[2 * e] = u.x; x[2 * e + 1] = u.y;
             }
         }
-        if (!wide) wait(M.bar_p[grp], 0);                   // k~ has been read
+        if (!wide) wait(M.bar_p[grp], ps++ & 1u);           // k~ has been read
         stage(ClusterSmem::kInc);
         fence_proxy_async_smem();
         sync();
@@ -390,10 +400,10 @@ __global__ void __launch_bounds__(kClusterThreads) gla_cluster_kernel(const __gr
             tile_mma<0, 1>(acc_slot(tmem, ACC_P), ta, tv, false);
         }
         __syncwarp();
-    } else {
+    } else if (opening) {
         cluster_wait();
     }
-    wait(M.inbox, 0);
+    wait(M.inbox, ph);
 
     // ---- the owned rows through all chunks, four columns a thread; 16 lanes have a row
     const int mine = owned * 16;
@@ -429,24 +439,25 @@ __global__ void __launch_bounds__(kClusterThreads) gla_cluster_kernel(const __gr
         for (int u = tid; u < mine; u += blockDim.x) {
             unit(u);
             const uint32_t fac = base + lay.in_f + (u >> 4) * 16u, fac_step = C.rows * 16u;
-            float4 S = initial();
-            for (int c0 = 0; c0 < P.NT; c0 += kAhead) {
+            float4 S = opening ? initial() : carry;
+            for (int c0 = 0; c0 < NT; c0 += kAhead) {
                 float2 f[kAhead];
                 float4 d[kAhead];
 #pragma unroll
                 for (int i = 0; i < kAhead; ++i)
-                    if (c0 + i < P.NT) {
+                    if (c0 + i < NT) {
                         f[i] = ld_shared_f2(fac + (c0 + i) * fac_step);
                         d[i] = ld_shared_f4(inc + (c0 + i) * step);
                     }
 #pragma unroll
                 for (int i = 0; i < kAhead; ++i)
-                    if (c0 + i < P.NT) {
+                    if (c0 + i < NT) {
                         give(c0 + i, times(f[i].y, S));
                         S = plus(f[i].x, S, d[i]);
                     }
             }
-            final(S);
+            if (kRounds && left > 0) carry = S;             // (a row's unit a thread, then)
+            else final(S);
         }
     } else {
         // segments times units, a warp always in one segment (what is left over of it does the last unit again)
@@ -538,10 +549,11 @@ __global__ void __launch_bounds__(kClusterThreads) gla_cluster_kernel(const __gr
     }
     fence_proxy_async_smem();
     __syncthreads();
+    if (kRounds && left > 0 && tid == 0) mbar_arrive_expect_tx(smem_u32(&M.inbox), owned * min(C.round, left) * 272);
     {
         const int warps = blockDim.x >> 5, c = (tid >> 5) + warps * l, who = c / C.groups, g = c - who * C.groups;
         static_assert(kClusterMax * kClusterGroups <= 32 * 4, "a lane for every chunk");
-        if (c < P.NT && owned > 0)
+        if (c < NT && owned > 0)
             cluster_copy(cluster_address(base + g * lay.group + OutSmem::kS16 + first * 128, who), mat + c * C.rows * 128, owned * 128,
                          cluster_address(smem_u32(&M.start[g]), who));
         __syncwarp();
@@ -556,16 +568,22 @@ __global__ void __launch_bounds__(kClusterThreads) gla_cluster_kernel(const __gr
     // ---- outputs
     if (live) {
         if (w == 0) {
-            wait(M.start[grp], 0);
+            wait(M.start[grp], ph);
             if (elect_one()) {
+                if (kRounds && place < left) mbar_arrive_expect_tx(smem_u32(&M.start[grp]), kTileBytes);
                 tc_fence_after();
                 tile_mma<0, 1>(acc_slot(tmem, ACC_P), tq, s16, true);
                 umma_commit(smem_u32(&M.bar_o[grp]));
             }
             __syncwarp();
         }
-        wait(M.bar_o[grp], 0);
-        cluster_arrive_relaxed();                           // every owner has what this chunk sent, and this chunk what they sent
+        wait(M.bar_o[grp], ph);
+        if (kRounds) cluster_arrive();
+        else cluster_arrive_relaxed();                      // every owner has what this chunk sent, and this chunk what they sent
+        if (kRounds && place < left && w == 0) {
+            if (elect_one()) load(chunk + C.round);
+            __syncwarp();
+        }
         tc_fence_after();
         half_row_read(tmem, ACC_P, w, x);
         tmem_ld_wait();
@@ -606,12 +624,20 @@ __global__ void __launch_bounds__(kClusterThreads) gla_cluster_kernel(const __gr
                 for (int m = 0; m < 4; ++m) reinterpret_cast<uint4*>(op)[m] = make_uint4(r[4 * m], r[4 * m + 1], r[4 * m + 2], r[4 * m + 3]);
             }
         }
+    } else if (kRounds) {
+        cluster_arrive();
     } else {
         cluster_arrive_relaxed();
     }
     tc_fence_before();
     __syncthreads();
     cluster_wait();                                         // nothing is read from this CTA any more
+    if (!kRounds || left == 0) break;
+    fill_constant(mat, [&](uint32_t r, uint32_t s) { return (rev ? s >= r : s <= r) ? 0.5f : -0.5f; });        // where start states were
+    fence_proxy_async_smem();
+    __syncthreads();
+    tc_fence_after();
+    }
     if (tid == 0) {
         if (M.gave_up) report_alone(P, P.clear);
         if (blockIdx.x == 0) P.ctrl[0] = 0u;

@@ -1,4 +1,4 @@
-"""The cluster kernel at the edges of what it serves -- clusters of two to sixteen, one to three chunks a CTA, ragged ends, owners of uneven and of no rows --
+"""The cluster kernel at the edges of what it serves -- clusters of two to sixteen, one to three chunks a CTA, one round and two, ragged ends, owners of uneven and of no rows --
 against the CPU oracle, and its block arithmetic against the persistent kernel, to the bit."""
 import ctypes
 
@@ -21,7 +21,13 @@ EDGES = [  # B, H, T, K, direction, states, fused, logits, gates
     (1, 12, 25 * 64, 64, 2, False, False, False, "weak"),    # clusters of nine, of which eight own rows
     (1, 2, 36 * 64, 64, 3, True, False, False, "weak"),      # sixteen CTAs for memory's sake, four of them without chunks
     (1, 2, 48 * 64, 64, 1, True, False, True, "weak"),       # the longest
-    (1, 2, 49 * 64, 64, 1, True, False, False, "weak"),      # and one that is too long
+    (1, 2, 49 * 64, 64, 1, True, False, False, "weak"),      # two rounds
+    (1, 7, 96 * 64 - 3, 64, 0, True, False, True, "weak"),   # two full ones
+    (1, 3, 70 * 64, 32, 2, True, True, False, "weak"),       # CTAs without a chunk in the second
+    (1, 3, 97 * 64, 64, 3, False, False, False, "weak"),     # too long
+    (1, 12, 32 * 64 - 9, 64, 1, True, True, True, "weak"),   # two rounds for many sequences' sake
+    (8, 3, 20 * 64, 64, 0, True, False, False, "weak"),      # clusters of four, owners of sixteen rows
+    (1, 2, 57 * 64, 64, 1, True, False, False, "strong"),    # the exact path in both rounds
     (15, 3, 6 * 64 - 1, 64, 0, True, False, False, "weak"),  # the most sequences
     (1, 2, 20 * 64 + 7, 64, 0, True, False, False, "strong"),    # every chunk pair by pair
     (1, 2, 40 * 64 + 7, 32, 3, True, True, False, "strong"),
